@@ -174,6 +174,24 @@ typedef struct {
                              over its 16 pixels */
 } mk_launch;
 
+/* A plan of the node form (mk_nodes_plan): which tiles are interpolated from
+ * how many Chebyshev nodes per patch, and the sizes its run needs. */
+typedef struct {
+    int n_frames, n_tiles;
+    int n0, n1;             /* nodes per axis of the coarse patches (0: no groups) and the fine ones */
+    int group_tiles;        /* tiles per group at most (0: no groups) */
+    int n_groups, n_members;/* groups and the tiles in them */
+    int n_mid;              /* tiles evaluated on the fine nodes directly */
+    int n_wide;             /* tiles left to the split kernel (their indices at off_wide) */
+    int n_src;              /* n_groups + n_mid */
+    int slices, src_per_slice, passes;
+    long long nodes0, patches1, weights, n_pix;
+    long long off_src, off_members, off_mid, off_wide, buf_bytes;
+    long long chunk_bytes, ws_bytes;
+    double radius1_m, radius2_m; /* widest tile of a group, widest source */
+    double nodes_s, direct_s;    /* estimated time of this form and of the split kernel */
+} mk_node_plan;
+
 /* --- library ---------------------------------------------------------- */
 int mk_version(void);
 const char *mk_last_error(void);
@@ -336,6 +354,47 @@ int mk_kin_scan_f32(const mk_tiles *tiles, const mk_species *sp, const mk_physic
                     const mk_pixels *px, int n_frames, const mk_frame_desc *frames_dev,
                     long long n_items, long long n_partial, const mk_launch *launch, double *out,
                     double *intensity_sums, void *workspace, size_t ws_bytes, void *stream);
+
+/* --- node form ----------------------------------------------------------- */
+/* The same sum for detectors whose pixels lie on a plane grid: the field of
+ * a compact group of atoms relative to its own centre is evaluated (FP32
+ * split-phase terms) on a few Chebyshev nodes of the detector's patches and
+ * interpolated to the pixels, n nodes per axis chosen so that
+ * 4 (phi/2)^n / n! <= 3e-8 for the phase half-range phi = k r (patch half
+ * extent)/|P| of the widest group. Replaces the per-(atom, pixel) loop of
+ * the reference (Beam.py:748-808, 8114-8632) where it is admitted.
+ *
+ * mk_plane_fit: per frame, (n_frames, 12) doubles: first pixel, mean column
+ * step, mean row step, largest distance of a pixel from the product grid of
+ * its own column and row coordinates [m], smallest |P| [m], largest
+ * departure of those coordinates from column and row number [pixels].
+ * shapes: device (n_frames, 3) first pixel, ny, nz; max_pix: pixels of the
+ * largest frame; xyz: device pixel coordinates [m]. */
+int mk_plane_fit(int n_frames, const long long *shapes, long long max_pix, const double *xyz,
+                 double *fit, void *stream);
+/* Host only: choose the form's radii, groups and node counts for these tiles
+ * (origins: host copy of mk_tiles.origin) and frames (shapes, fit: host
+ * copies; beam_dirs: (n_frames, 3)). phase_tol [rad] bounds the dropped
+ * third-order terms and the pixels' departure from their grid;
+ * direct_s_per_term is the split kernel's time per (atom, pixel);
+ * group_tiles < 0 chooses the tiles per group, 0 forbids groups. host_buf
+ * (mk_nodes_plan_bytes) receives the frame and source tables; its first
+ * plan->buf_bytes go to the device for mk_kin_nodes_f32. MK_EDECLINE where
+ * the geometry is outside the form or the split kernel is as fast. */
+size_t mk_nodes_plan_bytes(int n_frames, int n_tiles);
+int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const int64_t *counts,
+                  const double *origins, int n_frames, const long long *shapes, const double *fit,
+                  const double *beam_dirs, double k, double phase_tol, double direct_s_per_term,
+                  int group_tiles, mk_node_plan *plan, void *host_buf, size_t host_bytes);
+/* Run a plan: host_buf and its device copy, px with a factor table, the
+ * |d|^2 term kept (fresnel != 0) for tiles wider than fresnel_radius_m.
+ * Output as mk_kin_split_f32 / mk_kin_scan_f32; the plan's wide tiles are
+ * not in it (run them with the split kernel and accumulate). Kernel launches
+ * only: capturable. Workspace of plan->ws_bytes, 256-byte aligned. */
+int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, const mk_pixels *px,
+                     const mk_node_plan *plan, const void *host_buf, const void *dev_buf,
+                     int fresnel, double fresnel_radius_m, double *out, double *intensity_sums,
+                     int accumulate, void *workspace, size_t ws_bytes, void *stream);
 
 /* --- free-space propagation ------------------------------------------- */
 /* Replaces the pad / prop_mul_kernel / crop steps of

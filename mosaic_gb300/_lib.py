@@ -151,8 +151,28 @@ class MkLaunch(ctypes.Structure):
                 ("octet_radius_m", ctypes.c_double)]
 
 
+class MkNodePlan(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_int) for n in
+                ("n_frames", "n_tiles", "n0", "n1", "group_tiles", "n_groups", "n_members", "n_mid",
+                 "n_wide", "n_src", "slices", "src_per_slice", "passes")] + \
+               [(n, ctypes.c_longlong) for n in
+                ("nodes0", "patches1", "weights", "n_pix", "off_src", "off_members", "off_mid",
+                 "off_wide", "buf_bytes", "chunk_bytes", "ws_bytes")] + \
+               [(n, ctypes.c_double) for n in ("radius1_m", "radius2_m", "nodes_s", "direct_s")]
+
+
 # name -> (restype, argtypes)
 SIGNATURES = {
+    "mk_plane_fit": (ctypes.c_int, [ctypes.c_int, _vp, ctypes.c_longlong, _vp, _vp, _vp]),
+    "mk_nodes_plan_bytes": (ctypes.c_size_t, [ctypes.c_int, ctypes.c_int]),
+    "mk_nodes_plan": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_int, _vp, _vp, ctypes.c_int,
+                                     _vp, _vp, _vp, ctypes.c_double, ctypes.c_double,
+                                     ctypes.c_double, ctypes.c_int, ctypes.POINTER(MkNodePlan), _vp,
+                                     ctypes.c_size_t]),
+    "mk_kin_nodes_f32": (ctypes.c_int, [ctypes.POINTER(MkTiles), ctypes.POINTER(MkPhysics),
+                                        ctypes.POINTER(MkPixels), ctypes.POINTER(MkNodePlan), _vp,
+                                        _vp, ctypes.c_int, ctypes.c_double, _vp, _vp, ctypes.c_int,
+                                        _vp, ctypes.c_size_t, _vp]),
     "mk_version": (ctypes.c_int, []),
     "mk_last_error": (ctypes.c_char_p, []),
     "mk_sync_status": (ctypes.c_int, [_vp]),

@@ -54,6 +54,9 @@ class beam:
         self._kernel_phase_tol_rad = 1e-6
         self._kernel_tile_atoms = None      # None: autotuned (512 untuned)
         self._kernel_launch = None          # None: autotuned
+        # sums on plane detectors by node interpolation (engine.NodePlan) where
+        # its plan admits it; False: always per (atom, pixel)
+        self._use_nodes = True
         # tune tile size and launch shape on the first use of a detector size
         # (as the reference tunes its fast kernel on first use, Beam.py:8871-8940);
         # MOSAIC_GB300_AUTOTUNE=0 uses the cached choice or the defaults only
@@ -481,7 +484,44 @@ class beam:
         src = "cached" if autotune.cached(pix.n) is not None else "default"
         return su, tuned_launch(pix.n, su.level, tiles.tile_atoms), src, diag
 
+    def _scatter_nodes(self, atoms, pix, phys, out, accumulate):
+        """The node form of the FP32 sum (detectors on a plane grid, no
+        analyser, no remove_forward), its wide tiles through the split kernel;
+        None where its plan declines."""
+        tiles = engine.Tiles(atoms, self.k, int(self._kernel_tile_atoms or engine.DEFAULT_TILE_ATOMS),
+                             device=atoms.pos.device)
+        tol = min(float(self._kernel_phase_tol_rad), float(self._phase_tol_rad))
+        plan = engine.NodePlan.make(tiles, pix, self.k, tuple(phys.beam_dir), tol)
+        if plan is None:
+            return None
+        cfg = engine.default_launch(4 if pix.squares_fit() else 2, tiles.tile_atoms)
+        info = {}
+        if plan.wide is not None:
+            su, diag = self.split_setup(plan.wide, pix, phys)
+            if su is None:
+                return None
+            cfg = engine.grouping_launch(engine.default_launch(su.level, tiles.tile_atoms), su.level,
+                                         plan.wide, pix, self.k, su.info)
+            out = engine.run_split(plan.wide, pix, phys, atoms.table, launch=cfg, fresnel=su.fresnel,
+                                   out=out, accumulate=accumulate, fresnel_radius=su.fresnel_radius,
+                                   factor_table=True)
+            accumulate = True
+            info = dict(su.info)
+        _, fresnel, _, diag = self.split_budget(tiles, pix.r0_min())
+        res = engine.run_nodes(plan, tiles, pix, phys, atoms.table, out=out, accumulate=accumulate,
+                               fresnel=int(fresnel), fresnel_radius=diag["fresnel_radius_m"])
+        self.last_run = dict(path="split_f32", n_tiles=tiles.n_tiles, tile_atoms=tiles.tile_atoms,
+                             fresnel=bool(fresnel), factor_table=True, launch=dict(cfg),
+                             launch_source="nodes", **plan.info(), **info, **diag)
+        return res
+
     def _scatter_once(self, atoms, pix, phys, out=None, accumulate=False, launch=None):
+        if self._use_fast_kernel and self._use_nodes and not (launch or self._kernel_launch) and \
+                not phys.analyser and not phys.remove_forward and \
+                float(atoms.n) * pix.n >= engine.NODES_MIN_TERMS:
+            res = self._scatter_nodes(atoms, pix, phys, out, accumulate)
+            if res is not None:
+                return res
         if self._use_fast_kernel and atoms.n > 0:
             su, cfg, src, diag = self.choose_split(atoms, pix, phys, launch)
             if su is not None:

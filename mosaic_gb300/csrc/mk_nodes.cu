@@ -1,0 +1,1262 @@
+// Node form of the FP32 split-phase sum (sm_103a): tile fields on a few
+// Chebyshev nodes of the detector, interpolated to its pixels.
+//
+// The field of a compact group of atoms relative to its own centre o,
+//   F(P) = sum_a E_a exp(2 pi i [w(P, o).D_a + the |d|^2 term]),
+// is a smooth function of the pixel position: along one detector axis its
+// phase runs over +-phi, phi = k r (half the patch's extent) / |P|, so on
+// n Chebyshev nodes per axis it is interpolated with a relative error of at
+// most 4 J_n(phi) <= 4 (phi/2)^n / n!. A 512-atom tile (r ~ 2.5 nm) of the
+// 8.19M-atom exposure needs 12 nodes per axis for all of its 512 x 512
+// pixels: 144 terms an atom instead of 262,144. The steps are
+//   leaf    V0[tile][node] = F of every tile on its patch's nodes (the terms
+//           of the split kernel, phase and sin/cos in FP32),
+//   merge   V1[group][fine node]: the tiles of a group (consecutive on the
+//           Hilbert curve) interpolated from the coarse patch's nodes to the
+//           nodes of finer patches, each times exp(2 pi i phase of its origin
+//           relative to the group's), added,
+//   pixels  every group's field interpolated from the fine patch's nodes to
+//           the pixels, times exp(2 pi i phase of the group's origin), added
+//           (Kahan), times the species' factor (mk_factor_table); slices of
+//           groups are reduced in FP64 in fixed order.
+// Tiles wider than the tile radius of the plan skip the merge (their fine
+// nodes are evaluated directly), and tiles wider than the group radius are
+// left to the split kernel. With no groups every tile goes from the leaf
+// straight to the pixels.
+//
+// A phase q.d (q = k/2pi (b - u), up to 1e4 cycles) is formed in two-float
+// FP32 arithmetic (q = qh + ql, d = dh + dl, the product qh dh with its
+// rounding error from an FMA), mod 1 per component: good to ~1e-7 cycles at
+// 1/20 of the FP64 pipe's cost (2 FP64 operations per clock and SM).
+//
+// Measured against the split kernel on every (atom, pixel), through the entry
+// point: 8.19M atoms x 512^2 348 -> 21.0 ms, 5.3M x 1024^2 at 0.5 m 1043 ->
+// 31.0 ms, 2M x 256^2 29.2 -> 8.2 ms, 32k x 128^2 1.43 -> 1.22 ms; a staged
+// scan of 16 frames x 500k atoms 103.5 -> 1.73 ms. Error against FP64 at
+// pixels spread over the detector: peak-relative intensity 4.6e-7 (split
+// kernel 5.0e-7) on the first, 1.9e-6 (2.3e-6) on the second.
+//
+// Interpolation weights are FP64 Lagrange products rounded once; the pixel
+// coordinates they are taken at are the pixels' own (projected on the
+// detector's axes), so an uneven pitch is interpolated exactly; a detector
+// off its plane or off the (column, row) product grid is not admitted.
+#include <vector>
+
+#include "mk_split.cuh"
+
+#define MK_NODE_MAX 16       // nodes per axis at most
+#define MK_NODE_SB 4         // sources staged per step
+#define MK_PIX_COLS 32       // pixel block: 32 columns x 16 rows, 4 rows a thread
+#define MK_PIX_ROWS 16
+#define MK_NODE_PAD 0.25     // half pixel pitches the node interval exceeds the pixel centres
+
+// One frame of a plan. A frame is cut into p1y x p1z fine patches of
+// l1y x l1z pixels, and those into p0y x p0z coarse patches of
+// (ratio_y x ratio_z) fine ones.
+struct MkNodeFrame {
+    double p0[3], ey[3], ez[3], b[3];
+    int ny, nz;
+    int l1y, l1z, p1y, p1z;
+    int ratio_y, ratio_z, p0y, p0z;
+    int bpy, bpz;                       // pixel blocks per fine patch
+    long long pix_off;
+    long long node0_off, patch1_off;    // node1_off = patch1_off * n1^2
+    long long pblk_off, part_off, w_off;
+};
+
+// A source of the pixel step: a group of tiles (count > 0: nar[first ..]) or
+// a single tile (count 0).
+struct MkNodeSrc {
+    float dh[3];
+    int species;
+    float dl[3];
+    int count;
+    double o[3];
+    long long first;
+};
+
+struct MkNodeRec {       // one node's direction: 64 bytes
+    float4 w;            // b - u, 1/|P|
+    float4 u;            // u, b.x
+    float4 qh;           // k/2pi (b - u), high parts, b.y
+    float4 ql;           // low parts, b.z
+};
+
+// ------------------------------------------------------------- plane fit
+// Per frame: first pixel, mean column and row steps, and how far the pixels
+// are from the product grid p0 + y_col ey + z_row ez of their own projected
+// coordinates (fit[9], m), the smallest |P| (fit[10]) and the largest
+// departure of y_col, z_row from column and row number (fit[11], pixels).
+__device__ __forceinline__ void mk_fit_axes(const double *xyz, int ny, int nz, double *p0, double *ey,
+                                            double *ez)
+{
+    for (int c = 0; c < 3; ++c) {
+        p0[c] = xyz[c];
+        ey[c] = ny > 1 ? (xyz[3ll * (ny - 1) + c] - p0[c]) / (ny - 1) : 0.0;
+        ez[c] = nz > 1 ? (xyz[3ll * (nz - 1) * ny + c] - p0[c]) / (nz - 1) : 0.0;
+    }
+}
+
+// Coordinate of a first-row (first-column) pixel along its axis, in steps.
+__device__ __forceinline__ double mk_axis_coord(const double *p, const double *p0, const double *e)
+{
+    const double n2 = e[0] * e[0] + e[1] * e[1] + e[2] * e[2];
+    if (!(n2 > 0.0)) return 0.0;
+    return ((p[0] - p0[0]) * e[0] + (p[1] - p0[1]) * e[1] + (p[2] - p0[2]) * e[2]) / n2;
+}
+
+__global__ void mk_fit_init_kernel(int n_frames, const long long *__restrict__ shapes,
+                                   const double *__restrict__ xyz, double *__restrict__ fit)
+{
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= n_frames) return;
+    const double *p = xyz + 3 * shapes[3 * f];
+    double *o = fit + 12 * (long long)f;
+    mk_fit_axes(p, (int)shapes[3 * f + 1], (int)shapes[3 * f + 2], o, o + 3, o + 6);
+    o[9] = 0.0;
+    o[10] = 1e300;
+    o[11] = 0.0;
+}
+
+__global__ void mk_fit_kernel(const long long *__restrict__ shapes, const double *__restrict__ xyz,
+                              double *__restrict__ fit)
+{
+    const int f = blockIdx.x;
+    const long long off = shapes[3 * f];
+    const int ny = (int)shapes[3 * f + 1], nz = (int)shapes[3 * f + 2];
+    const double *P = xyz + 3 * off;
+    double *o = fit + 12 * (long long)f;
+    double p0[3], ey[3], ez[3];
+    mk_fit_axes(P, ny, nz, p0, ey, ez);
+    double dev = 0.0, rmin = 1e300, skew = 0.0;
+    const long long n = (long long)ny * nz;
+    for (long long i = (long long)blockIdx.y * blockDim.x + threadIdx.x; i < n;
+         i += (long long)gridDim.y * blockDim.x) {
+        const int row = (int)(i / ny), col = (int)(i - (long long)row * ny);
+        const double y = mk_axis_coord(P + 3ll * col, p0, ey);
+        const double z = mk_axis_coord(P + 3ll * row * ny, p0, ez);
+        double d2 = 0.0, r2 = 0.0;
+        for (int c = 0; c < 3; ++c) {
+            const double v = P[3 * i + c], m = p0[c] + y * ey[c] + z * ez[c];
+            d2 += (v - m) * (v - m);
+            r2 += v * v;
+        }
+        const double d = sqrt(d2), s = fmax(fabs(y - (ny > 1 ? col : 0)), fabs(z - (nz > 1 ? row : 0)));
+        dev = fmax(dev, d <= 1e300 ? d : INFINITY);         // a NaN counts as infinite
+        skew = fmax(skew, s <= 1e300 ? s : INFINITY);
+        rmin = fmin(rmin, r2 >= 0.0 ? sqrt(r2) : 0.0);
+    }
+    for (int w = 16; w > 0; w >>= 1) {
+        dev = fmax(dev, __shfl_xor_sync(0xffffffffu, dev, w));
+        skew = fmax(skew, __shfl_xor_sync(0xffffffffu, skew, w));
+        rmin = fmin(rmin, __shfl_xor_sync(0xffffffffu, rmin, w));
+    }
+    if ((threadIdx.x & 31) == 0) {      // non-negative doubles order as their bits
+        atomicMax(reinterpret_cast<unsigned long long *>(o + 9), (unsigned long long)__double_as_longlong(dev));
+        atomicMin(reinterpret_cast<unsigned long long *>(o + 10), (unsigned long long)__double_as_longlong(rmin));
+        atomicMax(reinterpret_cast<unsigned long long *>(o + 11), (unsigned long long)__double_as_longlong(skew));
+    }
+}
+
+extern "C" int mk_plane_fit(int n_frames, const long long *shapes, long long max_pix, const double *xyz,
+                            double *fit, void *stream)
+{
+    MK_REQUIRE(n_frames >= 1 && shapes && xyz && fit && max_pix >= 1, "mk_plane_fit: bad arguments");
+    cudaStream_t st = mk_stream(stream);
+    mk_fit_init_kernel<<<(n_frames + 127) / 128, 128, 0, st>>>(n_frames, shapes, xyz, fit);
+    const int gy = (int)std::max<long long>(1, std::min<long long>((max_pix + 1023) / 1024, 512));
+    mk_fit_kernel<<<dim3(n_frames, gy), 256, 0, st>>>(shapes, xyz, fit);
+    MK_CHECK_CUDA(cudaGetLastError());
+    return MK_OK;
+}
+
+// ------------------------------------------------------------------ plan
+#define MK_SUM_PARTS 64      // chunks a frame's intensity sum is added in
+namespace {
+
+const int kNodeCounts[] = {6, 8, 10, 12, 16};
+
+// Largest phase half-range phi [rad] n Chebyshev nodes interpolate to
+// 4 (phi/2)^n / n! <= 3e-8.
+double phi_max(int n)
+{
+    double f = 7.5e-9;
+    for (int i = 2; i <= n; ++i) f *= i;
+    return 2.0 * std::pow(f, 1.0 / n);
+}
+
+// Largest patch (pixels) whose phase half-range stays within `phi` for atoms
+// up to k r = kr [rad] off the centre, a rad of direction per pixel.
+double patch_limit(double phi, double kr, double a)
+{
+    const double half = phi / std::max(1.05 * kr * a, 1e-300);   // pixels, pad included
+    return std::min(2.0 * (half - MK_NODE_PAD) + 1.0, 1e9);
+}
+
+// Even cut of n pixels into patches of at most `most`, a multiple of `unit`
+// unless one patch holds all; false when even `unit` pixels are too many.
+bool cut(int n, double most, int unit, int *len, int *count)
+{
+    if (most >= n) { *len = n; *count = 1; return true; }
+    const int lim = (int)(most / unit) * unit;
+    if (lim < unit) return false;
+    const int c = (n + lim - 1) / lim;
+    *len = ((n + c - 1) / c + unit - 1) / unit * unit;
+    *count = (n + *len - 1) / *len;
+    return true;
+}
+
+// One ROI shape: the widest angular steps of its frames, and how many there are.
+struct Geo { double ay, az; int ny, nz, frames; };
+
+// Fine patches of every ROI shape for sources of radius r2 on n1 nodes, and
+// coarse ones (n0 > 0) for tiles of radius r1; the nodes of all frames.
+bool lay_out(const std::vector<Geo> &g, double k, double r2, int n1, double r1, int n0,
+             std::vector<MkNodeFrame> *out, double *nodes1, double *nodes0)
+{
+    *nodes1 = *nodes0 = 0.0;
+    for (size_t f = 0; f < g.size(); ++f) {
+        MkNodeFrame F{};
+        if (!cut(g[f].ny, patch_limit(phi_max(n1), k * r2, g[f].ay), MK_PIX_COLS, &F.l1y, &F.p1y) ||
+            !cut(g[f].nz, patch_limit(phi_max(n1), k * r2, g[f].az), MK_PIX_ROWS, &F.l1z, &F.p1z))
+            return false;
+        F.ratio_y = F.ratio_z = F.p0y = F.p0z = 1;
+        if (n0 > 0) {
+            const double ly = patch_limit(phi_max(n0), k * r1, g[f].ay), lz = patch_limit(phi_max(n0), k * r1, g[f].az);
+            const int ry = (int)std::min<double>(F.p1y, std::floor(ly / F.l1y));
+            const int rz = (int)std::min<double>(F.p1z, std::floor(lz / F.l1z));
+            if (ry < 1 || rz < 1) return false;
+            F.p0y = (F.p1y + ry - 1) / ry;
+            F.p0z = (F.p1z + rz - 1) / rz;
+            F.ratio_y = (F.p1y + F.p0y - 1) / F.p0y;
+            F.ratio_z = (F.p1z + F.p0z - 1) / F.p0z;
+            F.p0y = (F.p1y + F.ratio_y - 1) / F.ratio_y;
+            F.p0z = (F.p1z + F.ratio_z - 1) / F.ratio_z;
+            *nodes0 += (double)g[f].frames * F.p0y * F.p0z * n0 * n0;
+        }
+        F.ny = g[f].ny;
+        F.nz = g[f].nz;
+        F.bpy = (F.l1y + MK_PIX_COLS - 1) / MK_PIX_COLS;
+        F.bpz = (F.l1z + MK_PIX_ROWS - 1) / MK_PIX_ROWS;
+        *nodes1 += (double)g[f].frames * F.p1y * F.p1z * n1 * n1;
+        if (out) (*out)[f] = F;
+    }
+    return true;
+}
+
+struct Ball { double c[3], r; };
+
+// Ball around the tiles idx[a..b): centre of the box of their balls.
+Ball bound(const double *org, const std::vector<int> &idx, size_t a, size_t b)
+{
+    double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
+    for (size_t i = a; i < b; ++i) {
+        const double *o = org + 4ll * idx[i];
+        for (int c = 0; c < 3; ++c) {
+            lo[c] = std::min(lo[c], o[c] - o[3]);
+            hi[c] = std::max(hi[c], o[c] + o[3]);
+        }
+    }
+    Ball B;
+    for (int c = 0; c < 3; ++c) B.c[c] = 0.5 * (lo[c] + hi[c]);
+    B.r = 0.0;
+    for (size_t i = a; i < b; ++i) {
+        const double *o = org + 4ll * idx[i];
+        const double dx = o[0] - B.c[0], dy = o[1] - B.c[1], dz = o[2] - B.c[2];
+        B.r = std::max(B.r, std::sqrt(dx * dx + dy * dy + dz * dz) + o[3]);
+    }
+    return B;
+}
+
+double quantile(std::vector<double> v, double q)
+{
+    if (v.empty()) return 0.0;
+    const size_t i = std::min(v.size() - 1, (size_t)std::floor(q * (v.size() - 1) + 0.5));
+    std::nth_element(v.begin(), v.begin() + i, v.end());
+    return v[i];
+}
+
+size_t up256(size_t b) { return (b + 255) & ~(size_t)255; }
+
+// Costs [s] of one leaf term, one (source, pixel) and one (tile, fine node)
+// of the merge, and what a launch costs.
+const double kLeaf = 0.55e-12, kPix = 4.5e-12, kMerge = 6.0e-12, kLaunch = 4e-6;
+
+struct Choice {
+    double cost = 1e300, r1 = 0.0, r2 = 0.0;
+    int n0 = 0, n1 = 0, G = 0;
+};
+
+}  // namespace
+
+extern "C" size_t mk_nodes_plan_bytes(int n_frames, int n_tiles)
+{
+    if (n_frames < 1 || n_tiles < 0) return 0;
+    return up256(sizeof(MkNodeFrame) * (size_t)n_frames) + up256(sizeof(MkNodeSrc) * (size_t)n_tiles) +
+           3 * up256(sizeof(int) * (size_t)n_tiles);
+}
+
+extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const int64_t *counts,
+                             const double *origins, int n_frames, const long long *shapes,
+                             const double *fit, const double *beam_dirs, double k, double phase_tol,
+                             double direct_s_per_term, int group_tiles, mk_node_plan *plan,
+                             void *host_buf, size_t host_bytes)
+{
+    MK_REQUIRE(n_tiles >= 1 && n_frames >= 1 && counts && origins && shapes && fit && beam_dirs && plan &&
+                   host_buf && n_species >= 1 && n_species <= MK_MAX_SPECIES && tile_atoms >= 1,
+               "mk_nodes_plan: bad arguments");
+    MK_REQUIRE(host_bytes >= mk_nodes_plan_bytes(n_frames, n_tiles), "mk_nodes_plan: buffer too small");
+    memset(plan, 0, sizeof(*plan));
+    std::vector<Geo> geo;
+    std::vector<int> shape_of(n_frames);
+    double n_pix = 0.0, rmin = 1e300, dev = 0.0;
+    for (int f = 0; f < n_frames; ++f) {
+        const double *t = fit + 12ll * f;
+        // the fit's own sanity: on the grid, within a quarter pixel of it
+        if (!(t[9] <= 1e300) || !(t[11] <= 0.25) || !(t[10] > 0.0)) {
+            mk_set_error("mk_nodes_plan: frame %d is not a plane grid of pixels", f);
+            return MK_EDECLINE;
+        }
+        const int ny = (int)shapes[3 * f + 1], nz = (int)shapes[3 * f + 2];
+        size_t i = 0;
+        while (i < geo.size() && (geo[i].ny != ny || geo[i].nz != nz)) ++i;
+        if (i == geo.size()) geo.push_back(Geo{0.0, 0.0, ny, nz, 0});
+        shape_of[f] = (int)i;
+        geo[i].ay = std::max(geo[i].ay, std::sqrt(t[3] * t[3] + t[4] * t[4] + t[5] * t[5]) / t[10]);
+        geo[i].az = std::max(geo[i].az, std::sqrt(t[6] * t[6] + t[7] * t[7] + t[8] * t[8]) / t[10]);
+        ++geo[i].frames;
+        n_pix += (double)ny * nz;
+        rmin = std::min(rmin, t[10]);
+        dev = std::max(dev, t[9] / t[10]);
+    }
+    std::vector<int> tsp(n_tiles);
+    {
+        int t = 0;
+        for (int s = 0; s < n_species; ++s)
+            for (int64_t i = 0; i < (counts[s] + tile_atoms - 1) / tile_atoms; ++i)
+                if (t < n_tiles) tsp[t++] = s;
+        MK_REQUIRE(t == n_tiles, "mk_nodes_plan: %d tiles, the species counts give %d", n_tiles, t);
+    }
+    std::vector<double> rad(n_tiles);
+    double rmax = 0.0, omax = 0.0;
+    for (int t = 0; t < n_tiles; ++t) {
+        const double *o = origins + 4ll * t;
+        rad[t] = o[3];
+        const double on = std::sqrt(o[0] * o[0] + o[1] * o[1] + o[2] * o[2]);
+        if (!(o[3] < 1.0) || !(on < 1.0)) {
+            mk_set_error("mk_nodes_plan: tile %d has no finite extent", t);
+            return MK_EDECLINE;
+        }
+        rmax = std::max(rmax, o[3]);
+        omax = std::max(omax, on);
+    }
+    // the factor is taken at the pixels' own directions (as the split
+    // kernel's factor table), and third-order terms are dropped
+    auto admitted = [&](double r) {
+        const double third = k * (r * r * r + omax * omax * omax + 3.0 * omax * omax * r) / (rmin * rmin);
+        return third + k * r * dev <= phase_tol && 2.0 * (omax + r) / rmin < 1e-6;
+    };
+    const double T = tile_atoms;
+    auto direct = [&](double n) { return n * T * n_pix * direct_s_per_term; };
+    plan->direct_s = direct(n_tiles) + 2.0 * kLaunch;
+
+    Choice best;
+    const double q1[] = {1.0, 0.99, 0.9};
+    for (int iq = 0; iq < 3; ++iq) {
+        const double r1 = quantile(rad, q1[iq]);
+        if (iq > 0 && r1 == rmax) continue;
+        std::vector<int> nar;
+        for (int t = 0; t < n_tiles; ++t)
+            if (rad[t] <= r1) nar.push_back(t);
+        const double n_nar = (double)nar.size();
+        // no groups: every tile within r1 straight from its nodes
+        if (admitted(r1) && group_tiles <= 0)
+            for (int n1 : kNodeCounts) {
+                double N1, N0;
+                if (!lay_out(geo, k, r1, n1, 0.0, 0, nullptr, &N1, &N0)) continue;
+                const double c = n_nar * T * N1 * kLeaf + n_nar * n_pix * kPix * (0.4 + 0.05 * n1) +
+                                 direct(n_tiles - n_nar) + 4.0 * kLaunch;
+                if (c < best.cost) { best.cost = c; best.r1 = best.r2 = r1; best.n0 = 0; best.n1 = n1; best.G = 0; }
+            }
+        if (group_tiles == 0 || (group_tiles < 0 && n_tiles < 32)) continue;
+        for (int G = group_tiles > 0 ? group_tiles : 8; G <= (group_tiles > 0 ? group_tiles : 128); G *= 2) {
+            std::vector<double> gr;
+            std::vector<int> gn;
+            for (size_t a = 0; a < nar.size();) {
+                size_t b = a;
+                while (b < nar.size() && b < a + G && tsp[nar[b]] == tsp[nar[a]]) ++b;
+                gr.push_back(bound(origins, nar, a, b).r);
+                gn.push_back((int)(b - a));
+                a = b;
+            }
+            for (double q2 : {1.0, 0.95, 0.8}) {
+                const double r2 = std::max(quantile(gr, q2), r1);
+                if (!admitted(r2)) continue;
+                double groups = 0, in_groups = 0, mid = 0, wide = 0;
+                for (size_t i = 0; i < gr.size(); ++i) {
+                    if (gr[i] <= r2) { groups += 1; in_groups += gn[i]; }
+                    else mid += gn[i];
+                }
+                for (int t = 0; t < n_tiles; ++t)
+                    if (rad[t] > r1) (rad[t] <= r2 ? mid : wide) += 1;
+                for (int n1 : kNodeCounts) {
+                    if (n1 > 12) continue;
+                    for (int n0 : kNodeCounts) {
+                        if (n0 < 8) continue;
+                        double N1, N0;
+                        if (!lay_out(geo, k, r2, n1, r1, n0, nullptr, &N1, &N0)) continue;
+                        const double c = in_groups * T * N0 * kLeaf + mid * T * N1 * kLeaf +
+                                         in_groups * N1 * kMerge * (0.4 + 0.05 * n0) +
+                                         (groups + mid) * n_pix * kPix * (0.4 + 0.05 * n1) + direct(wide) +
+                                         6.0 * kLaunch;
+                        if (c < best.cost) { best.cost = c; best.r1 = r1; best.r2 = r2; best.n0 = n0; best.n1 = n1; best.G = G; }
+                    }
+                }
+            }
+        }
+    }
+    plan->nodes_s = best.cost;
+    if (!(best.cost < plan->direct_s)) {
+        mk_set_error("mk_nodes_plan: the direct sum is as fast (%.3g s against %.3g s) or the geometry "
+                     "leaves the error budget", plan->direct_s, best.cost);
+        return MK_EDECLINE;
+    }
+    // lay the chosen plan out
+    std::vector<MkNodeFrame> fr(n_frames), cuts(geo.size());
+    double N1, N0;
+    lay_out(geo, k, best.r2, best.n1, best.r1, best.n0, &cuts, &N1, &N0);
+    for (int f = 0; f < n_frames; ++f) fr[f] = cuts[shape_of[f]];
+    std::vector<MkNodeSrc> src;
+    std::vector<int> nar, members, mid, wide;
+    for (int t = 0; t < n_tiles; ++t) {
+        if (rad[t] <= best.r1) nar.push_back(t);
+        else if (rad[t] <= best.r2) mid.push_back(t);
+        else wide.push_back(t);
+    }
+    auto add_src = [&](const double *c, int species, int count, long long first) {
+        MkNodeSrc S{};
+        for (int i = 0; i < 3; ++i) {
+            S.o[i] = c[i];
+            S.dh[i] = (float)c[i];
+            S.dl[i] = (float)(c[i] - (double)S.dh[i]);
+        }
+        S.species = species;
+        S.count = count;
+        S.first = first;
+        src.push_back(S);
+    };
+    if (best.G == 0) {
+        mid.insert(mid.end(), nar.begin(), nar.end());
+    } else {
+        for (size_t a = 0; a < nar.size();) {
+            size_t b = a;
+            while (b < nar.size() && b < a + best.G && tsp[nar[b]] == tsp[nar[a]]) ++b;
+            const Ball B = bound(origins, nar, a, b);
+            if (B.r <= best.r2) {
+                add_src(B.c, tsp[nar[a]], (int)(b - a), (long long)members.size());
+                members.insert(members.end(), nar.begin() + a, nar.begin() + b);
+            } else {
+                mid.insert(mid.end(), nar.begin() + a, nar.begin() + b);
+            }
+            a = b;
+        }
+    }
+    std::sort(mid.begin(), mid.end());          // by species
+    plan->n_groups = (int)src.size();
+    for (int t : mid) add_src(origins + 4ll * t, tsp[t], 0, 0);
+    plan->n_src = (int)src.size();
+    plan->n_members = (int)members.size();
+    plan->n_mid = (int)mid.size();
+    plan->n_wide = (int)wide.size();
+    plan->n0 = best.G ? best.n0 : 0;
+    plan->n1 = best.n1;
+    plan->n_frames = n_frames;
+    plan->n_tiles = n_tiles;
+    plan->group_tiles = best.G;
+    plan->radius1_m = best.r1;
+    plan->radius2_m = best.r2;
+    plan->n_pix = (long long)n_pix;
+    if (plan->n_src < 1) {
+        mk_set_error("mk_nodes_plan: every tile is wider than the plan's radius");
+        return MK_EDECLINE;
+    }
+    long long pblk = 0, wf = 0, patch = 0, node0 = 0;
+    for (int f = 0; f < n_frames; ++f) {
+        MkNodeFrame &F = fr[f];
+        const double *t = fit + 12ll * f;
+        for (int c = 0; c < 3; ++c) {
+            F.p0[c] = t[c];
+            F.ey[c] = t[3 + c];
+            F.ez[c] = t[6 + c];
+            F.b[c] = beam_dirs[3ll * f + c];
+        }
+        F.pix_off = shapes[3 * f];
+        F.node0_off = node0;
+        F.patch1_off = patch;
+        F.pblk_off = pblk;
+        F.w_off = wf;
+        patch += (long long)F.p1y * F.p1z;
+        node0 += best.G ? (long long)F.p0y * F.p0z * best.n0 * best.n0 : 0;
+        pblk += (long long)F.p1y * F.p1z * F.bpy * F.bpz;
+        wf += (long long)best.n1 * (F.ny + F.nz) +
+              (best.G ? (long long)best.n1 * best.n0 * (F.ratio_y + F.ratio_z) : 0);
+    }
+    plan->nodes0 = node0;
+    plan->patches1 = patch;
+    plan->weights = wf;
+    // slices of sources: enough blocks for every SM several times over, at
+    // least two staging steps a slice
+    int sms = 152, devid = 0;
+    if (cudaGetDevice(&devid) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, devid);
+    const long long want = (12ll * sms + pblk - 1) / pblk;
+    plan->slices = (int)std::max<long long>(1, std::min<long long>(std::min<long long>(want, 256),
+                                                                   plan->n_src / (2 * MK_NODE_SB)));
+    plan->src_per_slice = (plan->n_src + plan->slices - 1) / plan->slices;
+    plan->slices = (plan->n_src + plan->src_per_slice - 1) / plan->src_per_slice;
+    for (int f = 0; f < n_frames; ++f) fr[f].part_off = fr[f].pix_off * plan->slices;
+    // frames per pass: as many as a few GB of node fields and partials hold
+    const double n1sq = (double)best.n1 * best.n1;
+    size_t need = 0;
+    const size_t budget = (size_t)4 << 30;
+    long long chunk_n0 = 0, chunk_p1 = 0, chunk_pix = 0;
+    int fa = 0;
+    auto bytes = [&](long long a, long long b, long long c) {
+        return up256(8 * (size_t)(a * (long long)members.size())) +
+               up256((size_t)(8.0 * b * n1sq * plan->n_src)) + up256(16 * (size_t)c * plan->slices);
+    };
+    int passes = 1;
+    for (int f = 0; f < n_frames; ++f) {
+        const long long a = best.G ? (long long)fr[f].p0y * fr[f].p0z * best.n0 * best.n0 : 0;
+        const long long b = (long long)fr[f].p1y * fr[f].p1z, c = (long long)fr[f].ny * fr[f].nz;
+        const bool too_many = (chunk_p1 + b) * std::max(plan->n_groups, 1) > (1ll << 30) ||
+                              (chunk_n0 + a) > 256ll * 60000 || (chunk_p1 + b) * n1sq > 256.0 * 60000;
+        if (f > fa && (bytes(chunk_n0 + a, chunk_p1 + b, chunk_pix + c) > budget || too_many)) {
+            ++passes;
+            fa = f;
+            chunk_n0 = chunk_p1 = chunk_pix = 0;
+        }
+        chunk_n0 += a;
+        chunk_p1 += b;
+        chunk_pix += c;
+        need = std::max(need, bytes(chunk_n0, chunk_p1, chunk_pix));
+    }
+    plan->passes = passes;
+    if (need > ((size_t)16 << 30)) {
+        mk_set_error("mk_nodes_plan: %zu bytes of node fields for one frame", need);
+        return MK_EDECLINE;
+    }
+    plan->chunk_bytes = need;
+    plan->ws_bytes = up256(sizeof(MkNodeRec) * (size_t)(node0 + patch * best.n1 * best.n1)) +
+                     up256(sizeof(float) * (size_t)wf) +
+                     std::max(need, up256(8 * (size_t)MK_SUM_PARTS * n_frames));
+    char *hb = static_cast<char *>(host_buf);
+    size_t off = 0;
+    auto put = [&](const void *p, size_t n) {
+        const size_t at = off;
+        if (n) memcpy(hb + at, p, n);
+        off += up256(n);
+        return (long long)at;
+    };
+    put(fr.data(), sizeof(MkNodeFrame) * fr.size());
+    plan->off_src = put(src.data(), sizeof(MkNodeSrc) * src.size());
+    plan->off_members = put(members.data(), sizeof(int) * members.size());
+    plan->off_mid = put(mid.data(), sizeof(int) * mid.size());
+    plan->off_wide = put(wide.data(), sizeof(int) * wide.size());
+    plan->buf_bytes = (long long)off;
+    return MK_OK;
+}
+
+// --------------------------------------------------------------- kernels
+struct MkNodeArgs {
+    const MkNodeFrame *frames;
+    int f_lo, f_hi;                  // frames of this pass
+    int n0, n1, n_groups, n_src, src_per_slice, tile_atoms;
+    long long nodes0, patches1;      // of this pass
+    long long node0_base, patch1_base, pblk_base, part_base;
+    const MkNodeSrc *src;
+    const int *members;
+    const MkNodeRec *rec0, *rec1;    // of every frame
+    const float *weights;
+    float2 *V0, *V1;
+    const double4 *origin;
+    const float4 *tpos;
+    const float2 *tamp;
+    const double4 *q;
+    const float4 *u;
+    const float2 *ftab;
+    long long ftab_n;
+    double2 *partial;
+    float kappa, fres_r;
+    double kappa_d;
+    int fresnel, decay;
+};
+
+// First frame f in [lo, hi) whose key(f+1) exceeds i.
+template <class Key>
+__device__ __forceinline__ int mk_find_frame(int lo, int hi, long long i, Key key)
+{
+    --hi;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (key(mid) <= i) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+
+__device__ __forceinline__ double mk_cheb(int i, int n) { return cospi((2 * i + 1) / (2.0 * n)); }
+
+// Lagrange weights at x of the n Chebyshev nodes, FP64 products rounded once.
+__device__ void mk_lagrange(double x, int n, float *out)
+{
+    double xs[MK_NODE_MAX];
+    for (int i = 0; i < n; ++i) xs[i] = mk_cheb(i, n);
+    for (int j = 0; j < n; ++j) {
+        double num = 1.0, den = 1.0;
+        for (int i = 0; i < n; ++i)
+            if (i != j) {
+                num *= x - xs[i];
+                den *= xs[j] - xs[i];
+            }
+        out[j] = (float)(num / den);
+    }
+}
+
+__device__ __forceinline__ double mk_half_range(int len) { return 0.5 * (len - 1) + MK_NODE_PAD; }
+
+// Node records and weight tables of every frame; one thread per node, pixel
+// column, pixel row and fine node position. A few thousand FP64 operations a
+// thread at most, launched once per sum: latency (7 us), not throughput.
+__global__ void mk_node_prep_kernel(const MkNodeFrame *__restrict__ frames, int n0, int n1, double kappa,
+                                    const double *__restrict__ xyz, MkNodeRec *__restrict__ rec0,
+                                    MkNodeRec *__restrict__ rec1, float *__restrict__ weights)
+{
+    const MkNodeFrame F = frames[blockIdx.x];
+    const int l0y = F.l1y * F.ratio_y, l0z = F.l1z * F.ratio_z;
+    const int a0 = n0 ? F.p0y * F.p0z * n0 * n0 : 0, a1 = F.p1y * F.p1z * n1 * n1;
+    const int wy = F.ny, wz = F.nz, my = n0 ? F.ratio_y * n1 : 0, mz = n0 ? F.ratio_z * n1 : 0;
+    const int total = a0 + a1 + wy + wz + my + mz;
+    float *W = weights + F.w_off;
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < total; i += gridDim.y * blockDim.x) {
+        int e = i;
+        if (e < a0 + a1) {
+            const bool fine = e >= a0;
+            if (fine) e -= a0;
+            const int n = fine ? n1 : n0, py = fine ? F.p1y : F.p0y;
+            const int ly = fine ? F.l1y : l0y, lz = fine ? F.l1z : l0z;
+            const int p = e / (n * n), r = e - p * n * n, j = r / n, c = r - j * n;
+            const int pz = p / py, pyi = p - pz * py;
+            const double y = pyi * (double)ly + 0.5 * (ly - 1) + mk_half_range(ly) * mk_cheb(c, n);
+            const double z = pz * (double)lz + 0.5 * (lz - 1) + mk_half_range(lz) * mk_cheb(j, n);
+            double P[3], u[3], q[3], r2 = 0.0;
+            for (int d = 0; d < 3; ++d) {
+                P[d] = F.p0[d] + y * F.ey[d] + z * F.ez[d];
+                r2 += P[d] * P[d];
+            }
+            const double inv = 1.0 / sqrt(r2);
+            for (int d = 0; d < 3; ++d) {
+                u[d] = P[d] * inv;
+                q[d] = kappa * (F.b[d] - u[d]);
+            }
+            const float hx = (float)q[0], hy = (float)q[1], hz = (float)q[2];
+            MkNodeRec R;
+            R.w = make_float4((float)(F.b[0] - u[0]), (float)(F.b[1] - u[1]), (float)(F.b[2] - u[2]), (float)inv);
+            R.u = make_float4((float)u[0], (float)u[1], (float)u[2], (float)F.b[0]);
+            R.qh = make_float4(hx, hy, hz, (float)F.b[1]);
+            R.ql = make_float4((float)(q[0] - hx), (float)(q[1] - hy), (float)(q[2] - hz), (float)F.b[2]);
+            if (fine) rec1[F.patch1_off * n1 * n1 + e] = R;
+            else rec0[F.node0_off + e] = R;
+            continue;
+        }
+        e -= a0 + a1;
+        float out[MK_NODE_MAX];
+        if (e < wy + wz) {                 // a pixel column or row in its fine patch
+            const bool row = e >= wy;
+            if (row) e -= wy;
+            const int len = row ? F.l1z : F.l1y;
+            const double *P = xyz + 3 * (F.pix_off + (row ? (long long)e * F.ny : e));
+            double v = mk_axis_coord(P, F.p0, row ? F.ez : F.ey);
+            const double c = (e / len) * (double)len + 0.5 * (len - 1);
+            mk_lagrange((v - c) / mk_half_range(len), n1, out);
+            float *o = W + (row ? (long long)n1 * F.ny : 0) + (long long)e * n1;
+            for (int j = 0; j < n1; ++j) o[j] = out[j];
+            continue;
+        }
+        e -= wy + wz;                      // a fine node's position in the coarse patch
+        const bool row = e >= my;
+        if (row) e -= my;
+        const int l1 = row ? F.l1z : F.l1y, l0 = row ? l0z : l0y;
+        const int sub = e / n1, c = e - sub * n1;
+        const double v = sub * (double)l1 + 0.5 * (l1 - 1) + mk_half_range(l1) * mk_cheb(c, n1);
+        mk_lagrange((v - 0.5 * (l0 - 1)) / mk_half_range(l0), n0, out);
+        float *o = W + (long long)n1 * (F.ny + F.nz) + (row ? (long long)F.ratio_y * n1 * n0 : 0) + (long long)e * n0;
+        for (int j = 0; j < n0; ++j) o[j] = out[j];
+    }
+}
+
+// A tile's field on the nodes: V[list position][node]. One node a thread,
+// the tile's atoms (interleaved pairs) from shared memory, two atoms per
+// packed instruction. Bound by the MUFU (two results a term, 16 per clock
+// and SM); the phase is always reduced mod 1, so __sincosf stays at its
+// 3.5e-7 absolute error.
+__global__ void __launch_bounds__(256) mk_node_leaf_kernel(const MkNodeArgs A, const int *__restrict__ list,
+                                                           const MkNodeRec *__restrict__ rec,
+                                                           long long n_nodes, float2 *__restrict__ V)
+{
+    extern __shared__ __align__(16) unsigned char leaf_smem[];
+    const int T = A.tile_atoms;
+    float4 *s_pos = reinterpret_cast<float4 *>(leaf_smem);
+    float4 *s_amp = s_pos + T;
+    const int t = list[blockIdx.x];
+    const float4 *gp = A.tpos + (size_t)t * T;
+    const float4 *ga = reinterpret_cast<const float4 *>(A.tamp + (size_t)t * T);
+    for (int i = threadIdx.x; i < T; i += blockDim.x) s_pos[i] = gp[i];
+    for (int i = threadIdx.x; i < T / 2; i += blockDim.x) s_amp[i] = ga[i];
+    __syncthreads();
+    const long long g = (long long)blockIdx.y * blockDim.x + threadIdx.x;
+    if (g >= n_nodes) return;
+    const double4 o = A.origin[t];
+    const float ox = (float)o.x, oy = (float)o.y, oz = (float)o.z;
+    const float4 w4 = rec[g].w, u4 = rec[g].u;
+    const float uo = fmaf(u4.z, oz, fmaf(u4.y, oy, u4.x * ox));
+    // w = b - u', u' the direction from the tile's origin
+    const mk_f2 wx = f2_splat(fmaf(ox - uo * u4.x, w4.w, w4.x));
+    const mk_f2 wy = f2_splat(fmaf(oy - uo * u4.y, w4.w, w4.y));
+    const mk_f2 wz = f2_splat(fmaf(oz - uo * u4.z, w4.w, w4.z));
+    const mk_f2 magic = f2_splat(MK_ROUND_MAGIC), two_pi = f2_splat(TWO_PI_F), m_one = f2_splat(-1.f);
+    mk_f2 ar = 0ull, ai = 0ull;
+    const ulonglong2 *P2 = reinterpret_cast<const ulonglong2 *>(s_pos);
+    const ulonglong2 *E2 = reinterpret_cast<const ulonglong2 *>(s_amp);
+    const bool fr = A.fresnel && (float)o.w > A.fres_r;
+    mk_f2 bx = 0ull, by = 0ull, bz = 0ull, hq = 0ull;
+    if (fr) {
+        bx = f2_splat(u4.w);
+        by = f2_splat(rec[g].qh.w);
+        bz = f2_splat(rec[g].ql.w);
+        hq = f2_splat(0.5f * w4.w / (A.kappa * fmaf(-uo, w4.w, 1.f)));
+    }
+#pragma unroll 4
+    for (int p = 0; p < T / 2; ++p) {
+        const ulonglong2 a = P2[2 * p], b = P2[2 * p + 1], e = E2[p];
+        mk_f2 lin = f2_fma(b.x, wz, f2_fma(a.y, wy, f2_mul(a.x, wx)));
+        if (fr) {
+            const mk_f2 sp = f2_sub(f2_fma(b.x, bz, f2_fma(a.y, by, f2_mul(a.x, bx))), lin);
+            lin = f2_fma(f2_fma(f2_mul(sp, m_one), sp, b.y), hq, lin);
+        }
+        const float2 r = f2_unpack(f2_mul(f2_sub(lin, f2_sub(f2_add(lin, magic), magic)), two_pi));
+        float s0, c0, s1, c1;
+        __sincosf(r.x, &s0, &c0);
+        __sincosf(r.y, &s1, &c1);
+        const mk_f2 c = f2_pack(c0, c1), s = f2_pack(s0, s1);
+        ar = f2_fma(e.x, c, f2_fma(f2_mul(e.y, m_one), s, ar));
+        ai = f2_fma(e.x, s, f2_fma(e.y, c, ai));
+    }
+    const float2 r2 = f2_unpack(ar), i2 = f2_unpack(ai);
+    V[(long long)blockIdx.x * n_nodes + g] = make_float2(r2.x + r2.y, i2.x + i2.y);
+}
+
+__device__ __forceinline__ void mk_cp16(void *dst, const void *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(mk_smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void mk_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void mk_cp_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// q.d in cycles, mod 1 per component: two-float products.
+__device__ __forceinline__ float mk_dot_frac(float3 qh, float3 ql, float3 dh, float3 dl)
+{
+    const float px = qh.x * dh.x, py = qh.y * dh.y, pz = qh.z * dh.z;
+    float lo = fmaf(qh.x, dh.x, -px) + fmaf(qh.y, dh.y, -py) + fmaf(qh.z, dh.z, -pz);
+    lo = fmaf(qh.x, dl.x, fmaf(ql.x, dh.x, lo));
+    lo = fmaf(qh.y, dl.y, fmaf(ql.y, dh.y, lo));
+    lo = fmaf(qh.z, dl.z, fmaf(ql.z, dh.z, lo));
+    return (mk_frac_nearest(px) + mk_frac_nearest(py)) + (mk_frac_nearest(pz) + lo);
+}
+
+// acc += v (Kahan: c carries what the sum's last bit lost).
+__device__ __forceinline__ void mk_kahan(float v, float &acc, float &c)
+{
+    const float y = __fsub_rn(v, c), z = __fadd_rn(acc, y);
+    c = __fsub_rn(__fsub_rn(z, acc), y);
+    acc = z;
+}
+
+// Sources s0 .. s0 + SB - 1's patch fields into shared memory (16-byte
+// chunks: n^2 even).
+template <int N>
+__device__ __forceinline__ void mk_stage_fields(float2 (*s_v)[N * N], const float2 *V, long long ld,
+                                                long long s0, int count)
+{
+    constexpr int CH = N * N / 2;
+    for (int i = threadIdx.x; i < count * CH; i += blockDim.x) {
+        const int s = i / CH, c = i - s * CH;
+        mk_cp16(&s_v[s][2 * c], V + (s0 + s) * ld + 2 * c);
+    }
+}
+
+// Merge: block = (group, fine patch), one fine node a thread. The group's
+// tiles come SB at a time: first the interpolation along z to the patch's
+// n1 node rows (shared by the row's nodes), then along y per node.
+template <int N0>
+__global__ void __launch_bounds__(256) mk_node_merge_kernel(const MkNodeArgs A)
+{
+    __shared__ __align__(16) float2 s_v[2][MK_NODE_SB][N0 * N0];
+    __shared__ __align__(16) float2 s_t[MK_NODE_SB][MK_NODE_MAX][N0];
+    __shared__ float s_wz[MK_NODE_MAX][N0];
+    __shared__ float s_d[2][MK_NODE_SB][6];
+    const long long patch = blockIdx.x % A.patches1;
+    const int grp = (int)(blockIdx.x / A.patches1);
+    const int n1 = A.n1;
+    const long long gpatch = A.patch1_base + patch;
+    const int f = mk_find_frame(A.f_lo, A.f_hi, gpatch, [&](int i) { return A.frames[i].patch1_off; });
+    const MkNodeFrame &F = A.frames[f];
+    const int lp = (int)(gpatch - F.patch1_off), pz = lp / F.p1y, py = lp - pz * F.p1y;
+    const int cy = py / F.ratio_y, cz = pz / F.ratio_z;
+    const int suby = py - cy * F.ratio_y, subz = pz - cz * F.ratio_z;
+    const float *W = A.weights + F.w_off + (long long)n1 * (F.ny + F.nz);
+    const float *Wy = W + suby * n1 * N0, *Wz = W + F.ratio_y * n1 * N0 + subz * n1 * N0;
+    for (int i = threadIdx.x; i < n1 * N0; i += blockDim.x) s_wz[i / N0][i % N0] = Wz[i];
+    const int oy = threadIdx.x % n1, oz = threadIdx.x / n1;
+    const bool live = oz < n1;
+    mk_f2 wy[N0];
+#pragma unroll
+    for (int i = 0; i < N0; ++i) wy[i] = f2_splat(Wy[oy * N0 + i]);
+    const MkNodeSrc &S = A.src[grp];
+    const double gx = S.o[0], gy = S.o[1], gz = S.o[2];
+    const MkNodeRec R = A.rec1[gpatch * n1 * n1 + (live ? oz * n1 + oy : 0)];
+    // directions from the group's origin
+    float3 qh = make_float3(R.qh.x, R.qh.y, R.qh.z), ql, u = make_float3(R.u.x, R.u.y, R.u.z);
+    float half;
+    {
+        const float ox = (float)gx, oy_ = (float)gy, oz_ = (float)gz;
+        const float uo = fmaf(u.z, oz_, fmaf(u.y, oy_, u.x * ox));
+        const float kr = A.kappa * R.w.w;
+        ql = make_float3(fmaf(ox - uo * u.x, kr, R.ql.x), fmaf(oy_ - uo * u.y, kr, R.ql.y),
+                         fmaf(oz_ - uo * u.z, kr, R.ql.z));
+        half = 0.5f * kr / fmaf(-uo, R.w.w, 1.f);
+    }
+    const float2 *V = A.V0 + (F.node0_off - A.node0_base) + (long long)(cz * F.p0y + cy) * N0 * N0;
+    const long long first = S.first;
+    const int count = S.count;
+    auto stage = [&](int s0, int buf) {
+        const int m = min(MK_NODE_SB, count - s0);
+        mk_stage_fields<N0>(s_v[buf], V, A.nodes0, first + s0, m);
+        mk_cp_commit();
+        if ((int)threadIdx.x < m) {
+            const double4 o = A.origin[A.members[first + s0 + threadIdx.x]];
+            const double d[3] = {o.x - gx, o.y - gy, o.z - gz};
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const float h = (float)d[c];
+                s_d[buf][threadIdx.x][c] = h;
+                s_d[buf][threadIdx.x][3 + c] = (float)(d[c] - (double)h);
+            }
+        }
+    };
+    float accr = 0.f, acci = 0.f, cr = 0.f, ci = 0.f;
+    stage(0, 0);
+    for (int s0 = 0, buf = 0; s0 < count; s0 += MK_NODE_SB, buf ^= 1) {
+        const int m = min(MK_NODE_SB, count - s0);
+        if (s0 + MK_NODE_SB < count) {
+            stage(s0 + MK_NODE_SB, buf ^ 1);
+            mk_cp_wait<1>();
+        } else {
+            mk_cp_wait<0>();
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < m * n1 * N0; i += blockDim.x) {
+            const int s = i / (n1 * N0), r = i - s * n1 * N0, row = r / N0, c = r - row * N0;
+            mk_f2 a = 0ull;
+#pragma unroll
+            for (int j = 0; j < N0; ++j)
+                a = f2_fma(f2_splat(s_wz[row][j]), *reinterpret_cast<const mk_f2 *>(&s_v[buf][s][j * N0 + c]), a);
+            *reinterpret_cast<mk_f2 *>(&s_t[s][row][c]) = a;
+        }
+        __syncthreads();
+        if (live) {
+#pragma unroll 2
+            for (int s = 0; s < m; ++s) {
+                mk_f2 v = 0ull;
+                const ulonglong2 *t2 = reinterpret_cast<const ulonglong2 *>(s_t[s][oz]);
+#pragma unroll
+                for (int i = 0; i < N0 / 2; ++i) {
+                    const ulonglong2 t = t2[i];
+                    v = f2_fma(wy[2 * i], t.x, v);
+                    v = f2_fma(wy[2 * i + 1], t.y, v);
+                }
+                const float *d = s_d[buf][s];
+                const float3 dh = make_float3(d[0], d[1], d[2]), dl = make_float3(d[3], d[4], d[5]);
+                const float ud = fmaf(u.z, dh.z, fmaf(u.y, dh.y, u.x * dh.x));
+                const float dd = fmaf(dh.z, dh.z, fmaf(dh.y, dh.y, dh.x * dh.x));
+                float ph = fmaf(fmaf(-ud, ud, dd), half, mk_dot_frac(qh, ql, dh, dl));
+                ph = mk_frac_nearest(ph);
+                float sn, cs;
+                __sincosf(ph * TWO_PI_F, &sn, &cs);
+                const float2 vv = f2_unpack(v);
+                mk_kahan(vv.x * cs - vv.y * sn, accr, cr);
+                mk_kahan(vv.x * sn + vv.y * cs, acci, ci);
+            }
+        }
+        __syncthreads();        // s_d and s_t are read; the next step may stage
+    }
+    if (live)
+        A.V1[(long long)grp * (A.patches1 * n1 * n1) + patch * n1 * n1 + threadIdx.x] =
+            make_float2(accr - cr, acci - ci);
+}
+
+// Pixels: block = (32 x 16 pixels of one fine patch, slice of sources), a
+// thread one column and four rows. Sources come SB at a time as in the
+// merge; bound by the FMA pipe (about 2 N + 45 FP32 operations a source and
+// pixel).
+template <int N>
+__global__ void __launch_bounds__(128) mk_node_pixels_kernel(const MkNodeArgs A)
+{
+    __shared__ __align__(16) float2 s_v[2][MK_NODE_SB][N * N];
+    __shared__ __align__(16) float2 s_t[MK_NODE_SB][MK_PIX_ROWS][N];
+    __shared__ float s_wz[MK_PIX_ROWS][N];
+    const long long blk = A.pblk_base + blockIdx.x;
+    const int f = mk_find_frame(A.f_lo, A.f_hi, blk, [&](int i) { return A.frames[i].pblk_off; });
+    const MkNodeFrame &F = A.frames[f];
+    const int per = F.bpy * F.bpz;
+    const int lb = (int)(blk - F.pblk_off), lp = lb / per, sub = lb - lp * per;
+    const int pz = lp / F.p1y, py = lp - pz * F.p1y, bz = sub / F.bpy, by = sub - bz * F.bpy;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int col_end = min((py + 1) * F.l1y, F.ny), row_end = min((pz + 1) * F.l1z, F.nz);
+    const int col = py * F.l1y + by * MK_PIX_COLS + lane;
+    const int row0 = pz * F.l1z + bz * MK_PIX_ROWS;
+    if (row0 >= row_end || py * F.l1y + by * MK_PIX_COLS >= col_end) return;   // whole block outside
+    const float *Wy = A.weights + F.w_off, *Wz = Wy + (long long)N * F.ny;
+    for (int i = threadIdx.x; i < MK_PIX_ROWS * N; i += blockDim.x)
+        s_wz[i / N][i % N] = Wz[(long long)min(row0 + i / N, row_end - 1) * N + i % N];
+    const int c0 = min(col, col_end - 1);
+    mk_f2 wy[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) wy[i] = f2_splat(Wy[(long long)c0 * N + i]);
+    float3 qh[4], ql[4], u[4];
+    float inv[4];
+    float accr[4], acci[4], cr[4], ci[4], tr[4], ti[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const long long g = F.pix_off + (long long)min(row0 + 4 * warp + r, row_end - 1) * F.ny + c0;
+        const double4 q = A.q[g];
+        const float4 uu = A.u[g];
+        qh[r] = make_float3((float)q.x, (float)q.y, (float)q.z);
+        ql[r] = make_float3((float)(q.x - (double)qh[r].x), (float)(q.y - (double)qh[r].y),
+                            (float)(q.z - (double)qh[r].z));
+        u[r] = make_float3(uu.x, uu.y, uu.z);
+        inv[r] = uu.w;
+        accr[r] = acci[r] = cr[r] = ci[r] = tr[r] = ti[r] = 0.f;
+    }
+    const int s_lo = blockIdx.y * A.src_per_slice, s_hi = min(A.n_src, s_lo + A.src_per_slice);
+    const long long ld = A.patches1 * N * N;
+    const float2 *V = A.V1 + (F.patch1_off - A.patch1_base + lp) * N * N;
+    int species = A.src[s_lo].species;
+    auto flush = [&](int s) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const long long g = F.pix_off + (long long)min(row0 + 4 * warp + r, row_end - 1) * F.ny + c0;
+            const float2 fc = A.ftab[(long long)s * A.ftab_n + g];
+            const float xr = accr[r] - cr[r], xi = acci[r] - ci[r];
+            tr[r] += fc.x * xr - fc.y * xi;
+            ti[r] += fc.x * xi + fc.y * xr;
+            accr[r] = acci[r] = cr[r] = ci[r] = 0.f;
+        }
+    };
+    mk_stage_fields<N>(s_v[0], V, ld, s_lo, min(MK_NODE_SB, s_hi - s_lo));
+    mk_cp_commit();
+    for (int s0 = s_lo, buf = 0; s0 < s_hi; s0 += MK_NODE_SB, buf ^= 1) {
+        const int m = min(MK_NODE_SB, s_hi - s0);
+        if (s0 + MK_NODE_SB < s_hi) {
+            mk_stage_fields<N>(s_v[buf ^ 1], V, ld, s0 + MK_NODE_SB, min(MK_NODE_SB, s_hi - s0 - MK_NODE_SB));
+            mk_cp_commit();
+            mk_cp_wait<1>();
+        } else {
+            mk_cp_wait<0>();
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < m * MK_PIX_ROWS * N; i += blockDim.x) {
+            const int s = i / (MK_PIX_ROWS * N), e = i - s * MK_PIX_ROWS * N, row = e / N, c = e - row * N;
+            mk_f2 a = 0ull;
+#pragma unroll
+            for (int j = 0; j < N; ++j)
+                a = f2_fma(f2_splat(s_wz[row][j]), *reinterpret_cast<const mk_f2 *>(&s_v[buf][s][j * N + c]), a);
+            *reinterpret_cast<mk_f2 *>(&s_t[s][row][c]) = a;
+        }
+        __syncthreads();
+        for (int s = 0; s < m; ++s) {
+            const float4 h4 = *reinterpret_cast<const float4 *>(A.src[s0 + s].dh);
+            const float4 l4 = *reinterpret_cast<const float4 *>(A.src[s0 + s].dl);
+            const int sp = __float_as_int(h4.w);
+            if (sp != species) {            // uniform across the block
+                flush(species);
+                species = sp;
+            }
+            const float3 dh = make_float3(h4.x, h4.y, h4.z), dl = make_float3(l4.x, l4.y, l4.z);
+            const float dd = fmaf(dh.z, dh.z, fmaf(dh.y, dh.y, dh.x * dh.x));
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                mk_f2 v = 0ull;
+                const ulonglong2 *t2 = reinterpret_cast<const ulonglong2 *>(s_t[s][4 * warp + r]);
+#pragma unroll
+                for (int i = 0; i < N / 2; ++i) {
+                    const ulonglong2 t = t2[i];
+                    v = f2_fma(wy[2 * i], t.x, v);
+                    v = f2_fma(wy[2 * i + 1], t.y, v);
+                }
+                const float ud = fmaf(u[r].z, dh.z, fmaf(u[r].y, dh.y, u[r].x * dh.x));
+                float ph = fmaf(fmaf(-ud, ud, dd), 0.5f * A.kappa * inv[r], mk_dot_frac(qh[r], ql[r], dh, dl));
+                ph = mk_frac_nearest(ph);
+                float sn, cs;
+                __sincosf(ph * TWO_PI_F, &sn, &cs);
+                if (A.decay) {
+                    const float dr = 1.f / fmaf(-ud, inv[r], 1.f);
+                    sn *= dr;
+                    cs *= dr;
+                }
+                const float2 vv = f2_unpack(v);
+                mk_kahan(vv.x * cs - vv.y * sn, accr[r], cr[r]);
+                mk_kahan(vv.x * sn + vv.y * cs, acci[r], ci[r]);
+            }
+        }
+        __syncthreads();
+    }
+    flush(species);
+    if (col >= col_end) return;
+    const long long n_pix = (long long)F.ny * F.nz;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int row = row0 + 4 * warp + r;
+        if (row < row_end)
+            A.partial[F.part_off - A.part_base + blockIdx.y * n_pix + (long long)row * F.ny + col] =
+                make_double2((double)tr[r], (double)ti[r]);
+    }
+}
+
+// out[g] (+)= r_e phasor[g] sum over slices (FP64, fixed order).
+__global__ void mk_node_reduce_kernel(const MkNodeFrame *__restrict__ frames, int f_lo, int f_hi,
+                                      long long g0, long long n, int slices, long long part_base,
+                                      const double2 *__restrict__ partial,
+                                      const double2 *__restrict__ phasor, double2 *__restrict__ out,
+                                      int accumulate)
+{
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const long long g = g0 + i;
+    const int f = mk_find_frame(f_lo, f_hi, g, [&](int j) { return frames[j].pix_off; });
+    const long long n_pix = (long long)frames[f].ny * frames[f].nz;
+    const double2 *p = partial + (frames[f].part_off - part_base) + (g - frames[f].pix_off);
+    double re = 0.0, im = 0.0;
+    for (int s = 0; s < slices; ++s) {
+        const double2 v = p[s * n_pix];
+        re += v.x;
+        im += v.y;
+    }
+    const double2 e = phasor[g];
+    double2 o = make_double2(MK_R_E * (re * e.x - im * e.y), MK_R_E * (re * e.y + im * e.x));
+    if (accumulate) {
+        o.x += out[g].x;
+        o.y += out[g].y;
+    }
+    out[g] = o;
+}
+
+// sums[f] = sum of |A|^2 over the frame's pixels: MK_SUM_PARTS fixed chunks a
+// frame, each a fixed-order tree, then the chunks in order.
+__global__ void __launch_bounds__(256) mk_node_sums_kernel(const MkNodeFrame *__restrict__ frames,
+                                                           const double2 *__restrict__ field,
+                                                           double *__restrict__ parts)
+{
+    __shared__ double red[256];
+    const MkNodeFrame &F = frames[blockIdx.x];
+    const long long n = (long long)F.ny * F.nz, step = (n + MK_SUM_PARTS - 1) / MK_SUM_PARTS;
+    const long long lo = blockIdx.y * step, hi = min(n, lo + step);
+    double acc = 0.0;
+    for (long long p = lo + threadIdx.x; p < hi; p += 256) {
+        const double2 v = field[F.pix_off + p];
+        acc += v.x * v.x + v.y * v.y;
+    }
+    red[threadIdx.x] = acc;
+    __syncthreads();
+    for (int w = 128; w > 0; w >>= 1) {
+        if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) parts[(long long)blockIdx.x * MK_SUM_PARTS + blockIdx.y] = red[0];
+}
+
+__global__ void mk_node_sums_final_kernel(int n_frames, const double *__restrict__ parts,
+                                          double *__restrict__ sums)
+{
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= n_frames) return;
+    double acc = 0.0;
+    for (int i = 0; i < MK_SUM_PARTS; ++i) acc += parts[(long long)f * MK_SUM_PARTS + i];
+    sums[f] = acc;
+}
+
+template <int N>
+static void mk_launch_pixels(const MkNodeArgs &A, dim3 grid, cudaStream_t st)
+{
+    mk_node_pixels_kernel<N><<<grid, 128, 0, st>>>(A);
+}
+template <int N>
+static void mk_launch_merge(const MkNodeArgs &A, unsigned grid, cudaStream_t st)
+{
+    mk_node_merge_kernel<N><<<grid, (A.n1 * A.n1 + 31) / 32 * 32, 0, st>>>(A);
+}
+
+extern "C" int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, const mk_pixels *px,
+                                const mk_node_plan *plan, const void *host_buf, const void *dev_buf,
+                                int fresnel, double fresnel_radius_m, double *out, double *intensity_sums,
+                                int accumulate, void *workspace, size_t ws_bytes, void *stream)
+{
+    MK_REQUIRE(tiles && phys && px && plan && host_buf && dev_buf && out, "mk_kin_nodes_f32: null argument");
+    MK_REQUIRE(px->xyz && px->q && px->u && px->phasor && px->factor,
+               "mk_kin_nodes_f32: pixels not prepared, or no factor table");
+    MK_REQUIRE(tiles->origin && tiles->pos && tiles->amp && tiles->n_tiles == plan->n_tiles,
+               "mk_kin_nodes_f32: the tiles are not the plan's");
+    MK_REQUIRE(((uintptr_t)tiles->pos & 15) == 0 && ((uintptr_t)tiles->amp & 15) == 0 &&
+                   ((uintptr_t)workspace & 255) == 0 && ((uintptr_t)dev_buf & 15) == 0,
+               "mk_kin_nodes_f32: misaligned buffer");
+    MK_REQUIRE(!phys->analyser && !phys->remove_forward && phys->k > 0.0,
+               "mk_kin_nodes_f32: no analyser and no remove_forward here");
+    MK_REQUIRE(plan->n_src >= 1 && plan->n_frames >= 1 && (long long)px->ny * px->nz >= plan->n_pix,
+               "mk_kin_nodes_f32: empty plan or too few pixels");
+    if (!workspace || ws_bytes < (size_t)plan->ws_bytes) {
+        mk_set_error("mk_kin_nodes_f32: workspace %zu bytes, need %lld", ws_bytes, plan->ws_bytes);
+        return MK_ENOMEM;
+    }
+    const int n0 = plan->n0, n1 = plan->n1, T = tiles->tile_atoms;
+    const MkNodeFrame *hf = static_cast<const MkNodeFrame *>(host_buf);
+    const char *db = static_cast<const char *>(dev_buf);
+    cudaStream_t st = mk_stream(stream);
+    MkNodeArgs A;
+    memset(&A, 0, sizeof(A));
+    A.frames = reinterpret_cast<const MkNodeFrame *>(db);
+    A.src = reinterpret_cast<const MkNodeSrc *>(db + plan->off_src);
+    A.members = reinterpret_cast<const int *>(db + plan->off_members);
+    const int *mid = reinterpret_cast<const int *>(db + plan->off_mid);
+    char *w = static_cast<char *>(workspace);
+    MkNodeRec *rec0 = reinterpret_cast<MkNodeRec *>(w);
+    MkNodeRec *rec1 = rec0 + plan->nodes0;
+    w += up256(sizeof(MkNodeRec) * (size_t)(plan->nodes0 + plan->patches1 * n1 * n1));
+    float *weights = reinterpret_cast<float *>(w);
+    w += up256(sizeof(float) * (size_t)plan->weights);
+    A.rec0 = rec0;
+    A.rec1 = rec1;
+    A.weights = weights;
+    A.n0 = n0;
+    A.n1 = n1;
+    A.n_groups = plan->n_groups;
+    A.n_src = plan->n_src;
+    A.src_per_slice = plan->src_per_slice;
+    A.tile_atoms = T;
+    A.origin = reinterpret_cast<const double4 *>(tiles->origin);
+    A.tpos = reinterpret_cast<const float4 *>(tiles->pos);
+    A.tamp = reinterpret_cast<const float2 *>(tiles->amp);
+    A.q = reinterpret_cast<const double4 *>(px->q);
+    A.u = reinterpret_cast<const float4 *>(px->u);
+    A.ftab = reinterpret_cast<const float2 *>(px->factor);
+    A.ftab_n = (long long)px->ny * px->nz;
+    A.kappa_d = phys->k / MK_TWO_PI;
+    A.kappa = (float)A.kappa_d;
+    A.fresnel = fresnel != 0;
+    A.fres_r = fresnel_radius_m > 0.0 ? (float)fresnel_radius_m : 0.f;
+    A.decay = phys->spherical_decay;
+
+    int most = 0;
+    for (int f = 0; f < plan->n_frames; ++f) {
+        const MkNodeFrame &F = hf[f];
+        const int items = (n0 ? F.p0y * F.p0z * n0 * n0 + (F.ratio_y + F.ratio_z) * n1 : 0) +
+                          F.p1y * F.p1z * n1 * n1 + F.ny + F.nz;
+        most = std::max(most, items);
+    }
+    mk_node_prep_kernel<<<dim3(plan->n_frames, std::min((most + 63) / 64, 1024)), 64, 0, st>>>(
+        A.frames, n0, n1, A.kappa_d, px->xyz, rec0, rec1, weights);
+    MK_CHECK_CUDA(cudaGetLastError());
+    const size_t leaf_smem = (size_t)T * 24;
+    MK_CHECK_CUDA(cudaFuncSetAttribute((const void *)mk_node_leaf_kernel,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)leaf_smem));
+    auto leaf = [&](const int *list, int n_list, const MkNodeRec *rec, long long nodes, float2 *V) {
+        const int th = (int)std::min<long long>(256, (nodes + 31) / 32 * 32);
+        mk_node_leaf_kernel<<<dim3(n_list, (unsigned)((nodes + th - 1) / th)), th, leaf_smem, st>>>(
+            A, list, rec, nodes, V);
+    };
+    // passes of whole frames whose node fields and partials fit the chunk
+    const size_t budget = std::max((size_t)plan->chunk_bytes, (size_t)1);
+    for (int fa = 0; fa < plan->n_frames;) {
+        long long a = 0, b = 0, c = 0, pb = 0;
+        int fb = fa;
+        auto bytes = [&](long long x, long long y, long long z) {
+            return up256(8 * (size_t)(x * plan->n_members)) +
+                   up256((size_t)(8.0 * y * (double)(n1 * n1) * plan->n_src)) + up256(16 * (size_t)z * plan->slices);
+        };
+        while (fb < plan->n_frames) {
+            const MkNodeFrame &F = hf[fb];
+            const long long da = n0 ? (long long)F.p0y * F.p0z * n0 * n0 : 0;
+            const long long dp = (long long)F.p1y * F.p1z, dc = (long long)F.ny * F.nz;
+            const bool too_many = (b + dp) * std::max(plan->n_groups, 1) > (1ll << 30) ||
+                                  (a + da) > 256ll * 60000 || (b + dp) * (double)(n1 * n1) > 256.0 * 60000;
+            if (fb > fa && (bytes(a + da, b + dp, c + dc) > budget || too_many)) break;
+            a += da;
+            b += dp;
+            c += dc;
+            pb += dp * F.bpy * F.bpz;
+            ++fb;
+        }
+        A.f_lo = fa;
+        A.f_hi = fb;
+        A.nodes0 = a;
+        A.patches1 = b;
+        A.node0_base = hf[fa].node0_off;
+        A.patch1_base = hf[fa].patch1_off;
+        A.pblk_base = hf[fa].pblk_off;
+        A.part_base = hf[fa].part_off;
+        char *cw = w;
+        A.V0 = reinterpret_cast<float2 *>(cw);
+        cw += up256(8 * (size_t)(a * plan->n_members));
+        A.V1 = reinterpret_cast<float2 *>(cw);
+        cw += up256((size_t)(8.0 * b * (double)(n1 * n1) * plan->n_src));
+        A.partial = reinterpret_cast<double2 *>(cw);
+        if (plan->n_members > 0) {
+            leaf(A.members, plan->n_members, rec0 + A.node0_base, a, A.V0);
+            const unsigned grid = (unsigned)(b * plan->n_groups);
+            switch (n0) {
+            case 8: mk_launch_merge<8>(A, grid, st); break;
+            case 10: mk_launch_merge<10>(A, grid, st); break;
+            case 12: mk_launch_merge<12>(A, grid, st); break;
+            case 16: mk_launch_merge<16>(A, grid, st); break;
+            default: mk_set_error("mk_kin_nodes_f32: %d coarse nodes", n0); return MK_EINVAL;
+            }
+        }
+        if (plan->n_mid > 0)
+            leaf(mid, plan->n_mid, rec1 + A.patch1_base * n1 * n1, b * n1 * n1,
+                 A.V1 + (long long)plan->n_groups * b * n1 * n1);
+        const dim3 grid((unsigned)pb, plan->slices);
+        switch (n1) {
+        case 6: mk_launch_pixels<6>(A, grid, st); break;
+        case 8: mk_launch_pixels<8>(A, grid, st); break;
+        case 10: mk_launch_pixels<10>(A, grid, st); break;
+        case 12: mk_launch_pixels<12>(A, grid, st); break;
+        case 16: mk_launch_pixels<16>(A, grid, st); break;
+        default: mk_set_error("mk_kin_nodes_f32: %d nodes", n1); return MK_EINVAL;
+        }
+        mk_node_reduce_kernel<<<(unsigned)((c + 255) / 256), 256, 0, st>>>(
+            A.frames, fa, fb, hf[fa].pix_off, c, plan->slices, A.part_base, A.partial,
+            reinterpret_cast<const double2 *>(px->phasor), reinterpret_cast<double2 *>(out), accumulate);
+        MK_CHECK_CUDA(cudaGetLastError());
+        fa = fb;
+    }
+    if (intensity_sums) {       // the node fields are read: their space holds the chunks' sums
+        double *parts = reinterpret_cast<double *>(w);
+        mk_node_sums_kernel<<<dim3(plan->n_frames, MK_SUM_PARTS), 256, 0, st>>>(
+            A.frames, reinterpret_cast<const double2 *>(out), parts);
+        mk_node_sums_final_kernel<<<(plan->n_frames + 127) / 128, 128, 0, st>>>(plan->n_frames, parts,
+                                                                                intensity_sums);
+        MK_CHECK_CUDA(cudaGetLastError());
+    }
+    return MK_OK;
+}

@@ -15,13 +15,14 @@ from __future__ import annotations
 
 import ctypes
 import math
+import types
 from dataclasses import dataclass, field
 
 import numpy as np
 import torch
 
 from . import _lib
-from ._lib import MkLaunch, MkPhysics, MkPixels, MkSpecies, MkTiles, check
+from ._lib import MkLaunch, MkNodePlan, MkPhysics, MkPixels, MkSpecies, MkTiles, check
 
 R_E = 2.81794092e-15
 
@@ -197,6 +198,23 @@ class Pixels:
                                 _stream_handle(stream)))
         self._ftab = (key, ftab)
         return ftab
+
+    def plane_fit(self, stream=None):
+        """(shapes (F, 3) int64, fit (F, 12) float64) on the host: every
+        frame's pixel grid as ``mk_plane_fit`` describes it (one read-back per
+        Pixels object)."""
+        if getattr(self, "_fit", None) is None:
+            shapes = np.array([(off, ny, nz) for (off, _), (ny, nz) in zip(self.spans, self.shapes)],
+                              dtype=np.int64)
+            dev = self.xyz.device
+            sd = torch.from_numpy(shapes).to(dev)
+            fit = torch.empty((len(shapes), 12), dtype=torch.float64, device=dev)
+            check(_require_cuda().mk_plane_fit(len(shapes), _ptr(sd),
+                                               int((shapes[:, 1] * shapes[:, 2]).max()),
+                                               _ptr(self.xyz), _ptr(fit), _stream_handle(stream)))
+            self._fit = (shapes, fit.cpu().numpy())
+            self._r0_min = float(self._fit[1][:, 10].min())
+        return self._fit
 
     def r0_min(self):
         """Smallest pixel distance (one read-back per Pixels object)."""
@@ -507,7 +525,7 @@ class Tiles:
         self.amp = torch.empty((max(n_tiles, 1) * T, 2), dtype=torch.float32, device=device)
         self.abi = MkTiles(n_tiles, T, self.origin.data_ptr(), self.species.data_ptr(),
                            self.pos.data_ptr(), self.amp.data_ptr())
-        self.table = atoms.table
+        self.table, self.counts = atoms.table, counts
         if atoms.n == 0:
             return
         ws_n = L.mk_tiles_workspace_size(atoms.n)
@@ -861,6 +879,79 @@ def run_split(tiles: Tiles, pix: Pixels, phys, table: SpeciesTable, launch=None,
     return out
 
 
+# The node form is planned from this many (atom, pixel) terms on: below it the
+# split kernel takes ~10 us, as long as the node form's launches alone.
+NODES_MIN_TERMS = 1e8
+
+
+class NodePlan:
+    """A plan of the node form (``mk_nodes_plan``) for these tiles and pixels:
+    its tables on the host and the device, and the tiles it leaves to the
+    split kernel (``wide``: a gathered TilesView, or None). ``make`` returns
+    None where the geometry is outside the form or the split kernel is as
+    fast."""
+
+    # the split kernel's time per (atom, pixel), octets to squares
+    DIRECT_S_PER_TERM = 0.18e-12
+
+    def __init__(self, plan, buf, tiles):
+        self.plan, self.buf = plan, buf
+        self.dev = torch.from_numpy(buf[: plan.buf_bytes]).to(tiles.origin.device)
+        self.wide = None
+        if plan.n_wide:
+            idx = np.frombuffer(buf, dtype=np.int32, count=plan.n_wide, offset=plan.off_wide)
+            self.wide = TilesView.gather(tiles, idx)
+
+    @classmethod
+    def make(cls, tiles, pix, k, beam_dirs, phase_tol, direct=DIRECT_S_PER_TERM, group_tiles=-1):
+        L = _require_cuda()
+        if not tiles.n_tiles or getattr(tiles, "counts", None) is None:
+            return None
+        shapes, fit = pix.plane_fit()
+        org = np.ascontiguousarray(origins_host(tiles))
+        nf = len(shapes)
+        nb = int(L.mk_nodes_plan_bytes(nf, tiles.n_tiles))
+        buf = np.empty(nb, dtype=np.uint8)
+        plan = MkNodePlan()
+        bd = np.ascontiguousarray(np.asarray(beam_dirs, dtype=np.float64).reshape(nf, 3))
+        rc = L.mk_nodes_plan(tiles.n_tiles, tiles.tile_atoms, len(tiles.counts),
+                             tiles.counts.ctypes.data, org.ctypes.data, nf, shapes.ctypes.data,
+                             fit.ctypes.data, bd.ctypes.data, float(k), float(phase_tol),
+                             float(direct), int(group_tiles), ctypes.byref(plan), buf.ctypes.data, nb)
+        if rc == _lib.MK_EDECLINE:
+            return None
+        check(rc)
+        return cls(plan, buf, tiles)
+
+    def info(self):
+        p = self.plan
+        return dict(form="nodes", nodes=(p.n0, p.n1), groups=p.n_groups, single_tiles=p.n_mid,
+                    wide_tiles=p.n_wide, group_radius_m=p.radius2_m)
+
+
+def run_nodes(np_, tiles, pix, phys, table, out=None, accumulate=False, fresnel=0, fresnel_radius=0.0,
+              factor=None, sums=None, ws=None, stream=None):
+    """Node-form sum of a plan's groups and single tiles (``mk_kin_nodes_f32``;
+    the plan's wide tiles are the caller's); float64 (P, 2). ``factor``: the
+    factor table (default: ``Pixels.factor_table`` of single exposures)."""
+    L = _require_cuda()
+    if out is None:
+        out = torch.empty((pix.n, 2), dtype=torch.float64, device=pix.xyz.device)
+        accumulate = False
+    if ws is None:
+        ws = torch.empty(np_.plan.ws_bytes, dtype=torch.uint8, device=pix.xyz.device)
+    if factor is None:
+        factor = pix.factor_table(table, phys, stream)
+    pabi = MkPixels.from_buffer_copy(pix.abi)
+    pabi.factor = factor.data_ptr()
+    check(L.mk_kin_nodes_f32(ctypes.byref(tiles.abi), ctypes.byref(phys), ctypes.byref(pabi),
+                             ctypes.byref(np_.plan), np_.buf.ctypes.data, _ptr(np_.dev), int(fresnel),
+                             float(fresnel_radius), _ptr(out), _ptr(sums), int(bool(accumulate)),
+                             _ptr(ws), int(ws.numel()), _stream_handle(stream)))
+    out._mk_keep = (ws, factor, np_.dev)
+    return out
+
+
 def run_plain(atoms: Atoms, pix: Pixels, phys, slices=0, out=None, accumulate=False, stream=None):
     """FP64 plain sum; returns float64 (P, 2)."""
     L = _require_cuda()
@@ -899,6 +990,19 @@ class TilesView:
         self.table = tiles.table
         self.abi = MkTiles(self.n_tiles, self.tile_atoms, self.origin.data_ptr(),
                            self.species.data_ptr(), self.pos.data_ptr(), self.amp.data_ptr())
+
+    @classmethod
+    def gather(cls, tiles, idx):
+        """The tiles ``idx`` (host int32) copied into arrays of their own."""
+        i = torch.from_numpy(np.ascontiguousarray(idx, dtype=np.int64)).to(tiles.origin.device)
+        n, T = tiles.n_tiles, tiles.tile_atoms
+        v = types.SimpleNamespace(
+            tile_atoms=T, table=tiles.table, origin=tiles.origin[i], species=tiles.species[i],
+            pos=tiles.pos[: n * T].view(n, T, 4)[i].view(-1, 4),
+            amp=tiles.amp[: n * T].view(n, T, 2)[i].view(-1, 2))
+        out = cls(v, len(idx))
+        out._origins_host = origins_host(tiles)[idx]
+        return out
 
     def amp_is_real(self):
         if getattr(self, "_real", None) is None:

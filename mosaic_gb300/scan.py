@@ -27,6 +27,7 @@ import numpy as np
 import torch
 
 from . import _lib, engine
+from .autotune import Setup
 from ._lib import MkFrameDesc, MkLaunch, MkPixels, check
 
 
@@ -121,8 +122,17 @@ class BatchedScan:
         self.phys = beam.physics(apply_polarization, spherical_decay, remove_forward, pol=pol)
         self.pix = engine.Pixels(np.concatenate(xyz, axis=1), n_total, 1, self.phys, device=dev,
                                  frames=fr)
-        su = self._setup(self.tiles)
         self.tune_results = []
+        self.out = torch.zeros((n_total, 2), dtype=torch.float64, device=dev)
+        self.sums = torch.zeros(len(self.frames), dtype=torch.float64, device=dev)
+        self.ws, self.ws_bytes = None, 0
+        self.terms = float(self.atoms.n) * n_total
+        self._ftab_key, self._ftab = None, None
+        self.nodes = None
+        if not launch and not beam._kernel_launch and self._plan_nodes():
+            self.launch_source = "nodes"
+            return
+        su = self._setup(self.tiles)
         if launch:
             cfg, src = dict(engine.default_launch(su.level, self.tiles.tile_atoms), **launch), "explicit"
         elif beam._kernel_launch:
@@ -147,11 +157,34 @@ class BatchedScan:
             cfg = (autotune.lookup(n_total, su.level, "scan", self.tiles.tile_atoms) if best
                    else engine.default_launch(su.level, self.tiles.tile_atoms))
         self.launch_source = src
-        self.out = torch.zeros((n_total, 2), dtype=torch.float64, device=dev)
-        self.sums = torch.zeros(len(self.frames), dtype=torch.float64, device=dev)
-        self.ws, self.ws_bytes = None, 0
         self.replan(self.tiles, su, cfg)
-        self.terms = float(self.atoms.n) * n_total
+
+    def _plan_nodes(self):
+        """Plan the node form (``engine.NodePlan``) for the whole scan, its
+        wide tiles through the split kernel; False where it declines."""
+        B = self.beam
+        if not B._use_nodes or self.phys.remove_forward or not self.tiles.n_tiles or \
+                self.terms < engine.NODES_MIN_TERMS:
+            return False
+        tol = min(float(B._kernel_phase_tol_rad), float(B._phase_tol_rad))
+        plan = engine.NodePlan.make(self.tiles, self.pix, B.k, self._bd, tol)
+        if plan is None:
+            return False
+        _, fresnel, _, self.diag = B.split_budget(self.tiles, self.pix.r0_min())
+        self._node_fresnel = (int(fresnel), self.diag["fresnel_radius_m"])
+        if plan.wide is not None:
+            su, _ = B.split_setup(plan.wide, self.pix)
+            if su is None:
+                return False
+            self.replan(plan.wide, su, engine.default_launch(su.level, self.tiles.tile_atoms))
+        else:
+            # nothing for the split kernel: a plan of its simplest shape keeps
+            # the frame table the factor table reads
+            self.replan(self.tiles, Setup(self.tiles, 0, {}), engine.default_launch(0), workspace=False)
+        self.nodes = plan
+        self._node_ws = torch.empty(plan.plan.ws_bytes, dtype=torch.uint8, device=self._dev)
+        self.diag = dict(self.diag, **plan.info())
+        return True
 
     def _setup(self, tiles):
         """The split form's set-up for these tiles (raises when the scan's
@@ -190,15 +223,16 @@ class BatchedScan:
                            launch=launch or engine.default_launch(0), device=self._dev,
                            **self._flags)
 
-    def replan(self, tiles, su, cfg):
+    def replan(self, tiles, su, cfg, workspace=True):
         """Plan the launch for ``tiles`` (this scan's, or a view of them) with
         launch dict ``cfg`` (clamped to what ``su`` allows)."""
+        self.nodes = None
         cfg = engine.grouping_launch(cfg, su.level, tiles, self.pix, self.beam.k, su.info)
         self.cfg = cfg
         self.setup = su
         self.tiles_run = tiles
         self.launch = MkLaunch(int(cfg["pix_per_thread"]), int(cfg["threads"]), int(cfg["slices"]),
-                               int(su.fresnel), int(tiles.amp_is_real()), float(su.fresnel_radius),
+                               int(su.fresnel), 1 if not workspace else int(tiles.amp_is_real()), float(su.fresnel_radius),
                                int(cfg["pairs"]), float(cfg["pair_short_radius_m"]),
                                float(cfg.get("sin_direct_max_rad", 0.0) or 0.0),
                                float(cfg.get("octet_radius_m", 0.0) or 0.0))
@@ -233,7 +267,7 @@ class BatchedScan:
             self.pix_abi = MkPixels.from_buffer_copy(self.pix.abi)
             self.pix_abi.factor = self.ftab.data_ptr()
         need = int(self.L.mk_scan_workspace_size(self.n_partial))
-        if self.ws is None or self.ws_bytes < need:
+        if workspace and (self.ws is None or self.ws_bytes < need):
             self.ws = torch.empty(need, dtype=torch.uint8, device=self._dev)
             self.ws_bytes = need
         self._graph = None
@@ -258,14 +292,26 @@ class BatchedScan:
 
     def run(self, stream=None):
         """Launch the whole scan (asynchronous); returns (fields, sums) on device."""
+        if self.nodes is not None:
+            if self.nodes.wide is not None:
+                self._run_split(self.out, None, stream)
+            engine.run_nodes(self.nodes, self.tiles, self.pix, self.phys, self.table, out=self.out,
+                             accumulate=self.nodes.wide is not None, fresnel=self._node_fresnel[0],
+                             fresnel_radius=self._node_fresnel[1], factor=self.ftab, sums=self.sums,
+                             ws=self._node_ws, stream=stream)
+        else:
+            self._run_split(self.out, self.sums, stream)
+        return self.out, self.sums
+
+    def _run_split(self, out, sums, stream):
         sp = self.table.abi()
         check(self.L.mk_kin_scan_f32(ctypes.byref(self.tiles_run.abi), ctypes.byref(sp),
                                      ctypes.byref(self.phys), ctypes.byref(self.pix_abi),
                                      len(self.frames), self.frames_dev.data_ptr(), self.n_items,
-                                     self.n_partial, ctypes.byref(self.launch), self.out.data_ptr(),
-                                     self.sums.data_ptr(), self.ws.data_ptr(), self.ws_bytes,
+                                     self.n_partial, ctypes.byref(self.launch), out.data_ptr(),
+                                     sums.data_ptr() if sums is not None else None,
+                                     self.ws.data_ptr(), self.ws_bytes,
                                      engine._stream_handle(stream)))
-        return self.out, self.sums
 
     def capture(self, warm=True):
         """Capture run() in a CUDA graph (frames > 1); replay() then re-runs it.

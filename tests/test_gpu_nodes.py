@@ -1,0 +1,134 @@
+"""The node form of the FP32 sum (engine.NodePlan / run_nodes) against the
+FP64 sum of the same atoms and pixels and against the split kernel with one
+sin/cos per term.
+
+Tolerances are the other FP32 forms': 1e-4 of the peak intensity against
+FP64, 2e-5 of max |A| against the one-sin/cos form (interpolation adds at
+most ~1e-6 of the sum of |E| by the plan's node counts)."""
+import numpy as np
+import pytest
+import torch
+
+from mosaic_gb300 import ChunkedSample, Detector, StaticStage, engine, workloads
+from mosaic_gb300.scan import BatchedScan, frames_from_motors
+
+from helpers import rel_intensity, rel_max
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(cells, dilute=0.0, seed=3):
+    rng = np.random.default_rng(seed)
+    w = workloads.fcc_cu_32k(cells=cells, npix=16)
+    pos = w.sample.load_chunk_positions(1)
+    u = rng.random(pos.shape[0])
+    spc = np.where(u < dilute, "Ag", np.where(u < 0.4, "Ni", "Cu"))
+    return w, ChunkedSample([(pos, spc)])
+
+
+def _det(w, shape, dist=1.0e10, mode="plane", pitch=5.5e5):
+    D = Detector()
+    D.create_detector(shape, (pitch, pitch), construction_mode=mode)
+    D.position_detector_absolute(dist, 2.0 * w.meta["theta_deg"], 0.0)
+    return D
+
+
+def _c(out, shape):
+    engine.sync()
+    return torch.view_as_complex(out).cpu().numpy().reshape(shape[1], shape[0])
+
+
+@pytest.mark.parametrize("shape, tile, group, dist, decay, cplx", [
+    ((64, 48), 512, 0, 1.0e10, False, False),     # one patch, tiles straight to the pixels
+    ((33, 17), 128, 0, 1.0e10, True, True),       # one past a pixel block each way, complex amplitudes
+    ((1, 40), 128, 0, 1.0e10, False, False),      # single column
+    ((50, 1), 128, 0, 1.0e10, False, False),      # single row
+    ((200, 90), 128, 8, 0.2e10, True, False),     # groups, several patches, last ones ragged
+    ((96, 64), 128, 16, 0.2e10, False, True),     # whole blocks
+    ((161, 47), 256, 8, 0.5e10, True, True),
+])
+def test_nodes_match_fp64_and_split(cuda, shape, tile, group, dist, decay, cplx):
+    w, sample = _case(14, dilute=0.005 if group else 0.0)
+    B = workloads._beam(10000.0, 200.0, pol_perp_rate=1.0)
+    if cplx:
+        rng = np.random.default_rng(2)
+        B.set_wavefield((B._beam_E0_map * np.exp(1j * rng.uniform(-np.pi, np.pi, B._beam_E0_map.shape))
+                         ).astype(np.complex64))
+    B.set_debye_waller({"Cu": 0.55})
+    st = StaticStage(w.stage.rotation, w.stage.translation)
+    D = _det(w, shape, dist)
+    phys = B.physics(apply_polarization=True, spherical_decay=decay)
+    atoms = B.stage_atoms(sample, st, device=cuda)
+    pix = engine.Pixels(np.asarray(D.pixel_coordinates) / 1e10, *shape, phys, device=cuda)
+    tiles = engine.Tiles(atoms, B.k, tile, device=cuda)
+    plan = engine.NodePlan.make(tiles, pix, B.k, (1.0, 0.0, 0.0), 1e-6, direct=1.0, group_tiles=group)
+    assert plan is not None and (plan.plan.n_groups > 0) == (group > 0)
+    assert plan.plan.n_members + plan.plan.n_mid + plan.plan.n_wide == tiles.n_tiles
+    acc = torch.full((pix.n, 2), float("nan"), dtype=torch.float64, device=cuda)
+    wide = plan.wide is not None
+    if wide:
+        engine.run_split(plan.wide, pix, phys, atoms.table, fresnel=1, out=acc, factor_table=True)
+    got = _c(engine.run_nodes(plan, tiles, pix, phys, atoms.table, out=acc, accumulate=wide, fresnel=1), shape)
+    one = _c(engine.run_split(tiles, pix, phys, atoms.table, fresnel=1), shape)
+    ref = _c(engine.run_plain(atoms, pix, phys), shape)
+    assert rel_intensity(got, ref) <= 1e-4, rel_intensity(got, ref)
+    assert rel_max(got, one) <= 2e-5, rel_max(got, one)
+    again = engine.run_nodes(plan, tiles, pix, phys, atoms.table, fresnel=1)
+    engine.sync()
+    if not wide:
+        assert torch.equal(again, acc)              # the same sum twice, to the bit
+
+
+def test_entry_point_takes_nodes_where_admitted(cuda):
+    """Large enough on a plane detector: nodes; a curved (shell) detector,
+    an explicit launch, remove_forward and an analyser: the other forms, with
+    the same field where the physics is the same."""
+    w, sample = _case(16)
+    B = workloads._beam(10000.0, 200.0, pol_perp_rate=1.0)
+    st = StaticStage(w.stage.rotation, w.stage.translation)
+    kw = dict(apply_polarization=True, return_double=True)
+    D = _det(w, (130, 90))
+    a = B.atomic_scattering_kinematic(sample, D, st, **kw)
+    assert B.last_run["launch_source"] == "nodes" and B.last_run["path"] == "split_f32"
+    B._kernel_launch = dict(pix_per_thread=4, threads=128, slices=0, pairs=0)
+    b = B.atomic_scattering_kinematic(sample, D, st, **kw)
+    assert B.last_run["launch_source"] == "beam"
+    assert rel_max(a, b) <= 2e-5, rel_max(a, b)
+    B._kernel_launch = None
+    for extra in (dict(remove_forward=True), dict(analyser_mode="top-hat", analyser_acceptance_angle_rad=1e-3)):
+        B.atomic_scattering_kinematic(sample, D, st, **kw, **extra)
+        assert B.last_run["launch_source"] != "nodes", extra
+    # 2 mm pixels: the sphere is 8 mm off its chord plane at the corners
+    S = _det(w, (130, 90), mode="shell", pitch=2.0e7)
+    c = B.atomic_scattering_kinematic(sample, S, st, **kw)
+    assert B.last_run["launch_source"] != "nodes"
+    B._use_fast_kernel = False
+    assert rel_intensity(c, B.atomic_scattering_kinematic(sample, S, st, **kw)) <= 1e-4
+
+
+def test_scan_nodes_match_single_fp64_exposures(cuda):
+    """Frames of several shapes in one node plan, their sums, and a captured
+    replay, bit for bit."""
+    w, sample = _case(16)
+    B = w.beam
+    theta = np.radians(w.meta["theta_deg"])
+    D = _det(w, (128, 128))
+    steps = [dict(mu=theta + np.radians(d), chi=np.radians(c)) for c in (-0.3, 0.2) for d in (-0.5, 0.0, 0.4)]
+    frames = frames_from_motors(w.stage, D, steps, [24, 128, 50, 64, 33, 128])
+    scan = BatchedScan(B, sample, frames, apply_polarization=True)
+    assert scan.launch_source == "nodes" and scan.nodes is not None
+    out, sums = scan.run()
+    engine.sync()
+    first, s1 = out.clone(), sums.clone()
+    B._use_fast_kernel = False
+    for f, fr in enumerate(frames):
+        ref = B.interact_beam_gpu(sample, fr.pixels, fr.shape, StaticStage(fr.rotation, fr.translation),
+                                  apply_polarization=True, spherical_decay=False, return_double=True)
+        assert rel_intensity(scan.frame_field(f), ref) <= 1e-4, f
+        I = float((np.abs(scan.frame_field(f)) ** 2).sum())
+        assert abs(float(s1[f]) - I) <= 1e-12 * I
+    scan.capture()
+    scan.out.zero_()
+    scan.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(scan.out, first) and torch.equal(scan.sums, s1)

@@ -232,6 +232,13 @@ int mk_atoms_lab(int64_t n, const float *pos_in, const float *rot, const float *
                  const float *e0, int grid_ny, int grid_nz, const double *grid,
                  double *pos_lab, float *amp, void *stream);
 
+/* Byte species codes of a chunk (device) -> species indices through lut
+ * (host, n_lut <= 256 entries in [0, n_species)), and the atoms of every
+ * species added to counts (device int64, n_species). Codes beyond n_lut are
+ * written as 0 and not counted. */
+int mk_species_index(int64_t n, const unsigned char *codes, const int *lut, int n_lut,
+                     int n_species, int *species, int64_t *counts, void *stream);
+
 /* --- depth-dependent incident field (Beam.py:956-1045, 4963-5140,
  * 5583-5618, 7118-7283) ---------------------------------------------------
  * Column sums of the forward scattering factors on the beam grid (the

@@ -163,6 +163,8 @@ class MkNodePlan(ctypes.Structure):
 
 # name -> (restype, argtypes)
 SIGNATURES = {
+    "mk_species_index": (ctypes.c_int, [ctypes.c_int64, _vp, _vp, ctypes.c_int, ctypes.c_int, _vp, _vp,
+                                        _vp]),
     "mk_plane_fit": (ctypes.c_int, [ctypes.c_int, _vp, ctypes.c_longlong, _vp, _vp, _vp]),
     "mk_nodes_plan_bytes": (ctypes.c_size_t, [ctypes.c_int, ctypes.c_int]),
     "mk_nodes_plan": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_int, _vp, _vp, ctypes.c_int,

@@ -262,6 +262,8 @@ class beam:
         dev = torch.device(device)
         pos_d = torch.empty((max(n_max, 1), 3), dtype=torch.float32, device=dev)
         idx_d = torch.empty(max(n_max, 1), dtype=torch.int32, device=dev)
+        counts_d = torch.zeros(engine.MAX_SPECIES, dtype=torch.int64, device=dev)
+        counts_h, mapped = np.zeros(max(16, len(self.tables.f0)), dtype=np.int64), 0
         labels, lab_index = [], {}
         off = 0
         self.last_stream_bytes = 0               # host -> device bytes of this call
@@ -289,7 +291,8 @@ class beam:
             # byte codes of known labels go to the device as they are and
             # are mapped to the global species there; anything else is
             # mapped (and filtered) on the host
-            on_device = codes.dtype == np.uint8 and bool((remap >= 0).all())
+            on_device = (codes.dtype == np.uint8 and bool((remap >= 0).all()) and
+                         0 < len(remap) <= 256 and len(labels) <= engine.MAX_SPECIES)
             g = None
             if not on_device:
                 g = remap[codes]
@@ -304,15 +307,19 @@ class beam:
             pos_d[off:off + n].copy_(torch.from_numpy(np.ascontiguousarray(pos, dtype=np.float32)))
             self.last_stream_bytes += 12 * n + (n + 4 * len(remap) if on_device else 4 * n)
             if on_device:
-                lut = torch.from_numpy(remap).to(dev)
                 raw = torch.from_numpy(np.ascontiguousarray(codes)).to(dev)
-                idx_d[off:off + n] = lut[raw.long()]
+                engine.species_index(raw, remap, len(labels), idx_d[off:off + n], counts_d)
+                mapped += n
             else:
                 idx_d[off:off + n].copy_(torch.from_numpy(np.ascontiguousarray(g, dtype=np.int32)))
+                counts_h[: len(labels)] += np.bincount(g, minlength=len(labels))[: len(labels)]
             off += n
-        counts = (torch.bincount(idx_d[:off].long(), minlength=len(labels)).cpu().numpy()
-                  if off and labels else np.zeros(len(labels), dtype=np.int64))
-        return pos_d[:off], idx_d[:off], labels, counts.astype(np.int64)
+        if mapped:
+            c = counts_d.cpu().numpy()
+            if int(c.sum()) != mapped:
+                raise IndexError("species codes beyond the chunk's label table")
+            counts_h[: len(c)] += c
+        return pos_d[:off], idx_d[:off], labels, counts_h[: len(labels)].copy()
 
     def stage_atoms(self, sample, stage, device="cuda"):
         """All atoms on the device, lab frame, with their incident amplitudes

@@ -72,6 +72,18 @@ struct MkRot {
     double grid[4];
 };
 
+// x / 1e10 correctly rounded: with y = RN(1e-10) = RN(1 / 1e10) the estimate
+// q = RN(x y) is within an ulp, its remainder x - q 1e10 is exact in an FMA
+// and RN(q + r y) is the rounded quotient (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Dev. 34, 111 (1990)). Three FP64 operations instead of a division's ~20:
+// the stage transform of 8.19M atoms was bound by the FP64 pipe.
+__device__ __forceinline__ double mk_metres(float x_A)
+{
+    const double x = (double)x_A, q = x * 1e-10;
+    return fma(fma(-q, 1e10, x), 1e-10, q);
+}
+
 __global__ void mk_atoms_lab_kernel(int64_t n, const float *__restrict__ pin, MkRot R,
                                     const float2 *__restrict__ e0, int gny, int gnz,
                                     double *__restrict__ pos_lab, float2 *__restrict__ amp)
@@ -87,9 +99,9 @@ __global__ void mk_atoms_lab_kernel(int64_t n, const float *__restrict__ pin, Mk
         acc = __fadd_rn(acc, __fmul_rn(z, R.r[3 * r + 2]));
         l[r] = __fadd_rn(acc, R.t[r]);
     }
-    pos_lab[3 * i] = __ddiv_rn((double)l[0], 1e10);
-    pos_lab[3 * i + 1] = __ddiv_rn((double)l[1], 1e10);
-    pos_lab[3 * i + 2] = __ddiv_rn((double)l[2], 1e10);
+    pos_lab[3 * i] = mk_metres(l[0]);
+    pos_lab[3 * i + 1] = mk_metres(l[1]);
+    pos_lab[3 * i + 2] = mk_metres(l[2]);
     float2 a = make_float2(1.f, 0.f);
     if (e0) {
         const float iu = __fadd_rn(__fdiv_rn(l[1], (float)R.grid[0]), (float)R.grid[2]);
@@ -138,6 +150,66 @@ extern "C" int mk_atoms_lab(int64_t n, const float *pos_in, const float *rot, co
     return MK_OK;
 }
 
+// ------------------------------------------------------------- species
+// Byte species codes of a chunk -> the call's species indices, and how many
+// atoms each has (added to counts), in one pass over the codes: 5 bytes an
+// atom. An indexing pass and a histogram took 907 us for 8.19M atoms. Codes
+// without an entry are written as 0 and not counted.
+struct MkSpeciesLut {
+    signed char to[256];
+};
+
+__global__ void __launch_bounds__(256) mk_species_kernel(int64_t n, const unsigned char *__restrict__ codes,
+                                                         const __grid_constant__ MkSpeciesLut lut, int n_species,
+                                                         int *__restrict__ out,
+                                                         unsigned long long *__restrict__ counts)
+{
+    __shared__ signed char s_to[256];
+    __shared__ int s_n[MK_MAX_SPECIES];
+    s_to[threadIdx.x] = lut.to[threadIdx.x];
+    if (threadIdx.x < MK_MAX_SPECIES) s_n[threadIdx.x] = 0;
+    __syncthreads();
+    const int64_t step = (int64_t)gridDim.x * 256;
+    int mine = 0;       // lane s of a warp counts species s
+    for (int64_t i0 = (int64_t)blockIdx.x * 256; i0 < n; i0 += step) {
+        const int64_t i = i0 + threadIdx.x;
+        int s = -1;
+        if (i < n) {
+            s = s_to[codes[i]];
+            out[i] = max(s, 0);
+        }
+        for (int k = 0; k < n_species; ++k) {
+            const int m = __popc(__ballot_sync(0xffffffffu, s == k));
+            if ((int)(threadIdx.x & 31) == k) mine += m;
+        }
+    }
+    if ((threadIdx.x & 31) < n_species && mine) atomicAdd(&s_n[threadIdx.x & 31], mine);
+    __syncthreads();
+    if (threadIdx.x < n_species && s_n[threadIdx.x])
+        atomicAdd(&counts[threadIdx.x], (unsigned long long)s_n[threadIdx.x]);
+}
+
+extern "C" int mk_species_index(int64_t n, const unsigned char *codes, const int *lut, int n_lut,
+                                int n_species, int *species, int64_t *counts, void *stream)
+{
+    MK_REQUIRE(n >= 0 && n_lut >= 1 && n_lut <= 256 && n_species >= 1 && n_species <= MK_MAX_SPECIES,
+               "mk_species_index: bad sizes");
+    if (n == 0) return MK_OK;
+    MK_REQUIRE(codes && lut && species && counts, "mk_species_index: null argument");
+    MkSpeciesLut L;
+    for (int i = 0; i < 256; ++i) {
+        const int v = i < n_lut ? lut[i] : -1;
+        MK_REQUIRE(i >= n_lut || (v >= 0 && v < n_species), "mk_species_index: code %d maps to species %d of %d",
+                   i, v, n_species);
+        L.to[i] = (signed char)v;
+    }
+    const unsigned nb = (unsigned)std::min<int64_t>((n + 1023) / 1024, 152 * 8);
+    mk_species_kernel<<<nb, 256, 0, mk_stream(stream)>>>(n, codes, L, n_species, species,
+                                                        reinterpret_cast<unsigned long long *>(counts));
+    MK_CHECK_CUDA(cudaGetLastError());
+    return MK_OK;
+}
+
 // ------------------------------------------------------------- tiles
 // Bounding box of all atoms (for the Morton quantisation): one block-level
 // min/max per block, combined with atomics on the ordered-integer image of
@@ -159,48 +231,43 @@ __global__ void mk_bbox_init(unsigned long long *bb)
     else if (threadIdx.x < 6) bb[threadIdx.x] = 0ull;   // max
 }
 
-__global__ void mk_bbox_kernel(int64_t n, const double *__restrict__ pos, unsigned long long *bb)
+// A thread always meets the same coordinate (the stride is a multiple of 3),
+// so the loads are whole lines; six atomics a block.
+#define MK_BBOX_NT 192
+__global__ void __launch_bounds__(MK_BBOX_NT) mk_bbox_kernel(int64_t n, const double *__restrict__ pos,
+                                                             unsigned long long *bb)
 {
-    unsigned long long lo[3] = {~0ull, ~0ull, ~0ull}, hi[3] = {0ull, 0ull, 0ull};
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const unsigned long long o = mk_ordered(pos[3 * i + c]);
-            lo[c] = o < lo[c] ? o : lo[c];
-            hi[c] = o > hi[c] ? o : hi[c];
-        }
+    __shared__ unsigned long long s_bb[6];
+    if (threadIdx.x < 6) s_bb[threadIdx.x] = threadIdx.x < 3 ? ~0ull : 0ull;
+    __syncthreads();
+    unsigned long long lo = ~0ull, hi = 0ull;
+    const int64_t step = (int64_t)gridDim.x * MK_BBOX_NT;
+    for (int64_t i = (int64_t)blockIdx.x * MK_BBOX_NT + threadIdx.x; i < 3 * n; i += step) {
+        const unsigned long long o = mk_ordered(pos[i]);
+        lo = o < lo ? o : lo;
+        hi = o > hi ? o : hi;
     }
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        for (int off = 16; off > 0; off >>= 1) {
-            const unsigned long long a = __shfl_xor_sync(0xffffffffu, lo[c], off);
-            const unsigned long long b = __shfl_xor_sync(0xffffffffu, hi[c], off);
-            lo[c] = a < lo[c] ? a : lo[c];
-            hi[c] = b > hi[c] ? b : hi[c];
-        }
-        if ((threadIdx.x & 31) == 0) {
-            atomicMin(&bb[c], lo[c]);
-            atomicMax(&bb[3 + c], hi[c]);
-        }
-    }
+    atomicMin(&s_bb[threadIdx.x % 3], lo);
+    atomicMax(&s_bb[3 + threadIdx.x % 3], hi);
+    __syncthreads();
+    if (threadIdx.x < 3) atomicMin(&bb[threadIdx.x], s_bb[threadIdx.x]);
+    else if (threadIdx.x < 6) atomicMax(&bb[threadIdx.x], s_bb[threadIdx.x]);
 }
 
-// Position along a 3-D Hilbert curve of 2^19 cells per axis (the
+// Position along a 3-D Hilbert curve of 2^bits cells per axis (the
 // axes-to-transpose construction of J. Skilling, "Programming the Hilbert
 // curve", AIP Conf. Proc. 707, 381 (2004)): undo the rotations/reflections
 // level by level, Gray-encode, then read the bits out MSB first, x first.
 // Unlike a Z-order (Morton) curve, consecutive cells are always face
 // neighbours, so a run of consecutive atoms never spans two distant corners
 // of the sample and every tile stays compact.
-#define MK_HILBERT_BITS 17   // per axis inside one cube: 51 bits
-#define MK_MAX_CUBES 128     // 7 bits of cube index
-#define MK_KEY_BITS 62       // + 4 bits of species (MK_MAX_SPECIES = 16)
+#define MK_HILBERT_BITS 10   // per axis inside one cube, at most
+#define MK_MAX_CUBES 128     // 7 bits of cube index at most
 
-__device__ __forceinline__ unsigned long long mk_hilbert3(uint32_t x, uint32_t y, uint32_t z)
+__device__ __forceinline__ uint32_t mk_hilbert3(uint32_t x, uint32_t y, uint32_t z, int bits)
 {
     uint32_t X[3] = {x, y, z};
-    for (uint32_t Q = 1u << (MK_HILBERT_BITS - 1); Q > 1; Q >>= 1) {
+    for (uint32_t Q = 1u << (bits - 1); Q > 1; Q >>= 1) {
         const uint32_t P = Q - 1;
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
@@ -216,13 +283,13 @@ __device__ __forceinline__ unsigned long long mk_hilbert3(uint32_t x, uint32_t y
     X[1] ^= X[0];
     X[2] ^= X[1];
     uint32_t t = 0;
-    for (uint32_t Q = 1u << (MK_HILBERT_BITS - 1); Q > 1; Q >>= 1)
+    for (uint32_t Q = 1u << (bits - 1); Q > 1; Q >>= 1)
         if (X[2] & Q) t ^= Q - 1;
     X[0] ^= t;
     X[1] ^= t;
     X[2] ^= t;
-    unsigned long long h = 0;
-    for (int b = MK_HILBERT_BITS - 1; b >= 0; --b) {
+    uint32_t h = 0;
+    for (int b = bits - 1; b >= 0; --b) {
         h = (h << 1) | ((X[0] >> b) & 1u);
         h = (h << 1) | ((X[1] >> b) & 1u);
         h = (h << 1) | ((X[2] >> b) & 1u);
@@ -230,47 +297,77 @@ __device__ __forceinline__ unsigned long long mk_hilbert3(uint32_t x, uint32_t y
     return h;
 }
 
-// Sort key: species in bits 58..61, then a row of cubes, then the Hilbert
-// index inside the atom's cube. The bounding box is cut into cubes whose
-// side is its shortest extent (enlarged until at most MK_MAX_CUBES), taken
-// x fastest. The curve runs from a cube's (0,0,0) corner to its (max,0,0)
+// The cubes and the key's layout, from the bounding box, once per build.
+struct MkKeyGrid {
+    double lo[3];
+    float inv;           // 1 / cube side
+    int nc[3];           // cubes per axis
+    int bits;            // Hilbert bits per axis
+    int cube_bits;
+};
+
+__global__ void mk_key_grid_kernel(const unsigned long long *__restrict__ bb, int key_bits,
+                                   int species_bits, MkKeyGrid *__restrict__ out)
+{
+    MkKeyGrid G;
+    double span[3], side = 0.0;
+    for (int c = 0; c < 3; ++c) {
+        G.lo[c] = mk_unordered(bb[c]);
+        span[c] = mk_unordered(bb[3 + c]) - G.lo[c];
+        if (!(span[c] < 1e30)) span[c] = 0.0;       // an atom at infinity or nowhere
+        if (span[c] > 0.0 && (side == 0.0 || span[c] < side)) side = span[c];
+    }
+    if (!(side > 0.0)) side = 1.0;
+    for (;;) {
+        double all = 1.0;
+        for (int c = 0; c < 3; ++c) {
+            const double m = ceil(span[c] / side - 1e-9);
+            G.nc[c] = (int)fmin(fmax(m, 1.0), 1e6);
+            all *= G.nc[c];
+        }
+        if (!(all > MK_MAX_CUBES)) break;
+        side *= 1.25;
+    }
+    G.inv = (float)(1.0 / side);
+    G.cube_bits = 0;
+    while ((1 << G.cube_bits) < G.nc[0] * G.nc[1] * G.nc[2]) ++G.cube_bits;
+    G.bits = min(MK_HILBERT_BITS, (key_bits - species_bits - G.cube_bits) / 3);
+    *out = G;
+}
+
+// Sort key: species on top, then a row of cubes, then the Hilbert index
+// inside the atom's cube. The bounding box is cut into cubes whose side is
+// its shortest extent (enlarged until at most MK_MAX_CUBES), taken x
+// fastest. The curve runs from a cube's (0,0,0) corner to its (max,0,0)
 // corner, so consecutive cubes along x join without a jump; only row ends
 // do. One cube size for all axes keeps tiles round, and filling every cube
 // keeps the curve out of empty space (where its excursions would put
 // far-apart atoms next to each other in the order).
+// The key has 32 bits, or 24 below MK_SHORT_KEY_ATOMS atoms (four or three
+// radix passes): the cells then still outnumber the atoms. 62-bit keys
+// (17 Hilbert bits an axis, cut in FP64 by every thread) took 1355 us to make
+// and 551 us to sort for 8.19M atoms, and eight passes, 63 us, for 32k.
+#define MK_SHORT_KEY_ATOMS (1 << 17)
 __global__ void mk_keys_kernel(int64_t n, const double *__restrict__ pos,
-                               const int *__restrict__ species,
-                               const unsigned long long *__restrict__ bb,
-                               unsigned long long *__restrict__ keys, int *__restrict__ idx)
+                               const int *__restrict__ species, const MkKeyGrid *__restrict__ grid,
+                               uint32_t *__restrict__ keys, int *__restrict__ idx)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    double lo[3], span[3], side = 0.0;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        lo[c] = mk_unordered(bb[c]);
-        span[c] = mk_unordered(bb[3 + c]) - lo[c];
-        if (span[c] > 0.0 && (side == 0.0 || span[c] < side)) side = span[c];
-    }
-    if (!(side > 0.0)) side = 1.0;
-    int nc[3];
-    for (;;) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) nc[c] = max(1, (int)ceil(span[c] / side - 1e-9));
-        if (nc[0] * nc[1] * nc[2] <= MK_MAX_CUBES) break;
-        side *= 1.25;
-    }
+    const MkKeyGrid &G = *grid;
+    const int bits = G.bits;
+    const float top = (float)((1u << bits) - 1);
     uint32_t q[3];
     int cube[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        const double t = (pos[3 * i + c] - lo[c]) / side;
-        cube[c] = min(nc[c] - 1, max(0, (int)floor(t)));
-        const double f = fmin(fmax(t - cube[c], 0.0), 1.0);
-        q[c] = (uint32_t)(f * (double)((1u << MK_HILBERT_BITS) - 1));
+        const float t = (float)(pos[3 * i + c] - G.lo[c]) * G.inv;
+        cube[c] = min(G.nc[c] - 1, max(0, (int)floorf(t)));
+        const float f = fminf(fmaxf(t - (float)cube[c], 0.f), 1.f);
+        q[c] = (uint32_t)(f * top);
     }
-    const unsigned long long ci = (unsigned long long)((cube[2] * nc[1] + cube[1]) * nc[0] + cube[0]);
-    keys[i] = ((unsigned long long)species[i] << 58) | (ci << 51) | mk_hilbert3(q[0], q[1], q[2]);
+    const uint32_t ci = (uint32_t)((cube[2] * G.nc[1] + cube[1]) * G.nc[0] + cube[0]);
+    keys[i] = ((((uint32_t)species[i] << G.cube_bits) | ci) << (3 * bits)) | mk_hilbert3(q[0], q[1], q[2], bits);
     idx[i] = (int)i;
 }
 
@@ -384,16 +481,15 @@ static size_t mk_align256(size_t b) { return (b + 255) & ~(size_t)255; }
 static size_t mk_cub_temp_bytes(int64_t n)
 {
     size_t tb = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, tb, (unsigned long long *)nullptr,
-                                    (unsigned long long *)nullptr, (int *)nullptr, (int *)nullptr,
-                                    (int)n, 0, MK_KEY_BITS);
+    cub::DeviceRadixSort::SortPairs(nullptr, tb, (uint32_t *)nullptr, (uint32_t *)nullptr, (int *)nullptr,
+                                    (int *)nullptr, (int)n, 0, 32);
     return tb;
 }
 
 extern "C" size_t mk_tiles_workspace_size(int64_t n)
 {
     if (n <= 0) return 256;
-    return mk_align256(64) + 2 * mk_align256(8 * (size_t)n) + 2 * mk_align256(4 * (size_t)n) +
+    return mk_align256(64) + mk_align256(sizeof(MkKeyGrid)) + 4 * mk_align256(4 * (size_t)n) +
            mk_align256(mk_cub_temp_bytes(n));
 }
 
@@ -439,10 +535,12 @@ extern "C" int mk_tiles_build(int64_t n, const double *pos, const int *species, 
     char *w = static_cast<char *>(workspace);
     unsigned long long *bb = reinterpret_cast<unsigned long long *>(w);
     w += mk_align256(64);
-    unsigned long long *k_in = reinterpret_cast<unsigned long long *>(w);
-    w += mk_align256(8 * (size_t)n);
-    unsigned long long *k_out = reinterpret_cast<unsigned long long *>(w);
-    w += mk_align256(8 * (size_t)n);
+    MkKeyGrid *grid = reinterpret_cast<MkKeyGrid *>(w);
+    w += mk_align256(sizeof(MkKeyGrid));
+    uint32_t *k_in = reinterpret_cast<uint32_t *>(w);
+    w += mk_align256(4 * (size_t)n);
+    uint32_t *k_out = reinterpret_cast<uint32_t *>(w);
+    w += mk_align256(4 * (size_t)n);
     int *i_in = reinterpret_cast<int *>(w);
     w += mk_align256(4 * (size_t)n);
     int *i_out = reinterpret_cast<int *>(w);
@@ -450,14 +548,17 @@ extern "C" int mk_tiles_build(int64_t n, const double *pos, const int *species, 
     size_t temp = mk_cub_temp_bytes(n);
     cudaStream_t st = mk_stream(stream);
 
+    const int key_bits = n <= MK_SHORT_KEY_ATOMS ? 24 : 32;
+    int species_bits = 0;
+    while ((1 << species_bits) < n_species) ++species_bits;
     mk_bbox_init<<<1, 32, 0, st>>>(bb);
+    const int nb = (int)std::min<int64_t>((3 * n + 4 * MK_BBOX_NT - 1) / (4 * MK_BBOX_NT), 152 * 10);
+    mk_bbox_kernel<<<nb, MK_BBOX_NT, 0, st>>>(n, pos, bb);
+    mk_key_grid_kernel<<<1, 1, 0, st>>>(bb, key_bits, species_bits, grid);
     const int th = 256;
-    const int nb = (int)std::min<int64_t>((n + th - 1) / th, 4096);
-    mk_bbox_kernel<<<nb, th, 0, st>>>(n, pos, bb);
-    mk_keys_kernel<<<(unsigned)((n + th - 1) / th), th, 0, st>>>(n, pos, species, bb, k_in, i_in);
+    mk_keys_kernel<<<(unsigned)((n + th - 1) / th), th, 0, st>>>(n, pos, species, grid, k_in, i_in);
     MK_CHECK_CUDA(cudaGetLastError());
-    MK_CHECK_CUDA(cub::DeviceRadixSort::SortPairs(w, temp, k_in, k_out, i_in, i_out, (int)n, 0,
-                                                  MK_KEY_BITS, st));
+    MK_CHECK_CUDA(cub::DeviceRadixSort::SortPairs(w, temp, k_in, k_out, i_in, i_out, (int)n, 0, key_bits, st));
     if (tiles_needed > 0) {
         mk_tile_kernel<256><<<tiles_needed, 256, 0, st>>>(
             M, k / MK_TWO_PI, pos, reinterpret_cast<const float2 *>(amp), i_out,

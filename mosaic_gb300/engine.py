@@ -25,6 +25,7 @@ from . import _lib
 from ._lib import MkLaunch, MkNodePlan, MkPhysics, MkPixels, MkSpecies, MkTiles, check
 
 R_E = 2.81794092e-15
+MAX_SPECIES = _lib.MAX_SPECIES
 
 
 def _require_cuda():
@@ -396,6 +397,16 @@ class Atoms:
     @property
     def n(self):
         return int(self.pos.shape[0])
+
+
+def species_index(codes, lut, n_species, out, counts, stream=None):
+    """Device byte codes -> species indices ``out`` (int32) through the host
+    table ``lut`` (int32), counted into the device ``counts`` (int64)
+    (mk_species_index)."""
+    lut = np.ascontiguousarray(lut, dtype=np.int32)
+    check(_require_cuda().mk_species_index(int(codes.numel()), _ptr(codes), lut.ctypes.data, len(lut),
+                                           int(n_species), _ptr(out), _ptr(counts),
+                                           _stream_handle(stream)))
 
 
 def atoms_lab(pos_A, species_idx, rot, trans, table, e0=None, grid=None, device="cuda",

@@ -44,7 +44,7 @@
 
 #include "mk_split.cuh"
 
-#define MK_NODE_MAX 16       // nodes per axis at most
+#define MK_NODE_MAX 20       // nodes per axis at most (fine nodes: 16)
 #define MK_NODE_SB 4         // sources staged per step
 #define MK_PIX_COLS 32       // pixel block: 32 columns x 16 rows, 4 rows a thread
 #define MK_PIX_ROWS 16
@@ -174,7 +174,7 @@ extern "C" int mk_plane_fit(int n_frames, const long long *shapes, long long max
 #define MK_SUM_PARTS 64      // chunks a frame's intensity sum is added in
 namespace {
 
-const int kNodeCounts[] = {6, 8, 10, 12, 16};
+const int kNodeCounts[] = {6, 8, 10, 12, 16, 20};
 
 // Largest phase half-range phi [rad] n Chebyshev nodes interpolate to
 // 4 (phi/2)^n / n! <= 3e-8.
@@ -244,43 +244,63 @@ bool lay_out(const std::vector<Geo> &g, double k, double r2, int n1, double r1, 
     return true;
 }
 
-struct Ball { double c[3], r; };
-
-// Ball around the tiles idx[a..b): centre of the box of their balls.
-Ball bound(const double *org, const std::vector<int> &idx, size_t a, size_t b)
-{
-    double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-    for (size_t i = a; i < b; ++i) {
-        const double *o = org + 4ll * idx[i];
+// A run of tiles being gathered into a group: the box of their origins and
+// their widest radius bound the group's radius about the box's centre.
+struct Run {
+    double lo[3], hi[3], rmax;
+    int count;
+    void start(const double *o)
+    {
+        for (int c = 0; c < 3; ++c) lo[c] = hi[c] = o[c];
+        rmax = o[3];
+        count = 1;
+    }
+    // Adds a tile if the group's radius stays within r2.
+    bool add(const double *o, double r2)
+    {
+        double l[3], h[3], d2 = 0.0;
         for (int c = 0; c < 3; ++c) {
-            lo[c] = std::min(lo[c], o[c] - o[3]);
-            hi[c] = std::max(hi[c], o[c] + o[3]);
+            l[c] = std::min(lo[c], o[c]);
+            h[c] = std::max(hi[c], o[c]);
+            d2 += (h[c] - l[c]) * (h[c] - l[c]);
         }
+        const double r = std::max(rmax, o[3]);
+        if (!(0.5 * std::sqrt(d2) + r <= r2)) return false;
+        for (int c = 0; c < 3; ++c) { lo[c] = l[c]; hi[c] = h[c]; }
+        rmax = r;
+        ++count;
+        return true;
     }
-    Ball B;
-    for (int c = 0; c < 3; ++c) B.c[c] = 0.5 * (lo[c] + hi[c]);
-    B.r = 0.0;
-    for (size_t i = a; i < b; ++i) {
-        const double *o = org + 4ll * idx[i];
-        const double dx = o[0] - B.c[0], dy = o[1] - B.c[1], dz = o[2] - B.c[2];
-        B.r = std::max(B.r, std::sqrt(dx * dx + dy * dy + dz * dz) + o[3]);
-    }
-    return B;
-}
+};
 
-double quantile(std::vector<double> v, double q)
+// Cuts the narrow tiles (radius <= r1) of [a, b), in order, into runs of one
+// species, radius <= r2 and at most `most` tiles: done(run, last) for each.
+template <class Done>
+void cut_runs(const double *org, const int *tsp, int a, int b, double r1, double r2, int most, Done done)
 {
-    if (v.empty()) return 0.0;
-    const size_t i = std::min(v.size() - 1, (size_t)std::floor(q * (v.size() - 1) + 0.5));
-    std::nth_element(v.begin(), v.begin() + i, v.end());
-    return v[i];
+    Run R;
+    R.count = 0;
+    int sp = -1;
+    for (int t = a; t < b; ++t) {
+        const double *o = org + 4ll * t;
+        if (!(o[3] <= r1)) continue;
+        if (R.count && tsp[t] == sp && R.count < most && R.add(o, r2)) continue;
+        if (R.count) done(R);
+        R.start(o);
+        sp = tsp[t];
+    }
+    if (R.count) done(R);
 }
 
 size_t up256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-// Costs [s] of one leaf term, one (source, pixel) and one (tile, fine node)
-// of the merge, and what a launch costs.
-const double kLeaf = 0.55e-12, kPix = 4.5e-12, kMerge = 6.0e-12, kLaunch = 4e-6;
+// Costs [s], measured: one leaf term (2.1e12 a second), one (source, pixel) and
+// one (tile, fine node) of the merge, both times 0.4 + 0.05 n for n nodes per
+// axis, what a launch costs, and a term and the set-up of the split kernel where
+// it takes a few wide tiles (its bounds, its plan, its own reduction).
+const double kLeaf = 0.48e-12, kPix = 4.1e-12, kMerge = 9.0e-12, kLaunch = 4e-6;
+const double kWide = 0.3e-12, kWideSetup = 150e-6;
+double per_node(int n) { return 0.4 + 0.05 * n; }
 
 struct Choice {
     double cost = 1e300, r1 = 0.0, r2 = 0.0;
@@ -357,60 +377,65 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
         return third + k * r * dev <= phase_tol && 2.0 * (omax + r) / rmin < 1e-6;
     };
     const double T = tile_atoms;
-    auto direct = [&](double n) { return n * T * n_pix * direct_s_per_term; };
-    plan->direct_s = direct(n_tiles) + 2.0 * kLaunch;
+    plan->direct_s = n_tiles * T * n_pix * direct_s_per_term + 2.0 * kLaunch;
+    auto split = [&](double n) { return n > 0.0 ? n * T * n_pix * kWide + n_pix * 30e-12 + kWideSetup : 0.0; };
 
+    // Search on a sample: at most 2048 tiles, in 8 stretches of the curve.
+    const int stretch = n_tiles <= 2048 ? n_tiles : 256, stretches = n_tiles <= 2048 ? 1 : 8;
+    std::vector<double> some;
+    std::vector<int> starts;
+    for (int i = 0; i < stretches; ++i) {
+        const int a = (int)((long long)(n_tiles - stretch) * i / std::max(stretches - 1, 1));
+        starts.push_back(a);
+        some.insert(some.end(), rad.begin() + a, rad.begin() + a + stretch);
+    }
+    std::sort(some.begin(), some.end());
+    const double up = (double)n_tiles / some.size();
+    auto q = [&](double x) { return some[(size_t)std::floor(x * (some.size() - 1) + 0.5)]; };
+    std::vector<double> tail;               // the widest tiles, all of them: few, but dear
+    for (double r : rad)
+        if (r > q(0.9)) tail.push_back(r);
+    std::sort(tail.begin(), tail.end());
     Choice best;
-    const double q1[] = {1.0, 0.99, 0.9};
-    for (int iq = 0; iq < 3; ++iq) {
-        const double r1 = quantile(rad, q1[iq]);
-        if (iq > 0 && r1 == rmax) continue;
-        std::vector<int> nar;
-        for (int t = 0; t < n_tiles; ++t)
-            if (rad[t] <= r1) nar.push_back(t);
-        const double n_nar = (double)nar.size();
+    const double q1[] = {rmax, q(0.99), q(0.95), q(0.8), q(0.5)};
+    const double f2[] = {1.0, 1.5, 2.2, 3.2, 4.5, 6.5};
+    for (int i1 = 0; i1 < 5; ++i1) {
+        const double r1 = q1[i1];
+        if (i1 > 0 && r1 == q1[i1 - 1]) continue;
+        auto above = [&](double r) {            // tiles wider than r (few: exactly)
+            if (r >= q(0.9)) return (double)(tail.end() - std::upper_bound(tail.begin(), tail.end(), r));
+            return up * (double)(some.end() - std::upper_bound(some.begin(), some.end(), r));
+        };
+        const double n_nar = n_tiles - above(r1);
+        if (n_nar < 1.0) continue;
         // no groups: every tile within r1 straight from its nodes
         if (admitted(r1) && group_tiles <= 0)
             for (int n1 : kNodeCounts) {
                 double N1, N0;
-                if (!lay_out(geo, k, r1, n1, 0.0, 0, nullptr, &N1, &N0)) continue;
-                const double c = n_nar * T * N1 * kLeaf + n_nar * n_pix * kPix * (0.4 + 0.05 * n1) +
-                                 direct(n_tiles - n_nar) + 4.0 * kLaunch;
+                if (n1 > 16 || !lay_out(geo, k, r1, n1, 0.0, 0, nullptr, &N1, &N0)) continue;
+                const double c = n_nar * T * N1 * kLeaf + n_nar * n_pix * kPix * per_node(n1) +
+                                 split(n_tiles - n_nar) + 4.0 * kLaunch;
                 if (c < best.cost) { best.cost = c; best.r1 = best.r2 = r1; best.n0 = 0; best.n1 = n1; best.G = 0; }
             }
         if (group_tiles == 0 || (group_tiles < 0 && n_tiles < 32)) continue;
-        for (int G = group_tiles > 0 ? group_tiles : 8; G <= (group_tiles > 0 ? group_tiles : 128); G *= 2) {
-            std::vector<double> gr;
-            std::vector<int> gn;
-            for (size_t a = 0; a < nar.size();) {
-                size_t b = a;
-                while (b < nar.size() && b < a + G && tsp[nar[b]] == tsp[nar[a]]) ++b;
-                gr.push_back(bound(origins, nar, a, b).r);
-                gn.push_back((int)(b - a));
-                a = b;
-            }
-            for (double q2 : {1.0, 0.95, 0.8}) {
-                const double r2 = std::max(quantile(gr, q2), r1);
-                if (!admitted(r2)) continue;
-                double groups = 0, in_groups = 0, mid = 0, wide = 0;
-                for (size_t i = 0; i < gr.size(); ++i) {
-                    if (gr[i] <= r2) { groups += 1; in_groups += gn[i]; }
-                    else mid += gn[i];
-                }
-                for (int t = 0; t < n_tiles; ++t)
-                    if (rad[t] > r1) (rad[t] <= r2 ? mid : wide) += 1;
-                for (int n1 : kNodeCounts) {
-                    if (n1 > 12) continue;
-                    for (int n0 : kNodeCounts) {
-                        if (n0 < 8) continue;
-                        double N1, N0;
-                        if (!lay_out(geo, k, r2, n1, r1, n0, nullptr, &N1, &N0)) continue;
-                        const double c = in_groups * T * N0 * kLeaf + mid * T * N1 * kLeaf +
-                                         in_groups * N1 * kMerge * (0.4 + 0.05 * n0) +
-                                         (groups + mid) * n_pix * kPix * (0.4 + 0.05 * n1) + direct(wide) +
-                                         6.0 * kLaunch;
-                        if (c < best.cost) { best.cost = c; best.r1 = r1; best.r2 = r2; best.n0 = n0; best.n1 = n1; best.G = G; }
-                    }
+        const int G = group_tiles > 0 ? group_tiles : 4096;
+        for (double f : f2) {
+            const double r2 = std::max(f * q(0.5), r1);
+            if ((f > 1.0 && r2 == r1) || !admitted(r2)) continue;
+            double groups = 0.0;
+            for (int a : starts)
+                cut_runs(origins, tsp.data(), a, a + stretch, r1, r2, G, [&](const Run &) { groups += up; });
+            const double wide = above(r2), mid = above(r1) - wide;
+            for (int n1 : kNodeCounts) {
+                if (n1 > 12) continue;
+                for (int n0 : kNodeCounts) {
+                    if (n0 < 8) continue;
+                    double N1, N0;
+                    if (!lay_out(geo, k, r2, n1, r1, n0, nullptr, &N1, &N0)) continue;
+                    const double c = n_nar * T * N0 * kLeaf + mid * T * N1 * kLeaf +
+                                     n_nar * N1 * kMerge * per_node(n0) +
+                                     (groups + mid) * n_pix * kPix * per_node(n1) + split(wide) + 6.0 * kLaunch;
+                    if (c < best.cost) { best.cost = c; best.r1 = r1; best.r2 = r2; best.n0 = n0; best.n1 = n1; best.G = G; }
                 }
             }
         }
@@ -427,12 +452,7 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
     lay_out(geo, k, best.r2, best.n1, best.r1, best.n0, &cuts, &N1, &N0);
     for (int f = 0; f < n_frames; ++f) fr[f] = cuts[shape_of[f]];
     std::vector<MkNodeSrc> src;
-    std::vector<int> nar, members, mid, wide;
-    for (int t = 0; t < n_tiles; ++t) {
-        if (rad[t] <= best.r1) nar.push_back(t);
-        else if (rad[t] <= best.r2) mid.push_back(t);
-        else wide.push_back(t);
-    }
+    std::vector<int> members, mid, wide;
     auto add_src = [&](const double *c, int species, int count, long long first) {
         MkNodeSrc S{};
         for (int i = 0; i < 3; ++i) {
@@ -445,23 +465,19 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
         S.first = first;
         src.push_back(S);
     };
-    if (best.G == 0) {
-        mid.insert(mid.end(), nar.begin(), nar.end());
-    } else {
-        for (size_t a = 0; a < nar.size();) {
-            size_t b = a;
-            while (b < nar.size() && b < a + best.G && tsp[nar[b]] == tsp[nar[a]]) ++b;
-            const Ball B = bound(origins, nar, a, b);
-            if (B.r <= best.r2) {
-                add_src(B.c, tsp[nar[a]], (int)(b - a), (long long)members.size());
-                members.insert(members.end(), nar.begin() + a, nar.begin() + b);
-            } else {
-                mid.insert(mid.end(), nar.begin() + a, nar.begin() + b);
-            }
-            a = b;
-        }
+    for (int t = 0; t < n_tiles; ++t) {
+        if (rad[t] > best.r2) wide.push_back(t);
+        else if (best.G == 0 || rad[t] > best.r1) mid.push_back(t);
+        else members.push_back(t);
     }
-    std::sort(mid.begin(), mid.end());          // by species
+    if (best.G) {
+        long long first = 0;
+        cut_runs(origins, tsp.data(), 0, n_tiles, best.r1, best.r2, best.G, [&](const Run &R) {
+            const double c[3] = {0.5 * (R.lo[0] + R.hi[0]), 0.5 * (R.lo[1] + R.hi[1]), 0.5 * (R.lo[2] + R.hi[2])};
+            add_src(c, tsp[members[first]], R.count, first);
+            first += R.count;
+        });
+    }
     plan->n_groups = (int)src.size();
     for (int t : mid) add_src(origins + 4ll * t, tsp[t], 0, 0);
     plan->n_src = (int)src.size();
@@ -804,8 +820,8 @@ template <int N0>
 __global__ void __launch_bounds__(256) mk_node_merge_kernel(const MkNodeArgs A)
 {
     __shared__ __align__(16) float2 s_v[2][MK_NODE_SB][N0 * N0];
-    __shared__ __align__(16) float2 s_t[MK_NODE_SB][MK_NODE_MAX][N0];
-    __shared__ float s_wz[MK_NODE_MAX][N0];
+    __shared__ __align__(16) float2 s_t[MK_NODE_SB][16][N0];
+    __shared__ float s_wz[16][N0];
     __shared__ float s_d[2][MK_NODE_SB][6];
     const long long patch = blockIdx.x % A.patches1;
     const int grp = (int)(blockIdx.x / A.patches1);
@@ -1229,6 +1245,7 @@ extern "C" int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, c
             case 10: mk_launch_merge<10>(A, grid, st); break;
             case 12: mk_launch_merge<12>(A, grid, st); break;
             case 16: mk_launch_merge<16>(A, grid, st); break;
+            case 20: mk_launch_merge<20>(A, grid, st); break;
             default: mk_set_error("mk_kin_nodes_f32: %d coarse nodes", n0); return MK_EINVAL;
             }
         }

@@ -300,7 +300,7 @@ __device__ __forceinline__ uint32_t mk_hilbert3(uint32_t x, uint32_t y, uint32_t
 // The cubes and the key's layout, from the bounding box, once per build.
 struct MkKeyGrid {
     double lo[3];
-    float inv;           // 1 / cube side
+    float inv[3];        // 1 / cube side, per axis
     int nc[3];           // cubes per axis
     int bits;            // Hilbert bits per axis
     int cube_bits;
@@ -321,14 +321,14 @@ __global__ void mk_key_grid_kernel(const unsigned long long *__restrict__ bb, in
     for (;;) {
         double all = 1.0;
         for (int c = 0; c < 3; ++c) {
-            const double m = ceil(span[c] / side - 1e-9);
+            const double m = floor(span[c] / side + 0.5);
             G.nc[c] = (int)fmin(fmax(m, 1.0), 1e6);
             all *= G.nc[c];
         }
         if (!(all > MK_MAX_CUBES)) break;
         side *= 1.25;
     }
-    G.inv = (float)(1.0 / side);
+    for (int c = 0; c < 3; ++c) G.inv[c] = span[c] > 0.0 ? (float)(G.nc[c] / span[c]) : 0.f;
     G.cube_bits = 0;
     while ((1 << G.cube_bits) < G.nc[0] * G.nc[1] * G.nc[2]) ++G.cube_bits;
     G.bits = min(MK_HILBERT_BITS, (key_bits - species_bits - G.cube_bits) / 3);
@@ -336,13 +336,16 @@ __global__ void mk_key_grid_kernel(const unsigned long long *__restrict__ bb, in
 }
 
 // Sort key: species on top, then a row of cubes, then the Hilbert index
-// inside the atom's cube. The bounding box is cut into cubes whose side is
-// its shortest extent (enlarged until at most MK_MAX_CUBES), taken x
-// fastest. The curve runs from a cube's (0,0,0) corner to its (max,0,0)
-// corner, so consecutive cubes along x join without a jump; only row ends
-// do. One cube size for all axes keeps tiles round, and filling every cube
-// keeps the curve out of empty space (where its excursions would put
-// far-apart atoms next to each other in the order).
+// inside the atom's cube. The bounding box is cut into near-cubes, along each
+// axis the whole number of the shortest extent (enlarged until at most
+// MK_MAX_CUBES) that is nearest, taken x fastest. The curve runs from a
+// cube's (0,0,0) corner to its (max,0,0) corner, so consecutive cubes along
+// x join without a jump; only row ends do. Filling every cube keeps the curve
+// out of empty space (where its excursions would put far-apart atoms next to
+// each other in the order): cubes of one exact side left slivers of the
+// longer extents as cubes of their own, a few atoms thick, and every tile
+// that crossed one spanned the sample (5.4M atoms of a cubic polycrystal: 14
+// tiles too wide for the node form, 2.1 ms in the split kernel at 1024^2).
 // The key has 32 bits, or 24 below MK_SHORT_KEY_ATOMS atoms (four or three
 // radix passes): the cells then still outnumber the atoms. 62-bit keys
 // (17 Hilbert bits an axis, cut in FP64 by every thread) took 1355 us to make
@@ -361,7 +364,7 @@ __global__ void mk_keys_kernel(int64_t n, const double *__restrict__ pos,
     int cube[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        const float t = (float)(pos[3 * i + c] - G.lo[c]) * G.inv;
+        const float t = (float)(pos[3 * i + c] - G.lo[c]) * G.inv[c];
         cube[c] = min(G.nc[c] - 1, max(0, (int)floorf(t)));
         const float f = fminf(fmaxf(t - (float)cube[c], 0.f), 1.f);
         q[c] = (uint32_t)(f * top);

@@ -46,6 +46,7 @@
 
 #define MK_NODE_MAX 20       // nodes per axis at most (fine nodes: 16)
 #define MK_NODE_SB 4         // sources staged per step
+#define MK_MERGE_NT 128      // threads of a merge block
 #define MK_PIX_COLS 32       // pixel block: 32 columns x 16 rows, 4 rows a thread
 #define MK_PIX_ROWS 16
 #define MK_NODE_PAD 0.25     // half pixel pitches the node interval exceeds the pixel centres
@@ -59,9 +60,11 @@ struct MkNodeFrame {
     int l1y, l1z, p1y, p1z;
     int ratio_y, ratio_z, p0y, p0z;
     int bpy, bpz;                       // pixel blocks per fine patch
+    int strip, strips;                  // merge: fine patches per strip, strips per coarse patch
+    int rowg, chunks;                   // row groups of a block, blocks per strip
     long long pix_off;
     long long node0_off, patch1_off;    // node1_off = patch1_off * n1^2
-    long long pblk_off, part_off, w_off;
+    long long pblk_off, part_off, w_off, item_off;
 };
 
 // A source of the pixel step: a group of tiles (count > 0: nar[first ..]) or
@@ -292,13 +295,32 @@ void cut_runs(const double *org, const int *tsp, int a, int b, double r1, double
     if (R.count) done(R);
 }
 
+// Rows a thread of the merge holds, a divisor of n1.
+int merge_rows(int n1) { return n1 == 10 ? 5 : n1 == 6 || n1 == 12 ? 3 : 4; }
+
+// Cuts a coarse patch's row of fine patches into strips of at most 128 node
+// columns for the merge's blocks, the strip length that keeps most of their
+// 128 threads busy.
+void lay_strips(MkNodeFrame *F, int n1)
+{
+    const int rows = merge_rows(n1), most = std::min(F->ratio_y, MK_MERGE_NT / n1);
+    double best = -1.0;
+    for (int sp = 1; sp <= most; ++sp) {
+        const int strips = (F->ratio_y + sp - 1) / sp;
+        const int rowg = std::min(MK_MERGE_NT / (sp * n1), n1 / rows);
+        const int chunks = (n1 / rows + rowg - 1) / rowg;
+        const double use = (double)F->ratio_y * n1 * n1 / ((double)strips * chunks * MK_MERGE_NT * rows) + 1e-3 * sp;
+        if (use > best) { best = use; F->strip = sp; F->strips = strips; F->rowg = rowg; F->chunks = chunks; }
+    }
+}
+
 size_t up256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 // Costs [s], measured: one leaf term (2.1e12 a second), one (source, pixel) and
 // one (tile, fine node) of the merge, both times 0.4 + 0.05 n for n nodes per
 // axis, what a launch costs, and a term and the set-up of the split kernel where
 // it takes a few wide tiles (its bounds, its plan, its own reduction).
-const double kLeaf = 0.48e-12, kPix = 4.1e-12, kMerge = 9.0e-12, kLaunch = 4e-6;
+const double kLeaf = 0.48e-12, kPix = 4.1e-12, kMerge = 3.8e-12, kLaunch = 4e-6;
 const double kWide = 0.3e-12, kWideSetup = 150e-6;
 double per_node(int n) { return 0.4 + 0.05 * n; }
 
@@ -496,7 +518,7 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
         mk_set_error("mk_nodes_plan: every tile is wider than the plan's radius");
         return MK_EDECLINE;
     }
-    long long pblk = 0, wf = 0, patch = 0, node0 = 0;
+    long long pblk = 0, wf = 0, patch = 0, node0 = 0, item = 0;
     for (int f = 0; f < n_frames; ++f) {
         MkNodeFrame &F = fr[f];
         const double *t = fit + 12ll * f;
@@ -511,6 +533,11 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
         F.patch1_off = patch;
         F.pblk_off = pblk;
         F.w_off = wf;
+        F.item_off = item;
+        if (best.G) {
+            lay_strips(&F, best.n1);
+            item += (long long)F.p1z * F.p0y * F.strips * F.chunks;
+        }
         patch += (long long)F.p1y * F.p1z;
         node0 += best.G ? (long long)F.p0y * F.p0z * best.n0 * best.n0 : 0;
         pblk += (long long)F.p1y * F.p1z * F.bpy * F.bpz;
@@ -534,7 +561,7 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
     const double n1sq = (double)best.n1 * best.n1;
     size_t need = 0;
     const size_t budget = (size_t)4 << 30;
-    long long chunk_n0 = 0, chunk_p1 = 0, chunk_pix = 0;
+    long long chunk_n0 = 0, chunk_p1 = 0, chunk_pix = 0, chunk_it = 0;
     int fa = 0;
     auto bytes = [&](long long a, long long b, long long c) {
         return up256(8 * (size_t)(a * (long long)members.size())) +
@@ -544,16 +571,18 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
     for (int f = 0; f < n_frames; ++f) {
         const long long a = best.G ? (long long)fr[f].p0y * fr[f].p0z * best.n0 * best.n0 : 0;
         const long long b = (long long)fr[f].p1y * fr[f].p1z, c = (long long)fr[f].ny * fr[f].nz;
-        const bool too_many = (chunk_p1 + b) * std::max(plan->n_groups, 1) > (1ll << 30) ||
+        const long long it = best.G ? (long long)fr[f].p1z * fr[f].p0y * fr[f].strips * fr[f].chunks : 0;
+        const bool too_many = (chunk_it + it) * std::max(plan->n_groups, 1) > (1ll << 30) ||
                               (chunk_n0 + a) > 256ll * 60000 || (chunk_p1 + b) * n1sq > 256.0 * 60000;
         if (f > fa && (bytes(chunk_n0 + a, chunk_p1 + b, chunk_pix + c) > budget || too_many)) {
             ++passes;
             fa = f;
-            chunk_n0 = chunk_p1 = chunk_pix = 0;
+            chunk_n0 = chunk_p1 = chunk_pix = chunk_it = 0;
         }
         chunk_n0 += a;
         chunk_p1 += b;
         chunk_pix += c;
+        chunk_it += it;
         need = std::max(need, bytes(chunk_n0, chunk_p1, chunk_pix));
     }
     plan->passes = passes;
@@ -588,7 +617,7 @@ struct MkNodeArgs {
     int f_lo, f_hi;                  // frames of this pass
     int n0, n1, n_groups, n_src, src_per_slice, tile_atoms;
     long long nodes0, patches1;      // of this pass
-    long long node0_base, patch1_base, pblk_base, part_base;
+    long long node0_base, patch1_base, pblk_base, part_base, item_base, items;
     const MkNodeSrc *src;
     const int *members;
     const MkNodeRec *rec0, *rec1;    // of every frame
@@ -813,46 +842,72 @@ __device__ __forceinline__ void mk_stage_fields(float2 (*s_v)[N * N], const floa
     }
 }
 
-// Merge: block = (group, fine patch), one fine node a thread. The group's
-// tiles come SB at a time: first the interpolation along z to the patch's
-// n1 node rows (shared by the row's nodes), then along y per node.
-template <int N0>
-__global__ void __launch_bounds__(256) mk_node_merge_kernel(const MkNodeArgs A)
+// Merge: block = (group, strip of neighbouring fine patches, rows of their
+// nodes); a thread one node column of the strip and ROWS rows. The group's
+// tiles come SB at a time: first the interpolation along z to the block's
+// rows, which all the strip's columns share, then along y per node. Bound by
+// the FMA pipe: 2 N0 + ~47 FP32 operations a (tile, fine node), N0 from the
+// interpolation along y. With one fine patch a block (the z interpolation,
+// N0^2 / n1 packed FMAs a node, made again for every patch of a row) it took
+// 6.72 ms for N0 = 20, n1 = 12 on the 1024 x 1024 detector and 1.46 ms for N0 =
+// 16 on the 512 x 512 one; here 2.34 and 0.70 ms (4.5 and 5.2 ps a (tile, fine
+// node)).
+template <int N0, int ROWS>
+__global__ void __launch_bounds__(MK_MERGE_NT) mk_node_merge_kernel(const MkNodeArgs A)
 {
+    constexpr int MAXR = 16;                 // rows of a block at most
     __shared__ __align__(16) float2 s_v[2][MK_NODE_SB][N0 * N0];
-    __shared__ __align__(16) float2 s_t[MK_NODE_SB][16][N0];
-    __shared__ float s_wz[16][N0];
-    __shared__ float s_d[2][MK_NODE_SB][6];
-    const long long patch = blockIdx.x % A.patches1;
-    const int grp = (int)(blockIdx.x / A.patches1);
+    __shared__ __align__(16) float2 s_t[MK_NODE_SB][MAXR][N0];
+    __shared__ float s_wz[MAXR][N0];
+    __shared__ __align__(16) float s_d[2][MK_NODE_SB][8];
+    const long long it = A.item_base + blockIdx.x % A.items;
+    const int grp = (int)(blockIdx.x / A.items);
     const int n1 = A.n1;
-    const long long gpatch = A.patch1_base + patch;
-    const int f = mk_find_frame(A.f_lo, A.f_hi, gpatch, [&](int i) { return A.frames[i].patch1_off; });
+    const int f = mk_find_frame(A.f_lo, A.f_hi, it, [&](int i) { return A.frames[i].item_off; });
     const MkNodeFrame &F = A.frames[f];
-    const int lp = (int)(gpatch - F.patch1_off), pz = lp / F.p1y, py = lp - pz * F.p1y;
-    const int cy = py / F.ratio_y, cz = pz / F.ratio_z;
-    const int suby = py - cy * F.ratio_y, subz = pz - cz * F.ratio_z;
+    int e = (int)(it - F.item_off);
+    const int chunk = e % F.chunks;
+    e /= F.chunks;
+    const int strip = e % F.strips;
+    e /= F.strips;
+    const int cy = e % F.p0y, pz = e / F.p0y;
+    const int suby0 = strip * F.strip;
+    const int patches = min(min(F.strip, F.ratio_y - suby0), F.p1y - (cy * F.ratio_y + suby0));
+    if (patches <= 0) return;                // a last coarse patch with fewer fine ones
+    const int width = F.strip * n1;          // node columns of a full strip
+    const int cz = pz / F.ratio_z, subz = pz - cz * F.ratio_z;
+    const int rows = F.rowg * ROWS, row0 = chunk * rows;      // rows of this block
     const float *W = A.weights + F.w_off + (long long)n1 * (F.ny + F.nz);
-    const float *Wy = W + suby * n1 * N0, *Wz = W + F.ratio_y * n1 * N0 + subz * n1 * N0;
-    for (int i = threadIdx.x; i < n1 * N0; i += blockDim.x) s_wz[i / N0][i % N0] = Wz[i];
-    const int oy = threadIdx.x % n1, oz = threadIdx.x / n1;
-    const bool live = oz < n1;
+    const float *Wy = W + (long long)suby0 * n1 * N0, *Wz = W + (F.ratio_y + subz) * n1 * N0;
+    const int nrow = min(rows, n1 - row0);
+    for (int i = threadIdx.x; i < nrow * N0; i += MK_MERGE_NT) s_wz[i / N0][i % N0] = Wz[row0 * N0 + i];
+    const int rg = threadIdx.x / width, oc = threadIdx.x - rg * width;
+    const bool live = oc < patches * n1 && rg * ROWS < nrow && rg < F.rowg;
+    const int oc1 = live ? oc : 0, lr = live ? rg * ROWS : 0;
     mk_f2 wy[N0];
 #pragma unroll
-    for (int i = 0; i < N0; ++i) wy[i] = f2_splat(Wy[oy * N0 + i]);
+    for (int i = 0; i < N0; ++i) wy[i] = f2_splat(Wy[oc1 * N0 + i]);
     const MkNodeSrc &S = A.src[grp];
     const double gx = S.o[0], gy = S.o[1], gz = S.o[2];
-    const MkNodeRec R = A.rec1[gpatch * n1 * n1 + (live ? oz * n1 + oy : 0)];
-    // directions from the group's origin
-    float3 qh = make_float3(R.qh.x, R.qh.y, R.qh.z), ql, u = make_float3(R.u.x, R.u.y, R.u.z);
-    float half;
-    {
-        const float ox = (float)gx, oy_ = (float)gy, oz_ = (float)gz;
-        const float uo = fmaf(u.z, oz_, fmaf(u.y, oy_, u.x * ox));
+    // the thread's nodes: patch of its column, rows lr .. lr + ROWS - 1
+    const int py = cy * F.ratio_y + suby0 + oc1 / n1;
+    const long long node = (F.patch1_off - A.patch1_base + (long long)pz * F.p1y + py) * n1 * n1 +
+                           (row0 + lr) * n1 + oc1 % n1;
+    const MkNodeRec *rec = A.rec1 + A.patch1_base * n1 * n1 + node;
+    float3 qh[ROWS], ql[ROWS], u[ROWS];
+    float half[ROWS], accr[ROWS], acci[ROWS], cr[ROWS], ci[ROWS];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {         // directions from the group's origin
+        const MkNodeRec R = rec[r * n1];
+        const float ox = (float)gx, oy = (float)gy, oz = (float)gz;
+        qh[r] = make_float3(R.qh.x, R.qh.y, R.qh.z);
+        u[r] = make_float3(R.u.x, R.u.y, R.u.z);
+        const float uo = fmaf(u[r].z, oz, fmaf(u[r].y, oy, u[r].x * ox));
         const float kr = A.kappa * R.w.w;
-        ql = make_float3(fmaf(ox - uo * u.x, kr, R.ql.x), fmaf(oy_ - uo * u.y, kr, R.ql.y),
-                         fmaf(oz_ - uo * u.z, kr, R.ql.z));
-        half = 0.5f * kr / fmaf(-uo, R.w.w, 1.f);
+        ql[r] = make_float3(fmaf(ox - uo * u[r].x, kr, R.ql.x), fmaf(oy - uo * u[r].y, kr, R.ql.y),
+                            fmaf(oz - uo * u[r].z, kr, R.ql.z));
+        half[r] = 0.5f * kr / fmaf(-uo, R.w.w, 1.f);
+        accr[r] = acci[r] = cr[r] = ci[r] = 0.f;
     }
     const float2 *V = A.V0 + (F.node0_off - A.node0_base) + (long long)(cz * F.p0y + cy) * N0 * N0;
     const long long first = S.first;
@@ -864,15 +919,17 @@ __global__ void __launch_bounds__(256) mk_node_merge_kernel(const MkNodeArgs A)
         if ((int)threadIdx.x < m) {
             const double4 o = A.origin[A.members[first + s0 + threadIdx.x]];
             const double d[3] = {o.x - gx, o.y - gy, o.z - gz};
+            float *sd = s_d[buf][threadIdx.x], dd = 0.f;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 const float h = (float)d[c];
-                s_d[buf][threadIdx.x][c] = h;
-                s_d[buf][threadIdx.x][3 + c] = (float)(d[c] - (double)h);
+                sd[c] = h;
+                sd[4 + c] = (float)(d[c] - (double)h);
+                dd = fmaf(h, h, dd);
             }
+            sd[3] = dd;
         }
     };
-    float accr = 0.f, acci = 0.f, cr = 0.f, ci = 0.f;
     stage(0, 0);
     for (int s0 = 0, buf = 0; s0 < count; s0 += MK_NODE_SB, buf ^= 1) {
         const int m = min(MK_NODE_SB, count - s0);
@@ -883,8 +940,8 @@ __global__ void __launch_bounds__(256) mk_node_merge_kernel(const MkNodeArgs A)
             mk_cp_wait<0>();
         }
         __syncthreads();
-        for (int i = threadIdx.x; i < m * n1 * N0; i += blockDim.x) {
-            const int s = i / (n1 * N0), r = i - s * n1 * N0, row = r / N0, c = r - row * N0;
+        for (int i = threadIdx.x; i < m * nrow * N0; i += MK_MERGE_NT) {
+            const int s = i / (nrow * N0), r = i - s * nrow * N0, row = r / N0, c = r - row * N0;
             mk_f2 a = 0ull;
 #pragma unroll
             for (int j = 0; j < N0; ++j)
@@ -893,34 +950,38 @@ __global__ void __launch_bounds__(256) mk_node_merge_kernel(const MkNodeArgs A)
         }
         __syncthreads();
         if (live) {
-#pragma unroll 2
             for (int s = 0; s < m; ++s) {
-                mk_f2 v = 0ull;
-                const ulonglong2 *t2 = reinterpret_cast<const ulonglong2 *>(s_t[s][oz]);
+                const float4 d4 = *reinterpret_cast<const float4 *>(s_d[buf][s]);
+                const float4 l4 = *reinterpret_cast<const float4 *>(s_d[buf][s] + 4);
+                const float3 dh = make_float3(d4.x, d4.y, d4.z), dl = make_float3(l4.x, l4.y, l4.z);
 #pragma unroll
-                for (int i = 0; i < N0 / 2; ++i) {
-                    const ulonglong2 t = t2[i];
-                    v = f2_fma(wy[2 * i], t.x, v);
-                    v = f2_fma(wy[2 * i + 1], t.y, v);
+                for (int r = 0; r < ROWS; ++r) {
+                    mk_f2 v = 0ull;
+                    const ulonglong2 *t2 = reinterpret_cast<const ulonglong2 *>(s_t[s][lr + r]);
+#pragma unroll
+                    for (int i = 0; i < N0 / 2; ++i) {
+                        const ulonglong2 t = t2[i];
+                        v = f2_fma(wy[2 * i], t.x, v);
+                        v = f2_fma(wy[2 * i + 1], t.y, v);
+                    }
+                    const float ud = fmaf(u[r].z, dh.z, fmaf(u[r].y, dh.y, u[r].x * dh.x));
+                    float ph = fmaf(fmaf(-ud, ud, d4.w), half[r], mk_dot_frac(qh[r], ql[r], dh, dl));
+                    ph = mk_frac_nearest(ph);
+                    float sn, cs;
+                    __sincosf(ph * TWO_PI_F, &sn, &cs);
+                    const float2 vv = f2_unpack(v);
+                    mk_kahan(vv.x * cs - vv.y * sn, accr[r], cr[r]);
+                    mk_kahan(vv.x * sn + vv.y * cs, acci[r], ci[r]);
                 }
-                const float *d = s_d[buf][s];
-                const float3 dh = make_float3(d[0], d[1], d[2]), dl = make_float3(d[3], d[4], d[5]);
-                const float ud = fmaf(u.z, dh.z, fmaf(u.y, dh.y, u.x * dh.x));
-                const float dd = fmaf(dh.z, dh.z, fmaf(dh.y, dh.y, dh.x * dh.x));
-                float ph = fmaf(fmaf(-ud, ud, dd), half, mk_dot_frac(qh, ql, dh, dl));
-                ph = mk_frac_nearest(ph);
-                float sn, cs;
-                __sincosf(ph * TWO_PI_F, &sn, &cs);
-                const float2 vv = f2_unpack(v);
-                mk_kahan(vv.x * cs - vv.y * sn, accr, cr);
-                mk_kahan(vv.x * sn + vv.y * cs, acci, ci);
             }
         }
         __syncthreads();        // s_d and s_t are read; the next step may stage
     }
-    if (live)
-        A.V1[(long long)grp * (A.patches1 * n1 * n1) + patch * n1 * n1 + threadIdx.x] =
-            make_float2(accr - cr, acci - ci);
+    if (live) {
+        float2 *out = A.V1 + (long long)grp * (A.patches1 * n1 * n1) + node;
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) out[r * n1] = make_float2(accr[r] - cr[r], acci[r] - ci[r]);
+    }
 }
 
 // Pixels: block = (32 x 16 pixels of one fine patch, slice of sources), a
@@ -1121,7 +1182,11 @@ static void mk_launch_pixels(const MkNodeArgs &A, dim3 grid, cudaStream_t st)
 template <int N>
 static void mk_launch_merge(const MkNodeArgs &A, unsigned grid, cudaStream_t st)
 {
-    mk_node_merge_kernel<N><<<grid, (A.n1 * A.n1 + 31) / 32 * 32, 0, st>>>(A);
+    switch (merge_rows(A.n1)) {
+    case 3: mk_node_merge_kernel<N, 3><<<grid, MK_MERGE_NT, 0, st>>>(A); break;
+    case 4: mk_node_merge_kernel<N, 4><<<grid, MK_MERGE_NT, 0, st>>>(A); break;
+    default: mk_node_merge_kernel<N, 5><<<grid, MK_MERGE_NT, 0, st>>>(A); break;
+    }
 }
 
 extern "C" int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, const mk_pixels *px,
@@ -1204,7 +1269,7 @@ extern "C" int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, c
     // passes of whole frames whose node fields and partials fit the chunk
     const size_t budget = std::max((size_t)plan->chunk_bytes, (size_t)1);
     for (int fa = 0; fa < plan->n_frames;) {
-        long long a = 0, b = 0, c = 0, pb = 0;
+        long long a = 0, b = 0, c = 0, pb = 0, items = 0;
         int fb = fa;
         auto bytes = [&](long long x, long long y, long long z) {
             return up256(8 * (size_t)(x * plan->n_members)) +
@@ -1214,13 +1279,15 @@ extern "C" int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, c
             const MkNodeFrame &F = hf[fb];
             const long long da = n0 ? (long long)F.p0y * F.p0z * n0 * n0 : 0;
             const long long dp = (long long)F.p1y * F.p1z, dc = (long long)F.ny * F.nz;
-            const bool too_many = (b + dp) * std::max(plan->n_groups, 1) > (1ll << 30) ||
+            const long long di = n0 ? (long long)F.p1z * F.p0y * F.strips * F.chunks : 0;
+            const bool too_many = (items + di) * std::max(plan->n_groups, 1) > (1ll << 30) ||
                                   (a + da) > 256ll * 60000 || (b + dp) * (double)(n1 * n1) > 256.0 * 60000;
             if (fb > fa && (bytes(a + da, b + dp, c + dc) > budget || too_many)) break;
             a += da;
             b += dp;
             c += dc;
             pb += dp * F.bpy * F.bpz;
+            items += di;
             ++fb;
         }
         A.f_lo = fa;
@@ -1230,6 +1297,8 @@ extern "C" int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, c
         A.node0_base = hf[fa].node0_off;
         A.patch1_base = hf[fa].patch1_off;
         A.pblk_base = hf[fa].pblk_off;
+        A.item_base = hf[fa].item_off;
+        A.items = items;
         A.part_base = hf[fa].part_off;
         char *cw = w;
         A.V0 = reinterpret_cast<float2 *>(cw);
@@ -1239,7 +1308,7 @@ extern "C" int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, c
         A.partial = reinterpret_cast<double2 *>(cw);
         if (plan->n_members > 0) {
             leaf(A.members, plan->n_members, rec0 + A.node0_base, a, A.V0);
-            const unsigned grid = (unsigned)(b * plan->n_groups);
+            const unsigned grid = (unsigned)(items * plan->n_groups);
             switch (n0) {
             case 8: mk_launch_merge<8>(A, grid, st); break;
             case 10: mk_launch_merge<10>(A, grid, st); break;

@@ -16,8 +16,8 @@ from mosaic_gb300 import _lib
 K = 2 * np.pi / 1.2398e-10
 FRAME = np.dtype([("p0", "f8", 3), ("ey", "f8", 3), ("ez", "f8", 3), ("b", "f8", 3)] +
                  [(n, "i4") for n in ("ny", "nz", "l1y", "l1z", "p1y", "p1z", "ratio_y", "ratio_z",
-                                      "p0y", "p0z", "bpy", "bpz")] +
-                 [(n, "i8") for n in ("pix_off", "node0_off", "patch1_off", "pblk_off", "part_off", "w_off")])
+                                      "p0y", "p0z", "bpy", "bpz", "strip", "strips", "rowg", "chunks")] +
+                 [(n, "i8") for n in ("pix_off", "node0_off", "patch1_off", "pblk_off", "part_off", "w_off", "item_off")])
 SRC = np.dtype([("dh", "f4", 3), ("species", "i4"), ("dl", "f4", 3), ("count", "i4"), ("o", "f8", 3),
                 ("first", "i8")])
 
@@ -108,6 +108,24 @@ def _run(plan, buf, org, atoms, shapes, P, n_pix):
         return np.array([np.exp(2j * np.pi * _phase(Pn, b, o, a - o)) for a in atoms[t]]).sum(0)
 
     for F in fr:
+        if n0:                  # the merge's blocks cover every fine node once
+            rows = {6: 3, 8: 4, 10: 5, 12: 3}[n1]
+            got = np.zeros((F["p1z"], F["p1y"], n1, n1), int)
+            for e in range(F["p1z"] * F["p0y"] * F["strips"] * F["chunks"]):
+                e, chunk = divmod(e, F["chunks"])
+                e, strip = divmod(e, F["strips"])
+                pz, cy = divmod(e, F["p0y"])
+                s0 = strip * F["strip"]
+                patches = min(F["strip"], F["ratio_y"] - s0, F["p1y"] - cy * F["ratio_y"] - s0)
+                row0 = chunk * F["rowg"] * rows
+                nrow = min(F["rowg"] * rows, n1 - row0)
+                assert F["rowg"] * rows <= 16 and F["strip"] * n1 * F["rowg"] <= 128 and nrow % rows == 0
+                for th in range(128 if patches > 0 else 0):
+                    rg, oc = divmod(th, F["strip"] * n1)
+                    if oc < patches * n1 and rg * rows < nrow and rg < F["rowg"]:
+                        r = row0 + rg * rows
+                        got[pz, cy * F["ratio_y"] + s0 + oc // n1, r:r + rows, oc % n1] += 1
+            assert (got == 1).all()
         l0y, l0z = F["l1y"] * F["ratio_y"], F["l1z"] * F["ratio_z"]
         V0 = {}
         for p in range(F["p0y"] * F["p0z"] if n0 else 0):

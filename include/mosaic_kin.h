@@ -203,6 +203,16 @@ int mk_sync_status(void *stream);
  * compute_scattering_cffi (Beam.py:716-746) and pixel_phasor (Beam.py:9241-9255). */
 int mk_pixels_prepare(const mk_pixels *px, const mk_physics *phys, void *stream);
 
+/* A scan's pixels in one launch: lab coordinates [A] of every frame into the
+ * sample frame, xyz = R^T (P - t) / 1e10, and the prologue of
+ * mk_pixels_prepare with each frame's own direction. frames: device
+ * (n_frames, 20) doubles R (9, row-major), t (3), b (3), first pixel, ny, nz,
+ * offset into lab, 1 unused; lab: device, a frame's (3, ny nz) array from its
+ * offset on (frames may share one); max_pix: pixels of the largest frame; xyz (n, 3) and px's arrays
+ * are written. */
+int mk_scan_pixels(int n_frames, const double *frames, int max_pix, const double *lab, double k,
+                   double *xyz, const mk_pixels *px, void *stream);
+
 /* The scattering factor (f0 + f' + i f'') e^{-B s^2} sqrt(P_pol) of every
  * species at every pixel's own direction, into px->factor (n_species, n_pix,
  * 2) float32: once per (species, pixel), where the reference evaluates f0,

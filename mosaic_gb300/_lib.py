@@ -163,6 +163,8 @@ class MkNodePlan(ctypes.Structure):
 
 # name -> (restype, argtypes)
 SIGNATURES = {
+    "mk_scan_pixels": (ctypes.c_int, [ctypes.c_int, _vp, ctypes.c_int, _vp, ctypes.c_double, _vp,
+                                      ctypes.POINTER(MkPixels), _vp]),
     "mk_species_index": (ctypes.c_int, [ctypes.c_int64, _vp, _vp, ctypes.c_int, ctypes.c_int, _vp, _vp,
                                         _vp]),
     "mk_plane_fit": (ctypes.c_int, [ctypes.c_int, _vp, ctypes.c_longlong, _vp, _vp, _vp]),

@@ -89,23 +89,19 @@ struct MkNodeRec {       // one node's direction: 64 bytes
 // Per frame: first pixel, mean column and row steps, and how far the pixels
 // are from the product grid p0 + y_col ey + z_row ez of their own projected
 // coordinates (fit[9], m), the smallest |P| (fit[10]) and the largest
-// departure of y_col, z_row from column and row number (fit[11], pixels).
-__device__ __forceinline__ void mk_fit_axes(const double *xyz, int ny, int nz, double *p0, double *ey,
-                                            double *ez)
-{
-    for (int c = 0; c < 3; ++c) {
-        p0[c] = xyz[c];
-        ey[c] = ny > 1 ? (xyz[3ll * (ny - 1) + c] - p0[c]) / (ny - 1) : 0.0;
-        ez[c] = nz > 1 ? (xyz[3ll * (nz - 1) * ny + c] - p0[c]) / (nz - 1) : 0.0;
-    }
-}
+// departure of y_col, z_row from column and row number (fit[11], pixels). The
+// three are gathered as squares; ~35 operations of the FP64 pipe a pixel.
 
-// Coordinate of a first-row (first-column) pixel along its axis, in steps.
-__device__ __forceinline__ double mk_axis_coord(const double *p, const double *p0, const double *e)
+// Coordinate of a first-row (first-column) pixel along its axis, in steps;
+// inv = 1 / |e|^2, 0 for an axis of one pixel.
+__device__ __forceinline__ double mk_axis_coord(const double *p, const double *p0, const double *e, double inv)
+{
+    return ((p[0] - p0[0]) * e[0] + (p[1] - p0[1]) * e[1] + (p[2] - p0[2]) * e[2]) * inv;
+}
+__device__ __forceinline__ double mk_axis_inv(const double *e)
 {
     const double n2 = e[0] * e[0] + e[1] * e[1] + e[2] * e[2];
-    if (!(n2 > 0.0)) return 0.0;
-    return ((p[0] - p0[0]) * e[0] + (p[1] - p0[1]) * e[1] + (p[2] - p0[2]) * e[2]) / n2;
+    return n2 > 0.0 ? 1.0 / n2 : 0.0;
 }
 
 __global__ void mk_fit_init_kernel(int n_frames, const long long *__restrict__ shapes,
@@ -114,8 +110,13 @@ __global__ void mk_fit_init_kernel(int n_frames, const long long *__restrict__ s
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= n_frames) return;
     const double *p = xyz + 3 * shapes[3 * f];
+    const long long ny = shapes[3 * f + 1], nz = shapes[3 * f + 2];
     double *o = fit + 12 * (long long)f;
-    mk_fit_axes(p, (int)shapes[3 * f + 1], (int)shapes[3 * f + 2], o, o + 3, o + 6);
+    for (int c = 0; c < 3; ++c) {
+        o[c] = p[c];
+        o[3 + c] = ny > 1 ? (p[3 * (ny - 1) + c] - p[c]) / (ny - 1) : 0.0;
+        o[6 + c] = nz > 1 ? (p[3 * (nz - 1) * ny + c] - p[c]) / (nz - 1) : 0.0;
+    }
     o[9] = 0.0;
     o[10] = 1e300;
     o[11] = 0.0;
@@ -129,25 +130,25 @@ __global__ void mk_fit_kernel(const long long *__restrict__ shapes, const double
     const int ny = (int)shapes[3 * f + 1], nz = (int)shapes[3 * f + 2];
     const double *P = xyz + 3 * off;
     double *o = fit + 12 * (long long)f;
-    double p0[3], ey[3], ez[3];
-    mk_fit_axes(P, ny, nz, p0, ey, ez);
+    const double p0[3] = {o[0], o[1], o[2]}, ey[3] = {o[3], o[4], o[5]}, ez[3] = {o[6], o[7], o[8]};
+    const double iy = mk_axis_inv(ey), iz = mk_axis_inv(ez);
     double dev = 0.0, rmin = 1e300, skew = 0.0;
     const long long n = (long long)ny * nz;
     for (long long i = (long long)blockIdx.y * blockDim.x + threadIdx.x; i < n;
          i += (long long)gridDim.y * blockDim.x) {
         const int row = (int)(i / ny), col = (int)(i - (long long)row * ny);
-        const double y = mk_axis_coord(P + 3ll * col, p0, ey);
-        const double z = mk_axis_coord(P + 3ll * row * ny, p0, ez);
+        const double y = mk_axis_coord(P + 3ll * col, p0, ey, iy);
+        const double z = mk_axis_coord(P + 3ll * row * ny, p0, ez, iz);
         double d2 = 0.0, r2 = 0.0;
         for (int c = 0; c < 3; ++c) {
             const double v = P[3 * i + c], m = p0[c] + y * ey[c] + z * ez[c];
             d2 += (v - m) * (v - m);
             r2 += v * v;
         }
-        const double d = sqrt(d2), s = fmax(fabs(y - (ny > 1 ? col : 0)), fabs(z - (nz > 1 ? row : 0)));
-        dev = fmax(dev, d <= 1e300 ? d : INFINITY);         // a NaN counts as infinite
+        const double s = fmax(fabs(y - (ny > 1 ? col : 0)), fabs(z - (nz > 1 ? row : 0)));
+        dev = fmax(dev, d2 <= 1e300 ? d2 : INFINITY);       // a NaN counts as infinite
         skew = fmax(skew, s <= 1e300 ? s : INFINITY);
-        rmin = fmin(rmin, r2 >= 0.0 ? sqrt(r2) : 0.0);
+        rmin = fmin(rmin, r2 >= 0.0 ? r2 : 0.0);
     }
     for (int w = 16; w > 0; w >>= 1) {
         dev = fmax(dev, __shfl_xor_sync(0xffffffffu, dev, w));
@@ -155,6 +156,8 @@ __global__ void mk_fit_kernel(const long long *__restrict__ shapes, const double
         rmin = fmin(rmin, __shfl_xor_sync(0xffffffffu, rmin, w));
     }
     if ((threadIdx.x & 31) == 0) {      // non-negative doubles order as their bits
+        dev = sqrt(dev);
+        rmin = sqrt(rmin);
         atomicMax(reinterpret_cast<unsigned long long *>(o + 9), (unsigned long long)__double_as_longlong(dev));
         atomicMin(reinterpret_cast<unsigned long long *>(o + 10), (unsigned long long)__double_as_longlong(rmin));
         atomicMax(reinterpret_cast<unsigned long long *>(o + 11), (unsigned long long)__double_as_longlong(skew));
@@ -719,7 +722,7 @@ __global__ void mk_node_prep_kernel(const MkNodeFrame *__restrict__ frames, int 
             if (row) e -= wy;
             const int len = row ? F.l1z : F.l1y;
             const double *P = xyz + 3 * (F.pix_off + (row ? (long long)e * F.ny : e));
-            double v = mk_axis_coord(P, F.p0, row ? F.ez : F.ey);
+            double v = mk_axis_coord(P, F.p0, row ? F.ez : F.ey, mk_axis_inv(row ? F.ez : F.ey));
             const double c = (e / len) * (double)len + 0.5 * (len - 1);
             mk_lagrange((v - c) / mk_half_range(len), n1, out);
             float *o = W + (row ? (long long)n1 * F.ny : 0) + (long long)e * n1;

@@ -5,6 +5,64 @@
 #include "mk_common.cuh"
 
 // ------------------------------------------------------------------ pixels
+// x / 1e10 correctly rounded: with y = RN(1e-10) = RN(1 / 1e10) the estimate
+// q = RN(x y) is within an ulp, its remainder x - q 1e10 is exact in an FMA
+// and RN(q + r y) is the rounded quotient (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Dev. 34, 111 (1990)). Three FP64 operations instead of a division's ~20:
+// the stage transform of 8.19M atoms was bound by the FP64 pipe.
+__device__ __forceinline__ double mk_metres(double x)
+{
+    const double q = x * 1e-10;
+    return fma(fma(-q, 1e10, x), 1e-10, q);
+}
+
+// x mod 2 pi for x >= 0 (2 pi the double), exactly as fmod: the remainder is
+// representable, so an FMA with the right integer quotient returns it; the
+// quotient from the product with 1 / 2 pi is at most one off.
+__device__ __forceinline__ double mk_mod_2pi(double x)
+{
+    double r = fma(-trunc(x * (1.0 / MK_TWO_PI)), MK_TWO_PI, x);
+    if (r < 0.0) r = fma(-(trunc(x * (1.0 / MK_TWO_PI)) - 1.0), MK_TWO_PI, x);
+    else if (r >= MK_TWO_PI) r = fma(-(trunc(x * (1.0 / MK_TWO_PI)) + 1.0), MK_TWO_PI, x);
+    return r;
+}
+
+// One pixel's prologue from its position and its two neighbours' (right and
+// upper; edge pixels the inner one): see mk_pixels_kernel.
+struct MkPixelOut {
+    double r0;
+    double4 q;
+    float4 u;
+    double2 phasor;
+};
+
+__device__ __forceinline__ MkPixelOut mk_pixel(const double (&t)[3], const double (&n0)[3], const double (&n1)[3],
+                                               double kappa, double k, const double (&b)[3])
+{
+    MkPixelOut o;
+    const double R = sqrt(t[0] * t[0] + t[1] * t[1] + t[2] * t[2]);
+    double ux = 0.0, uy = 0.0, uz = 0.0;
+    const double inv = R > 0.0 ? 1.0 / R : 0.0;
+    if (R > 0.0) { ux = t[0] * inv; uy = t[1] * inv; uz = t[2] * inv; }
+    o.r0 = R;
+    o.u = make_float4((float)ux, (float)uy, (float)uz, (float)inv);
+    double s, c;
+    sincos(mk_mod_2pi(k * R), &s, &c);
+    o.phasor = make_double2(c, s);
+    double q2 = 0.0;
+    for (int j = 0; j < 2; ++j) {
+        const double (&m)[3] = j ? n1 : n0;
+        const double Rr = sqrt(m[0] * m[0] + m[1] * m[1] + m[2] * m[2]);
+        double cd = (Rr > 0.0) ? (ux * m[0] + uy * m[1] + uz * m[2]) / Rr : 1.0;
+        cd = fmin(1.0, fmax(-1.0, cd));
+        const double qn = k * sqrt(fmax(0.0, 2.0 * (1.0 - cd)));
+        q2 += qn * qn;
+    }
+    o.q = make_double4(kappa * (b[0] - ux), kappa * (b[1] - uy), kappa * (b[2] - uz), 0.5 * sqrt(q2));
+    return o;
+}
+
 // One thread per pixel. Everything of magnitude |P| is kept in double here so
 // the sum kernels only ever see it as (i) an FP64 dot product with a tile
 // origin and (ii) the per-pixel phasor exp(i k |P|).
@@ -16,31 +74,80 @@ __global__ void mk_pixels_kernel(int ny, int nz, const double *__restrict__ xyz,
     const int n = ny * nz;
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
-    const double tx = xyz[3 * p], ty = xyz[3 * p + 1], tz = xyz[3 * p + 2];
-    const double R = sqrt(tx * tx + ty * ty + tz * tz);
-    double ux = 0.0, uy = 0.0, uz = 0.0;
-    if (R > 0.0) { ux = tx / R; uy = ty / R; uz = tz / R; }
-    r0[p] = R;
-    u[p] = make_float4((float)ux, (float)uy, (float)uz, R > 0.0 ? (float)(1.0 / R) : 0.f);
-    double s, c;
-    sincos(fmod(k * R, MK_TWO_PI), &s, &c);
-    phasor[p] = make_double2(c, s);
     // Q_cut: half the pixel diagonal in Q from the right and upper neighbours,
     // edge pixels taking the inner one (compute_scattering_cffi, Beam.py:716-746).
     const int col = p % ny, row = p / ny;
     const int nb0 = (col + 1 < ny) ? p + 1 : ((col > 0) ? p - 1 : p);
     const int nb1 = (row + 1 < nz) ? p + ny : ((row > 0) ? p - ny : p);
-    double q2 = 0.0;
-    for (int j = 0; j < 2; ++j) {
-        const int m = j ? nb1 : nb0;
-        const double rx = xyz[3 * m], ry = xyz[3 * m + 1], rz = xyz[3 * m + 2];
-        const double Rr = sqrt(rx * rx + ry * ry + rz * rz);
-        double cd = (Rr > 0.0) ? (ux * rx + uy * ry + uz * rz) / Rr : 1.0;
-        cd = fmin(1.0, fmax(-1.0, cd));
-        const double qn = k * sqrt(fmax(0.0, 2.0 * (1.0 - cd)));
-        q2 += qn * qn;
+    const double t[3] = {xyz[3 * p], xyz[3 * p + 1], xyz[3 * p + 2]};
+    const double n0[3] = {xyz[3 * nb0], xyz[3 * nb0 + 1], xyz[3 * nb0 + 2]};
+    const double n1[3] = {xyz[3 * nb1], xyz[3 * nb1 + 1], xyz[3 * nb1 + 2]};
+    const double b[3] = {bx, by, bz};
+    const MkPixelOut o = mk_pixel(t, n0, n1, kappa, k, b);
+    r0[p] = o.r0;
+    u[p] = o.u;
+    phasor[p] = o.phasor;
+    q[p] = o.q;
+}
+
+// A scan's frames: lab pixels (A) into the sample frame, P' = R^T (P - t) /
+// 1e10, and their prologue, all frames in one launch. `frames`: 20 doubles
+// each -- R (9), t (3), b (3), first pixel, ny, nz, lab offset, 1 unused -- and
+// lab holds a frame's (3, ny nz) coordinates from that offset on (frames of one
+// ROI may share them). FP64 pipe:
+// ~250 operations a pixel. 64 frames of 128 x 128: the frames' transforms in
+// NumPy and a launch each took 17 ms of host and 0.87 ms of GPU time; here
+// 0.41 ms.
+__global__ void __launch_bounds__(256) mk_scan_pixels_kernel(const double *__restrict__ frames,
+                                                             const double *__restrict__ lab, double kappa,
+                                                             double k, double *__restrict__ xyz,
+                                                             double *__restrict__ r0, double4 *__restrict__ q,
+                                                             float4 *__restrict__ u, double2 *__restrict__ phasor)
+{
+    const double *F = frames + 20ll * blockIdx.y;
+    const long long off = (long long)F[15];
+    const int ny = (int)F[16], nz = (int)F[17], n = ny * nz;
+    const double b[3] = {F[12], F[13], F[14]};
+    const double *L = lab + (long long)F[18];
+    for (int p = blockIdx.x * 256 + threadIdx.x; p < n; p += gridDim.x * 256) {
+        const int row = p / ny, col = p - row * ny;
+        const int i0 = (col + 1 < ny) ? p + 1 : ((col > 0) ? p - 1 : p);
+        const int i1 = (row + 1 < nz) ? p + ny : ((row > 0) ? p - ny : p);
+        double P[3][3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const int i = j == 0 ? p : (j == 1 ? i0 : i1);
+            const double x = L[i] - F[9], y = L[n + i] - F[10], z = L[2ll * n + i] - F[11];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) P[j][c] = mk_metres(F[c] * x + F[3 + c] * y + F[6 + c] * z);
+        }
+        const MkPixelOut o = mk_pixel(P[0], P[1], P[2], kappa, k, b);
+        const long long g = off + p;
+        xyz[3 * g] = P[0][0];
+        xyz[3 * g + 1] = P[0][1];
+        xyz[3 * g + 2] = P[0][2];
+        r0[g] = o.r0;
+        q[g] = o.q;
+        u[g] = o.u;
+        phasor[g] = o.phasor;
     }
-    q[p] = make_double4(kappa * (bx - ux), kappa * (by - uy), kappa * (bz - uz), 0.5 * sqrt(q2));
+}
+
+extern "C" int mk_scan_pixels(int n_frames, const double *frames, int max_pix, const double *lab, double k,
+                              double *xyz, const mk_pixels *px, void *stream)
+{
+    MK_REQUIRE(n_frames >= 1 && frames && max_pix >= 1 && lab && xyz && px && px->r0 && px->q && px->u &&
+                   px->phasor && k > 0.0,
+               "mk_scan_pixels: bad arguments");
+    const int gx = std::min((max_pix + 255) / 256, 1024);
+    for (int f = 0; f < n_frames; f += 65535) {
+        const int m = std::min(n_frames - f, 65535);
+        mk_scan_pixels_kernel<<<dim3(gx, m), 256, 0, mk_stream(stream)>>>(
+            frames + 20ll * f, lab, k / MK_TWO_PI, k, xyz, px->r0, reinterpret_cast<double4 *>(px->q),
+            reinterpret_cast<float4 *>(px->u), reinterpret_cast<double2 *>(px->phasor));
+        MK_CHECK_CUDA(cudaGetLastError());
+    }
+    return MK_OK;
 }
 
 extern "C" int mk_pixels_prepare(const mk_pixels *px, const mk_physics *phys, void *stream)
@@ -72,18 +179,6 @@ struct MkRot {
     double grid[4];
 };
 
-// x / 1e10 correctly rounded: with y = RN(1e-10) = RN(1 / 1e10) the estimate
-// q = RN(x y) is within an ulp, its remainder x - q 1e10 is exact in an FMA
-// and RN(q + r y) is the rounded quotient (P. Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
-// Dev. 34, 111 (1990)). Three FP64 operations instead of a division's ~20:
-// the stage transform of 8.19M atoms was bound by the FP64 pipe.
-__device__ __forceinline__ double mk_metres(float x_A)
-{
-    const double x = (double)x_A, q = x * 1e-10;
-    return fma(fma(-q, 1e10, x), 1e-10, q);
-}
-
 __global__ void mk_atoms_lab_kernel(int64_t n, const float *__restrict__ pin, MkRot R,
                                     const float2 *__restrict__ e0, int gny, int gnz,
                                     double *__restrict__ pos_lab, float2 *__restrict__ amp)
@@ -99,7 +194,7 @@ __global__ void mk_atoms_lab_kernel(int64_t n, const float *__restrict__ pin, Mk
         acc = __fadd_rn(acc, __fmul_rn(z, R.r[3 * r + 2]));
         l[r] = __fadd_rn(acc, R.t[r]);
     }
-    pos_lab[3 * i] = mk_metres(l[0]);
+    pos_lab[3 * i] = mk_metres(l[0]);       // float32 lab positions, widened
     pos_lab[3 * i + 1] = mk_metres(l[1]);
     pos_lab[3 * i + 2] = mk_metres(l[2]);
     float2 a = make_float2(1.f, 0.f);

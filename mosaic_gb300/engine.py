@@ -179,6 +179,50 @@ class Pixels:
         if off != P:
             raise ValueError(f"frames cover {off} pixels, xyz has {P}")
 
+    @classmethod
+    def of_scan(cls, frames, beam_dirs, phys, device="cuda", stream=None):
+        """The concatenated pixels of a scan's frames (``scan.Frame``: rotation,
+        translation, lab pixels (3, P) in A, shape) in the sample frame,
+        transformed and prepared on the device in one launch
+        (``mk_scan_pixels``), each with its own direction."""
+        L = _require_cuda()
+        self = cls.__new__(cls)
+        self.shapes = [(int(f.shape[0]), int(f.shape[1])) for f in frames]
+        sizes = [ny * nz for ny, nz in self.shapes]
+        offs = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+        self.spans = [(int(o), m) for o, m in zip(offs[:-1], sizes)]
+        P = int(offs[-1])
+        dd = dict(dtype=torch.float64, device=device)
+        rec = np.zeros((len(frames), 20))
+        arrays, first, size = [], {}, 0       # frames may share a pixel array: uploaded once
+        for i, f in enumerate(frames):
+            if np.shape(f.pixels) != (3, sizes[i]):
+                raise ValueError(f"frame {i}: pixels {np.shape(f.pixels)} do not match its shape {self.shapes[i]}")
+            if id(f.pixels) not in first:
+                first[id(f.pixels)] = size
+                arrays.append((size, f.pixels))
+                size += 3 * sizes[i]
+            rec[i, :9] = np.asarray(f.rotation, dtype=np.float64).reshape(9)
+            rec[i, 9:12] = np.asarray(f.translation, dtype=np.float64).reshape(3)
+            rec[i, 12:15] = beam_dirs[i]
+            rec[i, 15:19] = offs[i], *self.shapes[i], first[id(f.pixels)]
+        lab = torch.empty(size, **dd)
+        for a, px in arrays:
+            t = torch.from_numpy(np.array(px, dtype=np.float64, order="C")).view(-1)   # a copy: may be read-only
+            lab[a:a + t.numel()].copy_(t)
+        self.xyz = torch.empty((P, 3), **dd)
+        self.r0 = torch.empty(P, **dd)
+        self.q = torch.empty((P, 4), **dd)
+        self.u = torch.empty((P, 4), dtype=torch.float32, device=device)
+        self.phasor = torch.empty((P, 2), **dd)
+        self.ny, self.nz, self.n = P, 1, P
+        self.abi = MkPixels(P, 1, self.xyz.data_ptr(), self.r0.data_ptr(), self.q.data_ptr(),
+                            self.u.data_ptr(), self.phasor.data_ptr())
+        rec_d = torch.from_numpy(rec).to(device)
+        check(L.mk_scan_pixels(len(frames), _ptr(rec_d), max(sizes), _ptr(lab), float(phys.k),
+                               _ptr(self.xyz), ctypes.byref(self.abi), _stream_handle(stream)))
+        return self
+
     def factor_table(self, table, phys, stream=None):
         """(n_species, P, 2) float32 scattering factors of every species at
         every pixel's own direction (``mk_factor_table``), for single

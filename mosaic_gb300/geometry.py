@@ -267,6 +267,8 @@ class Stage:
         for coupled in self._motor_coupling[idx]:
             if coupled is None:
                 break
+            if self._motor_value[coupled] == 0.0:       # the identity, exactly
+                continue
             axes[idx] = axis_rotation(self.get_motor_axis(coupled), self._motor_value[coupled],
                                       dtype=np.float32) @ axes[idx]
         return axes[idx]
@@ -274,6 +276,8 @@ class Stage:
     def get_rotation(self):
         R = np.eye(3, dtype=np.float32)
         for i in np.where(self._motor_type == "R")[0]:
+            if self._motor_value[i] == 0.0:             # the identity, exactly
+                continue
             R = axis_rotation(self.get_motor_axis(i), self._motor_value[i], dtype=np.float32) @ R
         self._rotation = R
         return R
@@ -281,6 +285,8 @@ class Stage:
     def get_translation(self):
         t = np.zeros(3, dtype=np.float32)
         for i in np.where(self._motor_type == "T")[0]:
+            if self._motor_value[i] == 0.0:
+                continue
             t += self.get_motor_axis(i) * self._motor_value[i]
         self._translation = t
         return t

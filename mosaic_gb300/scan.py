@@ -66,12 +66,14 @@ class BatchedScan:
             else the autotuner's cached choice for this scan size, else tuned
             now on a probe of the first frames when ``tune`` (default: the
             beam's ``_autotune``), else the default).
+        nodes: False sums every (atom, pixel) in the split kernel even where
+            the node form is admitted.
         staged: an earlier BatchedScan of the same sample whose atoms and
             tiles this one reuses.
     """
 
     def __init__(self, beam, sample, frames, apply_polarization=False, spherical_decay=False,
-                 remove_forward=False, launch=None, device="cuda", staged=None, tune=None):
+                 remove_forward=False, launch=None, device="cuda", staged=None, tune=None, nodes=True):
         self.L = engine._require_cuda()
         self.beam = beam
         self.frames = list(frames)
@@ -85,18 +87,13 @@ class BatchedScan:
         pol = beam._polarization_state()
         e_lab = np.array(pol[1:4], dtype=np.float64)
         b_lab = np.array([1.0, 0.0, 0.0])
-        xyz, fr, bdirs, pols = [], [], [], []
+        bdirs, pols = [], []
         for f in self.frames:
             R = np.asarray(f.rotation, dtype=np.float64)
-            t = np.asarray(f.translation, dtype=np.float64)
-            P = np.asarray(f.pixels, dtype=np.float64)
-            xyz.append((R.T @ (P - t[:, None])) / 1e10)
-            b = R.T @ b_lab
-            fr.append((int(f.shape[0]), int(f.shape[1]), b))
-            bdirs.append(b)
+            bdirs.append(R.T @ b_lab)
             pols.append(R.T @ e_lab)
-        self.frame_pixels = np.array([int(s[0]) * int(s[1]) for s in fr], dtype=np.int32)
-        self.frame_rows = np.array([int(s[0]) for s in fr], dtype=np.int32)
+        self.frame_pixels = np.array([int(f.shape[0]) * int(f.shape[1]) for f in self.frames], dtype=np.int32)
+        self.frame_rows = np.array([int(f.shape[0]) for f in self.frames], dtype=np.int32)
         self.offsets = np.concatenate([[0], np.cumsum(self.frame_pixels)]).astype(np.int64)
         n_total = int(self.offsets[-1])
         self._bd = np.ascontiguousarray(np.array(bdirs, dtype=np.float64))
@@ -120,8 +117,7 @@ class BatchedScan:
             self.tiles = engine.Tiles(self.atoms, beam.k, beam.tile_atoms_for(n_total, "scan"),
                                       device=dev)
         self.phys = beam.physics(apply_polarization, spherical_decay, remove_forward, pol=pol)
-        self.pix = engine.Pixels(np.concatenate(xyz, axis=1), n_total, 1, self.phys, device=dev,
-                                 frames=fr)
+        self.pix = engine.Pixels.of_scan(self.frames, self._bd, self.phys, device=dev)
         self.tune_results = []
         self.out = torch.zeros((n_total, 2), dtype=torch.float64, device=dev)
         self.sums = torch.zeros(len(self.frames), dtype=torch.float64, device=dev)
@@ -129,7 +125,7 @@ class BatchedScan:
         self.terms = float(self.atoms.n) * n_total
         self._ftab_key, self._ftab = None, None
         self.nodes = None
-        if not launch and not beam._kernel_launch and self._plan_nodes():
+        if nodes and not launch and not beam._kernel_launch and self._plan_nodes():
             self.launch_source = "nodes"
             return
         su = self._setup(self.tiles)
@@ -356,18 +352,23 @@ def frames_from_motors(stage, detector, steps, rois=None):
     per-step ROI side (int) or None for the full detector."""
     saved = stage._motor_value.copy()
     out = []
+    full = np.asarray(detector.pixel_coordinates)
+    roi_pixels = {}             # the frames of one ROI share its pixel array (read-only)
     try:
         for i, st in enumerate(steps):
             stage._motor_value[:] = saved
             for name, v in st.items():
                 stage._motor_value[stage.motor_index(name)] = float(v)
             R, t = stage.get_rotation().copy(), stage.get_translation().copy()
-            coords = np.asarray(detector.pixel_coordinates)
+            coords, shape = full, tuple(detector.shape)
             if rois is not None and rois[i] is not None:
-                sel, shape = roi_indices(detector.shape, rois[i])
-                coords = coords[:, sel]
-            else:
-                shape = tuple(detector.shape)
+                side = int(rois[i])
+                if side not in roi_pixels:
+                    sel, shape = roi_indices(detector.shape, side)
+                    coords = full[:, sel]
+                    coords.flags.writeable = False
+                    roi_pixels[side] = (coords, shape)
+                coords, shape = roi_pixels[side]
             out.append(Frame(R, t, coords, shape))
     finally:
         stage._motor_value[:] = saved

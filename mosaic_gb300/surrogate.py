@@ -472,6 +472,7 @@ class SurrogateScan:
         if self._staged is not None:
             return
         self.exact(np.zeros(1, np.int64))
+        self.exact(np.zeros(1, np.int64), direct=True)
         n_nodes, P = len(self.nodes_t) * len(self.nodes_c), self.roi * self.roi
         n_tr = max(n_nodes, 2)
         I = torch.rand((n_tr, P), dtype=torch.float32, device=self.dev) + 0.5
@@ -542,8 +543,10 @@ class SurrogateScan:
         return basis.decode(net, D[:, :r].float().contiguous(), out=out, row_scale=scale,
                             row_map=rows, clamp=True)
 
-    def exact(self, idx, first=256):
-        """Exact intensities (len(idx), roi*roi) of the given frames, in
+    def exact(self, idx, first=256, direct=False):
+        """Exact intensities (len(idx), roi*roi) of the given frames
+        (``direct``: by the sum over every (atom, pixel), the reference that
+        the other frames are checked against, without the node form), in
         batched launches of at most ``batch_frames`` frames (the first of at
         most ``first``). The batches' sums run on a side stream, so that the
         set-up of the next batch (frame geometry on the host, pixel arrays
@@ -572,7 +575,7 @@ class SurrogateScan:
                 frames = frames * 2
             # no tuning inside the timed scan: the cached launch shape or the default
             scan = BatchedScan(self.beam, self.sample, frames, staged=self._staged, tune=False,
-                               **self.kw)
+                               nodes=not direct, **self.kw)
             self._staged = self._staged or scan
             side.wait_stream(cur)
             with torch.cuda.stream(side):
@@ -590,11 +593,15 @@ class SurrogateScan:
         return out
 
     def run(self, verify=0, exact_all=False):
-        """Run the scan. ``exact_all`` also computes every frame exactly (the
-        exact-only scan, timed) and the true error of every predicted frame;
-        otherwise the exact-only time is the exact launch's per-frame time
-        times the frame count, and ``verify`` > 0 computes that many unjudged
-        predicted frames exactly (untimed) to measure their true error."""
+        """Run the scan. ``exact_all`` also computes every frame by the direct
+        sum over (atom, pixel) pairs (the exact-only scan, timed), which the
+        true error of every returned frame is measured against -- a reference
+        that shares neither the surrogate's frames nor the node form they are
+        summed with; otherwise the exact-only time is the exact launch's
+        per-frame time times the frame count, and ``verify`` > 0 computes that
+        many unjudged predicted frames directly (untimed) to measure their
+        true error. Where the node form is admitted an exact scan of every
+        frame (``exact(np.arange(n))``) costs less than the networks' fit."""
         sync = torch.cuda.synchronize
         n = len(self.ij)
         t = {}
@@ -707,7 +714,7 @@ class SurrogateScan:
         if exact_all:
             sync()
             t0 = time.perf_counter()
-            I_all = self.exact(np.arange(n))
+            I_all = self.exact(np.arange(n), direct=True)
             sync()
             ex_s = time.perf_counter() - t0
             res.update(exact_seconds=ex_s, exact_measured=True)
@@ -731,7 +738,7 @@ class SurrogateScan:
             unjudged = np.setdiff1d(np.arange(len(pred_idx)), np.concatenate([judged, fb]))
             pick = rng.choice(unjudged, size=min(int(verify), unjudged.size), replace=False) \
                 if unjudged.size else np.zeros(0, np.int64)
-            I_true = self.exact(pred_idx[pick])
+            I_true = self.exact(pred_idx[pick], direct=True)
             res["verify_err"] = frame_rel_error(
                 frames[torch.as_tensor(pred_idx[pick], device=self.dev)], I_true).cpu().numpy()
         return res

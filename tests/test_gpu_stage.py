@@ -63,3 +63,31 @@ def test_tiles_hold_every_atom_and_stay_compact(cuda, n, box):
     dims = np.array([b for b in box if b > 0], float)
     share = (np.prod(dims) * T / (n / 2)) ** (1 / len(dims)) * 1e-10
     assert np.median(o[:, 3]) <= 1.5 * share
+
+
+@pytest.mark.parametrize("shapes", [[(5, 3)], [(1, 7), (33, 9), (7, 1), (16, 16)]])
+def test_scan_pixels_match_numpy(cuda, shapes):
+    """Frames into the sample frame and their prologue, against NumPy and the
+    single-exposure prologue; the frames of one ROI may share their array."""
+    from mosaic_gb300 import workloads
+    from mosaic_gb300.scan import Frame
+    rng = np.random.default_rng(7)
+    frames, bd = [], []
+    for i, (ny, nz) in enumerate(shapes + shapes[:1]):
+        R = workloads.random_rotations(1, rng)[0].astype(np.float32)
+        t = rng.uniform(-500, 500, 3).astype(np.float32)
+        P = frames[0].pixels if i == len(shapes) else rng.uniform(0.5e10, 1.5e10, (3, ny * nz))
+        frames.append(Frame(R, t, P, (ny, nz)))
+        bd.append(R.astype(np.float64).T @ np.array([1.0, 0, 0]))
+    phys = engine.physics(5.0e10)
+    px = engine.Pixels.of_scan(frames, np.array(bd), phys, device=cuda)
+    for (off, m), f, b in zip(px.spans, frames, bd):
+        R = np.asarray(f.rotation, np.float64)
+        want = (R.T @ (f.pixels - np.asarray(f.translation, np.float64)[:, None]) / 1e10).T
+        got = px.xyz[off:off + m].cpu().numpy()
+        # three products and two sums, in whatever order and contraction
+        assert np.abs(got - want).max() <= 4 * np.finfo(float).eps * np.abs(f.pixels).max() / 1e10 * 3
+        ph = engine.physics(5.0e10, beam_dir=b)
+        one = engine.Pixels(np.ascontiguousarray(got.T), *f.shape, ph, device=cuda)
+        for a, c in ((px.r0, one.r0), (px.q, one.q), (px.u, one.u), (px.phasor, one.phasor)):
+            assert torch.equal(a[off:off + m], c)

@@ -443,6 +443,14 @@ size_t mk_prop_cols_workspace_size(int ny2, int nz2);
 int mk_prop_cols(float *spectrum, int ny2, int nz2, double dy, double dz, double k, double z,
                  double k_axis, double k_perp_y, double k_perp_z, void *workspace, size_t ws_bytes,
                  void *stream);
+/* mk_prop_cols for a field padded along z: `spectrum` holds only the field's
+ * nz rows (nz, ny2), already transformed along y, which lie at rows
+ * [z0, z0 + nz) of the nz2; the other rows repeat the edge rows (mode 0) or are
+ * the constant (cval_re, cval_im) (mode 1). Only the field's rows are written
+ * back. */
+int mk_prop_cols_rows(float *spectrum, int ny2, int nz2, int z0, int nz, int mode, float cval_re,
+                      float cval_im, double dy, double dz, double k, double z, double k_axis,
+                      double k_perp_y, double k_perp_z, void *workspace, size_t ws_bytes, void *stream);
 /* Centre crop (nz, ny) at (z0, y0) of the inverse transform times `scale`,
  * fused with |A|^2: writes field (complex64) and/or intensity (float32). */
 int mk_prop_crop_abs2(const float *grid, int ny2, int nz2, int y0, int z0, int ny, int nz,

@@ -244,6 +244,8 @@ SIGNATURES = {
     "mk_prop_cols": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, ctypes.c_double, ctypes.c_double,
                                     ctypes.c_double, ctypes.c_double, ctypes.c_double, ctypes.c_double,
                                     ctypes.c_double, _vp, ctypes.c_size_t, _vp]),
+    "mk_prop_cols_rows": (ctypes.c_int, [_vp] + [ctypes.c_int] * 5 + [ctypes.c_float] * 2 +
+                          [ctypes.c_double] * 7 + [_vp, ctypes.c_size_t, _vp]),
     "mk_prop_cols_workspace_size": (ctypes.c_size_t, [ctypes.c_int, ctypes.c_int]),
     "mk_prop_crop_abs2": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                          ctypes.c_int, ctypes.c_int, ctypes.c_float, _vp, _vp, _vp]),

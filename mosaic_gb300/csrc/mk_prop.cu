@@ -91,180 +91,254 @@ __global__ void mk_prop_crop_kernel(const float2 *__restrict__ G, int ny2, int n
 // transforms (cuFFT, contiguous rows) the spectrum is read and written once
 // instead of three times (column FFT, multiply, inverse column FFT).
 //
-// A block loads W columns (each row's W neighbours are one contiguous
-// segment of 8 W bytes) into shared memory as W lines of N points in
-// bit-reversed order (stride N + 1, which spreads a row's W points over
-// different banks), transforms every line in place by radix-2
-// decimation-in-time stages fused three at a time (a butterfly keeps its 8
-// points in registers through the three stages and writes them back where
-// it read them), applies H in natural order, bit-reverses the lines and
-// transforms them back the same way, and writes the columns back. Twiddles come from a table of exp(-2 pi i t / N)
-// made in FP64. The transfer function is formed in FP32 as the reference's
-// prop_mul_kernel does (Beam.py:4763-4830), with the two large constant
-// phases, z (k - k_axis) and -z k_axis, reduced mod 2 pi in FP64 on the
-// host.
+// The padded rows need no memory: rows outside the field repeat its edge
+// rows (their transforms too) or are constant (their transform is one bin),
+// and only the field's rows are wanted back, so the kernel reads and writes
+// the field's nz rows and forms the nz2 - nz others as it loads.
+//
+// N = 2^logn points are P passes of radix 8 and a last one of radix 2, 4 or
+// 8, decimation in frequency forward and in time back, so that neither
+// transform is permuted: the forward one ends with frequency k0 + 8 k1 + ..
+// at position k0 N/8 + k1 N/64 + .., where H is applied. A thread holds 8
+// points in registers per item; the first forward pass reads global memory,
+// the last inverse pass writes it, and the radix-2/4/8 passes either side of
+// H stay in registers: 2 P + 2 passes over shared memory of 8 bytes a point.
+// A line's point i is at i + i/8 and lines are LD = 16/W (mod 16) points
+// apart, which keeps the 8-byte accesses of a half warp (W lines x 16/W
+// neighbouring points) on different banks at every stride; in place and
+// unpadded, radix-2 stages fused by threes with a bit-reversal pass between
+// the transforms ran 8-way conflicts and took 299 us for the 2048 x 4096
+// spectrum of a 2048 x 1500 field; this 91 us (98 MB at copy bandwidth: 15).
+// Twiddles come from a table of exp(-2 pi i t / N) made in FP64. The transfer
+// function is formed in FP32 as the reference's prop_mul_kernel does
+// (Beam.py:4763-4830), with the two large constant phases, z (k - k_axis) and
+// -z k_axis, reduced mod 2 pi in FP64 on the host.
 #define MK_FFT_NT 512
 #define MK_FFT_MAX 8192
-#define MK_FFT_PTS 16384          // W x N points a block holds
+#define MK_FFT_SMEM (74 << 10)    // a block's lines where three blocks fit an SM
 
 __device__ __forceinline__ float2 mk_cmul(float2 a, float2 b)
 {
     return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
-
-// Bit reversal of the low `bits` bits of i.
-__device__ __forceinline__ int mk_bitrev(int i, int bits)
-{
-    return (int)(__brev((unsigned)i) >> (32 - bits));
-}
-
-// G consecutive in-place radix-2 decimation-in-time stages (half sizes m,
-// 2m, .., 2^(G-1) m) fused into one pass over W lines of N points in shared
-// memory (line c at s + c * ld; the lines were loaded in bit-reversed
-// order). A butterfly owns the R = 2^G points b + i + r m (b a multiple of
-// R m, i < m), keeps them in registers through the G stages and writes them
-// back where it read them, so the pass works in place. Stage h pairs points
-// a and a + 2^h (bit h of a clear) with the twiddle
-// exp(-/+ 2 pi i j / (2^(h+1) m)), j = i + (a mod 2^h) m.
-template <int G, bool INV>
-__device__ __forceinline__ void mk_dit_pass(float2 *s, int ld, int W, int N, int m,
-                                            const float2 *__restrict__ tw)
-{
-    constexpr int R = 1 << G;
-    const int nb = N / R, total = W * nb;
-    for (int t = threadIdx.x; t < total; t += MK_FFT_NT) {
-        const int c = t / nb, q = t - c * nb;
-        const int i = q & (m - 1);
-        float2 *pts = s + c * ld + (q - i) * R + i;
-        float2 v[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = pts[r * m];
-#pragma unroll
-        for (int h = 0; h < G; ++h) {
-            const int hs = m << h;
-            const int tstep = N / (2 * hs);
-#pragma unroll
-            for (int a = 0; a < R; ++a) {
-                if (a & (1 << h)) continue;
-                const int j = i + (a & ((1 << h) - 1)) * m;
-                float2 w = __ldg(tw + j * tstep);
-                if (INV) w.y = -w.y;
-                const float2 x = v[a], y = mk_cmul(v[a + (1 << h)], w);
-                v[a] = make_float2(x.x + y.x, x.y + y.y);
-                v[a + (1 << h)] = make_float2(x.x - y.x, x.y - y.y);
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < R; ++r) pts[r * m] = v[r];
-    }
-    __syncthreads();
-}
-
-// FFT of W lines of N = 2^logn points loaded in bit-reversed order; the
-// result is in natural order, in place.
+__device__ __forceinline__ float2 mk_cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ float2 mk_csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+// a times -i (forward) or +i (inverse)
 template <bool INV>
-__device__ __forceinline__ void mk_fft_lines(float2 *s, int ld, int W, int N, int logn,
-                                             const float2 *__restrict__ tw)
+__device__ __forceinline__ float2 mk_crot(float2 a)
 {
-    int m = 1, left = logn;
-    for (; left >= 3; left -= 3, m <<= 3) mk_dit_pass<3, INV>(s, ld, W, N, m, tw);
-    if (left == 2) mk_dit_pass<2, INV>(s, ld, W, N, m, tw);
-    else if (left == 1) mk_dit_pass<1, INV>(s, ld, W, N, m, tw);
+    return INV ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
 }
 
-// In-place bit-reversal permutation of W lines (between the forward and the
-// inverse transform, whose input must again be bit-reversed).
-__device__ __forceinline__ void mk_bitrev_lines(float2 *s, int ld, int W, int N, int logn)
+// DFT of R points in registers, natural order in and out.
+template <int R, bool INV>
+__device__ __forceinline__ void mk_dft(float2 *v)
 {
-    for (int e = threadIdx.x; e < W * N; e += MK_FFT_NT) {
-        const int c = e / N, r = e - c * N;
-        const int q = mk_bitrev(r, logn);
-        if (q > r) {
-            float2 *line = s + c * ld;
-            const float2 t = line[r];
-            line[r] = line[q];
-            line[q] = t;
+    if constexpr (R == 2) {
+        const float2 a = v[0], b = v[1];
+        v[0] = mk_cadd(a, b);
+        v[1] = mk_csub(a, b);
+    } else if constexpr (R == 4) {
+        const float2 a = mk_cadd(v[0], v[2]), b = mk_csub(v[0], v[2]);
+        const float2 c = mk_cadd(v[1], v[3]), d = mk_crot<INV>(mk_csub(v[1], v[3]));
+        v[0] = mk_cadd(a, c);
+        v[1] = mk_cadd(b, d);
+        v[2] = mk_csub(a, c);
+        v[3] = mk_csub(b, d);
+    } else {
+        float2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
+        mk_dft<4, INV>(e);
+        mk_dft<4, INV>(o);
+        const float h = 0.70710678118654752f;
+        const float2 r1 = mk_crot<INV>(o[1]), r3 = mk_crot<INV>(o[3]);
+        o[1] = make_float2(h * (o[1].x + r1.x), h * (o[1].y + r1.y));        // times w8
+        o[2] = mk_crot<INV>(o[2]);
+        o[3] = make_float2(h * (r3.x - o[3].x), h * (r3.y - o[3].y));        // times w8^3
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            v[j] = mk_cadd(e[j], o[j]);
+            v[j + 4] = mk_csub(e[j], o[j]);
         }
     }
-    __syncthreads();
 }
 
-// F (nz2, ny2) row-transformed spectrum, in place: every column
-// z-transformed, multiplied by H(ky[col], kz[row]) and inverse
-// z-transformed (unnormalised). W columns a block; ky, kz: FP32 transverse
-// wavenumbers (2 pi fftfreq + carrier offset) of every column and row;
-// c_prop = z (k - k_axis) mod 2 pi, c_evan = -z k_axis mod 2 pi.
-__global__ void __launch_bounds__(MK_FFT_NT)
-    mk_prop_cols_kernel(float2 *__restrict__ F, int ny2, int nz2, int logn, int W,
-                        const float2 *__restrict__ tw, const float *__restrict__ ky,
-                        const float *__restrict__ kz, float k, float z, float c_prop, float c_evan)
+struct MkColsArgs {
+    float2 *F;             // (nz, ny2) rows of the field's spectrum, in place
+    int ny2, nz2, logn, W, ld;
+    int z0, nz, mode;      // field rows at [z0, z0 + nz); 0 repeat the edges, 1 constant
+    float2 cval;           // spectrum of a constant row at column 0
+    const float2 *tw;
+    const float *ky, *kz;
+    float k, z, c_prop, c_evan;
+};
+
+__device__ __forceinline__ int mk_pad8(int i) { return i + (i >> 3); }
+
+// Row r of column col of the padded, row-transformed field.
+__device__ __forceinline__ float2 mk_cols_load(const MkColsArgs &A, int r, int col)
+{
+    const int s = r - A.z0;
+    if (A.mode == 1 && (unsigned)s >= (unsigned)A.nz)
+        return col == 0 ? A.cval : make_float2(0.f, 0.f);
+    return A.F[(size_t)min(max(s, 0), A.nz - 1) * A.ny2 + col];
+}
+
+// H(ky, kz) times v.
+__device__ __forceinline__ float2 mk_cols_mul(const MkColsArgs &A, float2 v, float a, float b)
+{
+    const float kt2 = fmaf(a, a, b * b);
+    const float kt = sqrtf(kt2);
+    float ph, amp;
+    if (kt <= A.k) {
+        // sqrt(k^2 - kt^2) - k = -kt^2 / (sqrt(k^2 - kt^2) + k)
+        ph = -A.z * kt2 / (sqrtf((A.k - kt) * (A.k + kt)) + A.k) + A.c_prop;
+        amp = 1.f;
+    } else {
+        amp = expf(-fabsf(A.z) * sqrtf((kt - A.k) * (kt + A.k)));
+        ph = A.c_evan;
+    }
+    float sn, cs;
+    sincosf(ph, &sn, &cs);
+    return mk_cmul(v, make_float2(amp * cs, amp * sn));
+}
+
+// LAST: bits of the last radix (1, 2 or 3). Block = W neighbouring columns.
+template <int LAST>
+__global__ void __launch_bounds__(MK_FFT_NT, 2) mk_prop_cols_kernel(const __grid_constant__ MkColsArgs A)
 {
     extern __shared__ __align__(16) float2 s_lines[];
-    const int ld = nz2 + 1;
-    const int groups = ny2 / W, pts = W * nz2;
-    for (int g = blockIdx.x; g < groups; g += gridDim.x) {
-        const int c0 = g * W;
-        for (int e = threadIdx.x; e < pts; e += MK_FFT_NT) {
-            const int r = e / W, c = e - r * W;
-            s_lines[c * ld + mk_bitrev(r, logn)] = F[(size_t)r * ny2 + c0 + c];
-        }
-        __syncthreads();
-        mk_fft_lines<false>(s_lines, ld, W, nz2, logn, tw);
-        for (int e = threadIdx.x; e < pts; e += MK_FFT_NT) {
-            const int c = e / nz2, r = e - c * nz2;
-            const float a = ky[c0 + c], b = kz[r];
-            const float kt2 = fmaf(a, a, b * b);
-            const float kt = sqrtf(kt2);
-            float ph, amp;
-            if (kt <= k) {
-                // sqrt(k^2 - kt^2) - k = -kt^2 / (sqrt(k^2 - kt^2) + k)
-                ph = -z * kt2 / (sqrtf((k - kt) * (k + kt)) + k) + c_prop;
-                amp = 1.f;
-            } else {
-                amp = expf(-fabsf(z) * sqrtf((kt - k) * (kt + k)));
-                ph = c_evan;
-            }
-            float sn, cs;
-            sincosf(ph, &sn, &cs);
-            float2 *p = s_lines + c * ld + r;
-            *p = mk_cmul(*p, make_float2(amp * cs, amp * sn));
-        }
-        __syncthreads();
-        mk_bitrev_lines(s_lines, ld, W, nz2, logn);
-        mk_fft_lines<true>(s_lines, ld, W, nz2, logn, tw);
-        for (int e = threadIdx.x; e < pts; e += MK_FFT_NT) {
-            const int r = e / W, c = e - r * W;
-            F[(size_t)r * ny2 + c0 + c] = s_lines[c * ld + r];
+    constexpr int RL = 1 << LAST;
+    const int N = A.nz2, W = A.W, P = (A.logn - LAST) / 3;
+    const int logw = 31 - __clz(W), items = W * (N >> 3);
+    const int c0 = blockIdx.x * W;
+    // forward passes
+    for (int p = 0; p < P; ++p) {
+        const int logm = A.logn - 3 * (p + 1), m = 1 << logm;
+        for (int t = threadIdx.x; t < items; t += MK_FFT_NT) {
+            const int c = t & (W - 1), q = t >> logw;
+            const int i = q & (m - 1), base = ((q >> logm) << (logm + 3)) + i;
+            float2 *line = s_lines + c * A.ld;
+            float2 v[8];
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+                v[r] = p == 0 ? mk_cols_load(A, base + (r << logm), c0 + c) : line[mk_pad8(base + (r << logm))];
+            mk_dft<8, false>(v);
+            line[mk_pad8(base)] = v[0];
+#pragma unroll
+            for (int k = 1; k < 8; ++k)
+                line[mk_pad8(base + (k << logm))] = mk_cmul(v[k], __ldg(A.tw + ((i * k) << (3 * p))));
         }
         __syncthreads();
     }
+    // last radix, H, and back: 8 consecutive positions a thread
+    for (int t = threadIdx.x; t < items; t += MK_FFT_NT) {
+        const int c = t & (W - 1), q = t >> logw;
+        float2 *line = s_lines + c * A.ld + 9 * q;             // mk_pad8(8 q)
+        const float a = A.ky[c0 + c];
+        float2 v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = line[j];
+#pragma unroll
+        for (int g = 0; g < 8 / RL; ++g) {
+            mk_dft<RL, false>(v + g * RL);
+            // the frequency of position 8 q + g RL + k: its digits reversed
+            const int pos = 8 * q + g * RL;
+            int f = 0;
+            for (int p = 0; p < P; ++p) f |= ((pos >> (A.logn - 3 * (p + 1))) & 7) << (3 * p);
+#pragma unroll
+            for (int k = 0; k < RL; ++k)
+                v[g * RL + k] = mk_cols_mul(A, v[g * RL + k], a, A.kz[f + (k << (3 * P))]);
+            mk_dft<RL, true>(v + g * RL);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) line[j] = v[j];
+    }
+    __syncthreads();
+    // inverse passes
+    for (int p = P - 1; p >= 0; --p) {
+        const int logm = A.logn - 3 * (p + 1), m = 1 << logm;
+        for (int t = threadIdx.x; t < items; t += MK_FFT_NT) {
+            const int c = t & (W - 1), q = t >> logw;
+            const int i = q & (m - 1), base = ((q >> logm) << (logm + 3)) + i;
+            float2 *line = s_lines + c * A.ld;
+            float2 v[8];
+            v[0] = line[mk_pad8(base)];
+#pragma unroll
+            for (int k = 1; k < 8; ++k) {
+                float2 w = __ldg(A.tw + ((i * k) << (3 * p)));
+                w.y = -w.y;
+                v[k] = mk_cmul(line[mk_pad8(base + (k << logm))], w);
+            }
+            mk_dft<8, true>(v);
+            if (p > 0) {
+#pragma unroll
+                for (int r = 0; r < 8; ++r) line[mk_pad8(base + (r << logm))] = v[r];
+            } else {
+#pragma unroll
+                for (int r = 0; r < 8; ++r) {
+                    const int s = base + (r << logm) - A.z0;
+                    if ((unsigned)s < (unsigned)A.nz) A.F[(size_t)s * A.ny2 + c0 + c] = v[r];
+                }
+            }
+        }
+        if (p > 0) __syncthreads();
+    }
 }
 
-// exp(-2 pi i t / n), t < n, from FP64 sincospi.
-__global__ void mk_prop_twiddle_kernel(float2 *__restrict__ tw, int n)
+// Column lengths 2, 4 and 8: a thread a column, in registers.
+template <int N>
+__global__ void mk_prop_cols_short_kernel(const __grid_constant__ MkColsArgs A)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    double s, c;
-    sincospi(-2.0 * (double)t / (double)n, &s, &c);
-    tw[t] = make_float2((float)c, (float)s);
+    const int col = blockIdx.x * blockDim.x + threadIdx.x;
+    if (col >= A.ny2) return;
+    float2 v[N];
+#pragma unroll
+    for (int r = 0; r < N; ++r) v[r] = mk_cols_load(A, r, col);
+    mk_dft<N, false>(v);
+#pragma unroll
+    for (int r = 0; r < N; ++r) v[r] = mk_cols_mul(A, v[r], A.ky[col], A.kz[r]);
+    mk_dft<N, true>(v);
+#pragma unroll
+    for (int r = 0; r < N; ++r) {
+        const int s = r - A.z0;
+        if ((unsigned)s < (unsigned)A.nz) A.F[(size_t)s * A.ny2 + col] = v[r];
+    }
 }
 
-// 2 pi fftfreq(n, d) + off as float32 (numpy ordering), in FP64.
-__global__ void mk_prop_freq_kernel(float *__restrict__ out, int n, double d, double off)
+// The tables of a column pass: twiddles exp(-2 pi i t / nz2) from FP64
+// sincospi, and 2 pi fftfreq + offset of every column and row as float32
+// (numpy ordering, in FP64).
+__global__ void mk_prop_tables_kernel(float2 *__restrict__ tw, float *__restrict__ ky, float *__restrict__ kz,
+                                      int ny2, int nz2, double dy, double dz, double offy, double offz)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    out[i] = (float)(MK_TWO_PI * mk_fftfreq(i, n, d) + off);
+    if (i < nz2) {
+        double s, c;
+        sincospi(-2.0 * (double)i / (double)nz2, &s, &c);
+        tw[i] = make_float2((float)c, (float)s);
+        kz[i] = (float)(MK_TWO_PI * mk_fftfreq(i, nz2, dz) + offz);
+    }
+    if (i < ny2) ky[i] = (float)(MK_TWO_PI * mk_fftfreq(i, ny2, dy) + offy);
 }
 
-// Columns a block: W x nz2 <= MK_FFT_PTS, at most 16 and the row length.
+// Points between a line's start and the next: its padded length, rounded up to
+// 16 / W (mod 16) points.
+static int mk_prop_ld(int nz2, int W)
+{
+    int ld = nz2 + nz2 / 8;
+    while (ld % 16 != (16 / W) % 16) ++ld;
+    return ld;
+}
+
+// Columns a block: as many as three blocks an SM leave room for, at least 4
+// (whole 32-byte sectors) where one block can hold them, at most 16 and the
+// row length.
 static int mk_prop_cols_width(int ny2, int nz2)
 {
-    int W = MK_FFT_PTS / nz2;
-    W = std::min(W, 16);
-    W = std::min(W, ny2);
-    return std::max(W, 1);
+    int W = 16;
+    while (W > 4 && sizeof(float2) * (size_t)W * mk_prop_ld(nz2, W) > MK_FFT_SMEM) W /= 2;
+    while (W > 1 && sizeof(float2) * (size_t)W * mk_prop_ld(nz2, W) > (227u << 10)) W /= 2;
+    return std::max(1, std::min(W, ny2));
 }
 
 extern "C" size_t mk_prop_cols_workspace_size(int ny2, int nz2)
@@ -273,9 +347,10 @@ extern "C" size_t mk_prop_cols_workspace_size(int ny2, int nz2)
     return sizeof(float2) * (size_t)nz2 + sizeof(float) * ((size_t)ny2 + (size_t)nz2) + 256;
 }
 
-extern "C" int mk_prop_cols(float *spectrum, int ny2, int nz2, double dy, double dz, double k,
-                            double z, double k_axis, double k_perp_y, double k_perp_z,
-                            void *workspace, size_t ws_bytes, void *stream)
+extern "C" int mk_prop_cols_rows(float *spectrum, int ny2, int nz2, int z0, int nz, int mode,
+                                 float cval_re, float cval_im, double dy, double dz, double k,
+                                 double z, double k_axis, double k_perp_y, double k_perp_z,
+                                 void *workspace, size_t ws_bytes, void *stream)
 {
     MK_REQUIRE(spectrum && ny2 > 0 && nz2 > 0 && dy > 0.0 && dz > 0.0 && k > 0.0,
                "mk_prop_cols: bad arguments");
@@ -284,6 +359,8 @@ extern "C" int mk_prop_cols(float *spectrum, int ny2, int nz2, double dy, double
                MK_FFT_MAX);
     MK_REQUIRE((ny2 & (ny2 - 1)) == 0, "mk_prop_cols: the row length %d must be a power of two",
                ny2);
+    MK_REQUIRE(nz > 0 && z0 >= 0 && z0 + nz <= nz2 && (mode == 0 || mode == 1),
+               "mk_prop_cols: %d rows at %d do not fit %d", nz, z0, nz2);
     const size_t need = mk_prop_cols_workspace_size(ny2, nz2);
     if (!workspace || ws_bytes < need) {
         mk_set_error("mk_prop_cols: workspace %zu bytes, need %zu", ws_bytes, need);
@@ -292,34 +369,54 @@ extern "C" int mk_prop_cols(float *spectrum, int ny2, int nz2, double dy, double
     MK_REQUIRE(((uintptr_t)workspace & 15) == 0, "mk_prop_cols: workspace must be 16-byte aligned");
     int logn = 0;
     while ((1 << logn) < nz2) ++logn;
-    const int W = mk_prop_cols_width(ny2, nz2);
     cudaStream_t st = mk_stream(stream);
     float2 *tw = reinterpret_cast<float2 *>(workspace);
     float *ky = reinterpret_cast<float *>(tw + nz2);
     float *kz = ky + ny2;
-    mk_prop_twiddle_kernel<<<(nz2 + 255) / 256, 256, 0, st>>>(tw, nz2);
+    mk_prop_tables_kernel<<<(std::max(ny2, nz2) + 255) / 256, 256, 0, st>>>(tw, ky, kz, ny2, nz2, dy, dz,
+                                                                           k_perp_y, k_perp_z);
     MK_CHECK_CUDA(cudaGetLastError());
-    mk_prop_freq_kernel<<<(ny2 + 255) / 256, 256, 0, st>>>(ky, ny2, dy, k_perp_y);
-    MK_CHECK_CUDA(cudaGetLastError());
-    mk_prop_freq_kernel<<<(nz2 + 255) / 256, 256, 0, st>>>(kz, nz2, dz, k_perp_z);
-    MK_CHECK_CUDA(cudaGetLastError());
-    const double c_prop = fmod(z * (k - k_axis), MK_TWO_PI);
-    const double c_evan = fmod(-z * k_axis, MK_TWO_PI);
-    const size_t smem = sizeof(float2) * (size_t)W * (size_t)(nz2 + 1);
-    MK_CHECK_CUDA(cudaFuncSetAttribute((const void *)mk_prop_cols_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int dev = 0, sms = 0, bps = 0;
-    MK_CHECK_CUDA(cudaGetDevice(&dev));
-    MK_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    MK_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, (const void *)mk_prop_cols_kernel,
-                                                                MK_FFT_NT, smem));
-    MK_REQUIRE(bps >= 1, "mk_prop_cols: %d columns of %d points do not fit on an SM", W, nz2);
-    const int grid = std::min(ny2 / W, sms * bps);
-    mk_prop_cols_kernel<<<grid, MK_FFT_NT, smem, st>>>(reinterpret_cast<float2 *>(spectrum), ny2, nz2,
-                                                      logn, W, tw, ky, kz, (float)k, (float)z,
-                                                      (float)c_prop, (float)c_evan);
+    MkColsArgs A;
+    memset(&A, 0, sizeof(A));
+    A.F = reinterpret_cast<float2 *>(spectrum);
+    A.ny2 = ny2;
+    A.nz2 = nz2;
+    A.logn = logn;
+    A.z0 = z0;
+    A.nz = nz;
+    A.mode = mode;
+    A.cval = make_float2(cval_re * (float)ny2, cval_im * (float)ny2);
+    A.tw = tw;
+    A.ky = ky;
+    A.kz = kz;
+    A.k = (float)k;
+    A.z = (float)z;
+    A.c_prop = (float)fmod(z * (k - k_axis), MK_TWO_PI);
+    A.c_evan = (float)fmod(-z * k_axis, MK_TWO_PI);
+    if (logn <= 3) {
+        auto fn = logn == 1 ? mk_prop_cols_short_kernel<2>
+                            : (logn == 2 ? mk_prop_cols_short_kernel<4> : mk_prop_cols_short_kernel<8>);
+        fn<<<(ny2 + 127) / 128, 128, 0, st>>>(A);
+        MK_CHECK_CUDA(cudaGetLastError());
+        return MK_OK;
+    }
+    A.W = mk_prop_cols_width(ny2, nz2);
+    A.ld = mk_prop_ld(nz2, A.W);
+    const size_t smem = sizeof(float2) * (size_t)A.W * (size_t)A.ld;
+    const int last = logn % 3 == 0 ? 3 : logn % 3;
+    auto fn = last == 1 ? mk_prop_cols_kernel<1> : (last == 2 ? mk_prop_cols_kernel<2> : mk_prop_cols_kernel<3>);
+    MK_CHECK_CUDA(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    fn<<<ny2 / A.W, MK_FFT_NT, smem, st>>>(A);
     MK_CHECK_CUDA(cudaGetLastError());
     return MK_OK;
+}
+
+extern "C" int mk_prop_cols(float *spectrum, int ny2, int nz2, double dy, double dz, double k,
+                            double z, double k_axis, double k_perp_y, double k_perp_z,
+                            void *workspace, size_t ws_bytes, void *stream)
+{
+    return mk_prop_cols_rows(spectrum, ny2, nz2, 0, nz2, 0, 0.f, 0.f, dy, dz, k, z, k_axis, k_perp_y,
+                             k_perp_z, workspace, ws_bytes, stream);
 }
 
 extern "C" int mk_prop_pad(const float *field, int ny, int nz, float *padded, int ny2, int nz2,

@@ -101,17 +101,20 @@ def propagate(field, dy, dz, z, wavelength, step_max=None, pad_factor=1.0, paddi
         Ny2, Nz2 = choose_optimal_pad(Ny, Nz, dy, dz, wavelength, dz_step,
                                       min_pad_factor=max(1.0, float(pad_factor)))
         y0, z0 = (Ny2 - Ny) // 2, (Nz2 - Nz) // 2
-        P = torch.empty((Nz2, Ny2), dtype=torch.complex64, device=E.device)
         mode = 1 if str(padding_mode or "edge").lower() == "constant" else 0
         c = complex(pad_constant)
-        check(L.mk_prop_pad(E.data_ptr(), Ny, Nz, P.data_ptr(), Ny2, Nz2, y0, z0, mode,
+        # fused: only the field's rows exist; the column pass forms the others
+        rows, r0 = (Nz, 0) if fused else (Nz2, z0)
+        P = torch.empty((rows, Ny2), dtype=torch.complex64, device=E.device)
+        check(L.mk_prop_pad(E.data_ptr(), Ny, Nz, P.data_ptr(), Ny2, rows, y0, r0, mode,
                             c.real, c.imag, sh))
         if fused:
             F = torch.fft.fft(P, dim=-1).contiguous()   # rows (y); already contiguous
             ws_n = int(L.mk_prop_cols_workspace_size(Ny2, Nz2))
             ws = torch.empty(ws_n, dtype=torch.uint8, device=E.device)
-            check(L.mk_prop_cols(F.data_ptr(), Ny2, Nz2, float(dy), float(dz), k, dz_step, kga,
-                                 float(k_perp_y), float(k_perp_z), ws.data_ptr(), ws_n, sh))
+            check(L.mk_prop_cols_rows(F.data_ptr(), Ny2, Nz2, z0, Nz, mode, c.real, c.imag, float(dy),
+                                      float(dz), k, dz_step, kga, float(k_perp_y), float(k_perp_z),
+                                      ws.data_ptr(), ws_n, sh))
             G = torch.fft.ifft(F, dim=-1, norm="forward")   # unnormalised; 1/N in the crop
         else:
             F = torch.fft.fft2(P)
@@ -121,7 +124,7 @@ def propagate(field, dy, dz, z, wavelength, step_max=None, pad_factor=1.0, paddi
         out = torch.empty((Nz, Ny), dtype=torch.complex64, device=E.device)
         if intensity and last:
             I = torch.empty((Nz, Ny), dtype=torch.float32, device=E.device)
-        check(L.mk_prop_crop_abs2(G.data_ptr(), Ny2, Nz2, y0, z0, Ny, Nz,
+        check(L.mk_prop_crop_abs2(G.data_ptr(), Ny2, rows, y0, r0, Ny, Nz,
                                   1.0 / float(Ny2 * Nz2), out.data_ptr(),
                                   I.data_ptr() if I is not None else None, sh))
         E = out

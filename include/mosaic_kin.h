@@ -413,6 +413,15 @@ int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, const mk_pix
                      int fresnel, double fresnel_radius_m, double *out, double *intensity_sums,
                      int accumulate, void *workspace, size_t ws_bytes, void *stream);
 
+/* A top-hat analyser (phys->analyser 1) in the factor table: factor_out
+ * (n_species, n_pix, 2) takes px->factor where every direction within
+ * `excursion` [rad] of the pixel's own is accepted and 0 elsewhere; pixels the
+ * acceptance edge may cut are 0 too and listed in edge (device, 1 + edge_cap
+ * ints: how many there are, then the first edge_cap of them, in any order),
+ * for mk_kin_plain_f64 to sum. */
+int mk_analyser_mask(const mk_pixels *px, const mk_physics *phys, double excursion, int n_species,
+                     float *factor_out, int *edge, int edge_cap, void *stream);
+
 /* --- free-space propagation ------------------------------------------- */
 /* Replaces the pad / prop_mul_kernel / crop steps of
  * _angular_spectrum_propagate_gpu (Beam.py:7829-7943, 4747-4834); the FFTs

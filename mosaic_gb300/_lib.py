@@ -163,6 +163,8 @@ class MkNodePlan(ctypes.Structure):
 
 # name -> (restype, argtypes)
 SIGNATURES = {
+    "mk_analyser_mask": (ctypes.c_int, [ctypes.POINTER(MkPixels), ctypes.POINTER(MkPhysics),
+                                        ctypes.c_double, ctypes.c_int, _vp, _vp, ctypes.c_int, _vp]),
     "mk_scan_pixels": (ctypes.c_int, [ctypes.c_int, _vp, ctypes.c_int, _vp, ctypes.c_double, _vp,
                                       ctypes.POINTER(MkPixels), _vp]),
     "mk_species_index": (ctypes.c_int, [ctypes.c_int64, _vp, _vp, ctypes.c_int, ctypes.c_int, _vp, _vp,

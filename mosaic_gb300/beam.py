@@ -492,9 +492,10 @@ class beam:
         return su, tuned_launch(pix.n, su.level, tiles.tile_atoms), src, diag
 
     def _scatter_nodes(self, atoms, pix, phys, out, accumulate):
-        """The node form of the FP32 sum (detectors on a plane grid, no
-        analyser, no remove_forward), its wide tiles through the split kernel;
-        None where its plan declines."""
+        """The node form of the FP32 sum (detectors on a plane grid, no Darwin
+        analyser, no remove_forward), its wide tiles through the split kernel
+        and the pixels a top-hat's edge cuts through the FP64 sum; None where
+        its plan declines."""
         tiles = engine.Tiles(atoms, self.k, int(self._kernel_tile_atoms or engine.DEFAULT_TILE_ATOMS),
                              device=atoms.pos.device)
         tol = min(float(self._kernel_phase_tol_rad), float(self._phase_tol_rad))
@@ -502,7 +503,15 @@ class beam:
         if plan is None:
             return None
         cfg = engine.default_launch(4 if pix.squares_fit() else 2, tiles.tile_atoms)
-        info = {}
+        info, factor, edge, full = {}, True, None, phys
+        if phys.analyser:
+            masked = engine.analyser_mask(tiles, pix, phys, atoms.table)
+            if masked is None:
+                return None
+            factor, edge = masked
+            phys = type(full).from_buffer_copy(full)
+            phys.analyser = 0
+            info["edge_pixels"] = int(edge.numel())
         if plan.wide is not None:
             su, diag = self.split_setup(plan.wide, pix, phys)
             if su is None:
@@ -511,12 +520,16 @@ class beam:
                                          plan.wide, pix, self.k, su.info)
             out = engine.run_split(plan.wide, pix, phys, atoms.table, launch=cfg, fresnel=su.fresnel,
                                    out=out, accumulate=accumulate, fresnel_radius=su.fresnel_radius,
-                                   factor_table=True)
+                                   factor_table=factor)
             accumulate = True
-            info = dict(su.info)
+            info.update(su.info)
         _, fresnel, _, diag = self.split_budget(tiles, pix.r0_min())
         res = engine.run_nodes(plan, tiles, pix, phys, atoms.table, out=out, accumulate=accumulate,
-                               fresnel=int(fresnel), fresnel_radius=diag["fresnel_radius_m"])
+                               fresnel=int(fresnel), fresnel_radius=diag["fresnel_radius_m"],
+                               factor=None if factor is True else factor)
+        if edge is not None and edge.numel():
+            sub = engine.Pixels(pix.xyz[edge].t(), int(edge.numel()), 1, full, device=pix.xyz.device)
+            res[edge] += engine.run_plain(atoms, sub, full)
         self.last_run = dict(path="split_f32", n_tiles=tiles.n_tiles, tile_atoms=tiles.tile_atoms,
                              fresnel=bool(fresnel), factor_table=True, launch=dict(cfg),
                              launch_source="nodes", **plan.info(), **info, **diag)
@@ -524,7 +537,7 @@ class beam:
 
     def _scatter_once(self, atoms, pix, phys, out=None, accumulate=False, launch=None):
         if self._use_fast_kernel and self._use_nodes and not (launch or self._kernel_launch) and \
-                not phys.analyser and not phys.remove_forward and \
+                phys.analyser != 2 and not phys.remove_forward and \
                 float(atoms.n) * pix.n >= engine.NODES_MIN_TERMS:
             res = self._scatter_nodes(atoms, pix, phys, out, accumulate)
             if res is not None:

@@ -1177,6 +1177,56 @@ __global__ void mk_node_sums_final_kernel(int n_frames, const double *__restrict
     sums[f] = acc;
 }
 
+// ------------------------------------------------------- top-hat analyser
+// Every atom's direction to a pixel is within `exc` of the pixel's own, so x =
+// |u' - c|^2 is within 2 sqrt(x) exc + exc^2 of the pixel's: a pixel whose own
+// x is farther than that from the acceptance edge takes one factor, 0 or 1,
+// for every atom, which its factor-table entries carry; the others (the edge
+// passes them within 1e-7 rad: a pixel or two of a detector) are zeroed and
+// listed for the FP64 sum. FP64, one pass: 24 B read, 16 B a species.
+__global__ void __launch_bounds__(256) mk_analyser_mask_kernel(long long n, const double *__restrict__ xyz,
+                                                               double cx, double cy, double cz, double x_acc,
+                                                               double exc, int n_species,
+                                                               const float2 *__restrict__ in,
+                                                               float2 *__restrict__ out,
+                                                               int *__restrict__ edge, int cap)
+{
+    const long long p = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (p >= n) return;
+    const double x0 = xyz[3 * p], y0 = xyz[3 * p + 1], z0 = xyz[3 * p + 2];
+    const double inv = 1.0 / sqrt(x0 * x0 + y0 * y0 + z0 * z0);
+    const double vx = x0 * inv - cx, vy = y0 * inv - cy, vz = z0 * inv - cz;
+    const double x = vx * vx + vy * vy + vz * vz, m = 2.0 * sqrt(x) * exc + exc * exc + 1e-15;
+    const bool inside = x + m <= x_acc, outside = x - m > x_acc;
+    for (int s = 0; s < n_species; ++s)
+        out[s * n + p] = inside ? in[s * n + p] : make_float2(0.f, 0.f);
+    if (!inside && !outside) {          // NaN too
+        const int i = atomicAdd(edge, 1);
+        if (i < cap) edge[1 + i] = (int)p;
+    }
+}
+
+extern "C" int mk_analyser_mask(const mk_pixels *px, const mk_physics *phys, double excursion, int n_species,
+                                float *factor_out, int *edge, int edge_cap, void *stream)
+{
+    MK_REQUIRE(px && phys && px->xyz && px->factor && factor_out && edge && edge_cap >= 0 && n_species >= 1 &&
+                   excursion >= 0.0,
+               "mk_analyser_mask: bad arguments");
+    MK_REQUIRE(phys->analyser == 1, "mk_analyser_mask: a top-hat analyser is needed");
+    int kind;
+    double ax, ay, az, xacc, hw;
+    const int rc = mk_analyser_pack(phys, &kind, &ax, &ay, &az, &xacc, &hw);
+    if (rc != MK_OK) return rc;
+    const long long n = (long long)px->ny * px->nz;
+    cudaStream_t st = mk_stream(stream);
+    MK_CHECK_CUDA(cudaMemsetAsync(edge, 0, sizeof(int), st));
+    mk_analyser_mask_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
+        n, px->xyz, ax, ay, az, xacc, excursion, n_species, reinterpret_cast<const float2 *>(px->factor),
+        reinterpret_cast<float2 *>(factor_out), edge, edge_cap);
+    MK_CHECK_CUDA(cudaGetLastError());
+    return MK_OK;
+}
+
 template <int N>
 static void mk_launch_pixels(const MkNodeArgs &A, dim3 grid, cudaStream_t st)
 {
@@ -1206,7 +1256,8 @@ extern "C" int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, c
                    ((uintptr_t)workspace & 255) == 0 && ((uintptr_t)dev_buf & 15) == 0,
                "mk_kin_nodes_f32: misaligned buffer");
     MK_REQUIRE(!phys->analyser && !phys->remove_forward && phys->k > 0.0,
-               "mk_kin_nodes_f32: no analyser and no remove_forward here");
+               "mk_kin_nodes_f32: no analyser (a top-hat comes in the factor table, mk_analyser_mask) and "
+               "no remove_forward here");
     MK_REQUIRE(plan->n_src >= 1 && plan->n_frames >= 1 && (long long)px->ny * px->nz >= plan->n_pix,
                "mk_kin_nodes_f32: empty plan or too few pixels");
     if (!workspace || ws_bytes < (size_t)plan->ws_bytes) {

@@ -893,7 +893,7 @@ def run_split(tiles: Tiles, pix: Pixels, phys, table: SpeciesTable, launch=None,
     """FP32 split-phase sum; returns float64 (P, 2) (a view of `out` if given).
     ``factor_table`` None: the per-(species, pixel) factor table where
     ``factor_table_ok`` admits it (else the factor per tile and pixel);
-    False: never; True: always.
+    False: never; True: always; a tensor: that table.
     With ``fresnel`` set, only tiles wider than ``fresnel_radius`` [m] keep the
     |d|^2 term (0: all tiles). ``launch["pairs"]`` = 1 shares one sin/cos
     between pixels 2j and 2j+1; only legal where ``pairs_allowed`` holds;
@@ -921,10 +921,11 @@ def run_split(tiles: Tiles, pix: Pixels, phys, table: SpeciesTable, launch=None,
     if out is None:
         out = torch.zeros((pix.n, 2), dtype=torch.float64, device=pix.xyz.device)
     sp = table.abi()
-    use_tab = factor_table_ok(tiles, pix, phys) if factor_table is None else bool(factor_table)
+    given = isinstance(factor_table, torch.Tensor)
+    use_tab = given or (factor_table_ok(tiles, pix, phys) if factor_table is None else bool(factor_table))
     pabi, ftab = pix.abi, None
     if use_tab:
-        ftab = pix.factor_table(table, phys, stream)
+        ftab = factor_table if given else pix.factor_table(table, phys, stream)
         pabi = MkPixels.from_buffer_copy(pix.abi)
         pabi.factor = ftab.data_ptr()
     check(L.mk_kin_split_f32(ctypes.byref(tiles.abi), ctypes.byref(sp), ctypes.byref(phys),
@@ -982,6 +983,30 @@ class NodePlan:
         p = self.plan
         return dict(form="nodes", nodes=(p.n0, p.n1), groups=p.n_groups, single_tiles=p.n_mid,
                     wide_tiles=p.n_wide, group_radius_m=p.radius2_m)
+
+
+EDGE_PIXELS = 1024      # pixels the acceptance edge may cut that the FP64 sum takes
+
+
+def analyser_mask(tiles, pix, phys, table, stream=None):
+    """(factor table with a top-hat analyser's 0 or 1 in it, int64 indices of
+    the pixels the acceptance edge cuts for some atom, zeroed in the table) by
+    ``mk_analyser_mask``; None when there are more than EDGE_PIXELS of them.
+    Directions from the tiles' atoms differ from the pixel's own by at most
+    (|o| + r) / R0 (here with 1 % to spare)."""
+    L = _require_cuda()
+    exc = 1.01 * (tiles.max_origin_norm() + tiles.max_radius()) / max(pix.r0_min(), 1e-300)
+    factor = pix.factor_table(table, phys, stream)
+    out = torch.empty_like(factor)
+    edge = torch.empty(1 + EDGE_PIXELS, dtype=torch.int32, device=factor.device)
+    abi = MkPixels.from_buffer_copy(pix.abi)
+    abi.factor = factor.data_ptr()
+    check(L.mk_analyser_mask(ctypes.byref(abi), ctypes.byref(phys), exc, int(factor.shape[0]), _ptr(out),
+                             _ptr(edge), EDGE_PIXELS, _stream_handle(stream)))
+    n = int(edge[0])
+    if n > EDGE_PIXELS:
+        return None
+    return out, edge[1:1 + n].long()
 
 
 def run_nodes(np_, tiles, pix, phys, table, out=None, accumulate=False, fresnel=0, fresnel_radius=0.0,

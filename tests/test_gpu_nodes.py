@@ -81,8 +81,8 @@ def test_nodes_match_fp64_and_split(cuda, shape, tile, group, dist, decay, cplx)
 
 def test_entry_point_takes_nodes_where_admitted(cuda):
     """Large enough on a plane detector: nodes; a curved (shell) detector,
-    an explicit launch, remove_forward and an analyser: the other forms, with
-    the same field where the physics is the same."""
+    an explicit launch, remove_forward and a Darwin analyser: the other forms,
+    with the same field where the physics is the same."""
     w, sample = _case(16)
     B = workloads._beam(10000.0, 200.0, pol_perp_rate=1.0)
     st = StaticStage(w.stage.rotation, w.stage.translation)
@@ -95,7 +95,7 @@ def test_entry_point_takes_nodes_where_admitted(cuda):
     assert B.last_run["launch_source"] == "beam"
     assert rel_max(a, b) <= 2e-5, rel_max(a, b)
     B._kernel_launch = None
-    for extra in (dict(remove_forward=True), dict(analyser_mode="top-hat", analyser_acceptance_angle_rad=1e-3)):
+    for extra in (dict(remove_forward=True), dict(analyser_mode="darwin", analyser_darwin_halfwidth_rad=1e-3)):
         B.atomic_scattering_kinematic(sample, D, st, **kw, **extra)
         assert B.last_run["launch_source"] != "nodes", extra
     # 2 mm pixels: the sphere is 8 mm off its chord plane at the corners
@@ -132,3 +132,35 @@ def test_scan_nodes_match_single_fp64_exposures(cuda):
     scan.replay()
     torch.cuda.synchronize()
     assert torch.equal(scan.out, first) and torch.equal(scan.sums, s1)
+
+
+@pytest.mark.parametrize("acceptance", [0.0, 1.1e-3, "edge", 1.0])
+def test_top_hat_nodes_match_fp64(cuda, acceptance):
+    """A top-hat analyser in the factor table: nothing, some and everything
+    accepted, and an edge through one pixel's atoms (that pixel goes to the
+    FP64 sum), against the FP64 sum of every (atom, pixel)."""
+    w, sample = _case(16)
+    B = workloads._beam(10000.0, 200.0, pol_perp_rate=1.0)
+    st = StaticStage(w.stage.rotation, w.stage.translation)
+    shape = (120, 90)
+    D = _det(w, shape)
+    xyz = np.asarray(D.pixel_coordinates, np.float64) / 1e10
+    c = (np.asarray(D.pixel_coordinates)[:, 45 * 120 + 60].astype(np.float32) / np.float32(1e10)).astype(np.float64)
+    c /= np.linalg.norm(c)
+    if acceptance == "edge":
+        u = xyz[:, 30 * 120 + 17] / np.linalg.norm(xyz[:, 30 * 120 + 17])
+        acceptance = 2.0 * np.arcsin(0.5 * np.linalg.norm(u - c))
+    kw = dict(apply_polarization=True, spherical_decay=True, return_double=True, analyser_mode="top-hat",
+              analyser_acceptance_angle_rad=acceptance)
+    got = B.atomic_scattering_kinematic(sample, D, st, **kw)
+    run = dict(B.last_run)
+    assert run["launch_source"] == "nodes", run
+    if acceptance not in (0.0, 1.1e-3, 1.0):
+        assert 1 <= run["edge_pixels"] <= 8, run
+    B._use_fast_kernel = False
+    ref = B.atomic_scattering_kinematic(sample, D, st, **kw)
+    one = B.atomic_scattering_kinematic(sample, D, st, apply_polarization=True, spherical_decay=True,
+                                        return_double=True)
+    scale = np.abs(one).max()
+    assert np.abs(got - ref).max() <= 1e-4 * scale
+    assert ((got == 0) == (ref == 0)).all()

@@ -651,41 +651,60 @@ __device__ __forceinline__ int mk_find_frame(int lo, int hi, long long i, Key ke
     return lo;
 }
 
-__device__ __forceinline__ double mk_cheb(int i, int n) { return cospi((2 * i + 1) / (2.0 * n)); }
-
-// Lagrange weights at x of the n Chebyshev nodes, FP64 products rounded once.
-__device__ void mk_lagrange(double x, int n, float *out)
-{
-    double xs[MK_NODE_MAX];
-    for (int i = 0; i < n; ++i) xs[i] = mk_cheb(i, n);
-    for (int j = 0; j < n; ++j) {
-        double num = 1.0, den = 1.0;
-        for (int i = 0; i < n; ++i)
-            if (i != j) {
-                num *= x - xs[i];
-                den *= xs[j] - xs[i];
-            }
-        out[j] = (float)(num / den);
-    }
-}
-
 __device__ __forceinline__ double mk_half_range(int len) { return 0.5 * (len - 1) + MK_NODE_PAD; }
 
-// Node records and weight tables of every frame; one thread per node, pixel
-// column, pixel row and fine node position. A few thousand FP64 operations a
-// thread at most, launched once per sum: latency (7 us), not throughput.
-__global__ void mk_node_prep_kernel(const MkNodeFrame *__restrict__ frames, int n0, int n1, double kappa,
-                                    const double *__restrict__ xyz, MkNodeRec *__restrict__ rec0,
-                                    MkNodeRec *__restrict__ rec1, float *__restrict__ weights)
+// The Chebyshev nodes of one count and the inverse products of their Lagrange
+// weights, in shared memory.
+struct MkCheb {
+    double x[MK_NODE_MAX], inv[MK_NODE_MAX];
+};
+
+// Lagrange weight j of n nodes at x: FP64 products rounded once.
+__device__ __forceinline__ float mk_lagrange(const MkCheb &C, double x, int n, int j)
 {
-    const MkNodeFrame F = frames[blockIdx.x];
+    double num = C.inv[j];
+    for (int i = 0; i < n; ++i)
+        if (i != j) num *= x - C.x[i];
+    return (float)num;
+}
+
+// Node records and weight tables of every frame; one thread per node and per
+// weight. A chain of ~n FP64 products a thread, launched once per sum:
+// latency. With all n weights (and the nodes' cosines) in one thread it took
+// 35 us on a 128 x 128 detector and 99 us for 16 frames; here 8.5 and 51.
+__global__ void __launch_bounds__(128) mk_node_prep_kernel(const MkNodeFrame *__restrict__ frames, int n0,
+                                                           int n1, double kappa,
+                                                           const double *__restrict__ xyz,
+                                                           MkNodeRec *__restrict__ rec0,
+                                                           MkNodeRec *__restrict__ rec1,
+                                                           float *__restrict__ weights)
+{
+    __shared__ MkCheb s_c[2];              // of n0 and n1
+    const int th = threadIdx.x;
+    if (th < 64) {
+        const int n = th < 32 ? n0 : n1, i = th & 31;
+        if (i < n) s_c[th >> 5].x[i] = cospi((2 * i + 1) / (2.0 * n));
+    }
+    __syncthreads();
+    if (th < 64) {
+        const int n = th < 32 ? n0 : n1, j = th & 31;
+        MkCheb &C = s_c[th >> 5];
+        if (j < n) {
+            double den = 1.0;
+            for (int i = 0; i < n; ++i)
+                if (i != j) den *= C.x[j] - C.x[i];
+            C.inv[j] = 1.0 / den;
+        }
+    }
+    __syncthreads();
+    const MkNodeFrame &F = frames[blockIdx.x];
     const int l0y = F.l1y * F.ratio_y, l0z = F.l1z * F.ratio_z;
     const int a0 = n0 ? F.p0y * F.p0z * n0 * n0 : 0, a1 = F.p1y * F.p1z * n1 * n1;
-    const int wy = F.ny, wz = F.nz, my = n0 ? F.ratio_y * n1 : 0, mz = n0 ? F.ratio_z * n1 : 0;
-    const int total = a0 + a1 + wy + wz + my + mz;
+    const int wp = (F.ny + F.nz) * n1, wm = n0 ? (F.ratio_y + F.ratio_z) * n1 * n0 : 0;
+    const int total = a0 + a1 + wp + wm;
     float *W = weights + F.w_off;
-    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < total; i += gridDim.y * blockDim.x) {
-        int e = i;
+    for (int t = blockIdx.y * blockDim.x + th; t < total; t += gridDim.y * blockDim.x) {
+        int e = t;
         if (e < a0 + a1) {
             const bool fine = e >= a0;
             if (fine) e -= a0;
@@ -693,8 +712,9 @@ __global__ void mk_node_prep_kernel(const MkNodeFrame *__restrict__ frames, int 
             const int ly = fine ? F.l1y : l0y, lz = fine ? F.l1z : l0z;
             const int p = e / (n * n), r = e - p * n * n, j = r / n, c = r - j * n;
             const int pz = p / py, pyi = p - pz * py;
-            const double y = pyi * (double)ly + 0.5 * (ly - 1) + mk_half_range(ly) * mk_cheb(c, n);
-            const double z = pz * (double)lz + 0.5 * (lz - 1) + mk_half_range(lz) * mk_cheb(j, n);
+            const double *X = s_c[fine].x;
+            const double y = pyi * (double)ly + 0.5 * (ly - 1) + mk_half_range(ly) * X[c];
+            const double z = pz * (double)lz + 0.5 * (lz - 1) + mk_half_range(lz) * X[j];
             double P[3], u[3], q[3], r2 = 0.0;
             for (int d = 0; d < 3; ++d) {
                 P[d] = F.p0[d] + y * F.ey[d] + z * F.ez[d];
@@ -716,28 +736,24 @@ __global__ void mk_node_prep_kernel(const MkNodeFrame *__restrict__ frames, int 
             continue;
         }
         e -= a0 + a1;
-        float out[MK_NODE_MAX];
-        if (e < wy + wz) {                 // a pixel column or row in its fine patch
-            const bool row = e >= wy;
-            if (row) e -= wy;
-            const int len = row ? F.l1z : F.l1y;
-            const double *P = xyz + 3 * (F.pix_off + (row ? (long long)e * F.ny : e));
-            double v = mk_axis_coord(P, F.p0, row ? F.ez : F.ey, mk_axis_inv(row ? F.ez : F.ey));
-            const double c = (e / len) * (double)len + 0.5 * (len - 1);
-            mk_lagrange((v - c) / mk_half_range(len), n1, out);
-            float *o = W + (row ? (long long)n1 * F.ny : 0) + (long long)e * n1;
-            for (int j = 0; j < n1; ++j) o[j] = out[j];
+        if (e < wp) {                      // weight j of a pixel column, then row, in its fine patch
+            const int i = e / n1, j = e - i * n1;
+            const bool row = i >= F.ny;
+            const int k = row ? i - F.ny : i, len = row ? F.l1z : F.l1y;
+            const double *P = xyz + 3 * (F.pix_off + (row ? (long long)k * F.ny : k));
+            const double v = mk_axis_coord(P, F.p0, row ? F.ez : F.ey, mk_axis_inv(row ? F.ez : F.ey));
+            const double c = (k / len) * (double)len + 0.5 * (len - 1);
+            W[e] = mk_lagrange(s_c[1], (v - c) / mk_half_range(len), n1, j);
             continue;
         }
-        e -= wy + wz;                      // a fine node's position in the coarse patch
-        const bool row = e >= my;
-        if (row) e -= my;
+        e -= wp;                           // of a fine node's position in the coarse patch
+        const int i = e / n0, j = e - i * n0;
+        const bool row = i >= F.ratio_y * n1;
+        const int k = row ? i - F.ratio_y * n1 : i;
         const int l1 = row ? F.l1z : F.l1y, l0 = row ? l0z : l0y;
-        const int sub = e / n1, c = e - sub * n1;
-        const double v = sub * (double)l1 + 0.5 * (l1 - 1) + mk_half_range(l1) * mk_cheb(c, n1);
-        mk_lagrange((v - 0.5 * (l0 - 1)) / mk_half_range(l0), n0, out);
-        float *o = W + (long long)n1 * (F.ny + F.nz) + (row ? (long long)F.ratio_y * n1 * n0 : 0) + (long long)e * n0;
-        for (int j = 0; j < n0; ++j) o[j] = out[j];
+        const int sub = k / n1, c = k - sub * n1;
+        const double v = sub * (double)l1 + 0.5 * (l1 - 1) + mk_half_range(l1) * s_c[1].x[c];
+        W[wp + e] = mk_lagrange(s_c[0], (v - 0.5 * (l0 - 1)) / mk_half_range(l0), n0, j);
     }
 }
 
@@ -1305,11 +1321,11 @@ extern "C" int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, c
     int most = 0;
     for (int f = 0; f < plan->n_frames; ++f) {
         const MkNodeFrame &F = hf[f];
-        const int items = (n0 ? F.p0y * F.p0z * n0 * n0 + (F.ratio_y + F.ratio_z) * n1 : 0) +
-                          F.p1y * F.p1z * n1 * n1 + F.ny + F.nz;
+        const int items = (n0 ? F.p0y * F.p0z * n0 * n0 + (F.ratio_y + F.ratio_z) * n1 * n0 : 0) +
+                          F.p1y * F.p1z * n1 * n1 + (F.ny + F.nz) * n1;
         most = std::max(most, items);
     }
-    mk_node_prep_kernel<<<dim3(plan->n_frames, std::min((most + 63) / 64, 1024)), 64, 0, st>>>(
+    mk_node_prep_kernel<<<dim3(plan->n_frames, std::min((most + 127) / 128, 1024)), 128, 0, st>>>(
         A.frames, n0, n1, A.kappa_d, px->xyz, rec0, rec1, weights);
     MK_CHECK_CUDA(cudaGetLastError());
     const size_t leaf_smem = (size_t)T * 24;

@@ -477,9 +477,15 @@ struct MkTileMap {
     int tile_start[MK_MAX_SPECIES + 1];   // first tile of each species
 };
 
-// One block per tile: gather its atoms in sorted order, FP64 bounding-box
-// centre as origin, offsets k/2pi (a - o) rounded once to float32.
-template <int NT>
+// One block per tile: gather its atoms in sorted order; origin the centre of
+// their bounding box, offsets k/2pi (a - o) formed in FP64 and rounded once to
+// float32. The box is taken of the offsets from the tile's first atom, exact
+// differences rounded to float32, so that its ~40 minima and maxima a thread
+// stay off the FP64 pipe (2 lane operations per clock and SM), which bound
+// the build at 39 operations an atom (645 us for 8.19M atoms; here 358). Tiles of
+// up to 2 NT atoms hold their positions in registers, larger ones gather them
+// again for the offsets.
+template <int NT, bool HOLD>
 __global__ void __launch_bounds__(NT) mk_tile_kernel(MkTileMap M, double kappa,
                                                       const double *__restrict__ pos,
                                                       const float2 *__restrict__ amp,
@@ -494,28 +500,47 @@ __global__ void __launch_bounds__(NT) mk_tile_kernel(MkTileMap M, double kappa,
     while (s + 1 < M.n_species && t >= M.tile_start[s + 1]) ++s;
     const long long first = M.run_start[s] + (long long)(t - M.tile_start[s]) * M.tile_atoms;
     const long long end = M.run_start[s] + M.run_count[s];
-    __shared__ double red[6][NT / 32];
-    __shared__ double org[3];
-    __shared__ double rad2[NT / 32];
+    __shared__ float red[6][NT / 32];
+    __shared__ float rad2[NT / 32];
+    const long long a0 = order[first];
+    const double fx = pos[3 * a0], fy = pos[3 * a0 + 1], fz = pos[3 * a0 + 2];
 
-    double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-    for (int j = threadIdx.x; j < M.tile_atoms; j += NT) {
-        const long long si = first + j;
-        if (si < end) {
-            const int a = order[si];
+    double hx[2], hy[2], hz[2];             // HOLD: offsets from the first atom
+    int ha[2];
+    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    auto meet = [&](double x, double y, double z) {
+        const float v[3] = {(float)x, (float)y, (float)z};
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const double v = pos[3 * (long long)a + c];
-                lo[c] = fmin(lo[c], v);
-                hi[c] = fmax(hi[c], v);
+        for (int c = 0; c < 3; ++c) {
+            lo[c] = fminf(lo[c], v[c]);
+            hi[c] = fmaxf(hi[c], v[c]);
+        }
+    };
+    if constexpr (HOLD) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int j = threadIdx.x + i * NT;
+            const long long si = first + j;
+            ha[i] = j < M.tile_atoms && si < end ? order[si] : -1;
+            hx[i] = hy[i] = hz[i] = 0.0;
+            if (ha[i] >= 0) {
+                hx[i] = pos[3 * (long long)ha[i]] - fx;
+                hy[i] = pos[3 * (long long)ha[i] + 1] - fy;
+                hz[i] = pos[3 * (long long)ha[i] + 2] - fz;
+                meet(hx[i], hy[i], hz[i]);
             }
+        }
+    } else {
+        for (int j = threadIdx.x; j < M.tile_atoms && first + j < end; j += NT) {
+            const long long a = order[first + j];
+            meet(pos[3 * a] - fx, pos[3 * a + 1] - fy, pos[3 * a + 2] - fz);
         }
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         for (int off = 16; off > 0; off >>= 1) {
-            lo[c] = fmin(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], off));
-            hi[c] = fmax(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], off));
+            lo[c] = fminf(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], off));
+            hi[c] = fmaxf(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], off));
         }
         if ((threadIdx.x & 31) == 0) {
             red[c][threadIdx.x >> 5] = lo[c];
@@ -523,31 +548,27 @@ __global__ void __launch_bounds__(NT) mk_tile_kernel(MkTileMap M, double kappa,
         }
     }
     __syncthreads();
-    if (threadIdx.x < 3) {
-        double l = 1e300, h = -1e300;
+    double org[3];                          // the box's centre, from the first atom
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        float l = INFINITY, h = -INFINITY;
         for (int w = 0; w < NT / 32; ++w) {
-            l = fmin(l, red[threadIdx.x][w]);
-            h = fmax(h, red[3 + threadIdx.x][w]);
+            l = fminf(l, red[c][w]);
+            h = fmaxf(h, red[3 + c][w]);
         }
-        org[threadIdx.x] = 0.5 * (l + h);
+        org[c] = (double)(0.5f * (l + h));
     }
-    __syncthreads();
-    const double ox = org[0], oy = org[1], oz = org[2];
-    double r2max = 0.0;
+    float r2max = 0.f;
     const long long base = (long long)t * M.tile_atoms;
-    for (int j = threadIdx.x; j < M.tile_atoms; j += NT) {
-        const long long si = first + j;
+    auto put = [&](int j, int a, double x, double y, double z) {
         float4 P = make_float4(0.f, 0.f, 0.f, 0.f);
         float2 E = make_float2(0.f, 0.f);
-        if (si < end) {
-            const int a = order[si];
-            const double dx = pos[3 * (long long)a] - ox;
-            const double dy = pos[3 * (long long)a + 1] - oy;
-            const double dz = pos[3 * (long long)a + 2] - oz;
+        if (a >= 0) {
+            const double dx = x - org[0], dy = y - org[1], dz = z - org[2];
             const double d2 = dx * dx + dy * dy + dz * dz;
-            r2max = fmax(r2max, d2);
             P = make_float4((float)(kappa * dx), (float)(kappa * dy), (float)(kappa * dz),
                             (float)(kappa * kappa * d2));
+            r2max = fmaxf(r2max, P.w);
             E = amp[a];
         }
         // atom pairs interleaved: per pair (2q, 2q+1) the floats
@@ -562,14 +583,32 @@ __global__ void __launch_bounds__(NT) mk_tile_kernel(MkTileMap M, double kappa,
         pf[6 + h] = P.w;
         af[h] = E.x;
         af[2 + h] = E.y;
+    };
+    if constexpr (HOLD) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int j = threadIdx.x + i * NT;
+            if (j < M.tile_atoms) put(j, ha[i], hx[i], hy[i], hz[i]);
+        }
+    } else {
+        for (int j = threadIdx.x; j < M.tile_atoms; j += NT) {
+            const int a = first + j < end ? order[first + j] : -1;
+            if (a >= 0)
+                put(j, a, pos[3 * (long long)a] - fx, pos[3 * (long long)a + 1] - fy,
+                    pos[3 * (long long)a + 2] - fz);
+            else
+                put(j, a, 0.0, 0.0, 0.0);
+        }
     }
-    for (int off = 16; off > 0; off >>= 1) r2max = fmax(r2max, __shfl_xor_sync(0xffffffffu, r2max, off));
+    for (int off = 16; off > 0; off >>= 1) r2max = fmaxf(r2max, __shfl_xor_sync(0xffffffffu, r2max, off));
     if ((threadIdx.x & 31) == 0) rad2[threadIdx.x >> 5] = r2max;
     __syncthreads();
     if (threadIdx.x == 0) {
-        double m = 0.0;
-        for (int w = 0; w < NT / 32; ++w) m = fmax(m, rad2[w]);
-        origin[t] = make_double4(ox, oy, oz, sqrt(m));
+        float m = 0.f;
+        for (int w = 0; w < NT / 32; ++w) m = fmaxf(m, rad2[w]);
+        // |D|^2 was rounded to float32 (in cycles): a whole ulp up bounds it
+        origin[t] = make_double4(fx + org[0], fy + org[1], fz + org[2],
+                                 sqrt((double)m * (1.0 + 1.2e-7)) / kappa);
         tspecies[t] = s;
     }
 }
@@ -658,7 +697,8 @@ extern "C" int mk_tiles_build(int64_t n, const double *pos, const int *species, 
     MK_CHECK_CUDA(cudaGetLastError());
     MK_CHECK_CUDA(cub::DeviceRadixSort::SortPairs(w, temp, k_in, k_out, i_in, i_out, (int)n, 0, key_bits, st));
     if (tiles_needed > 0) {
-        mk_tile_kernel<256><<<tiles_needed, 256, 0, st>>>(
+        auto fn = T <= 512 ? mk_tile_kernel<256, true> : mk_tile_kernel<256, false>;
+        fn<<<tiles_needed, 256, 0, st>>>(
             M, k / MK_TWO_PI, pos, reinterpret_cast<const float2 *>(amp), i_out,
             reinterpret_cast<double4 *>(tiles->origin), tiles->species,
             reinterpret_cast<float4 *>(tiles->pos), reinterpret_cast<float2 *>(tiles->amp));

@@ -185,11 +185,13 @@ typedef struct {
     int n_wide;             /* tiles left to the split kernel (their indices at off_wide) */
     int n_src;              /* n_groups + n_mid */
     int slices, src_per_slice, passes;
-    long long nodes0, patches1, weights, n_pix;
+    int ns;                 /* nodes per axis of a tile's eighths (0: tiles evaluated whole) */
+    long long nodes0, patches1, weights, n_pix, nodes_s, sub_w_off;
     long long off_src, off_members, off_mid, off_wide, buf_bytes;
     long long chunk_bytes, ws_bytes;
     double radius1_m, radius2_m; /* widest tile of a group, widest source */
-    double nodes_s, direct_s;    /* estimated time of this form and of the split kernel */
+    double sub_radius_m;         /* widest eighth that its nodes take */
+    double form_s, direct_s;     /* estimated time of this form and of the split kernel */
 } mk_node_plan;
 
 /* --- library ---------------------------------------------------------- */

@@ -79,6 +79,34 @@ def test_nodes_match_fp64_and_split(cuda, shape, tile, group, dist, decay, cplx)
         assert torch.equal(again, acc)              # the same sum twice, to the bit
 
 
+@pytest.mark.parametrize("cells, dilute, shape, dist, n0", [
+    (24, 0.005, (200, 90), 0.2e10, 20),     # dilute tiles among the groups: eighths too wide for their nodes
+    (20, 0.02, (257, 33), 0.5e10, 16),
+    (24, 0.0, (400, 130), 0.1e10, 20),      # several coarse patches, tiles with the |d|^2 term
+])
+def test_leaf_by_eighths_matches_fp64_and_split(cuda, cells, dilute, shape, dist, n0):
+    """Tiles of 512 atoms whose coarse nodes are filled from their eighths'."""
+    w, sample = _case(cells, dilute=dilute)
+    B = workloads._beam(10000.0, 200.0, pol_perp_rate=1.0)
+    st = StaticStage(w.stage.rotation, w.stage.translation)
+    D = _det(w, shape, dist)
+    phys = B.physics(apply_polarization=True)
+    atoms = B.stage_atoms(sample, st, device=cuda)
+    pix = engine.Pixels(np.asarray(D.pixel_coordinates) / 1e10, *shape, phys, device=cuda)
+    tiles = engine.Tiles(atoms, B.k, 512, device=cuda)
+    plan = engine.NodePlan.make(tiles, pix, B.k, (1.0, 0.0, 0.0), 1e-6, direct=1.0, group_tiles=8)
+    assert plan is not None and plan.plan.n0 == n0 and plan.plan.ns > 0 and plan.plan.n_members > 0
+    acc = torch.full((pix.n, 2), float("nan"), dtype=torch.float64, device=cuda)
+    wide = plan.wide is not None
+    if wide:
+        engine.run_split(plan.wide, pix, phys, atoms.table, fresnel=1, out=acc, factor_table=True)
+    got = _c(engine.run_nodes(plan, tiles, pix, phys, atoms.table, out=acc, accumulate=wide, fresnel=1), shape)
+    one = _c(engine.run_split(tiles, pix, phys, atoms.table, fresnel=1), shape)
+    ref = _c(engine.run_plain(atoms, pix, phys), shape)
+    assert rel_intensity(got, ref) <= 1e-4, rel_intensity(got, ref)
+    assert rel_max(got, one) <= 2e-5, rel_max(got, one)
+
+
 def test_entry_point_takes_nodes_where_admitted(cuda):
     """Large enough on a plane detector: nodes; a curved (shell) detector,
     an explicit launch, remove_forward and a Darwin analyser: the other forms,

@@ -522,6 +522,9 @@ int mk_relu_backward(long long n, const float *grad, const float *pre, float *go
 int mk_bias_grad(int M, int N, const float *g, float *db, void *stream);
 int mk_bias_grad_groups(int groups, int M, int N, const float *g, long long g_stride, float *db,
                         long long db_stride, void *stream);
+/* mk_bias_grad_groups added into db. */
+int mk_bias_grad_add_groups(int groups, int M, int N, const float *g, long long g_stride, float *db,
+                            long long db_stride, void *stream);
 /* MSE over n entries: grad = 2(y - t)/n (float and/or bf16), partial sums of
  * squares per 256-block in `partials` (ceil(n/256) doubles). */
 int mk_mse(long long n, const float *y, const float *t, float *grad, void *grad_bf16,

@@ -22,11 +22,17 @@
 // and returns.
 #include <cuda_bf16.h>
 
+#include <atomic>
+
 #include "mk_tc.cuh"
 
 #define MK_TCG_BM 128
 #define MK_TCG_BK 64
-#define MK_TCG_STAGES 3
+// Stages: wide outputs (BN 128, the frame decode) 3, which lets two CTAs share
+// an SM; 64-column tiles 5, so that all four chunks of a 256-deep layer are in
+// flight before its first MMA (few CTAs, latency-bound: 11.0 -> 10.1 us a launch of
+// two 1272 x 256 x 256 networks).
+#define MK_TCG_STAGES(BN) ((BN) >= 128 ? 3 : 5)
 #define MK_TCG_NT 256
 
 #define MK_GEMM_ACCUMULATE 1
@@ -192,7 +198,7 @@ __global__ void __launch_bounds__(MK_TCG_NT) mk_gemm_tc_kernel(MkTcGemm g, int *
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem);            // MK_TCG_STAGES barriers
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + 64);
     unsigned char *stages = smem + 1024;
-    constexpr int S = MK_TCG_STAGES;
+    constexpr int S = MK_TCG_STAGES(BN);
     constexpr int A_BYTES = MK_TCG_BM * MK_TCG_BK * 2;
     constexpr int STAGE_BYTES = A_BYTES + BN * MK_TCG_BK * 2;
     constexpr uint32_t NCOLS = BN < 32 ? 32u : (uint32_t)BN;
@@ -399,9 +405,16 @@ static int mk_tcg_read_status(cudaStream_t st)
 template <int BN>
 static int mk_tcg_launch(const MkTcGemm &g, dim3 grid, cudaStream_t st, int *status)
 {
-    const size_t smem = 2048 + (size_t)MK_TCG_STAGES * (MK_TCG_BM + BN) * MK_TCG_BK * 2;
-    MK_CHECK_CUDA(cudaFuncSetAttribute((const void *)mk_gemm_tc_kernel<BN>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const size_t smem = 2048 + (size_t)MK_TCG_STAGES(BN) * (MK_TCG_BM + BN) * MK_TCG_BK * 2;
+    // the attribute is set once per device: it belongs to the loaded function
+    static std::atomic<unsigned long long> done{0};
+    int dev = 0;
+    MK_CHECK_CUDA(cudaGetDevice(&dev));
+    if (dev >= 64 || !(done.load(std::memory_order_acquire) >> dev & 1ull)) {
+        MK_CHECK_CUDA(cudaFuncSetAttribute((const void *)mk_gemm_tc_kernel<BN>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (dev < 64) done.fetch_or(1ull << dev, std::memory_order_release);
+    }
     mk_gemm_tc_kernel<BN><<<grid, MK_TCG_NT, smem, st>>>(g, status);
     MK_CHECK_CUDA(cudaGetLastError());
     return MK_OK;

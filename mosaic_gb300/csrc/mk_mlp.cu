@@ -276,19 +276,32 @@ __global__ void __launch_bounds__(256) mk_colsum_kernel(int M, int N, const floa
     }
 }
 
-extern "C" int mk_bias_grad_groups(int groups, int M, int N, const float *g, long long g_stride,
-                                   float *db, long long db_stride, void *stream)
+static int mk_bias_grad_run(int groups, int M, int N, const float *g, long long g_stride, float *db,
+                            long long db_stride, bool add, void *stream)
 {
     MK_REQUIRE(groups >= 1 && M > 0 && N > 0 && g && db, "mk_bias_grad: bad arguments");
     MK_REQUIRE(groups == 1 || db_stride >= N, "mk_bias_grad: groups' gradients overlap");
     dim3 grid((N + 31) / 32, (M + MK_COLSUM_ROWS - 1) / MK_COLSUM_ROWS, groups);
     MK_REQUIRE(grid.y < 65536 && groups < 65536, "mk_bias_grad: M or groups too large");
     cudaStream_t st = mk_stream(stream);
-    for (int q = 0; q < groups; ++q)
-        MK_CHECK_CUDA(cudaMemsetAsync(db + q * db_stride, 0, sizeof(float) * (size_t)N, st));
+    if (!add)
+        for (int q = 0; q < groups; ++q)
+            MK_CHECK_CUDA(cudaMemsetAsync(db + q * db_stride, 0, sizeof(float) * (size_t)N, st));
     mk_colsum_kernel<<<grid, 256, 0, st>>>(M, N, g, g_stride, db, db_stride);
     MK_CHECK_CUDA(cudaGetLastError());
     return MK_OK;
+}
+
+extern "C" int mk_bias_grad_groups(int groups, int M, int N, const float *g, long long g_stride,
+                                   float *db, long long db_stride, void *stream)
+{
+    return mk_bias_grad_run(groups, M, N, g, g_stride, db, db_stride, false, stream);
+}
+
+extern "C" int mk_bias_grad_add_groups(int groups, int M, int N, const float *g, long long g_stride,
+                                       float *db, long long db_stride, void *stream)
+{
+    return mk_bias_grad_run(groups, M, N, g, g_stride, db, db_stride, true, stream);
 }
 
 extern "C" int mk_bias_grad(int M, int N, const float *g, float *db, void *stream)

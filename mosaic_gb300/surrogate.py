@@ -158,12 +158,13 @@ class MLP:
         gradient of a hidden layer carries the ReLU derivative in its
         GEMM's epilogue (the layer's outputs as the mask)."""
         B = int(G.shape[-2])
+        self.gP.zero_()     # every layer's gradient is added into the flat buffer
         for l in range(len(self.dims) - 2, -1, -1):
             K, N = self.dims[l], self.dims[l + 1]
             gx = 0 if (l == 0 and acts[0].dim() == 2) else B * K
-            self._gemm(N, K, B, Gb, 1, N, acts[l], K, 1, self.dW[l], K, None, 0, None, 0,
+            self._gemm(N, K, B, Gb, 1, N, acts[l], K, 1, self.dW[l], K, None, GEMM_ACC, None, 0,
                        gstrides=(B * N, gx, self._wpad[l], 0, 0, 0))
-            check(self.L.mk_bias_grad_groups(self.G, B, N, _p(G), B * N, _p(self.db[l]),
+            check(self.L.mk_bias_grad_add_groups(self.G, B, N, _p(G), B * N, _p(self.db[l]),
                                              self._bpad[l], engine._stream_handle()))
             if l == 0:
                 break

@@ -14,7 +14,8 @@
 //   merge   V1[group][fine node]: the tiles of a group (consecutive on the
 //           Hilbert curve) interpolated from the coarse patch's nodes to the
 //           nodes of finer patches, each times exp(2 pi i phase of its origin
-//           relative to the group's), added,
+//           relative to the group's), added; in two steps by way of runs of
+//           a few tiles on middle patches where that is cheaper,
 //   pixels  every group's field interpolated from the fine patch's nodes to
 //           the pixels, times exp(2 pi i phase of the group's origin), added
 //           (Kahan), times the species' factor (mk_factor_table); slices of
@@ -58,24 +59,32 @@
 #define MK_SINCOS_SHORT 7.3e-8f
 __device__ __forceinline__ float mk_unshort(float v) { return fmaf(v, MK_SINCOS_SHORT, v); }
 
-// One frame of a plan. A frame is cut into p1y x p1z fine patches of
-// l1y x l1z pixels, and those into p0y x p0z coarse patches of
-// (ratio_y x ratio_z) fine ones.
+// Levels of patches: tiles' coarse ones, the middle ones of runs of a few tiles
+// (only in plans with two merges), the fine ones of groups. Patches of one
+// level are ratio_y x ratio_z of the next finer one.
+enum { MK_COARSE = 0, MK_MIDDLE = 1, MK_FINE = 2 };
+
+// A merge step of a frame: into the middle patches (0), into the fine ones (1).
+struct MkNodeMerge {
+    int ratio_y, ratio_z;               // finer patches per patch
+    int strip, strips;                  // finer patches per strip, strips per patch
+    int rowg, chunks;                   // row groups of a block, blocks per strip
+    long long w_off, item_off;
+};
+
+// One frame of a plan: py[L] x pz[L] patches of ly[L] x lz[L] pixels.
 struct MkNodeFrame {
     double p0[3], ey[3], ez[3], b[3];
     int ny, nz;
-    int l1y, l1z, p1y, p1z;
-    int ratio_y, ratio_z, p0y, p0z;
+    int ly[3], lz[3], py[3], pz[3];
     int bpy, bpz;                       // pixel blocks per fine patch
-    int strip, strips;                  // merge: fine patches per strip, strips per coarse patch
-    int rowg, chunks;                   // row groups of a block, blocks per strip
-    long long pix_off;
-    long long node0_off, patch1_off;    // node1_off = patch1_off * n1^2
-    long long pblk_off, part_off, w_off, item_off;
+    MkNodeMerge mg[2];
+    long long off[3];                   // patches of each level before this frame
+    long long pix_off, pblk_off, part_off, w_off;
 };
 
-// A source of the pixel step: a group of tiles (count > 0: nar[first ..]) or
-// a single tile (count 0).
+// A source of the pixel step: a group of `count` tiles (or runs) from `first`
+// on, or a single tile (count 0). A run of tiles on middle nodes is one too.
 struct MkNodeSrc {
     float dh[3];
     int species;
@@ -191,12 +200,18 @@ const int kNodeCounts[] = {6, 8, 10, 12, 16, 20};
 
 // Largest phase half-range phi [rad] n Chebyshev nodes interpolate to
 // 4 (phi/2)^n / n! <= 3e-8.
-double phi_max(int n)
+double phi_of(int n)
 {
     double f = 7.5e-9;
     for (int i = 2; i <= n; ++i) f *= i;
     return 2.0 * std::pow(f, 1.0 / n);
 }
+struct PhiTable {
+    double v[MK_NODE_MAX + 1];
+    PhiTable() { for (int n = 1; n <= MK_NODE_MAX; ++n) v[n] = phi_of(n); }
+};
+const PhiTable kPhi;
+double phi_max(int n) { return kPhi.v[n]; }
 
 // Largest patch (pixels) whose phase half-range stays within `phi` for atoms
 // up to k r = kr [rad] off the centre, a rad of direction per pixel.
@@ -222,62 +237,80 @@ bool cut(int n, double most, int unit, int *len, int *count)
 // One ROI shape: the widest angular steps of its frames, and how many there are.
 struct Geo { double ay, az; int ny, nz, frames; };
 
-// Fine patches of every ROI shape for sources of radius r2 on n1 nodes, and
-// coarse ones (n0 > 0) for tiles of radius r1; the nodes of all frames.
-bool lay_out(const std::vector<Geo> &g, double k, double r2, int n1, double r1, int n0,
-             std::vector<MkNodeFrame> *out, double *nodes1, double *nodes0)
+// A level's patches of one ROI shape: py x pz of ly x lz pixels, each ry x rz of
+// the finer level's.
+struct Cut { int ly, lz, py, pz, ry, rz; };
+
+// Fine patches of every ROI shape for sources of radius r on n nodes; the nodes
+// of all frames.
+bool fine_cut(const std::vector<Geo> &g, double k, double r, int n, std::vector<Cut> *out, double *nodes)
 {
-    *nodes1 = *nodes0 = 0.0;
+    *nodes = 0.0;
     for (size_t f = 0; f < g.size(); ++f) {
-        MkNodeFrame F{};
-        if (!cut(g[f].ny, patch_limit(phi_max(n1), k * r2, g[f].ay), MK_PIX_COLS, &F.l1y, &F.p1y) ||
-            !cut(g[f].nz, patch_limit(phi_max(n1), k * r2, g[f].az), MK_PIX_ROWS, &F.l1z, &F.p1z))
+        Cut &C = (*out)[f];
+        if (!cut(g[f].ny, patch_limit(phi_max(n), k * r, g[f].ay), MK_PIX_COLS, &C.ly, &C.py) ||
+            !cut(g[f].nz, patch_limit(phi_max(n), k * r, g[f].az), MK_PIX_ROWS, &C.lz, &C.pz))
             return false;
-        F.ratio_y = F.ratio_z = F.p0y = F.p0z = 1;
-        if (n0 > 0) {
-            const double ly = patch_limit(phi_max(n0), k * r1, g[f].ay), lz = patch_limit(phi_max(n0), k * r1, g[f].az);
-            const int ry = (int)std::min<double>(F.p1y, std::floor(ly / F.l1y));
-            const int rz = (int)std::min<double>(F.p1z, std::floor(lz / F.l1z));
-            if (ry < 1 || rz < 1) return false;
-            F.p0y = (F.p1y + ry - 1) / ry;
-            F.p0z = (F.p1z + rz - 1) / rz;
-            F.ratio_y = (F.p1y + F.p0y - 1) / F.p0y;
-            F.ratio_z = (F.p1z + F.p0z - 1) / F.p0z;
-            F.p0y = (F.p1y + F.ratio_y - 1) / F.ratio_y;
-            F.p0z = (F.p1z + F.ratio_z - 1) / F.ratio_z;
-            *nodes0 += (double)g[f].frames * F.p0y * F.p0z * n0 * n0;
-        }
-        F.ny = g[f].ny;
-        F.nz = g[f].nz;
-        F.bpy = (F.l1y + MK_PIX_COLS - 1) / MK_PIX_COLS;
-        F.bpz = (F.l1z + MK_PIX_ROWS - 1) / MK_PIX_ROWS;
-        *nodes1 += (double)g[f].frames * F.p1y * F.p1z * n1 * n1;
-        if (out) (*out)[f] = F;
+        C.ry = C.rz = 1;
+        *nodes += (double)g[f].frames * C.py * C.pz * n * n;
     }
     return true;
 }
 
-// A run of tiles being gathered into a group: the box of their origins and
-// their widest radius bound the group's radius about the box's centre.
+// Even blocks of at most `most` of p patches: how many patches a block, how many blocks.
+void blocks_of(int p, int most, int *ratio, int *count)
+{
+    *count = (p + most - 1) / most;
+    *ratio = (p + *count - 1) / *count;
+    *count = (p + *ratio - 1) / *ratio;
+}
+
+// Patches of sources of radius r on n nodes, each a block of the finer level's.
+bool parent_cut(const std::vector<Geo> &g, double k, double r, int n, const std::vector<Cut> &finer,
+                std::vector<Cut> *out, double *nodes)
+{
+    *nodes = 0.0;
+    for (size_t f = 0; f < g.size(); ++f) {
+        const Cut &S = finer[f];
+        Cut &C = (*out)[f];
+        const int ry = (int)std::min<double>(S.py, std::floor(patch_limit(phi_max(n), k * r, g[f].ay) / S.ly));
+        const int rz = (int)std::min<double>(S.pz, std::floor(patch_limit(phi_max(n), k * r, g[f].az) / S.lz));
+        if (ry < 1 || rz < 1) return false;
+        blocks_of(S.py, ry, &C.ry, &C.py);
+        blocks_of(S.pz, rz, &C.rz, &C.pz);
+        C.ly = S.ly * C.ry;
+        C.lz = S.lz * C.rz;
+        *nodes += (double)g[f].frames * C.py * C.pz * n * n;
+    }
+    return true;
+}
+
+// A run of tiles being gathered: the box of their origins and their widest
+// radius bound its radius about the box's centre.
 struct Run {
     double lo[3], hi[3], rmax;
-    int count;
-    void start(const double *o)
+    int count, species;
+    bool single;                         // one tile, too wide for the coarse nodes
+    long long first;
+    void start(const double *o, int sp)
     {
         for (int c = 0; c < 3; ++c) lo[c] = hi[c] = o[c];
         rmax = o[3];
         count = 1;
+        species = sp;
+        single = false;
     }
-    // Adds a tile if the group's radius stays within r2.
-    bool add(const double *o, double r2)
+    // Takes in a box of origins and their widest radius if the run's radius
+    // stays within r2.
+    bool add(const double *bl, const double *bh, double br, double r2)
     {
         double l[3], h[3], d2 = 0.0;
         for (int c = 0; c < 3; ++c) {
-            l[c] = std::min(lo[c], o[c]);
-            h[c] = std::max(hi[c], o[c]);
+            l[c] = std::min(lo[c], bl[c]);
+            h[c] = std::max(hi[c], bh[c]);
             d2 += (h[c] - l[c]) * (h[c] - l[c]);
         }
-        const double r = std::max(rmax, o[3]);
+        const double r = std::max(rmax, br);
         if (!(0.5 * std::sqrt(d2) + r <= r2)) return false;
         for (int c = 0; c < 3; ++c) { lo[c] = l[c]; hi[c] = h[c]; }
         rmax = r;
@@ -287,20 +320,18 @@ struct Run {
 };
 
 // Cuts the narrow tiles (radius <= r1) of [a, b), in order, into runs of one
-// species, radius <= r2 and at most `most` tiles: done(run, last) for each.
+// species, radius <= r2 and at most `most` tiles: done(run) for each.
 template <class Done>
 void cut_runs(const double *org, const int *tsp, int a, int b, double r1, double r2, int most, Done done)
 {
     Run R;
     R.count = 0;
-    int sp = -1;
     for (int t = a; t < b; ++t) {
         const double *o = org + 4ll * t;
         if (!(o[3] <= r1)) continue;
-        if (R.count && tsp[t] == sp && R.count < most && R.add(o, r2)) continue;
+        if (R.count && tsp[t] == R.species && R.count < most && R.add(o, o, o[3], r2)) continue;
         if (R.count) done(R);
-        R.start(o);
-        sp = tsp[t];
+        R.start(o, tsp[t]);
     }
     if (R.count) done(R);
 }
@@ -308,19 +339,19 @@ void cut_runs(const double *org, const int *tsp, int a, int b, double r1, double
 // Rows a thread of the merge holds, a divisor of n1.
 int merge_rows(int n1) { return n1 == 10 ? 5 : n1 == 6 || n1 == 12 ? 3 : 4; }
 
-// Cuts a coarse patch's row of fine patches into strips of at most 128 node
+// Cuts a patch's row of finer patches (n1 nodes) into strips of at most 128 node
 // columns for the merge's blocks, the strip length that keeps most of their
 // 128 threads busy.
-void lay_strips(MkNodeFrame *F, int n1)
+void lay_strips(MkNodeMerge *M, int n1)
 {
-    const int rows = merge_rows(n1), most = std::min(F->ratio_y, MK_MERGE_NT / n1);
+    const int rows = merge_rows(n1), most = std::min(M->ratio_y, MK_MERGE_NT / n1);
     double best = -1.0;
     for (int sp = 1; sp <= most; ++sp) {
-        const int strips = (F->ratio_y + sp - 1) / sp;
+        const int strips = (M->ratio_y + sp - 1) / sp;
         const int rowg = std::min(MK_MERGE_NT / (sp * n1), n1 / rows);
         const int chunks = (n1 / rows + rowg - 1) / rowg;
-        const double use = (double)F->ratio_y * n1 * n1 / ((double)strips * chunks * MK_MERGE_NT * rows) + 1e-3 * sp;
-        if (use > best) { best = use; F->strip = sp; F->strips = strips; F->rowg = rowg; F->chunks = chunks; }
+        const double use = (double)M->ratio_y * n1 * n1 / ((double)strips * chunks * MK_MERGE_NT * rows) + 1e-3 * sp;
+        if (use > best) { best = use; M->strip = sp; M->strips = strips; M->rowg = rowg; M->chunks = chunks; }
     }
 }
 
@@ -348,18 +379,66 @@ double leaf_terms(int n0, int tile_atoms)
     return ns ? 1.2 * ns * ns : (double)n0 * n0;
 }
 
+// Radii and nodes of tiles (r1, n0), runs (rm, nm; nm 0: no middle level) and
+// groups (r2, n1; G 0: none).
 struct Choice {
-    double cost = 1e300, r1 = 0.0, r2 = 0.0;
-    int n0 = 0, n1 = 0, G = 0;
+    double cost = 1e300, r1 = 0.0, rm = 0.0, r2 = 0.0;
+    int n0 = 0, nm = 0, n1 = 0, G = 0;
 };
+
+// Node records of a plan: coarse, middle, fine, and the eighths' on the coarse patches.
+long long records(const mk_node_plan &P)
+{
+    return P.patches0 * (P.n0 * P.n0 + P.ns * P.ns) + P.patchesm * P.nm * P.nm + P.patches1 * P.n1 * P.n1;
+}
+
+// Whole frames from f on whose node fields and partials fit `budget` bytes (one
+// at least), and their launches fit a grid: their patches of each level, pixels,
+// pixel blocks, merge blocks per source and bytes. Returns the frame after them.
+struct Pass {
+    long long patches[3], pix, pblk, items[2];
+    size_t bytes, field[3];
+};
+int next_pass(const mk_node_plan &plan, const MkNodeFrame *fr, int f, size_t budget, Pass *out)
+{
+    const int n[3] = {plan.n0, plan.nm, plan.n1};
+    const double rows[3] = {(double)plan.n_members, (double)plan.n_msrc, (double)plan.n_src};
+    Pass P{};
+    for (int g = f; g < plan.n_frames; ++g) {
+        const MkNodeFrame &F = fr[g];
+        Pass Q = P;
+        bool too_many = false;
+        for (int l = 0; l < 3; ++l) {
+            Q.patches[l] += (long long)F.py[l] * F.pz[l];
+            const double nodes = (double)Q.patches[l] * n[l] * n[l];
+            too_many |= nodes > 256.0 * 60000;
+            Q.field[l] = up256((size_t)(8.0 * nodes * rows[l]));
+        }
+        Q.pix += (long long)F.ny * F.nz;
+        Q.pblk += (long long)F.py[MK_FINE] * F.pz[MK_FINE] * F.bpy * F.bpz;
+        for (int m = 0; m < 2; ++m) {
+            const int in = m == 0 || !plan.nm ? MK_COARSE : MK_MIDDLE, to = m == 0 ? MK_MIDDLE : MK_FINE;
+            Q.items[m] += (long long)F.pz[to] * F.py[in] * F.mg[m].strips * F.mg[m].chunks;
+            too_many |= Q.items[m] * std::max(m == 0 ? plan.n_msrc : plan.n_groups, 1) > (1ll << 30);
+        }
+        Q.bytes = Q.field[0] + Q.field[1] + Q.field[2] + up256(16 * (size_t)Q.pix * plan.slices);
+        if (g > f && (Q.bytes > budget || too_many)) {
+            *out = P;
+            return g;
+        }
+        P = Q;
+    }
+    *out = P;
+    return plan.n_frames;
+}
 
 }  // namespace
 
 extern "C" size_t mk_nodes_plan_bytes(int n_frames, int n_tiles)
 {
     if (n_frames < 1 || n_tiles < 0) return 0;
-    return up256(sizeof(MkNodeFrame) * (size_t)n_frames) + up256(sizeof(MkNodeSrc) * (size_t)n_tiles) +
-           3 * up256(sizeof(int) * (size_t)n_tiles);
+    return up256(sizeof(MkNodeFrame) * (size_t)n_frames) + 2 * up256(sizeof(MkNodeSrc) * (size_t)n_tiles) +
+           up256(sizeof(double4) * (size_t)n_tiles) + 5 * up256(sizeof(int) * (size_t)n_tiles);
 }
 
 extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const int64_t *counts,
@@ -426,8 +505,8 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
     plan->direct_s = n_tiles * T * n_pix * direct_s_per_term + 2.0 * kLaunch;
     auto split = [&](double n) { return n > 0.0 ? n * T * n_pix * kWide + n_pix * 30e-12 + kWideSetup : 0.0; };
 
-    // Search on a sample: at most 2048 tiles, in 8 stretches of the curve.
-    const int stretch = n_tiles <= 2048 ? n_tiles : 256, stretches = n_tiles <= 2048 ? 1 : 8;
+    // Search on a sample: at most 2048 tiles, in 4 stretches of the curve.
+    const int stretch = n_tiles <= 2048 ? n_tiles : 512, stretches = n_tiles <= 2048 ? 1 : 4;
     std::vector<double> some;
     std::vector<int> starts;
     for (int i = 0; i < stretches; ++i) {
@@ -443,9 +522,20 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
         if (r > q(0.9)) tail.push_back(r);
     std::sort(tail.begin(), tail.end());
     Choice best;
-    const double q1[] = {rmax, q(0.99), q(0.95), q(0.8), q(0.5)};
-    const double f2[] = {1.0, 1.5, 2.2, 3.2, 4.5, 6.5};
-    for (int i1 = 0; i1 < 5; ++i1) {
+    std::vector<Cut> c1(geo.size()), cm(geo.size()), c0(geo.size());
+    const double q1[] = {rmax, q(0.99), q(0.95), q(0.8)};
+    const double f2[] = {1.0, 1.5, 2.2, 3.2, 4.5, 6.5, 9.0};
+    const int nf2 = sizeof(f2) / sizeof(f2[0]);
+    const int G = group_tiles > 0 ? group_tiles : 4096;
+    const bool groups = group_tiles != 0 && (group_tiles > 0 || n_tiles >= 32);
+    double run_count[nf2];                  // runs of all tiles within every radius
+    for (int i = 0; groups && i < nf2; ++i) {
+        run_count[i] = 0.0;
+        for (int a : starts)
+            cut_runs(origins, tsp.data(), a, a + stretch, q(0.95), std::max(f2[i] * q(0.5), q(0.95)), G,
+                     [&](const Run &) { run_count[i] += up / 0.95; });
+    }
+    for (int i1 = 0; i1 < 4; ++i1) {
         const double r1 = q1[i1];
         if (i1 > 0 && r1 == q1[i1 - 1]) continue;
         auto above = [&](double r) {            // tiles wider than r (few: exactly)
@@ -457,34 +547,61 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
         // no groups: every tile within r1 straight from its nodes
         if (admitted(r1) && group_tiles <= 0)
             for (int n1 : kNodeCounts) {
-                double N1, N0;
-                if (n1 > 16 || !lay_out(geo, k, r1, n1, 0.0, 0, nullptr, &N1, &N0)) continue;
+                double N1;
+                if (n1 > 16 || !fine_cut(geo, k, r1, n1, &c1, &N1)) continue;
                 const double c = n_nar * T * N1 * kLeaf + n_nar * n_pix * kPix * per_node(n1) +
                                  split(n_tiles - n_nar) + 4.0 * kLaunch;
-                if (c < best.cost) { best.cost = c; best.r1 = best.r2 = r1; best.n0 = 0; best.n1 = n1; best.G = 0; }
+                if (c < best.cost) { best = Choice(); best.cost = c; best.r1 = best.r2 = r1; best.n1 = n1; }
             }
-        if (group_tiles == 0 || (group_tiles < 0 && n_tiles < 32)) continue;
-        const int G = group_tiles > 0 ? group_tiles : 4096;
-        for (double f : f2) {
-            const double r2 = std::max(f * q(0.5), r1);
-            if ((f > 1.0 && r2 == r1) || !admitted(r2)) continue;
-            double groups = 0.0;
-            for (int a : starts)
-                cut_runs(origins, tsp.data(), a, a + stretch, r1, r2, G, [&](const Run &) { groups += up; });
-            const double wide = above(r2), mid = above(r1) - wide;
+        if (!groups) continue;
+        double rads[nf2], runs[nf2], wider[nf2];     // radii, runs within them, single tiles beyond them
+        int nr = 0;
+        for (int i = 0; i < nf2; ++i) {
+            const double r = f2[i] * q(0.5);
+            if (r < r1 || !admitted(r)) continue;
+            rads[nr] = r;
+            runs[nr] = run_count[i] * n_nar / n_tiles;
+            wider[nr++] = above(r);
+        }
+        for (int i2 = 0; i2 < nr; ++i2)
             for (int n1 : kNodeCounts) {
-                if (n1 > 12) continue;
-                for (int n0 : kNodeCounts) {
-                    if (n0 < 8) continue;
-                    double N1, N0;
-                    if (!lay_out(geo, k, r2, n1, r1, n0, nullptr, &N1, &N0)) continue;
-                    const double c = n_nar * T * N0 / (n0 * n0) * leaf_terms(n0, tile_atoms) * kLeaf + mid * T * N1 * kLeaf +
-                                     n_nar * N1 * kMerge * per_node(n0) +
-                                     (groups + mid) * n_pix * kPix * per_node(n1) + split(wide) + 6.0 * kLaunch;
-                    if (c < best.cost) { best.cost = c; best.r1 = r1; best.r2 = r2; best.n0 = n0; best.n1 = n1; best.G = G; }
+                double N1, Nm, N0;
+                if (n1 > 12 || !fine_cut(geo, k, rads[i2], n1, &c1, &N1)) continue;
+                const double pixel = runs[i2] * n_pix * kPix * per_node(n1) + split(wider[i2]) + 6.0 * kLaunch;
+                const double one = T * N1 * kLeaf + n_pix * kPix * per_node(n1);     // a single tile
+                for (int im = -1; im < i2; ++im) {
+                    // im < 0: tiles straight into groups; else by runs of radius rads[im]
+                    const double single = (im < 0 ? above(r1) : wider[im]) - wider[i2];
+                    const double rest = pixel + single * one;
+                    if (rest >= best.cost) continue;
+                    for (int nm : kNodeCounts) {
+                        double part = rest, Nt = N1;
+                        if (im < 0) {
+                            if (nm != kNodeCounts[0]) break;
+                        } else {
+                            if (nm < 8 || nm > 16 || !parent_cut(geo, k, rads[im], nm, c1, &cm, &Nm)) continue;
+                            const double own = above(r1) - wider[im];
+                            part += own * T * Nm * kLeaf + (runs[im] + own) * N1 * kMerge * per_node(nm) + 2.0 * kLaunch;
+                            Nt = Nm;
+                        }
+                        if (part >= best.cost) continue;
+                        for (int n0 : kNodeCounts) {
+                            if (n0 < 8 || !parent_cut(geo, k, r1, n0, im < 0 ? c1 : cm, &c0, &N0)) continue;
+                            const double c = part + n_nar * T * N0 / (n0 * n0) * leaf_terms(n0, tile_atoms) * kLeaf +
+                                             n_nar * Nt * kMerge * per_node(n0);
+                            if (c >= best.cost) continue;
+                            best.cost = c;
+                            best.r1 = r1;
+                            best.rm = im < 0 ? 0.0 : rads[im];
+                            best.r2 = rads[i2];
+                            best.n0 = n0;
+                            best.nm = im < 0 ? 0 : nm;
+                            best.n1 = n1;
+                            best.G = G;
+                        }
+                    }
                 }
             }
-        }
     }
     plan->form_s = best.cost;
     if (!(best.cost < plan->direct_s)) {
@@ -493,13 +610,44 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
         return MK_EDECLINE;
     }
     // lay the chosen plan out
-    std::vector<MkNodeFrame> fr(n_frames), cuts(geo.size());
-    double N1, N0;
-    lay_out(geo, k, best.r2, best.n1, best.r1, best.n0, &cuts, &N1, &N0);
-    for (int f = 0; f < n_frames; ++f) fr[f] = cuts[shape_of[f]];
-    std::vector<MkNodeSrc> src;
-    std::vector<int> members, mid, wide;
-    auto add_src = [&](const double *c, int species, int count, long long first) {
+    std::vector<MkNodeFrame> fr(n_frames);
+    double nodes;
+    fine_cut(geo, k, best.r2, best.n1, &c1, &nodes);
+    if (best.nm) parent_cut(geo, k, best.rm, best.nm, c1, &cm, &nodes);
+    if (best.G) parent_cut(geo, k, best.r1, best.n0, best.nm ? cm : c1, &c0, &nodes);
+    auto level = [&](MkNodeFrame *F, int l, const Cut &C) {
+        F->ly[l] = C.ly;
+        F->lz[l] = C.lz;
+        F->py[l] = C.py;
+        F->pz[l] = C.pz;
+    };
+    auto merge = [&](MkNodeMerge *M, const Cut &C, int n_out) {     // patches of C from the finer level's
+        M->ratio_y = C.ry;
+        M->ratio_z = C.rz;
+        lay_strips(M, n_out);
+    };
+    for (int f = 0; f < n_frames; ++f) {
+        MkNodeFrame &F = fr[f];
+        const int g = shape_of[f];
+        F = MkNodeFrame{};
+        F.ny = geo[g].ny;
+        F.nz = geo[g].nz;
+        level(&F, MK_FINE, c1[g]);
+        F.bpy = (c1[g].ly + MK_PIX_COLS - 1) / MK_PIX_COLS;
+        F.bpz = (c1[g].lz + MK_PIX_ROWS - 1) / MK_PIX_ROWS;
+        if (best.G) {
+            level(&F, MK_COARSE, c0[g]);
+            merge(&F.mg[1], best.nm ? cm[g] : c0[g], best.n1);
+        }
+        if (best.nm) {
+            level(&F, MK_MIDDLE, cm[g]);
+            merge(&F.mg[0], c0[g], best.nm);
+        }
+    }
+    std::vector<MkNodeSrc> src, msrc;
+    std::vector<double4> morg;
+    std::vector<int> members, mid, wide, msingle, mrow;
+    auto source = [&](const double *c, int species, int count, long long first) {
         MkNodeSrc S{};
         for (int i = 0; i < 3; ++i) {
             S.o[i] = c[i];
@@ -509,40 +657,110 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
         S.species = species;
         S.count = count;
         S.first = first;
-        src.push_back(S);
+        return S;
     };
+    auto centre = [&](const Run &R, double *c) {
+        for (int i = 0; i < 3; ++i) c[i] = 0.5 * (R.lo[i] + R.hi[i]);
+    };
+    const double reach = best.nm ? best.rm : best.r1;       // widest tile of a group
     for (int t = 0; t < n_tiles; ++t) {
         if (rad[t] > best.r2) wide.push_back(t);
-        else if (best.G == 0 || rad[t] > best.r1) mid.push_back(t);
-        else members.push_back(t);
+        else if (best.G == 0 || rad[t] > reach) mid.push_back(t);
+        else if (rad[t] <= best.r1) members.push_back(t);
     }
-    if (best.G) {
+    if (best.nm) {
+        // runs of tiles within rm, and the tiles between r1 and rm by themselves, in
+        // the order of the curve; then groups of those
+        std::vector<Run> list;
+        long long first = 0;
+        Run R;
+        R.count = 0;
+        auto close = [&]() {
+            if (!R.count) return;
+            R.first = first;
+            first += R.count;
+            list.push_back(R);
+            R.count = 0;
+        };
+        for (int t = 0; t < n_tiles; ++t) {
+            const double *o = origins + 4ll * t;
+            if (o[3] > best.rm) continue;
+            if (o[3] > best.r1) {
+                Run S;
+                S.start(o, tsp[t]);
+                S.single = true;
+                S.first = t;
+                list.push_back(S);
+                continue;
+            }
+            if (R.count && tsp[t] == R.species && R.count < best.G && R.add(o, o, o[3], best.rm)) continue;
+            close();
+            R.start(o, tsp[t]);
+        }
+        close();
+        std::stable_sort(list.begin(), list.end(), [](const Run &a, const Run &b) { return a.species < b.species; });
+        Run Q;
+        int tiles_in = 0;
+        Q.count = 0;
+        auto emit = [&]() {
+            double c[3];
+            if (!Q.count) return;
+            centre(Q, c);
+            src.push_back(source(c, Q.species, Q.count, (long long)msrc.size() - Q.count));
+            Q.count = 0;
+        };
+        for (const Run &L : list) {
+            const int n = L.single ? 1 : L.count;
+            if (!(Q.count && L.species == Q.species && tiles_in + n <= best.G && Q.add(L.lo, L.hi, L.rmax, best.r2))) {
+                emit();
+                Q = L;
+                Q.count = 1;
+                tiles_in = 0;
+            }
+            tiles_in += n;
+            double c[3];
+            centre(L, c);
+            msrc.push_back(source(c, L.species, L.single ? 0 : L.count, L.single ? 0 : L.first));
+            morg.push_back(double4{c[0], c[1], c[2], 0.0});
+            if (L.single) {
+                msingle.push_back((int)L.first);
+                mrow.push_back((int)msrc.size() - 1);
+            }
+        }
+        emit();
+    } else if (best.G) {
         long long first = 0;
         cut_runs(origins, tsp.data(), 0, n_tiles, best.r1, best.r2, best.G, [&](const Run &R) {
-            const double c[3] = {0.5 * (R.lo[0] + R.hi[0]), 0.5 * (R.lo[1] + R.hi[1]), 0.5 * (R.lo[2] + R.hi[2])};
-            add_src(c, tsp[members[first]], R.count, first);
+            double c[3];
+            centre(R, c);
+            src.push_back(source(c, R.species, R.count, first));
             first += R.count;
         });
     }
     plan->n_groups = (int)src.size();
-    for (int t : mid) add_src(origins + 4ll * t, tsp[t], 0, 0);
+    for (int t : mid) src.push_back(source(origins + 4ll * t, tsp[t], 0, 0));
     plan->n_src = (int)src.size();
     plan->n_members = (int)members.size();
     plan->n_mid = (int)mid.size();
     plan->n_wide = (int)wide.size();
     plan->n0 = best.G ? best.n0 : 0;
+    plan->nm = best.nm;
+    plan->n_msrc = (int)msrc.size();
+    plan->n_msingle = (int)msingle.size();
     plan->n1 = best.n1;
     plan->n_frames = n_frames;
     plan->n_tiles = n_tiles;
     plan->group_tiles = best.G;
     plan->radius1_m = best.r1;
+    plan->radiusm_m = best.rm;
     plan->radius2_m = best.r2;
     plan->n_pix = (long long)n_pix;
     if (plan->n_src < 1) {
         mk_set_error("mk_nodes_plan: every tile is wider than the plan's radius");
         return MK_EDECLINE;
     }
-    long long pblk = 0, wf = 0, patch = 0, node0 = 0, item = 0;
+    const int n[3] = {plan->n0, plan->nm, plan->n1};
+    long long pblk = 0, wf = 0, patches[3] = {0, 0, 0}, item[2] = {0, 0};
     for (int f = 0; f < n_frames; ++f) {
         MkNodeFrame &F = fr[f];
         const double *t = fit + 12ll * f;
@@ -553,25 +771,28 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
             F.b[c] = beam_dirs[3ll * f + c];
         }
         F.pix_off = shapes[3 * f];
-        F.node0_off = node0;
-        F.patch1_off = patch;
         F.pblk_off = pblk;
         F.w_off = wf;
-        F.item_off = item;
-        if (best.G) {
-            lay_strips(&F, best.n1);
-            item += (long long)F.p1z * F.p0y * F.strips * F.chunks;
+        pblk += (long long)F.py[MK_FINE] * F.pz[MK_FINE] * F.bpy * F.bpz;
+        wf += (long long)best.n1 * (F.ny + F.nz);
+        for (int l = 0; l < 3; ++l) {
+            F.off[l] = patches[l];
+            patches[l] += (long long)F.py[l] * F.pz[l];
         }
-        patch += (long long)F.p1y * F.p1z;
-        node0 += best.G ? (long long)F.p0y * F.p0z * best.n0 * best.n0 : 0;
-        pblk += (long long)F.p1y * F.p1z * F.bpy * F.bpz;
-        wf += (long long)best.n1 * (F.ny + F.nz) +
-              (best.G ? (long long)best.n1 * best.n0 * (F.ratio_y + F.ratio_z) : 0);
+        for (int m = 0; m < 2; ++m) {
+            MkNodeMerge &M = F.mg[m];
+            const int in = m == 0 || !best.nm ? MK_COARSE : MK_MIDDLE, to = m == 0 ? MK_MIDDLE : MK_FINE;
+            M.w_off = wf;
+            M.item_off = item[m];
+            wf += (long long)(M.ratio_y + M.ratio_z) * n[to] * n[in];
+            item[m] += (long long)F.pz[to] * F.py[in] * M.strips * M.chunks;
+        }
     }
-    plan->nodes0 = node0;
+    const long long patch = patches[MK_FINE];
+    plan->patches0 = patches[MK_COARSE];
+    plan->patchesm = patches[MK_MIDDLE];
     plan->ns = best.G ? sub_nodes(best.n0, tile_atoms) : 0;
     if (plan->ns) {
-        plan->nodes_s = node0 / (best.n0 * best.n0) * plan->ns * plan->ns;
         plan->sub_radius_m = best.r1 * phi_max(plan->ns) / phi_max(best.n0);
         plan->sub_w_off = wf;
         wf += best.n0 * plan->ns;
@@ -589,32 +810,17 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
     plan->slices = (plan->n_src + plan->src_per_slice - 1) / plan->src_per_slice;
     for (int f = 0; f < n_frames; ++f) fr[f].part_off = fr[f].pix_off * plan->slices;
     // frames per pass: as many as a few GB of node fields and partials hold
-    const double n1sq = (double)best.n1 * best.n1;
     size_t need = 0;
-    const size_t budget = (size_t)4 << 30;
-    long long chunk_n0 = 0, chunk_p1 = 0, chunk_pix = 0, chunk_it = 0;
-    int fa = 0;
-    auto bytes = [&](long long a, long long b, long long c) {
-        return up256(8 * (size_t)(a * (long long)members.size())) +
-               up256((size_t)(8.0 * b * n1sq * plan->n_src)) + up256(16 * (size_t)c * plan->slices);
-    };
-    int passes = 1;
-    for (int f = 0; f < n_frames; ++f) {
-        const long long a = best.G ? (long long)fr[f].p0y * fr[f].p0z * best.n0 * best.n0 : 0;
-        const long long b = (long long)fr[f].p1y * fr[f].p1z, c = (long long)fr[f].ny * fr[f].nz;
-        const long long it = best.G ? (long long)fr[f].p1z * fr[f].p0y * fr[f].strips * fr[f].chunks : 0;
-        const bool too_many = (chunk_it + it) * std::max(plan->n_groups, 1) > (1ll << 30) ||
-                              (chunk_n0 + a) > 256ll * 60000 || (chunk_p1 + b) * n1sq > 256.0 * 60000;
-        if (f > fa && (bytes(chunk_n0 + a, chunk_p1 + b, chunk_pix + c) > budget || too_many)) {
-            ++passes;
-            fa = f;
-            chunk_n0 = chunk_p1 = chunk_pix = chunk_it = 0;
-        }
-        chunk_n0 += a;
-        chunk_p1 += b;
-        chunk_pix += c;
-        chunk_it += it;
-        need = std::max(need, bytes(chunk_n0, chunk_p1, chunk_pix));
+    int passes = 0;
+    for (int f = 0; f < n_frames; ++passes) {
+        Pass P;
+        f = next_pass(*plan, fr.data(), f, (size_t)4 << 30, &P);
+        need = std::max(need, P.bytes);
+        for (int l = 0; l < 3; ++l)
+            if (P.patches[l] * n[l] * n[l] > 256ll * 65535) {
+                mk_set_error("mk_nodes_plan: too many nodes in one frame");
+                return MK_EDECLINE;
+            }
     }
     plan->passes = passes;
     if (need > ((size_t)16 << 30)) {
@@ -622,7 +828,7 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
         return MK_EDECLINE;
     }
     plan->chunk_bytes = need;
-    plan->ws_bytes = up256(sizeof(MkNodeRec) * (size_t)(node0 + plan->nodes_s + patch * best.n1 * best.n1)) +
+    plan->ws_bytes = up256(sizeof(MkNodeRec) * (size_t)records(*plan)) +
                      up256(sizeof(float) * (size_t)wf) +
                      std::max(need, up256(8 * (size_t)MK_SUM_PARTS * n_frames));
     char *hb = static_cast<char *>(host_buf);
@@ -638,6 +844,10 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
     plan->off_members = put(members.data(), sizeof(int) * members.size());
     plan->off_mid = put(mid.data(), sizeof(int) * mid.size());
     plan->off_wide = put(wide.data(), sizeof(int) * wide.size());
+    plan->off_msrc = put(msrc.data(), sizeof(MkNodeSrc) * msrc.size());
+    plan->off_morg = put(morg.data(), sizeof(double4) * morg.size());
+    plan->off_msingle = put(msingle.data(), sizeof(int) * msingle.size());
+    plan->off_mrow = put(mrow.data(), sizeof(int) * mrow.size());
     plan->buf_bytes = (long long)off;
     return MK_OK;
 }
@@ -646,14 +856,11 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
 struct MkNodeArgs {
     const MkNodeFrame *frames;
     int f_lo, f_hi;                  // frames of this pass
-    int n0, n1, n_groups, n_src, src_per_slice, tile_atoms;
-    long long nodes0, patches1;      // of this pass
-    long long node0_base, patch1_base, pblk_base, part_base, item_base, items;
+    int n1, n_groups, n_src, src_per_slice, tile_atoms;
+    long long patches1, patch1_base; // fine patches of this pass, and before it
+    long long pblk_base, part_base;
     const MkNodeSrc *src;
-    const int *members;
-    const MkNodeRec *rec0, *rec1;    // of every frame
-    const float *weights;
-    float2 *V0, *V1;
+    float2 *V1;
     const double4 *origin;
     const float4 *tpos;
     const float2 *tamp;
@@ -661,13 +868,30 @@ struct MkNodeArgs {
     const float4 *u;
     const float2 *ftab;
     long long ftab_n;
+    const float *weights;
     double2 *partial;
     float kappa, fres_r;
     double kappa_d;
     int fresnel, decay;
-    const MkNodeRec *rec_s;          // eighths of tiles: node records, weights, widest radius [cycles]
-    const float *w_s;
+    const float *w_s;                // weights and widest radius [cycles] of a tile's eighths
     float sub_r;
+};
+
+// One merge: sources on n_in nodes per axis of level `in` to n_out of level
+// `to`, patches and bases of this pass.
+struct MkMergeArgs {
+    const MkNodeFrame *frames;
+    int f_lo, f_hi;
+    int step, in, to, n_out;
+    long long in_patches, in_base, to_patches, to_base, item_base, items;
+    const MkNodeSrc *src;            // the runs or groups made
+    const int *members;              // their tiles (null: sources in order)
+    const double4 *origin;
+    const MkNodeRec *rec;            // of level `to`, every frame
+    const float *weights;
+    const float2 *Vin;
+    float2 *Vout;
+    float kappa;
 };
 
 // First frame f in [lo, hi) whose key(f+1) exceeds i.
@@ -730,44 +954,40 @@ __device__ __forceinline__ float mk_lagrange(const MkCheb &C, double x, int n, i
 // well: blocks enough for a few an SM, each over several points. With all n
 // weights (and the nodes' cosines) in one thread it took 35 us on a 128 x 128
 // detector and 99 us for 16 frames; here 7 and 56 us.
-__global__ void __launch_bounds__(128) mk_node_prep_kernel(const MkNodeFrame *__restrict__ frames, int n0,
-                                                           int n1, int ns, int node_blocks, double kappa,
-                                                           const double *__restrict__ xyz,
-                                                           MkNodeRec *__restrict__ rec0,
-                                                           MkNodeRec *__restrict__ rec1,
-                                                           MkNodeRec *__restrict__ rec_s,
-                                                           float *__restrict__ weights,
-                                                           float *__restrict__ w_s)
+struct MkPrepArgs {
+    const MkNodeFrame *frames;
+    int n[4];                            // nodes per axis of the levels, and of eighths
+    MkNodeRec *rec[4];
+    int node_blocks;
+    double kappa;
+    const double *xyz;
+    float *weights, *w_s;
+};
+__global__ void __launch_bounds__(128) mk_node_prep_kernel(const MkPrepArgs A)
 {
-    __shared__ MkCheb s_c[3];              // of n0, n1 and ns
-    const int th = threadIdx.x;
-    if (th < 96) {
-        const int n = th < 32 ? n0 : (th < 64 ? n1 : ns), i = th & 31;
-        if (i < n) s_c[th >> 5].x[i] = cospi((2 * i + 1) / (2.0 * n));
+    __shared__ MkCheb s_c[4];              // of every level, and of eighths
+    const int th = threadIdx.x, mine = A.n[th >> 5], lane32 = th & 31;
+    MkCheb &C = s_c[th >> 5];
+    if (lane32 < mine) C.x[lane32] = cospi((2 * lane32 + 1) / (2.0 * mine));
+    __syncwarp();
+    if (lane32 < mine) {
+        double den = 1.0;
+        for (int i = 0; i < mine; ++i)
+            if (i != lane32) den *= C.x[lane32] - C.x[i];
+        C.inv[lane32] = 1.0 / den;
     }
     __syncthreads();
-    if (th < 96) {
-        const int n = th < 32 ? n0 : (th < 64 ? n1 : ns), j = th & 31;
-        MkCheb &C = s_c[th >> 5];
-        if (j < n) {
-            double den = 1.0;
-            for (int i = 0; i < n; ++i)
-                if (i != j) den *= C.x[j] - C.x[i];
-            C.inv[j] = 1.0 / den;
+    const MkNodeFrame &F = A.frames[blockIdx.x];
+    if ((int)blockIdx.y < A.node_blocks) {
+        int end[4], sum = 0;
+        for (int l = 0; l < 4; ++l) {
+            const int g = l == 3 ? MK_COARSE : l;
+            end[l] = sum += F.py[g] * F.pz[g] * A.n[l] * A.n[l];
         }
-    }
-    __syncthreads();
-    const MkNodeFrame &F = frames[blockIdx.x];
-    const int l0y = F.l1y * F.ratio_y, l0z = F.l1z * F.ratio_z;
-    if ((int)blockIdx.y < node_blocks) {
-        const int a0 = n0 ? F.p0y * F.p0z * n0 * n0 : 0, a1 = F.p1y * F.p1z * n1 * n1;
-        const int as = n0 ? F.p0y * F.p0z * ns * ns : 0;
-        for (int t = blockIdx.y * 128 + th; t < a0 + a1 + as; t += node_blocks * 128) {
-            const int lv = t < a0 ? 0 : (t < a0 + a1 ? 1 : 2);     // coarse, fine, eighths
-            const int e = t - (lv == 0 ? 0 : (lv == 1 ? a0 : a0 + a1));
-            const bool fine = lv == 1;
-            const int n = lv == 0 ? n0 : (fine ? n1 : ns), py = fine ? F.p1y : F.p0y;
-            const int ly = fine ? F.l1y : l0y, lz = fine ? F.l1z : l0z;
+        for (int t = blockIdx.y * 128 + th; t < sum; t += A.node_blocks * 128) {
+            const int lv = (t >= end[0]) + (t >= end[1]) + (t >= end[2]), g = lv == 3 ? MK_COARSE : lv;
+            const int e = t - (lv == 0 ? 0 : lv == 1 ? end[0] : lv == 2 ? end[1] : end[2]);
+            const int n = A.n[lv], py = F.py[g], ly = F.ly[g], lz = F.lz[g];
             const int p = e / (n * n), r = e - p * n * n, j = r / n, c = r - j * n;
             const int pz = p / py, pyi = p - pz * py;
             const double *X = s_c[lv].x;
@@ -781,7 +1001,7 @@ __global__ void __launch_bounds__(128) mk_node_prep_kernel(const MkNodeFrame *__
             const double inv = 1.0 / sqrt(r2);
             for (int d = 0; d < 3; ++d) {
                 u[d] = P[d] * inv;
-                q[d] = kappa * (F.b[d] - u[d]);
+                q[d] = A.kappa * (F.b[d] - u[d]);
             }
             const float hx = (float)q[0], hy = (float)q[1], hz = (float)q[2];
             MkNodeRec R;
@@ -789,59 +1009,64 @@ __global__ void __launch_bounds__(128) mk_node_prep_kernel(const MkNodeFrame *__
             R.u = make_float4((float)u[0], (float)u[1], (float)u[2], (float)F.b[0]);
             R.qh = make_float4(hx, hy, hz, (float)F.b[1]);
             R.ql = make_float4((float)(q[0] - hx), (float)(q[1] - hy), (float)(q[2] - hz), (float)F.b[2]);
-            if (fine) rec1[F.patch1_off * n1 * n1 + e] = R;
-            else if (lv == 0) rec0[F.node0_off + e] = R;
-            else rec_s[F.node0_off / (n0 * n0) * (ns * ns) + e] = R;
+            A.rec[lv][F.off[g] * n * n + e] = R;
         }
         return;
     }
-    // points: pixel columns and rows in their fine patches, fine nodes in the
-    // coarse patch, and (frame 0) a tile's nodes among its eighths'
-    const int wp = F.ny + F.nz, wm = n0 ? (F.ratio_y + F.ratio_z) * n1 : 0;
-    const int points = wp + wm + (blockIdx.x == 0 && ns ? n0 : 0);
-    const int width = max(max(n0, n1), ns) > 16 ? 32 : 16, lane = th & (width - 1), per = 128 / width;
-    const int step = (gridDim.y - node_blocks) * per;
-    float *W = weights + F.w_off;
+    // points: pixel columns and rows in their fine patches, the nodes of a finer
+    // level in a patch of the coarser one, and (frame 0) a tile's nodes among its
+    // eighths'
+    const MkNodeMerge &M1 = F.mg[1], &M0 = F.mg[0];
+    const int above = A.n[MK_MIDDLE] ? MK_MIDDLE : MK_COARSE;
+    const int e0 = F.ny + F.nz, e1 = e0 + (A.n[0] ? (M1.ratio_y + M1.ratio_z) * A.n[MK_FINE] : 0);
+    const int e2 = e1 + (A.n[MK_MIDDLE] ? (M0.ratio_y + M0.ratio_z) * A.n[MK_MIDDLE] : 0);
+    const int points = e2 + (blockIdx.x == 0 && A.n[3] ? A.n[0] : 0);
+    const int width = max(max(A.n[0], A.n[1]), max(A.n[2], A.n[3])) > 16 ? 32 : 16, lane = th & (width - 1);
+    const int per = 128 / width, step = (gridDim.y - A.node_blocks) * per;
     // whole warps stay in the loop: the lanes of a warp's groups shuffle together
-    for (int i0 = (blockIdx.y - node_blocks) * per + (th >> 5) * (32 / width); i0 < points; i0 += step) {
+    for (int i0 = (blockIdx.y - A.node_blocks) * per + (th >> 5) * (32 / width); i0 < points; i0 += step) {
         const int at = i0 + (th & 31) / width, i = min(at, points - 1);
         double x;
         float *out;
-        int lv = 1;
-        if (i < wp) {
+        int lv = MK_FINE;
+        if (i < e0) {
             const bool row = i >= F.ny;
-            const int k = row ? i - F.ny : i, len = row ? F.l1z : F.l1y;
-            const double *P = xyz + 3 * (F.pix_off + (row ? (long long)k * F.ny : k));
+            const int k = row ? i - F.ny : i, len = row ? F.lz[MK_FINE] : F.ly[MK_FINE];
+            const double *P = A.xyz + 3 * (F.pix_off + (row ? (long long)k * F.ny : k));
             const double v = mk_axis_coord(P, F.p0, row ? F.ez : F.ey, mk_axis_inv(row ? F.ez : F.ey));
             x = (v - ((k / len) * (double)len + 0.5 * (len - 1))) / mk_half_range(len);
-            out = W + (long long)i * n1;
-        } else if (i < wp + wm) {
-            const int m = i - wp;
-            const bool row = m >= F.ratio_y * n1;
-            const int k = row ? m - F.ratio_y * n1 : m;
-            const int l1 = row ? F.l1z : F.l1y, l0 = row ? l0z : l0y;
-            const int sub = k / n1, c = k - sub * n1;
-            const double v = sub * (double)l1 + 0.5 * (l1 - 1) + mk_half_range(l1) * s_c[1].x[c];
+            out = A.weights + F.w_off + (long long)i * A.n[MK_FINE];
+        } else if (i < e2) {
+            const bool low = i < e1;             // into the fine patches
+            const MkNodeMerge &M = low ? M1 : M0;
+            const int m = i - (low ? e0 : e1), to = low ? MK_FINE : MK_MIDDLE, n_to = A.n[to];
+            lv = low ? above : MK_COARSE;
+            const bool row = m >= M.ratio_y * n_to;
+            const int k = row ? m - M.ratio_y * n_to : m;
+            const int l1 = row ? F.lz[to] : F.ly[to], l0 = row ? F.lz[lv] : F.ly[lv];
+            const int sub = k / n_to, c = k - sub * n_to;
+            const double v = sub * (double)l1 + 0.5 * (l1 - 1) + mk_half_range(l1) * s_c[to].x[c];
             x = (v - 0.5 * (l0 - 1)) / mk_half_range(l0);
-            out = W + (long long)wp * n1 + (long long)m * n0;
-            lv = 0;
+            out = A.weights + M.w_off + (long long)m * A.n[lv];
         } else {
-            x = s_c[0].x[i - wp - wm];
-            out = w_s + (i - wp - wm) * ns;
-            lv = 2;
+            x = s_c[MK_COARSE].x[i - e2];
+            out = A.w_s + (i - e2) * A.n[3];
+            lv = 3;
         }
-        const int n = lv == 0 ? n0 : (lv == 1 ? n1 : ns);
+        const int n = A.n[lv];
         const float w = mk_lagrange(s_c[lv], x, n, lane, width);
         if (lane < n && at < points) out[lane] = w;
     }
 }
 
-// A tile's field on the nodes: V[list position][node]. One node a thread,
+// A tile's field on the nodes: V[rows[list position]][node] (rows null: the list
+// position). One node a thread,
 // the tile's atoms (interleaved pairs) from shared memory, two atoms per
 // packed instruction. Bound by the MUFU (two results a term, 16 per clock
 // and SM); the phase is always reduced mod 1, so __sincosf stays at its
 // 3.5e-7 absolute error.
 __global__ void __launch_bounds__(256) mk_node_leaf_kernel(const MkNodeArgs A, const int *__restrict__ list,
+                                                           const int *__restrict__ rows,
                                                            const MkNodeRec *__restrict__ rec,
                                                            long long n_nodes, float2 *__restrict__ V)
 {
@@ -894,7 +1119,7 @@ __global__ void __launch_bounds__(256) mk_node_leaf_kernel(const MkNodeArgs A, c
         ai = f2_fma(e.x, s, f2_fma(e.y, c, ai));
     }
     const float2 r2 = f2_unpack(ar), i2 = f2_unpack(ai);
-    V[(long long)blockIdx.x * n_nodes + g] = make_float2(mk_unshort(r2.x + r2.y), mk_unshort(i2.x + i2.y));
+    V[(long long)(rows ? rows[blockIdx.x] : (int)blockIdx.x) * n_nodes + g] = make_float2(mk_unshort(r2.x + r2.y), mk_unshort(i2.x + i2.y));
 }
 
 // A tile's field on its coarse nodes by way of its eighths (64 atoms, a
@@ -1122,7 +1347,7 @@ __device__ __forceinline__ void mk_stage_fields(float2 (*s_v)[N * N], const floa
 // 16 on the 512 x 512 one; here 2.34 and 0.70 ms (4.5 and 5.2 ps a (tile, fine
 // node)).
 template <int N0, int ROWS>
-__global__ void __launch_bounds__(MK_MERGE_NT) mk_node_merge_kernel(const MkNodeArgs A)
+__global__ void __launch_bounds__(MK_MERGE_NT) mk_node_merge_kernel(const MkMergeArgs A)
 {
     constexpr int MAXR = 16;                 // rows of a block at most
     __shared__ __align__(16) float2 s_v[2][MK_NODE_SB][N0 * N0];
@@ -1131,38 +1356,41 @@ __global__ void __launch_bounds__(MK_MERGE_NT) mk_node_merge_kernel(const MkNode
     __shared__ __align__(16) float s_d[2][MK_NODE_SB][8];
     const long long it = A.item_base + blockIdx.x % A.items;
     const int grp = (int)(blockIdx.x / A.items);
-    const int n1 = A.n1;
-    const int f = mk_find_frame(A.f_lo, A.f_hi, it, [&](int i) { return A.frames[i].item_off; });
+    const int n1 = A.n_out;
+    const int f = mk_find_frame(A.f_lo, A.f_hi, it, [&](int i) { return A.frames[i].mg[A.step].item_off; });
     const MkNodeFrame &F = A.frames[f];
-    int e = (int)(it - F.item_off);
-    const int chunk = e % F.chunks;
-    e /= F.chunks;
-    const int strip = e % F.strips;
-    e /= F.strips;
-    const int cy = e % F.p0y, pz = e / F.p0y;
-    const int suby0 = strip * F.strip;
-    const int patches = min(min(F.strip, F.ratio_y - suby0), F.p1y - (cy * F.ratio_y + suby0));
+    const MkNodeMerge &M = F.mg[A.step];
+    int e = (int)(it - M.item_off);
+    const int chunk = e % M.chunks;
+    e /= M.chunks;
+    const int strip = e % M.strips;
+    e /= M.strips;
+    const int p0y = F.py[A.in], p1y = F.py[A.to];
+    const int cy = e % p0y, pz = e / p0y;
+    const int suby0 = strip * M.strip;
+    const int patches = min(min(M.strip, M.ratio_y - suby0), p1y - (cy * M.ratio_y + suby0));
     if (patches <= 0) return;                // a last coarse patch with fewer fine ones
-    const int width = F.strip * n1;          // node columns of a full strip
-    const int cz = pz / F.ratio_z, subz = pz - cz * F.ratio_z;
-    const int rows = F.rowg * ROWS, row0 = chunk * rows;      // rows of this block
-    const float *W = A.weights + F.w_off + (long long)n1 * (F.ny + F.nz);
-    const float *Wy = W + (long long)suby0 * n1 * N0, *Wz = W + (F.ratio_y + subz) * n1 * N0;
+    const int width = M.strip * n1;          // node columns of a full strip
+    const int cz = pz / M.ratio_z, subz = pz - cz * M.ratio_z;
+    const int rows = M.rowg * ROWS, row0 = chunk * rows;      // rows of this block
+    const float *W = A.weights + M.w_off;
+    const float *Wy = W + (long long)suby0 * n1 * N0, *Wz = W + (M.ratio_y + subz) * n1 * N0;
     const int nrow = min(rows, n1 - row0);
     for (int i = threadIdx.x; i < nrow * N0; i += MK_MERGE_NT) s_wz[i / N0][i % N0] = Wz[row0 * N0 + i];
     const int rg = threadIdx.x / width, oc = threadIdx.x - rg * width;
-    const bool live = oc < patches * n1 && rg * ROWS < nrow && rg < F.rowg;
+    const bool live = oc < patches * n1 && rg * ROWS < nrow && rg < M.rowg;
     const int oc1 = live ? oc : 0, lr = live ? rg * ROWS : 0;
     mk_f2 wy[N0];
 #pragma unroll
     for (int i = 0; i < N0; ++i) wy[i] = f2_splat(Wy[oc1 * N0 + i]);
     const MkNodeSrc &S = A.src[grp];
+    if (S.count == 0) return;                // a single tile: its leaf wrote its row
     const double gx = S.o[0], gy = S.o[1], gz = S.o[2];
     // the thread's nodes: patch of its column, rows lr .. lr + ROWS - 1
-    const int py = cy * F.ratio_y + suby0 + oc1 / n1;
-    const long long node = (F.patch1_off - A.patch1_base + (long long)pz * F.p1y + py) * n1 * n1 +
+    const int py = cy * M.ratio_y + suby0 + oc1 / n1;
+    const long long node = (F.off[A.to] - A.to_base + (long long)pz * p1y + py) * n1 * n1 +
                            (row0 + lr) * n1 + oc1 % n1;
-    const MkNodeRec *rec = A.rec1 + A.patch1_base * n1 * n1 + node;
+    const MkNodeRec *rec = A.rec + A.to_base * n1 * n1 + node;
     float3 qh[ROWS], ql[ROWS], u[ROWS];
     float half[ROWS], accr[ROWS], acci[ROWS], cr[ROWS], ci[ROWS];
 #pragma unroll
@@ -1178,15 +1406,16 @@ __global__ void __launch_bounds__(MK_MERGE_NT) mk_node_merge_kernel(const MkNode
         half[r] = 0.5f * kr / fmaf(-uo, R.w.w, 1.f);
         accr[r] = acci[r] = cr[r] = ci[r] = 0.f;
     }
-    const float2 *V = A.V0 + (F.node0_off - A.node0_base) + (long long)(cz * F.p0y + cy) * N0 * N0;
+    const float2 *V = A.Vin + (F.off[A.in] - A.in_base + cz * p0y + cy) * N0 * N0;
     const long long first = S.first;
     const int count = S.count;
     auto stage = [&](int s0, int buf) {
         const int m = min(MK_NODE_SB, count - s0);
-        mk_stage_fields<N0>(s_v[buf], V, A.nodes0, first + s0, m);
+        mk_stage_fields<N0>(s_v[buf], V, A.in_patches * N0 * N0, first + s0, m);
         mk_cp_commit();
         if ((int)threadIdx.x < m) {
-            const double4 o = A.origin[A.members[first + s0 + threadIdx.x]];
+            const long long j = first + s0 + threadIdx.x;
+            const double4 o = A.origin[A.members ? A.members[j] : j];
             const double d[3] = {o.x - gx, o.y - gy, o.z - gz};
             float *sd = s_d[buf][threadIdx.x], dd = 0.f;
 #pragma unroll
@@ -1247,7 +1476,7 @@ __global__ void __launch_bounds__(MK_MERGE_NT) mk_node_merge_kernel(const MkNode
         __syncthreads();        // s_d and s_t are read; the next step may stage
     }
     if (live) {
-        float2 *out = A.V1 + (long long)grp * (A.patches1 * n1 * n1) + node;
+        float2 *out = A.Vout + (long long)grp * (A.to_patches * n1 * n1) + node;
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) out[r * n1] = make_float2(mk_unshort(accr[r] - cr[r]), mk_unshort(acci[r] - ci[r]));
     }
@@ -1268,12 +1497,13 @@ __global__ void __launch_bounds__(128) mk_node_pixels_kernel(const MkNodeArgs A)
     const MkNodeFrame &F = A.frames[f];
     const int per = F.bpy * F.bpz;
     const int lb = (int)(blk - F.pblk_off), lp = lb / per, sub = lb - lp * per;
-    const int pz = lp / F.p1y, py = lp - pz * F.p1y, bz = sub / F.bpy, by = sub - bz * F.bpy;
+    const int p1y = F.py[MK_FINE], l1y = F.ly[MK_FINE], l1z = F.lz[MK_FINE];
+    const int pz = lp / p1y, py = lp - pz * p1y, bz = sub / F.bpy, by = sub - bz * F.bpy;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int col_end = min((py + 1) * F.l1y, F.ny), row_end = min((pz + 1) * F.l1z, F.nz);
-    const int col = py * F.l1y + by * MK_PIX_COLS + lane;
-    const int row0 = pz * F.l1z + bz * MK_PIX_ROWS;
-    if (row0 >= row_end || py * F.l1y + by * MK_PIX_COLS >= col_end) return;   // whole block outside
+    const int col_end = min((py + 1) * l1y, F.ny), row_end = min((pz + 1) * l1z, F.nz);
+    const int col = py * l1y + by * MK_PIX_COLS + lane;
+    const int row0 = pz * l1z + bz * MK_PIX_ROWS;
+    if (row0 >= row_end || py * l1y + by * MK_PIX_COLS >= col_end) return;   // whole block outside
     const float *Wy = A.weights + F.w_off, *Wz = Wy + (long long)N * F.ny;
     for (int i = threadIdx.x; i < MK_PIX_ROWS * N; i += blockDim.x)
         s_wz[i / N][i % N] = Wz[(long long)min(row0 + i / N, row_end - 1) * N + i % N];
@@ -1298,7 +1528,7 @@ __global__ void __launch_bounds__(128) mk_node_pixels_kernel(const MkNodeArgs A)
     }
     const int s_lo = blockIdx.y * A.src_per_slice, s_hi = min(A.n_src, s_lo + A.src_per_slice);
     const long long ld = A.patches1 * N * N;
-    const float2 *V = A.V1 + (F.patch1_off - A.patch1_base + lp) * N * N;
+    const float2 *V = A.V1 + (F.off[MK_FINE] - A.patch1_base + lp) * N * N;
     int species = A.src[s_lo].species;
     auto flush = [&](int s) {
 #pragma unroll
@@ -1499,13 +1729,26 @@ static void mk_launch_pixels(const MkNodeArgs &A, dim3 grid, cudaStream_t st)
     mk_node_pixels_kernel<N><<<grid, 128, 0, st>>>(A);
 }
 template <int N>
-static void mk_launch_merge(const MkNodeArgs &A, unsigned grid, cudaStream_t st)
+static void mk_launch_merge(const MkMergeArgs &A, unsigned grid, cudaStream_t st)
 {
-    switch (merge_rows(A.n1)) {
+    switch (merge_rows(A.n_out)) {
     case 3: mk_node_merge_kernel<N, 3><<<grid, MK_MERGE_NT, 0, st>>>(A); break;
     case 4: mk_node_merge_kernel<N, 4><<<grid, MK_MERGE_NT, 0, st>>>(A); break;
     default: mk_node_merge_kernel<N, 5><<<grid, MK_MERGE_NT, 0, st>>>(A); break;
     }
+}
+static int mk_merge(const MkMergeArgs &A, int n_in, int n_runs, cudaStream_t st)
+{
+    const unsigned grid = (unsigned)(A.items * n_runs);
+    switch (n_in) {
+    case 8: mk_launch_merge<8>(A, grid, st); break;
+    case 10: mk_launch_merge<10>(A, grid, st); break;
+    case 12: mk_launch_merge<12>(A, grid, st); break;
+    case 16: mk_launch_merge<16>(A, grid, st); break;
+    case 20: mk_launch_merge<20>(A, grid, st); break;
+    default: mk_set_error("mk_kin_nodes_f32: %d nodes to merge", n_in); return MK_EINVAL;
+    }
+    return MK_OK;
 }
 
 template <int N0, int NS>
@@ -1541,7 +1784,7 @@ extern "C" int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, c
         mk_set_error("mk_kin_nodes_f32: workspace %zu bytes, need %lld", ws_bytes, plan->ws_bytes);
         return MK_ENOMEM;
     }
-    const int n0 = plan->n0, n1 = plan->n1, T = tiles->tile_atoms;
+    const int n0 = plan->n0, nm = plan->nm, n1 = plan->n1, ns = plan->ns, T = tiles->tile_atoms;
     const MkNodeFrame *hf = static_cast<const MkNodeFrame *>(host_buf);
     const char *db = static_cast<const char *>(dev_buf);
     cudaStream_t st = mk_stream(stream);
@@ -1549,22 +1792,28 @@ extern "C" int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, c
     memset(&A, 0, sizeof(A));
     A.frames = reinterpret_cast<const MkNodeFrame *>(db);
     A.src = reinterpret_cast<const MkNodeSrc *>(db + plan->off_src);
-    A.members = reinterpret_cast<const int *>(db + plan->off_members);
+    const int *members = reinterpret_cast<const int *>(db + plan->off_members);
     const int *mid = reinterpret_cast<const int *>(db + plan->off_mid);
     char *w = static_cast<char *>(workspace);
-    MkNodeRec *rec0 = reinterpret_cast<MkNodeRec *>(w);
-    MkNodeRec *rec1 = rec0 + plan->nodes0;
-    MkNodeRec *rec_s = rec1 + plan->patches1 * n1 * n1;
-    w += up256(sizeof(MkNodeRec) * (size_t)(plan->nodes0 + plan->nodes_s + plan->patches1 * n1 * n1));
+    MkPrepArgs prep;
+    memset(&prep, 0, sizeof(prep));
+    prep.frames = A.frames;
+    prep.n[MK_COARSE] = n0;
+    prep.n[MK_MIDDLE] = nm;
+    prep.n[MK_FINE] = n1;
+    prep.n[3] = ns;
+    MkNodeRec *rec[4];
+    rec[0] = reinterpret_cast<MkNodeRec *>(w);
+    rec[1] = rec[0] + plan->patches0 * n0 * n0;
+    rec[2] = rec[1] + plan->patchesm * nm * nm;
+    rec[3] = rec[2] + plan->patches1 * n1 * n1;
+    for (int l = 0; l < 4; ++l) prep.rec[l] = rec[l];
+    w += up256(sizeof(MkNodeRec) * (size_t)records(*plan));
     float *weights = reinterpret_cast<float *>(w);
     w += up256(sizeof(float) * (size_t)plan->weights);
-    A.rec0 = rec0;
-    A.rec1 = rec1;
     A.weights = weights;
-    A.rec_s = rec_s;
     A.w_s = weights + plan->sub_w_off;
     A.sub_r = (float)(plan->sub_radius_m * phys->k / MK_TWO_PI);
-    A.n0 = n0;
     A.n1 = n1;
     A.n_groups = plan->n_groups;
     A.n_src = plan->n_src;
@@ -1586,87 +1835,110 @@ extern "C" int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, c
     int nodes = 0, points = 0;             // of the largest frame
     for (int f = 0; f < plan->n_frames; ++f) {
         const MkNodeFrame &F = hf[f];
-        nodes = std::max(nodes, (n0 ? F.p0y * F.p0z * (n0 * n0 + plan->ns * plan->ns) : 0) + F.p1y * F.p1z * n1 * n1);
-        points = std::max(points, F.ny + F.nz + (n0 ? (F.ratio_y + F.ratio_z) * n1 + n0 : 0));
+        nodes = std::max(nodes, F.py[0] * F.pz[0] * (n0 * n0 + ns * ns) + F.py[1] * F.pz[1] * nm * nm +
+                                    F.py[2] * F.pz[2] * n1 * n1);
+        points = std::max(points, F.ny + F.nz + n0 + (F.mg[1].ratio_y + F.mg[1].ratio_z) * n1 +
+                                      (F.mg[0].ratio_y + F.mg[0].ratio_z) * nm);
     }
     const int most = std::max(1, 1216 / plan->n_frames);
-    const int node_blocks = std::min((nodes + 127) / 128, most), point_blocks = std::min((points + 3) / 4, most);
-    mk_node_prep_kernel<<<dim3(plan->n_frames, node_blocks + point_blocks), 128, 0, st>>>(
-        A.frames, n0, n1, plan->ns, node_blocks, A.kappa_d, px->xyz, rec0, rec1, rec_s, weights,
-        weights + plan->sub_w_off);
+    prep.node_blocks = std::min((nodes + 127) / 128, most);
+    prep.kappa = A.kappa_d;
+    prep.xyz = px->xyz;
+    prep.weights = weights;
+    prep.w_s = weights + plan->sub_w_off;
+    mk_node_prep_kernel<<<dim3(plan->n_frames, prep.node_blocks + std::min((points + 3) / 4, most)), 128, 0, st>>>(
+        prep);
     MK_CHECK_CUDA(cudaGetLastError());
     const size_t leaf_smem = (size_t)T * 24;
     MK_CHECK_CUDA(cudaFuncSetAttribute((const void *)mk_node_leaf_kernel,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)leaf_smem));
-    auto leaf = [&](const int *list, int n_list, const MkNodeRec *rec, long long nodes, float2 *V) {
+    auto leaf = [&](const int *list, const int *rows, int n_list, const MkNodeRec *rec, long long nodes, float2 *V) {
         const int th = (int)std::min<long long>(256, (nodes + 31) / 32 * 32);
         mk_node_leaf_kernel<<<dim3(n_list, (unsigned)((nodes + th - 1) / th)), th, leaf_smem, st>>>(
-            A, list, rec, nodes, V);
+            A, list, rows, rec, nodes, V);
     };
     // passes of whole frames whose node fields and partials fit the chunk
     const size_t budget = std::max((size_t)plan->chunk_bytes, (size_t)1);
     for (int fa = 0; fa < plan->n_frames;) {
-        long long a = 0, b = 0, c = 0, pb = 0, items = 0;
-        int fb = fa;
-        auto bytes = [&](long long x, long long y, long long z) {
-            return up256(8 * (size_t)(x * plan->n_members)) +
-                   up256((size_t)(8.0 * y * (double)(n1 * n1) * plan->n_src)) + up256(16 * (size_t)z * plan->slices);
-        };
-        while (fb < plan->n_frames) {
-            const MkNodeFrame &F = hf[fb];
-            const long long da = n0 ? (long long)F.p0y * F.p0z * n0 * n0 : 0;
-            const long long dp = (long long)F.p1y * F.p1z, dc = (long long)F.ny * F.nz;
-            const long long di = n0 ? (long long)F.p1z * F.p0y * F.strips * F.chunks : 0;
-            const bool too_many = (items + di) * std::max(plan->n_groups, 1) > (1ll << 30) ||
-                                  (a + da) > 256ll * 60000 || (b + dp) * (double)(n1 * n1) > 256.0 * 60000;
-            if (fb > fa && (bytes(a + da, b + dp, c + dc) > budget || too_many)) break;
-            a += da;
-            b += dp;
-            c += dc;
-            pb += dp * F.bpy * F.bpz;
-            items += di;
-            ++fb;
-        }
+        Pass P;
+        const int fb = next_pass(*plan, hf, fa, budget, &P);
+        const MkNodeFrame &F = hf[fa];
         A.f_lo = fa;
         A.f_hi = fb;
-        A.nodes0 = a;
-        A.patches1 = b;
-        A.node0_base = hf[fa].node0_off;
-        A.patch1_base = hf[fa].patch1_off;
-        A.pblk_base = hf[fa].pblk_off;
-        A.item_base = hf[fa].item_off;
-        A.items = items;
-        A.part_base = hf[fa].part_off;
+        A.patches1 = P.patches[MK_FINE];
+        A.patch1_base = F.off[MK_FINE];
+        A.pblk_base = F.pblk_off;
+        A.part_base = F.part_off;
+        float2 *V[3];
         char *cw = w;
-        A.V0 = reinterpret_cast<float2 *>(cw);
-        cw += up256(8 * (size_t)(a * plan->n_members));
-        A.V1 = reinterpret_cast<float2 *>(cw);
-        cw += up256((size_t)(8.0 * b * (double)(n1 * n1) * plan->n_src));
+        for (int l = 0; l < 3; ++l) {
+            V[l] = reinterpret_cast<float2 *>(cw);
+            cw += P.field[l];
+        }
+        A.V1 = V[MK_FINE];
         A.partial = reinterpret_cast<double2 *>(cw);
         if (plan->n_members > 0) {
-            const MkNodeRec *rs = plan->ns ? rec_s + A.node0_base / (n0 * n0) * plan->ns * plan->ns : nullptr;
+            const long long nodes0 = P.patches[MK_COARSE] * n0 * n0;
+            const MkNodeRec *r0 = rec[MK_COARSE] + F.off[MK_COARSE] * n0 * n0, *rs = rec[3] + F.off[MK_COARSE] * ns * ns;
             int rc = MK_OK;
-            if (plan->ns == 14 && n0 == 20)
-                rc = mk_launch_leaf8<20, 14>(A, A.members, plan->n_members, rec0 + A.node0_base, rs, a, A.V0, st);
-            else if (plan->ns == 12 && n0 == 16)
-                rc = mk_launch_leaf8<16, 12>(A, A.members, plan->n_members, rec0 + A.node0_base, rs, a, A.V0, st);
+            if (ns == 14 && n0 == 20)
+                rc = mk_launch_leaf8<20, 14>(A, members, plan->n_members, r0, rs, nodes0, V[0], st);
+            else if (ns == 12 && n0 == 16)
+                rc = mk_launch_leaf8<16, 12>(A, members, plan->n_members, r0, rs, nodes0, V[0], st);
             else
-                leaf(A.members, plan->n_members, rec0 + A.node0_base, a, A.V0);
+                leaf(members, nullptr, plan->n_members, r0, nodes0, V[0]);
             if (rc != MK_OK) return rc;
-            const unsigned grid = (unsigned)(items * plan->n_groups);
-            switch (n0) {
-            case 8: mk_launch_merge<8>(A, grid, st); break;
-            case 10: mk_launch_merge<10>(A, grid, st); break;
-            case 12: mk_launch_merge<12>(A, grid, st); break;
-            case 16: mk_launch_merge<16>(A, grid, st); break;
-            case 20: mk_launch_merge<20>(A, grid, st); break;
-            default: mk_set_error("mk_kin_nodes_f32: %d coarse nodes", n0); return MK_EINVAL;
-            }
+        }
+        if (plan->n_msingle > 0)
+            leaf(reinterpret_cast<const int *>(db + plan->off_msingle), reinterpret_cast<const int *>(db + plan->off_mrow),
+                 plan->n_msingle, rec[MK_MIDDLE] + F.off[MK_MIDDLE] * nm * nm, P.patches[MK_MIDDLE] * nm * nm,
+                 V[MK_MIDDLE]);
+        MkMergeArgs G;
+        memset(&G, 0, sizeof(G));
+        G.frames = A.frames;
+        G.f_lo = fa;
+        G.f_hi = fb;
+        G.weights = weights;
+        G.kappa = A.kappa;
+        auto merge = [&](int step, int in, int to, int n_runs) {
+            G.step = step;
+            G.in = in;
+            G.to = to;
+            G.n_out = prep.n[to];
+            G.in_patches = P.patches[in];
+            G.in_base = F.off[in];
+            G.to_patches = P.patches[to];
+            G.to_base = F.off[to];
+            G.item_base = F.mg[step].item_off;
+            G.items = P.items[step];
+            G.rec = rec[to];
+            G.Vin = V[in];
+            G.Vout = V[to];
+            return mk_merge(G, prep.n[in], n_runs, st);
+        };
+        if (nm) {
+            // runs of no tiles (single ones) hold the leaf's field already
+            G.src = reinterpret_cast<const MkNodeSrc *>(db + plan->off_msrc);
+            G.members = members;
+            G.origin = A.origin;
+            int rc = merge(0, MK_COARSE, MK_MIDDLE, plan->n_msrc);
+            if (rc != MK_OK) return rc;
+            G.src = A.src;
+            G.members = nullptr;
+            G.origin = reinterpret_cast<const double4 *>(db + plan->off_morg);
+            rc = merge(1, MK_MIDDLE, MK_FINE, plan->n_groups);
+            if (rc != MK_OK) return rc;
+        } else if (plan->n_groups > 0) {
+            G.src = A.src;
+            G.members = members;
+            G.origin = A.origin;
+            const int rc = merge(1, MK_COARSE, MK_FINE, plan->n_groups);
+            if (rc != MK_OK) return rc;
         }
         if (plan->n_mid > 0)
-            leaf(mid, plan->n_mid, rec1 + A.patch1_base * n1 * n1, b * n1 * n1,
-                 A.V1 + (long long)plan->n_groups * b * n1 * n1);
-        const dim3 grid((unsigned)pb, plan->slices);
+            leaf(mid, nullptr, plan->n_mid, rec[MK_FINE] + A.patch1_base * n1 * n1, A.patches1 * n1 * n1,
+                 A.V1 + (long long)plan->n_groups * A.patches1 * n1 * n1);
+        const dim3 grid((unsigned)P.pblk, plan->slices);
         switch (n1) {
         case 6: mk_launch_pixels<6>(A, grid, st); break;
         case 8: mk_launch_pixels<8>(A, grid, st); break;
@@ -1675,8 +1947,8 @@ extern "C" int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, c
         case 16: mk_launch_pixels<16>(A, grid, st); break;
         default: mk_set_error("mk_kin_nodes_f32: %d nodes", n1); return MK_EINVAL;
         }
-        mk_node_reduce_kernel<<<(unsigned)((c + 255) / 256), 256, 0, st>>>(
-            A.frames, fa, fb, hf[fa].pix_off, c, plan->slices, A.part_base, A.partial,
+        mk_node_reduce_kernel<<<(unsigned)((P.pix + 255) / 256), 256, 0, st>>>(
+            A.frames, fa, fb, hf[fa].pix_off, P.pix, plan->slices, A.part_base, A.partial,
             reinterpret_cast<const double2 *>(px->phasor), reinterpret_cast<double2 *>(out), accumulate);
         MK_CHECK_CUDA(cudaGetLastError());
         fa = fb;

@@ -107,6 +107,35 @@ def test_leaf_by_eighths_matches_fp64_and_split(cuda, cells, dilute, shape, dist
     assert rel_max(got, one) <= 2e-5, rel_max(got, one)
 
 
+@pytest.mark.parametrize("cells, dilute, tile, shape, dist", [
+    (28, 0.01, 256, (256, 256), 0.2e10),
+    (24, 0.0, 512, (301, 187), 0.2e10),
+    (24, 0.0, 128, (256, 256), 0.1e10),     # tiles on the fine nodes and wide ones too
+])
+def test_middle_level_matches_fp64_and_split(cuda, cells, dilute, tile, shape, dist):
+    """Tiles merged into runs on middle nodes, single tiles among them, and
+    those into groups."""
+    w, sample = _case(cells, dilute=dilute)
+    B = workloads._beam(10000.0, 200.0, pol_perp_rate=1.0)
+    st = StaticStage(w.stage.rotation, w.stage.translation)
+    D = _det(w, shape, dist)
+    phys = B.physics(apply_polarization=True)
+    atoms = B.stage_atoms(sample, st, device=cuda)
+    pix = engine.Pixels(np.asarray(D.pixel_coordinates) / 1e10, *shape, phys, device=cuda)
+    tiles = engine.Tiles(atoms, B.k, tile, device=cuda)
+    plan = engine.NodePlan.make(tiles, pix, B.k, (1.0, 0.0, 0.0), 1e-6, direct=1.0)
+    assert plan is not None and plan.plan.nm > 0 and plan.plan.n_msingle > 0
+    acc = torch.full((pix.n, 2), float("nan"), dtype=torch.float64, device=cuda)
+    wide = plan.wide is not None
+    if wide:
+        engine.run_split(plan.wide, pix, phys, atoms.table, fresnel=1, out=acc, factor_table=True)
+    got = _c(engine.run_nodes(plan, tiles, pix, phys, atoms.table, out=acc, accumulate=wide, fresnel=1), shape)
+    one = _c(engine.run_split(tiles, pix, phys, atoms.table, fresnel=1), shape)
+    ref = _c(engine.run_plain(atoms, pix, phys), shape)
+    assert rel_intensity(got, ref) <= 1e-4, rel_intensity(got, ref)
+    assert rel_max(got, one) <= 2e-5, rel_max(got, one)
+
+
 def test_entry_point_takes_nodes_where_admitted(cuda):
     """Large enough on a plane detector: nodes; a curved (shell) detector,
     an explicit launch, remove_forward and a Darwin analyser: the other forms,

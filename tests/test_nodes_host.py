@@ -2,10 +2,10 @@
 the kernels' index arithmetic: leaf, merge and pixel steps over the plan's own
 tables, every array access in range, against the direct sum.
 
-Tolerance: the plan interpolates with 4 (phi/2)^n / n! <= 3e-8 per axis and
-step; two axes, at most two steps and Lebesgue constants below 2.8 give
-3e-8 * (1 + 2.8) * (1 + 2.8^2) < 1.1e-6 of the sum of |E| at worst; the
-dropped third-order phase is below 1e-6 rad."""
+Tolerance: the plan interpolates with e = 4 (phi/2)^n / n! <= 3e-8 per axis
+and step; two axes and Lebesgue constants L below 2.8 give e (1 + L) (1 + L^2)
+< 1.1e-6 of the sum of |E| at worst for two steps, e (1 + L) (1 + L^2 + L^4)
+< 8.0e-6 for three; the dropped third-order phase is below 1e-6 rad."""
 import ctypes
 
 import numpy as np
@@ -14,10 +14,11 @@ import pytest
 from mosaic_gb300 import _lib
 
 K = 2 * np.pi / 1.2398e-10
-FRAME = np.dtype([("p0", "f8", 3), ("ey", "f8", 3), ("ez", "f8", 3), ("b", "f8", 3)] +
-                 [(n, "i4") for n in ("ny", "nz", "l1y", "l1z", "p1y", "p1z", "ratio_y", "ratio_z",
-                                      "p0y", "p0z", "bpy", "bpz", "strip", "strips", "rowg", "chunks")] +
-                 [(n, "i8") for n in ("pix_off", "node0_off", "patch1_off", "pblk_off", "part_off", "w_off", "item_off")])
+MERGE = np.dtype([(n, "i4") for n in ("ratio_y", "ratio_z", "strip", "strips", "rowg", "chunks")] +
+                 [(n, "i8") for n in ("w_off", "item_off")])
+FRAME = np.dtype([("p0", "f8", 3), ("ey", "f8", 3), ("ez", "f8", 3), ("b", "f8", 3), ("ny", "i4"), ("nz", "i4")] +
+                 [(n, "i4", 3) for n in ("ly", "lz", "py", "pz")] + [("bpy", "i4"), ("bpz", "i4"), ("mg", MERGE, 2)] +
+                 [("off", "i8", 3)] + [(n, "i8") for n in ("pix_off", "pblk_off", "part_off", "w_off")])
 SRC = np.dtype([("dh", "f4", 3), ("species", "i4"), ("dl", "f4", 3), ("count", "i4"), ("o", "f8", 3),
                 ("first", "i8")])
 
@@ -89,77 +90,94 @@ def _phase(P, b, o_ref, d):
 
 def _run(plan, buf, org, atoms, shapes, P, n_pix):
     fr = np.frombuffer(buf, FRAME, plan.n_frames, 0)
+    ints = lambda n, off: np.frombuffer(buf, np.int32, n, off)
     src = np.frombuffer(buf, SRC, plan.n_src, plan.off_src)
-    mem = np.frombuffer(buf, np.int32, plan.n_members, plan.off_members)
-    mid = np.frombuffer(buf, np.int32, plan.n_mid, plan.off_mid)
-    n0, n1 = plan.n0, plan.n1
+    msrc = np.frombuffer(buf, SRC, plan.n_msrc, plan.off_msrc)
+    morg = np.frombuffer(buf, np.float64, 4 * plan.n_msrc, plan.off_morg).reshape(-1, 4)
+    mem, mid = ints(plan.n_members, plan.off_members), ints(plan.n_mid, plan.off_mid)
+    n = (plan.n0, plan.nm, plan.n1)
     out = np.zeros(n_pix, complex)
     hit = np.zeros(n_pix, int)
 
-    def nodes(F, p, py, ly, lz, n):
-        pz, pyi = divmod(p, py)
-        y = pyi * ly + 0.5 * (ly - 1) + _half(ly) * _cheb(n)
-        z = pz * lz + 0.5 * (lz - 1) + _half(lz) * _cheb(n)
+    def nodes(F, p, lv):
+        pz, pyi = divmod(p, F["py"][lv])
+        ly, lz = F["ly"][lv], F["lz"][lv]
+        y = pyi * ly + 0.5 * (ly - 1) + _half(ly) * _cheb(n[lv])
+        z = pz * lz + 0.5 * (lz - 1) + _half(lz) * _cheb(n[lv])
         Z, Y = np.meshgrid(z, y, indexing="ij")
         return F["p0"] + Y.ravel()[:, None] * F["ey"] + Z.ravel()[:, None] * F["ez"]
 
-    def leaf(t, Pn, b):
+    def leaf(F, t, lv):         # a tile's field on every patch of a level
         o = org[t, :3]
-        return np.array([np.exp(2j * np.pi * _phase(Pn, b, o, a - o)) for a in atoms[t]]).sum(0)
+        one = lambda Pn: np.array([np.exp(2j * np.pi * _phase(Pn, F["b"], o, a - o)) for a in atoms[t]]).sum(0)
+        return np.array([one(nodes(F, p, lv)) for p in range(F["py"][lv] * F["pz"][lv])]).reshape(-1, n[lv], n[lv])
+
+    def blocks(M, F, lo, hi):   # the merge's blocks cover every node of the finer level once
+        rows = {6: 3, 8: 4, 10: 5, 12: 3, 16: 4}[n[hi]]
+        got = np.zeros((F["pz"][hi], F["py"][hi], n[hi], n[hi]), int)
+        for e in range(F["pz"][hi] * F["py"][lo] * M["strips"] * M["chunks"]):
+            e, chunk = divmod(e, M["chunks"])
+            e, strip = divmod(e, M["strips"])
+            pz, cy = divmod(e, F["py"][lo])
+            s0 = strip * M["strip"]
+            patches = min(M["strip"], M["ratio_y"] - s0, F["py"][hi] - cy * M["ratio_y"] - s0)
+            row0 = chunk * M["rowg"] * rows
+            nrow = min(M["rowg"] * rows, n[hi] - row0)
+            assert M["rowg"] * rows <= 16 and M["strip"] * n[hi] * M["rowg"] <= 128 and nrow % rows == 0
+            for th in range(128 if patches > 0 else 0):
+                rg, oc = divmod(th, M["strip"] * n[hi])
+                if oc < patches * n[hi] and rg * rows < nrow and rg < M["rowg"]:
+                    r = row0 + rg * rows
+                    got[pz, cy * M["ratio_y"] + s0 + oc // n[hi], r:r + rows, oc % n[hi]] += 1
+        assert (got == 1).all()
+
+    def merge(M, F, lo, hi, sources, V, where):
+        """sources' runs of V's rows, at `where`, onto the finer level."""
+        blocks(M, F, lo, hi)
+        full = np.zeros((len(sources), F["py"][hi] * F["pz"][hi], n[hi], n[hi]), complex)
+        for p in range(F["py"][hi] * F["pz"][hi]):
+            pz, py = divmod(p, F["py"][hi])
+            Pn = nodes(F, p, hi)
+            cy, cz = py // M["ratio_y"], pz // M["ratio_z"]
+            assert cy < F["py"][lo] and cz < F["pz"][lo]
+            pos = lambda sub, l1, l0: (sub * l1 + 0.5 * (l1 - 1) + _half(l1) * _cheb(n[hi]) - 0.5 * (l0 - 1)) / _half(l0)
+            Wy = np.array([_lagrange(x, n[lo]) for x in pos(py - cy * M["ratio_y"], F["ly"][hi], F["ly"][lo])])
+            Wz = np.array([_lagrange(x, n[lo]) for x in pos(pz - cz * M["ratio_z"], F["lz"][hi], F["lz"][lo])])
+            for s, S in enumerate(sources):
+                for i in range(S["first"], S["first"] + S["count"]):
+                    v = Wz @ V[i, cz * F["py"][lo] + cy] @ Wy.T
+                    ph = _phase(Pn, F["b"], S["o"], where[i] - S["o"])
+                    full[s, p] += v * np.exp(2j * np.pi * ph).reshape(n[hi], n[hi])
+        return full
 
     for F in fr:
-        if n0:                  # the merge's blocks cover every fine node once
-            rows = {6: 3, 8: 4, 10: 5, 12: 3}[n1]
-            got = np.zeros((F["p1z"], F["p1y"], n1, n1), int)
-            for e in range(F["p1z"] * F["p0y"] * F["strips"] * F["chunks"]):
-                e, chunk = divmod(e, F["chunks"])
-                e, strip = divmod(e, F["strips"])
-                pz, cy = divmod(e, F["p0y"])
-                s0 = strip * F["strip"]
-                patches = min(F["strip"], F["ratio_y"] - s0, F["p1y"] - cy * F["ratio_y"] - s0)
-                row0 = chunk * F["rowg"] * rows
-                nrow = min(F["rowg"] * rows, n1 - row0)
-                assert F["rowg"] * rows <= 16 and F["strip"] * n1 * F["rowg"] <= 128 and nrow % rows == 0
-                for th in range(128 if patches > 0 else 0):
-                    rg, oc = divmod(th, F["strip"] * n1)
-                    if oc < patches * n1 and rg * rows < nrow and rg < F["rowg"]:
-                        r = row0 + rg * rows
-                        got[pz, cy * F["ratio_y"] + s0 + oc // n1, r:r + rows, oc % n1] += 1
-            assert (got == 1).all()
-        l0y, l0z = F["l1y"] * F["ratio_y"], F["l1z"] * F["ratio_z"]
-        V0 = {}
-        for p in range(F["p0y"] * F["p0z"] if n0 else 0):
-            Pn = nodes(F, p, F["p0y"], l0y, l0z, n0)
-            for i, t in enumerate(mem):
-                V0[i, p] = leaf(t, Pn, F["b"]).reshape(n0, n0)
-        for p in range(F["p1y"] * F["p1z"]):
-            pz, py = divmod(p, F["p1y"])
-            Pn = nodes(F, p, F["p1y"], F["l1y"], F["l1z"], n1)
-            V1 = np.zeros((plan.n_src, n1, n1), complex)
-            for s in range(plan.n_groups):
-                S = src[s]
-                cy, cz = py // F["ratio_y"], pz // F["ratio_z"]
-                sy, sz = py - cy * F["ratio_y"], pz - cz * F["ratio_z"]
-                assert cy < F["p0y"] and cz < F["p0z"]
-                pos = lambda sub, l1, l0: (sub * l1 + 0.5 * (l1 - 1) + _half(l1) * _cheb(n1) - 0.5 * (l0 - 1)) / _half(l0)
-                Wy = np.array([_lagrange(x, n0) for x in pos(sy, F["l1y"], l0y)])
-                Wz = np.array([_lagrange(x, n0) for x in pos(sz, F["l1z"], l0z)])
-                for i in range(S["first"], S["first"] + S["count"]):
-                    v = Wz @ V0[i, cz * F["p0y"] + cy] @ Wy.T
-                    ph = _phase(Pn, F["b"], S["o"], org[mem[i], :3] - S["o"])
-                    V1[s] += v * np.exp(2j * np.pi * ph).reshape(n1, n1)
-            for j, t in enumerate(mid):
-                V1[plan.n_groups + j] = leaf(t, Pn, F["b"]).reshape(n1, n1)
-            cols = np.arange(py * F["l1y"], min((py + 1) * F["l1y"], F["ny"]))
-            rows = np.arange(pz * F["l1z"], min((pz + 1) * F["l1z"], F["nz"]))
+        V1 = np.zeros((0, F["py"][2] * F["pz"][2], n[2], n[2]), complex)
+        if n[0]:
+            V = np.array([leaf(F, t, 0) for t in mem])
+            lo, where = 0, org[mem, :3]
+            if n[1]:
+                V = merge(F["mg"][0], F, 0, 1, msrc, V, where)
+                for row, t in zip(ints(plan.n_msingle, plan.off_mrow), ints(plan.n_msingle, plan.off_msingle)):
+                    assert msrc[row]["count"] == 0
+                    V[row] = leaf(F, t, 1)
+                assert sum(msrc["count"]) == len(mem) and (msrc["count"] == 0).sum() == plan.n_msingle
+                lo, where = 1, morg[:, :3]
+            V1 = merge(F["mg"][1], F, lo, 2, src[:plan.n_groups], V, where)
+        if plan.n_mid:
+            V1 = np.concatenate([V1, np.array([leaf(F, t, 2) for t in mid])])
+        n1, ly, lz = n[2], F["ly"][2], F["lz"][2]
+        for p in range(F["py"][2] * F["pz"][2]):
+            pz, py = divmod(p, F["py"][2])
+            cols = np.arange(py * ly, min((py + 1) * ly, F["ny"]))
+            rows = np.arange(pz * lz, min((pz + 1) * lz, F["nz"]))
             assert F["bpy"] * 32 >= len(cols) and F["bpz"] * 16 >= len(rows)
-            Wy = np.array([_lagrange((c - py * F["l1y"] - 0.5 * (F["l1y"] - 1)) / _half(F["l1y"]), n1) for c in cols])
-            Wz = np.array([_lagrange((r - pz * F["l1z"] - 0.5 * (F["l1z"] - 1)) / _half(F["l1z"]), n1) for r in rows])
+            Wy = np.array([_lagrange((c - py * ly - 0.5 * (ly - 1)) / _half(ly), n1) for c in cols])
+            Wz = np.array([_lagrange((r - pz * lz - 0.5 * (lz - 1)) / _half(lz), n1) for r in rows])
             g = (F["pix_off"] + rows[:, None] * F["ny"] + cols[None, :]).ravel()
             for s in range(plan.n_src):
                 S = src[s]
                 o = S["dh"].astype(float) + S["dl"]
-                v = (Wz @ V1[s] @ Wy.T).ravel()
+                v = (Wz @ V1[s, p] @ Wy.T).ravel()
                 out[g] += v * np.exp(2j * np.pi * _phase(P[g], F["b"], np.zeros(3), o))
             hit[g] += 1
     assert (hit == 1).all()
@@ -197,6 +215,33 @@ def test_plan_reproduces_the_direct_sum(shapes, tiles, side, group):
     d = num / (np.sqrt(R[:, None] ** 2 + num) + R[:, None])
     ref = np.exp(1j * K * (a[:, 0][None] + d)).sum(1)
     assert np.abs(got - ref).max() <= 2.1e-6 * len(a)
+
+
+def test_plan_with_a_middle_level():
+    """Tiles in runs on middle nodes and runs in groups; a few tiles too wide
+    for the coarse nodes on the middle ones by themselves."""
+    rng = np.random.default_rng(7)
+    T, g, (ny, nz) = 3, 6, (400, 300)
+    cells = np.array([(x, y, z) for x in range(g) for y in range(g) for z in range(g)])
+    # octants first, as a space-filling curve visits them
+    cells = cells[np.lexsort((*(cells % 2).T[::-1], *(cells // 2 % 2).T[::-1], *(cells // 4).T[::-1]))]
+    org, atoms = _tiles(rng, (cells - g / 2) * 2.8e-9, 8, 2.6e-9)
+    atoms = atoms[:, :T].copy()
+    for t in (5, 100, 101, 215):            # spread out about their centres
+        atoms[t] = org[t, :3] + 2.0 * (atoms[t] - org[t, :3])
+        org[t, 3] *= 2.0
+    P = _grid(ny, nz, 0.3, 55e-6, 0.4)
+    n = len(org)
+    rc, plan, buf = _plan(org, [40 * T, (n - 40) * T], T, [(0, ny, nz)], [_fit(P, ny, nz)], [[1.0, 0, 0]])
+    assert rc == _lib.MK_OK and plan.nm > 0 and plan.n_msingle > 0
+    got = _run(plan, buf, org, atoms, [(ny, nz)], P, len(P))
+    a = atoms.reshape(-1, 3)
+    R = np.linalg.norm(P, axis=1)
+    ref = np.zeros(len(P), complex)
+    for x in a:
+        num = x @ x - 2 * P @ x
+        ref += np.exp(1j * K * (x[0] + num / (np.sqrt(R ** 2 + num) + R)))
+    assert np.abs(got - ref).max() <= 9.0e-6 * len(a)
 
 
 def test_plan_declines():

@@ -185,14 +185,17 @@ typedef struct {
     int n_wide;             /* tiles left to the split kernel (their indices at off_wide) */
     int n_src;              /* n_groups + n_mid */
     int slices, src_per_slice, passes;
-    int ns;                 /* nodes per axis of a tile's eighths (0: tiles evaluated whole) */
+    int ns[2];              /* nodes per axis of a tile's eighths, narrow tiles and others (0: tiles
+                             evaluated whole) */
+    int n_narrow;           /* narrow tiles (the first of off_leaf) */
     int nm;                 /* nodes per axis of the middle patches (0: tiles go straight into groups) */
     int n_msrc, n_msingle;  /* runs and single tiles on middle nodes, the single tiles among them */
-    long long patches0, patchesm, patches1, weights, n_pix, sub_w_off;
-    long long off_src, off_members, off_mid, off_wide, off_msrc, off_morg, off_msingle, off_mrow, buf_bytes;
+    long long patches0, patchesm, patches1, weights, n_pix, sub_w_off[2];
+    long long off_src, off_members, off_mid, off_wide, off_msrc, off_morg, off_msingle, off_mrow, off_leaf, off_leaf_row,
+        buf_bytes;
     long long chunk_bytes, ws_bytes;
     double radius1_m, radiusm_m, radius2_m; /* widest tile on coarse nodes, run, source */
-    double sub_radius_m;         /* widest eighth that its nodes take */
+    double sub_radius_m[2];      /* widest eighth that its nodes take */
     double form_s, direct_s;     /* estimated time of this form and of the split kernel */
 } mk_node_plan;
 

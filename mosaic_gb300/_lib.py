@@ -154,13 +154,15 @@ class MkLaunch(ctypes.Structure):
 class MkNodePlan(ctypes.Structure):
     _fields_ = [(n, ctypes.c_int) for n in
                 ("n_frames", "n_tiles", "n0", "n1", "group_tiles", "n_groups", "n_members", "n_mid",
-                 "n_wide", "n_src", "slices", "src_per_slice", "passes", "ns", "nm", "n_msrc", "n_msingle")] + \
+                 "n_wide", "n_src", "slices", "src_per_slice", "passes")] + \
+               [("ns", ctypes.c_int * 2)] + [(n, ctypes.c_int) for n in ("n_narrow", "nm", "n_msrc", "n_msingle")] + \
+               [(n, ctypes.c_longlong) for n in ("patches0", "patchesm", "patches1", "weights", "n_pix")] + \
+               [("sub_w_off", ctypes.c_longlong * 2)] + \
                [(n, ctypes.c_longlong) for n in
-                ("patches0", "patchesm", "patches1", "weights", "n_pix", "sub_w_off", "off_src", "off_members",
-                 "off_mid", "off_wide", "off_msrc", "off_morg", "off_msingle", "off_mrow", "buf_bytes",
-                 "chunk_bytes", "ws_bytes")] + \
-               [(n, ctypes.c_double) for n in ("radius1_m", "radiusm_m", "radius2_m", "sub_radius_m", "form_s",
-                                               "direct_s")]
+                ("off_src", "off_members", "off_mid", "off_wide", "off_msrc", "off_morg", "off_msingle", "off_mrow",
+                 "off_leaf", "off_leaf_row", "buf_bytes", "chunk_bytes", "ws_bytes")] + \
+               [(n, ctypes.c_double) for n in ("radius1_m", "radiusm_m", "radius2_m")] + \
+               [("sub_radius_m", ctypes.c_double * 2)] + [(n, ctypes.c_double) for n in ("form_s", "direct_s")]
 
 
 # name -> (restype, argtypes)

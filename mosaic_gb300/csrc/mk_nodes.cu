@@ -366,16 +366,34 @@ const double kWide = 0.3e-12, kWideSetup = 150e-6;
 double per_node(int n) { return 0.4 + 0.05 * n; }
 
 // Nodes per axis an eighth of a tile is evaluated on before it is interpolated
-// to the tile's n0 (0: no eighths): on the Hilbert curve an eighth has about
-// half the tile's radius, and 14^2 or 12^2 nodes take 0.49 or 0.53 of the
-// phase of 20^2 or 16^2. From 12 nodes down the interpolation eats the gain.
-int sub_nodes(int n0, int tile_atoms) { return tile_atoms < 512 ? 0 : n0 == 20 ? 14 : n0 == 16 ? 12 : 0; }
-
-// Leaf terms an atom costs per coarse patch, interpolation of the eighths and
-// the wide ones among them included.
-double leaf_terms(int n0, int tile_atoms)
+// to the tile's n0, in two classes (0: evaluated whole): on the Hilbert curve an
+// eighth has about half the tile's radius, and most tiles are much narrower than
+// the widest one, r1. The phase that fewer nodes take is 0.49 (14 of 20), 0.34 (12
+// of 20), 0.53 (12 of 16), 0.33 (10 of 16), 0.63 (10 of 12), 0.33 (8 of 12), 0.52
+// (8 of 10) and 0.37 (6 of 8) of the tile's.
+int sub_nodes(int n0, int tile_atoms, bool narrow)
 {
-    const int ns = sub_nodes(n0, tile_atoms);
+    if (tile_atoms < 512) return 0;
+    switch (n0) {
+    case 20: return narrow ? 12 : 14;
+    case 16: return narrow ? 10 : 12;
+    case 12: return narrow ? 8 : 10;
+    case 10: return narrow ? 8 : 0;
+    case 8: return narrow ? 6 : 0;
+    }
+    return 0;
+}
+
+// Widest tile that goes with the narrow class, for tiles up to r1 on n0 nodes: an
+// eighth is half of it where tiles are whole cubes (at 0.55 of it 1.48 + 1.03 ms
+// went on the 5.3M-atom exposure, at 0.51 and 0.47 2.3 ms).
+double narrow_radius(int n0, int nt, double r1) { return r1 * phi_max(nt) / phi_max(n0) / 0.50; }
+
+// Leaf terms per coarse patch of an atom of the two classes, interpolation of
+// the eighths and the wide ones among them included.
+double leaf_terms(int n0, int tile_atoms, bool narrow)
+{
+    const int ns = sub_nodes(n0, tile_atoms, narrow);
     return ns ? 1.2 * ns * ns : (double)n0 * n0;
 }
 
@@ -389,7 +407,7 @@ struct Choice {
 // Node records of a plan: coarse, middle, fine, and the eighths' on the coarse patches.
 long long records(const mk_node_plan &P)
 {
-    return P.patches0 * (P.n0 * P.n0 + P.ns * P.ns) + P.patchesm * P.nm * P.nm + P.patches1 * P.n1 * P.n1;
+    return P.patches0 * (P.n0 * P.n0 + P.ns[0] * P.ns[0] + P.ns[1] * P.ns[1]) + P.patchesm * P.nm * P.nm + P.patches1 * P.n1 * P.n1;
 }
 
 // Whole frames from f on whose node fields and partials fit `budget` bytes (one
@@ -438,7 +456,7 @@ extern "C" size_t mk_nodes_plan_bytes(int n_frames, int n_tiles)
 {
     if (n_frames < 1 || n_tiles < 0) return 0;
     return up256(sizeof(MkNodeFrame) * (size_t)n_frames) + 2 * up256(sizeof(MkNodeSrc) * (size_t)n_tiles) +
-           up256(sizeof(double4) * (size_t)n_tiles) + 5 * up256(sizeof(int) * (size_t)n_tiles);
+           up256(sizeof(double4) * (size_t)n_tiles) + 7 * up256(sizeof(int) * (size_t)n_tiles);
 }
 
 extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const int64_t *counts,
@@ -587,8 +605,11 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
                         if (part >= best.cost) continue;
                         for (int n0 : kNodeCounts) {
                             if (n0 < 8 || !parent_cut(geo, k, r1, n0, im < 0 ? c1 : cm, &c0, &N0)) continue;
-                            const double c = part + n_nar * T * N0 / (n0 * n0) * leaf_terms(n0, tile_atoms) * kLeaf +
-                                             n_nar * Nt * kMerge * per_node(n0);
+                            const int nt = sub_nodes(n0, tile_atoms, true);
+                            const double narrow = nt ? std::min(n_tiles - above(narrow_radius(n0, nt, r1)), n_nar) : 0.0;
+                            const double leaf = narrow * leaf_terms(n0, tile_atoms, true) +
+                                                (n_nar - narrow) * leaf_terms(n0, tile_atoms, false);
+                            const double c = part + T * N0 / (n0 * n0) * leaf * kLeaf + n_nar * Nt * kMerge * per_node(n0);
                             if (c >= best.cost) continue;
                             best.cost = c;
                             best.r1 = r1;
@@ -791,11 +812,24 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
     const long long patch = patches[MK_FINE];
     plan->patches0 = patches[MK_COARSE];
     plan->patchesm = patches[MK_MIDDLE];
-    plan->ns = best.G ? sub_nodes(best.n0, tile_atoms) : 0;
-    if (plan->ns) {
-        plan->sub_radius_m = best.r1 * phi_max(plan->ns) / phi_max(best.n0);
-        plan->sub_w_off = wf;
-        wf += best.n0 * plan->ns;
+    // leaves by eighths: the narrow class's tiles first, and the rows of their fields
+    std::vector<int> leaf, leaf_row;
+    for (int c = 0; c < 2 && best.G; ++c) {
+        const int ns = sub_nodes(best.n0, tile_atoms, c == 0);
+        if (!sub_nodes(best.n0, tile_atoms, true)) break;
+        // a second launch pays where both fill the chip: eight blocks an SM
+        const bool two = (long long)members.size() * plan->patches0 >= 8 * 152;
+        const double split_at = two ? narrow_radius(best.n0, sub_nodes(best.n0, tile_atoms, true), best.r1) : -1.0;
+        for (size_t i = 0; i < members.size(); ++i)
+            if ((rad[members[i]] <= split_at) == (c == 0)) {
+                leaf.push_back(members[i]);
+                leaf_row.push_back((int)i);
+            }
+        if (c == 0) plan->n_narrow = (int)leaf.size();
+        plan->ns[c] = ns;
+        plan->sub_radius_m[c] = ns ? best.r1 * phi_max(ns) / phi_max(best.n0) : 0.0;
+        plan->sub_w_off[c] = wf;
+        wf += best.n0 * ns;
     }
     plan->patches1 = patch;
     plan->weights = wf;
@@ -844,6 +878,8 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
     plan->off_members = put(members.data(), sizeof(int) * members.size());
     plan->off_mid = put(mid.data(), sizeof(int) * mid.size());
     plan->off_wide = put(wide.data(), sizeof(int) * wide.size());
+    plan->off_leaf = put(leaf.data(), sizeof(int) * leaf.size());
+    plan->off_leaf_row = put(leaf_row.data(), sizeof(int) * leaf_row.size());
     plan->off_msrc = put(msrc.data(), sizeof(MkNodeSrc) * msrc.size());
     plan->off_morg = put(morg.data(), sizeof(double4) * morg.size());
     plan->off_msingle = put(msingle.data(), sizeof(int) * msingle.size());
@@ -873,8 +909,6 @@ struct MkNodeArgs {
     float kappa, fres_r;
     double kappa_d;
     int fresnel, decay;
-    const float *w_s;                // weights and widest radius [cycles] of a tile's eighths
-    float sub_r;
 };
 
 // One merge: sources on n_in nodes per axis of level `in` to n_out of level
@@ -909,9 +943,19 @@ __device__ __forceinline__ int mk_find_frame(int lo, int hi, long long i, Key ke
 __device__ __forceinline__ double mk_half_range(int len) { return 0.5 * (len - 1) + MK_NODE_PAD; }
 
 // The Chebyshev nodes of one count and the inverse products of their Lagrange
-// weights, in shared memory.
+// weights.
 struct MkCheb {
     double x[MK_NODE_MAX], inv[MK_NODE_MAX];
+    void fill(int n)
+    {
+        for (int i = 0; i < n; ++i) x[i] = std::cos((2 * i + 1) * MK_PI / (2.0 * n));
+        for (int j = 0; j < n; ++j) {
+            double den = 1.0;
+            for (int i = 0; i < n; ++i)
+                if (i != j) den *= x[j] - x[i];
+            inv[j] = 1.0 / den;
+        }
+    }
 };
 
 // Lagrange weight j of n nodes at x (FP64 products), rounded to float32 so that
@@ -950,43 +994,42 @@ __device__ __forceinline__ float mk_lagrange(const MkCheb &C, double x, int n, i
 // Node records and weight tables of every frame: one thread per node, 16 or 32
 // lanes per point's weights (blocks before `node_blocks` the one, the rest the
 // other). On one frame a chain of ~n FP64 products' latency, on many the FP64
-// pipe, which each block's own nodes (~100 operations of three warps) load as
-// well: blocks enough for a few an SM, each over several points. With all n
-// weights (and the nodes' cosines) in one thread it took 35 us on a 128 x 128
-// detector and 99 us for 16 frames; here 7 and 56 us.
+// pipe: the nodes of every count come with the arguments (a block that made
+// them itself spent ~100 operations of it a warp). With all n weights (and the
+// nodes' cosines) in one thread it took 35 us on a 128 x 128 detector and 99 us
+// for 16 frames; here 6 and 55 us.
 struct MkPrepArgs {
     const MkNodeFrame *frames;
-    int n[4];                            // nodes per axis of the levels, and of eighths
-    MkNodeRec *rec[4];
+    int n[5];                            // nodes per axis of the levels, and of eighths of either class
+    MkNodeRec *rec[5];
     int node_blocks;
     double kappa;
     const double *xyz;
-    float *weights, *w_s;
+    float *weights, *w_s[2];
+    MkCheb cheb[5];
 };
-__global__ void __launch_bounds__(128) mk_node_prep_kernel(const MkPrepArgs A)
+#define MK_PREP_NT 128
+__global__ void __launch_bounds__(MK_PREP_NT) mk_node_prep_kernel(const MkPrepArgs A)
 {
-    __shared__ MkCheb s_c[4];              // of every level, and of eighths
-    const int th = threadIdx.x, mine = A.n[th >> 5], lane32 = th & 31;
-    MkCheb &C = s_c[th >> 5];
-    if (lane32 < mine) C.x[lane32] = cospi((2 * lane32 + 1) / (2.0 * mine));
-    __syncwarp();
-    if (lane32 < mine) {
-        double den = 1.0;
-        for (int i = 0; i < mine; ++i)
-            if (i != lane32) den *= C.x[lane32] - C.x[i];
-        C.inv[lane32] = 1.0 / den;
-    }
+    __shared__ MkCheb s_c[5];              // of every level, and of eighths
+    const int th = threadIdx.x;
+    for (int i = th; i < 5 * 2 * MK_NODE_MAX; i += MK_PREP_NT)
+        reinterpret_cast<double *>(s_c)[i] = reinterpret_cast<const double *>(A.cheb)[i];
     __syncthreads();
     const MkNodeFrame &F = A.frames[blockIdx.x];
     if ((int)blockIdx.y < A.node_blocks) {
-        int end[4], sum = 0;
-        for (int l = 0; l < 4; ++l) {
-            const int g = l == 3 ? MK_COARSE : l;
-            end[l] = sum += F.py[g] * F.pz[g] * A.n[l] * A.n[l];
+        int first[6] = {0};
+#pragma unroll
+        for (int l = 0; l < 5; ++l) {
+            const int g = l > 2 ? MK_COARSE : l;
+            first[l + 1] = first[l] + F.py[g] * F.pz[g] * A.n[l] * A.n[l];
         }
-        for (int t = blockIdx.y * 128 + th; t < sum; t += A.node_blocks * 128) {
-            const int lv = (t >= end[0]) + (t >= end[1]) + (t >= end[2]), g = lv == 3 ? MK_COARSE : lv;
-            const int e = t - (lv == 0 ? 0 : lv == 1 ? end[0] : lv == 2 ? end[1] : end[2]);
+        for (int t = blockIdx.y * MK_PREP_NT + th; t < first[5]; t += A.node_blocks * MK_PREP_NT) {
+            int lv = 0, e = t;
+#pragma unroll
+            for (int l = 1; l < 5; ++l)
+                if (t >= first[l]) { lv = l; e = t - first[l]; }
+            const int g = lv > 2 ? MK_COARSE : lv;
             const int n = A.n[lv], py = F.py[g], ly = F.ly[g], lz = F.lz[g];
             const int p = e / (n * n), r = e - p * n * n, j = r / n, c = r - j * n;
             const int pz = p / py, pyi = p - pz * py;
@@ -1020,9 +1063,9 @@ __global__ void __launch_bounds__(128) mk_node_prep_kernel(const MkPrepArgs A)
     const int above = A.n[MK_MIDDLE] ? MK_MIDDLE : MK_COARSE;
     const int e0 = F.ny + F.nz, e1 = e0 + (A.n[0] ? (M1.ratio_y + M1.ratio_z) * A.n[MK_FINE] : 0);
     const int e2 = e1 + (A.n[MK_MIDDLE] ? (M0.ratio_y + M0.ratio_z) * A.n[MK_MIDDLE] : 0);
-    const int points = e2 + (blockIdx.x == 0 && A.n[3] ? A.n[0] : 0);
-    const int width = max(max(A.n[0], A.n[1]), max(A.n[2], A.n[3])) > 16 ? 32 : 16, lane = th & (width - 1);
-    const int per = 128 / width, step = (gridDim.y - A.node_blocks) * per;
+    const int points = e2 + (blockIdx.x == 0 && A.n[3] ? 2 * A.n[0] : 0);
+    const int width = max(A.n[0], max(A.n[1], A.n[2])) > 16 ? 32 : 16, lane = th & (width - 1);
+    const int per = MK_PREP_NT / width, step = (gridDim.y - A.node_blocks) * per;
     // whole warps stay in the loop: the lanes of a warp's groups shuffle together
     for (int i0 = (blockIdx.y - A.node_blocks) * per + (th >> 5) * (32 / width); i0 < points; i0 += step) {
         const int at = i0 + (th & 31) / width, i = min(at, points - 1);
@@ -1049,9 +1092,10 @@ __global__ void __launch_bounds__(128) mk_node_prep_kernel(const MkPrepArgs A)
             x = (v - 0.5 * (l0 - 1)) / mk_half_range(l0);
             out = A.weights + M.w_off + (long long)m * A.n[lv];
         } else {
-            x = s_c[MK_COARSE].x[i - e2];
-            out = A.w_s + (i - e2) * A.n[3];
-            lv = 3;
+            const int c = i - e2 >= A.n[0], j = i - e2 - c * A.n[0];
+            x = s_c[MK_COARSE].x[j];
+            lv = 3 + c;
+            out = A.w_s[c] + j * A.n[lv];
         }
         const int n = A.n[lv];
         const float w = mk_lagrange(s_c[lv], x, n, lane, width);
@@ -1129,15 +1173,27 @@ __global__ void __launch_bounds__(256) mk_node_leaf_kernel(const MkNodeArgs A, c
 // coarse patch). An eighth wider than its nodes take (and every eighth of a
 // tile that keeps the |d|^2 term) is added term by term at the tile's nodes.
 // NS^2 terms an atom instead of N0^2: still bound by the MUFU. 10,321 tiles
-// on four 20 x 20 node patches 3.88 ms directly, 2.78 so; 15,756 on one of 16 x 16
-// 0.95 and 0.74.
+// on four 20 x 20 node patches 3.88 ms directly, 2.32 so; 15,814 on one of 16 x 16
+// 0.95 and 0.57 (all of them on 14 x 14 and 12 x 12 nodes: 2.78 and 0.74).
+struct MkSubArgs {
+    const int *list, *rows;              // tiles and the rows of their fields
+    const MkNodeRec *rec;                // the eighths' nodes
+    const float *w;                      // from those to the tile's, (N0, NS)
+    float radius;                        // widest eighth [cycles]
+    int patches;                         // of a block
+};
+// 256 threads, but 96 where there are only 288 eighth nodes (6 x 6; 466 us with
+// 288 threads, 436 with 96). Blocks of 16 NS threads for the others too, which
+// leave no round part empty, hold fewer warps an SM: 573 us instead of 524 for
+// 10 x 10.
+__host__ __device__ constexpr int mk_leaf8_threads(int ns) { return ns == 6 ? 96 : 256; }
 template <int N0, int NS>
-__global__ void __launch_bounds__(256) mk_node_leaf8_kernel(const MkNodeArgs A, const int *__restrict__ list,
-                                                            const MkNodeRec *__restrict__ rec,
-                                                            const MkNodeRec *__restrict__ rec_s,
-                                                            long long n_nodes, float2 *__restrict__ V)
+__global__ void __launch_bounds__(mk_leaf8_threads(NS)) mk_node_leaf8_kernel(const MkNodeArgs A, const MkSubArgs B,
+                                                                             const MkNodeRec *__restrict__ rec,
+                                                                             long long n_nodes,
+                                                                             float2 *__restrict__ V)
 {
-    constexpr int SQ = NS * NS;
+    constexpr int SQ = NS * NS, NT = mk_leaf8_threads(NS);
     extern __shared__ __align__(16) unsigned char leaf_smem[];
     const int T = A.tile_atoms, pairs = T / 16;          // atom pairs of an eighth
     float4 *s_pos = reinterpret_cast<float4 *>(leaf_smem);
@@ -1146,18 +1202,18 @@ __global__ void __launch_bounds__(256) mk_node_leaf8_kernel(const MkNodeArgs A, 
     float2 *s_t = s_v + 8 * SQ;                                     // [8][N0][NS]
     float *s_w = reinterpret_cast<float *>(s_t + 8 * N0 * NS);      // [N0][NS]
     __shared__ float4 s_c[8];                            // centre; 1 where the eighth has nodes
-    const int t = list[blockIdx.x];
+    const int t = B.list[blockIdx.x];
     const float4 *gp = A.tpos + (size_t)t * T;
     const float4 *ga = reinterpret_cast<const float4 *>(A.tamp + (size_t)t * T);
-    for (int i = threadIdx.x; i < T; i += 256) s_pos[i] = gp[i];
-    for (int i = threadIdx.x; i < T / 2; i += 256) s_amp[i] = ga[i];
-    for (int i = threadIdx.x; i < N0 * NS; i += 256) s_w[i] = A.w_s[i];
+    for (int i = threadIdx.x; i < T; i += NT) s_pos[i] = gp[i];
+    for (int i = threadIdx.x; i < T / 2; i += NT) s_amp[i] = ga[i];
+    for (int i = threadIdx.x; i < N0 * NS; i += NT) s_w[i] = B.w[i];
     __syncthreads();
     const double4 o = A.origin[t];
     const float ox = (float)o.x, oy = (float)o.y, oz = (float)o.z;
     const bool fr = A.fresnel && (float)o.w > A.fres_r;
-    {
-        const int s = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int s = threadIdx.x >> 5; s < 8; s += NT / 32) {
+        const int lane = threadIdx.x & 31;
         float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
         for (int p = s * pairs + lane; p < (s + 1) * pairs; p += 32) {
             const float4 a = s_pos[2 * p], b = s_pos[2 * p + 1];    // x0 x1 y0 y1, z0 z1
@@ -1182,7 +1238,7 @@ __global__ void __launch_bounds__(256) mk_node_leaf8_kernel(const MkNodeArgs A, 
         }
         for (int w = 16; w > 0; w >>= 1) r2 = fmaxf(r2, __shfl_xor_sync(0xffffffffu, r2, w));
         if (lane == 0)
-            s_c[s] = make_float4(c[0], c[1], c[2], !fr && r2 <= A.sub_r * A.sub_r ? 1.f : 0.f);
+            s_c[s] = make_float4(c[0], c[1], c[2], !fr && r2 <= B.radius * B.radius ? 1.f : 0.f);
     }
     __syncthreads();
     const mk_f2 magic = f2_splat(MK_ROUND_MAGIC), two_pi = f2_splat(TWO_PI_F), m_one = f2_splat(-1.f);
@@ -1213,84 +1269,87 @@ __global__ void __launch_bounds__(256) mk_node_leaf8_kernel(const MkNodeArgs A, 
         return make_float3(fmaf(ox - uo * u4.x, w4.w, w4.x), fmaf(oy - uo * u4.y, w4.w, w4.y),
                            fmaf(oz - uo * u4.z, w4.w, w4.z));
     };
-    const MkNodeRec *rs = rec_s + (long long)blockIdx.y * SQ;
-    for (int i = threadIdx.x; i < 8 * SQ; i += 256) {
-        const int s = i / SQ, q = i - s * SQ;
-        const float4 c = s_c[s];
-        if (c.w == 0.f) {
-            s_v[i] = make_float2(0.f, 0.f);
-            continue;
-        }
-        const float3 w = direction(rs[q].w, rs[q].u);
-        s_v[i] = terms(s * pairs, (s + 1) * pairs, w.x, w.y, w.z, fmaf(c.z, w.z, fmaf(c.y, w.y, c.x * w.x)));
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < 8 * N0 * NS; i += 256) {
-        const int s = i / (N0 * NS), r = i - s * N0 * NS, row = r / NS, c = r - row * NS;
-        mk_f2 a = 0ull;
-#pragma unroll
-        for (int j = 0; j < NS; ++j)
-            a = f2_fma(f2_splat(s_w[row * NS + j]), *reinterpret_cast<const mk_f2 *>(&s_v[s * SQ + j * NS + c]), a);
-        *reinterpret_cast<mk_f2 *>(&s_t[i]) = a;
-    }
-    __syncthreads();
-    const MkNodeRec *rn = rec + (long long)blockIdx.y * N0 * N0;
-    float2 *out = V + (long long)blockIdx.x * n_nodes + (long long)blockIdx.y * N0 * N0;
-    for (int g = threadIdx.x; g < N0 * N0; g += 256) {
-        const int row = g / N0, col = g - row * N0;
-        const float4 w4 = rn[g].w, u4 = rn[g].u;
-        const float3 w = direction(w4, u4);
-        float re = 0.f, im = 0.f;
-        for (int s = 0; s < 8; ++s) {
+    const int patches = (int)(n_nodes / (N0 * N0)), p_end = min((int)(blockIdx.y + 1) * B.patches, patches);
+    for (int patch = blockIdx.y * B.patches; patch < p_end; ++patch) {
+        const MkNodeRec *rs = B.rec + (long long)patch * SQ;
+        for (int i = threadIdx.x; i < 8 * SQ; i += NT) {
+            const int s = i / SQ, q = i - s * SQ;
             const float4 c = s_c[s];
-            if (c.w == 0.f) {               // uniform across the block
-                float2 v;
-                if (fr) {
-                    // the |d|^2 term: 1 / (2 kappa |P - o|), db = D.b
-                    const float uo = fmaf(u4.z, oz, fmaf(u4.y, oy, u4.x * ox));
-                    const float hq = 0.5f * w4.w / (A.kappa * fmaf(-uo, w4.w, 1.f));
-                    const float bx = u4.w, by = rn[g].qh.w, bz = rn[g].ql.w;
-                    v = make_float2(0.f, 0.f);
-                    for (int p = s * pairs; p < (s + 1) * pairs; ++p) {
-                        MkAtom m[2];
-                        mk_atom_pair(s_pos, s_amp, p, m[0], m[1]);
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            const float4 a = m[h].a;
-                            float lin = fmaf(a.z, w.z, fmaf(a.y, w.y, a.x * w.x));
-                            const float sp = fmaf(a.z, bz, fmaf(a.y, by, a.x * bx)) - lin;
-                            lin = fmaf(fmaf(-sp, sp, a.w), hq, lin);
-                            float sn, cs;
-                            __sincosf(mk_frac_nearest(lin) * TWO_PI_F, &sn, &cs);
-                            v.x += m[h].e.x * cs - m[h].e.y * sn;
-                            v.y += m[h].e.x * sn + m[h].e.y * cs;
-                        }
-                    }
-                    v = make_float2(mk_unshort(v.x), mk_unshort(v.y));
-                } else {
-                    v = terms(s * pairs, (s + 1) * pairs, w.x, w.y, w.z, 0.f);
-                }
-                re += v.x;
-                im += v.y;
+            if (c.w == 0.f) {
+                s_v[i] = make_float2(0.f, 0.f);
                 continue;
             }
-            mk_f2 v = 0ull;
-            const ulonglong2 *t2 = reinterpret_cast<const ulonglong2 *>(s_t + (s * N0 + row) * NS);
-            const float *wy = s_w + col * NS;
-#pragma unroll
-            for (int i = 0; i < NS / 2; ++i) {
-                const ulonglong2 tt = t2[i];
-                v = f2_fma(f2_splat(wy[2 * i]), tt.x, v);
-                v = f2_fma(f2_splat(wy[2 * i + 1]), tt.y, v);
-            }
-            float sn, cs;
-            __sincosf(mk_frac_nearest(fmaf(c.z, w.z, fmaf(c.y, w.y, c.x * w.x))) * TWO_PI_F, &sn, &cs);
-            const float2 vv = f2_unpack(v);
-            re += mk_unshort(vv.x * cs - vv.y * sn);
-            im += mk_unshort(vv.x * sn + vv.y * cs);
+            const float3 w = direction(rs[q].w, rs[q].u);
+            s_v[i] = terms(s * pairs, (s + 1) * pairs, w.x, w.y, w.z, fmaf(c.z, w.z, fmaf(c.y, w.y, c.x * w.x)));
         }
-        out[g] = make_float2(re, im);
-    }
+        __syncthreads();
+        for (int i = threadIdx.x; i < 8 * N0 * NS; i += NT) {
+            const int s = i / (N0 * NS), r = i - s * N0 * NS, row = r / NS, c = r - row * NS;
+            mk_f2 a = 0ull;
+#pragma unroll
+            for (int j = 0; j < NS; ++j)
+                a = f2_fma(f2_splat(s_w[row * NS + j]), *reinterpret_cast<const mk_f2 *>(&s_v[s * SQ + j * NS + c]), a);
+            *reinterpret_cast<mk_f2 *>(&s_t[i]) = a;
+        }
+        __syncthreads();
+        const MkNodeRec *rn = rec + (long long)patch * N0 * N0;
+        float2 *out = V + (long long)B.rows[blockIdx.x] * n_nodes + (long long)patch * N0 * N0;
+        for (int g = threadIdx.x; g < N0 * N0; g += NT) {
+            const int row = g / N0, col = g - row * N0;
+            const float4 w4 = rn[g].w, u4 = rn[g].u;
+            const float3 w = direction(w4, u4);
+            float re = 0.f, im = 0.f;
+            for (int s = 0; s < 8; ++s) {
+                const float4 c = s_c[s];
+                if (c.w == 0.f) {               // uniform across the block
+                    float2 v;
+                    if (fr) {
+                        // the |d|^2 term: 1 / (2 kappa |P - o|), db = D.b
+                        const float uo = fmaf(u4.z, oz, fmaf(u4.y, oy, u4.x * ox));
+                        const float hq = 0.5f * w4.w / (A.kappa * fmaf(-uo, w4.w, 1.f));
+                        const float bx = u4.w, by = rn[g].qh.w, bz = rn[g].ql.w;
+                        v = make_float2(0.f, 0.f);
+                        for (int p = s * pairs; p < (s + 1) * pairs; ++p) {
+                            MkAtom m[2];
+                            mk_atom_pair(s_pos, s_amp, p, m[0], m[1]);
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                const float4 a = m[h].a;
+                                float lin = fmaf(a.z, w.z, fmaf(a.y, w.y, a.x * w.x));
+                                const float sp = fmaf(a.z, bz, fmaf(a.y, by, a.x * bx)) - lin;
+                                lin = fmaf(fmaf(-sp, sp, a.w), hq, lin);
+                                float sn, cs;
+                                __sincosf(mk_frac_nearest(lin) * TWO_PI_F, &sn, &cs);
+                                v.x += m[h].e.x * cs - m[h].e.y * sn;
+                                v.y += m[h].e.x * sn + m[h].e.y * cs;
+                            }
+                        }
+                        v = make_float2(mk_unshort(v.x), mk_unshort(v.y));
+                    } else {
+                        v = terms(s * pairs, (s + 1) * pairs, w.x, w.y, w.z, 0.f);
+                    }
+                    re += v.x;
+                    im += v.y;
+                    continue;
+                }
+                mk_f2 v = 0ull;
+                const ulonglong2 *t2 = reinterpret_cast<const ulonglong2 *>(s_t + (s * N0 + row) * NS);
+                const float *wy = s_w + col * NS;
+#pragma unroll
+                for (int i = 0; i < NS / 2; ++i) {
+                    const ulonglong2 tt = t2[i];
+                    v = f2_fma(f2_splat(wy[2 * i]), tt.x, v);
+                    v = f2_fma(f2_splat(wy[2 * i + 1]), tt.y, v);
+                }
+                float sn, cs;
+                __sincosf(mk_frac_nearest(fmaf(c.z, w.z, fmaf(c.y, w.y, c.x * w.x))) * TWO_PI_F, &sn, &cs);
+                const float2 vv = f2_unpack(v);
+                re += mk_unshort(vv.x * cs - vv.y * sn);
+                im += mk_unshort(vv.x * sn + vv.y * cs);
+            }
+            out[g] = make_float2(re, im);
+        }
+    }       // s_v is written again only after every thread has left the reads of s_t's making
 }
 
 __device__ __forceinline__ void mk_cp16(void *dst, const void *src)
@@ -1752,13 +1811,16 @@ static int mk_merge(const MkMergeArgs &A, int n_in, int n_runs, cudaStream_t st)
 }
 
 template <int N0, int NS>
-static int mk_launch_leaf8(const MkNodeArgs &A, const int *list, int n_list, const MkNodeRec *rec,
-                           const MkNodeRec *rec_s, long long nodes, float2 *V, cudaStream_t st)
+static int mk_launch_leaf8(const MkNodeArgs &A, MkSubArgs B, int n_list, const MkNodeRec *rec,
+                           long long nodes, float2 *V, cudaStream_t st)
 {
     const size_t smem = (size_t)A.tile_atoms * 24 + 8 * 8 * (size_t)NS * (NS + N0) + 4 * (size_t)N0 * NS;
     auto fn = mk_node_leaf8_kernel<N0, NS>;
     MK_CHECK_CUDA(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    fn<<<dim3(n_list, (unsigned)(nodes / (N0 * N0))), 256, smem, st>>>(A, list, rec, rec_s, nodes, V);
+    // a block's patches share its tile's atoms and boxes; 16 blocks an SM first
+    const int patches = (int)(nodes / (N0 * N0));
+    B.patches = (int)std::max<long long>(1, std::min<long long>(8, (long long)n_list * patches / (16 * 152)));
+    fn<<<dim3(n_list, (patches + B.patches - 1) / B.patches), mk_leaf8_threads(NS), smem, st>>>(A, B, rec, nodes, V);
     return MK_OK;
 }
 
@@ -1784,7 +1846,7 @@ extern "C" int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, c
         mk_set_error("mk_kin_nodes_f32: workspace %zu bytes, need %lld", ws_bytes, plan->ws_bytes);
         return MK_ENOMEM;
     }
-    const int n0 = plan->n0, nm = plan->nm, n1 = plan->n1, ns = plan->ns, T = tiles->tile_atoms;
+    const int n0 = plan->n0, nm = plan->nm, n1 = plan->n1, T = tiles->tile_atoms;
     const MkNodeFrame *hf = static_cast<const MkNodeFrame *>(host_buf);
     const char *db = static_cast<const char *>(dev_buf);
     cudaStream_t st = mk_stream(stream);
@@ -1801,19 +1863,27 @@ extern "C" int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, c
     prep.n[MK_COARSE] = n0;
     prep.n[MK_MIDDLE] = nm;
     prep.n[MK_FINE] = n1;
-    prep.n[3] = ns;
-    MkNodeRec *rec[4];
+    MkNodeRec *rec[5];
     rec[0] = reinterpret_cast<MkNodeRec *>(w);
     rec[1] = rec[0] + plan->patches0 * n0 * n0;
     rec[2] = rec[1] + plan->patchesm * nm * nm;
     rec[3] = rec[2] + plan->patches1 * n1 * n1;
-    for (int l = 0; l < 4; ++l) prep.rec[l] = rec[l];
+    rec[4] = rec[3] + plan->patches0 * plan->ns[0] * plan->ns[0];
+    for (int l = 0; l < 5; ++l) prep.rec[l] = rec[l];
     w += up256(sizeof(MkNodeRec) * (size_t)records(*plan));
     float *weights = reinterpret_cast<float *>(w);
     w += up256(sizeof(float) * (size_t)plan->weights);
     A.weights = weights;
-    A.w_s = weights + plan->sub_w_off;
-    A.sub_r = (float)(plan->sub_radius_m * phys->k / MK_TWO_PI);
+    MkSubArgs sub[2];
+    for (int c = 0; c < 2; ++c) {
+        const int from = c ? plan->n_narrow : 0;
+        sub[c].list = reinterpret_cast<const int *>(db + plan->off_leaf) + from;
+        sub[c].rows = reinterpret_cast<const int *>(db + plan->off_leaf_row) + from;
+        sub[c].w = weights + plan->sub_w_off[c];
+        sub[c].radius = (float)(plan->sub_radius_m[c] * phys->k / MK_TWO_PI);
+        prep.n[3 + c] = plan->ns[c];
+        prep.w_s[c] = weights + plan->sub_w_off[c];
+    }
     A.n1 = n1;
     A.n_groups = plan->n_groups;
     A.n_src = plan->n_src;
@@ -1835,19 +1905,19 @@ extern "C" int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, c
     int nodes = 0, points = 0;             // of the largest frame
     for (int f = 0; f < plan->n_frames; ++f) {
         const MkNodeFrame &F = hf[f];
-        nodes = std::max(nodes, F.py[0] * F.pz[0] * (n0 * n0 + ns * ns) + F.py[1] * F.pz[1] * nm * nm +
+        nodes = std::max(nodes, F.py[0] * F.pz[0] * (n0 * n0 + plan->ns[0] * plan->ns[0] + plan->ns[1] * plan->ns[1]) + F.py[1] * F.pz[1] * nm * nm +
                                     F.py[2] * F.pz[2] * n1 * n1);
-        points = std::max(points, F.ny + F.nz + n0 + (F.mg[1].ratio_y + F.mg[1].ratio_z) * n1 +
+        points = std::max(points, F.ny + F.nz + 2 * n0 + (F.mg[1].ratio_y + F.mg[1].ratio_z) * n1 +
                                       (F.mg[0].ratio_y + F.mg[0].ratio_z) * nm);
     }
+    for (int l = 0; l < 5; ++l) prep.cheb[l].fill(prep.n[l]);
     const int most = std::max(1, 1216 / plan->n_frames);
-    prep.node_blocks = std::min((nodes + 127) / 128, most);
+    prep.node_blocks = std::min((nodes + MK_PREP_NT - 1) / MK_PREP_NT, most);
     prep.kappa = A.kappa_d;
     prep.xyz = px->xyz;
     prep.weights = weights;
-    prep.w_s = weights + plan->sub_w_off;
-    mk_node_prep_kernel<<<dim3(plan->n_frames, prep.node_blocks + std::min((points + 3) / 4, most)), 128, 0, st>>>(
-        prep);
+    mk_node_prep_kernel<<<dim3(plan->n_frames, prep.node_blocks + std::min((points + 3) / 4, most)), MK_PREP_NT, 0,
+                          st>>>(prep);
     MK_CHECK_CUDA(cudaGetLastError());
     const size_t leaf_smem = (size_t)T * 24;
     MK_CHECK_CUDA(cudaFuncSetAttribute((const void *)mk_node_leaf_kernel,
@@ -1879,15 +1949,27 @@ extern "C" int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, c
         A.partial = reinterpret_cast<double2 *>(cw);
         if (plan->n_members > 0) {
             const long long nodes0 = P.patches[MK_COARSE] * n0 * n0;
-            const MkNodeRec *r0 = rec[MK_COARSE] + F.off[MK_COARSE] * n0 * n0, *rs = rec[3] + F.off[MK_COARSE] * ns * ns;
-            int rc = MK_OK;
-            if (ns == 14 && n0 == 20)
-                rc = mk_launch_leaf8<20, 14>(A, members, plan->n_members, r0, rs, nodes0, V[0], st);
-            else if (ns == 12 && n0 == 16)
-                rc = mk_launch_leaf8<16, 12>(A, members, plan->n_members, r0, rs, nodes0, V[0], st);
-            else
-                leaf(members, nullptr, plan->n_members, r0, nodes0, V[0]);
-            if (rc != MK_OK) return rc;
+            const MkNodeRec *r0 = rec[MK_COARSE] + F.off[MK_COARSE] * n0 * n0;
+            if (!plan->ns[0]) leaf(members, nullptr, plan->n_members, r0, nodes0, V[0]);
+            for (int c = 0; c < 2 && plan->ns[0]; ++c) {
+                const int n = c ? plan->n_members - plan->n_narrow : plan->n_narrow, ns = plan->ns[c];
+                if (n == 0) continue;
+                MkSubArgs B = sub[c];
+                B.rec = rec[3 + c] + F.off[MK_COARSE] * ns * ns;
+                int rc = MK_OK;
+                switch (n0 * 100 + ns) {
+                case 2014: rc = mk_launch_leaf8<20, 14>(A, B, n, r0, nodes0, V[0], st); break;
+                case 2012: rc = mk_launch_leaf8<20, 12>(A, B, n, r0, nodes0, V[0], st); break;
+                case 1612: rc = mk_launch_leaf8<16, 12>(A, B, n, r0, nodes0, V[0], st); break;
+                case 1610: rc = mk_launch_leaf8<16, 10>(A, B, n, r0, nodes0, V[0], st); break;
+                case 1210: rc = mk_launch_leaf8<12, 10>(A, B, n, r0, nodes0, V[0], st); break;
+                case 1208: rc = mk_launch_leaf8<12, 8>(A, B, n, r0, nodes0, V[0], st); break;
+                case 1008: rc = mk_launch_leaf8<10, 8>(A, B, n, r0, nodes0, V[0], st); break;
+                case 806: rc = mk_launch_leaf8<8, 6>(A, B, n, r0, nodes0, V[0], st); break;
+                default: leaf(B.list, B.rows, n, r0, nodes0, V[0]);
+                }
+                if (rc != MK_OK) return rc;
+            }
         }
         if (plan->n_msingle > 0)
             leaf(reinterpret_cast<const int *>(db + plan->off_msingle), reinterpret_cast<const int *>(db + plan->off_mrow),

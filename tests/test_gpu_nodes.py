@@ -95,7 +95,7 @@ def test_leaf_by_eighths_matches_fp64_and_split(cuda, cells, dilute, shape, dist
     pix = engine.Pixels(np.asarray(D.pixel_coordinates) / 1e10, *shape, phys, device=cuda)
     tiles = engine.Tiles(atoms, B.k, 512, device=cuda)
     plan = engine.NodePlan.make(tiles, pix, B.k, (1.0, 0.0, 0.0), 1e-6, direct=1.0, group_tiles=8)
-    assert plan is not None and plan.plan.n0 == n0 and plan.plan.ns > 0 and plan.plan.n_members > 0
+    assert plan is not None and plan.plan.n0 == n0 and plan.plan.ns[0] > 0 and plan.plan.n_members > 0
     acc = torch.full((pix.n, 2), float("nan"), dtype=torch.float64, device=cuda)
     wide = plan.wide is not None
     if wide:
@@ -189,6 +189,33 @@ def test_scan_nodes_match_single_fp64_exposures(cuda):
     scan.replay()
     torch.cuda.synchronize()
     assert torch.equal(scan.out, first) and torch.equal(scan.sums, s1)
+
+
+@pytest.mark.parametrize("npix, dist, n0", [(48, 0.5e10, 8), (32, 0.2e10, 10), (48, 0.2e10, 12), (96, 0.2e10, 16),
+                                            (128, 0.2e10, 20)])
+def test_eighths_of_either_class_match_the_direct_sum(cuda, npix, dist, n0):
+    """Enough tiles and frames for two classes of tiles, on every count of
+    coarse nodes: the scan in node form against the scan by the split kernel,
+    and one frame against FP64."""
+    w, sample = _case(28)
+    B = w.beam
+    theta = np.radians(w.meta["theta_deg"])
+    frames = frames_from_motors(w.stage, _det(w, (128, 128), dist), [dict(mu=theta + np.radians(0.1 * i)) for i in range(12)],
+                                [npix] * 12)
+    scan = BatchedScan(B, sample, frames, apply_polarization=True)
+    plan = scan.nodes.plan
+    assert plan.n0 == n0 and plan.ns[0] > 0 and 0 < plan.n_narrow <= plan.n_members
+    assert (plan.ns[1] > 0) == (n0 >= 12)
+    got = scan.run()[0].clone()
+    direct = BatchedScan(B, sample, frames, apply_polarization=True, nodes=False)
+    ref = direct.run()[0]
+    engine.sync()
+    assert float((got - ref).norm(dim=1).max() / ref.norm(dim=1).max()) <= 2e-5
+    B._use_fast_kernel = False
+    exact = B.interact_beam_gpu(sample, frames[5].pixels, frames[5].shape,
+                                StaticStage(frames[5].rotation, frames[5].translation),
+                                apply_polarization=True, spherical_decay=False, return_double=True)
+    assert rel_intensity(scan.frame_field(5), exact) <= 1e-4
 
 
 @pytest.mark.parametrize("acceptance", [0.0, 1.1e-3, "edge", 1.0])

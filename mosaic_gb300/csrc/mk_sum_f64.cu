@@ -5,6 +5,8 @@
 // uncontracted C oracle, every product and sum rounds separately: the
 // absolute phase k (x + r) is ~1e10 rad, where one double ulp is ~2e-6 rad,
 // and a contracted build would differ from the CPU result at that level.
+#include <type_traits>
+
 #include "mk_common.cuh"
 
 int mk_launch_reduce(const double2 *partial, int slices, int n_pix, const double2 *phasor,
@@ -40,28 +42,56 @@ struct MkPlainArgs {
 
 // Largest |a| / |P| at which the direction-dependent factors are taken from
 // their expansion about the pixel's own direction. Per pixel and species the
-// kernel holds f0 and its first two derivatives in cos(2 theta); per term only
-// the CHANGE from the pixel's direction is formed in FP32 and added to the
-// FP64 value. At the limit, with c = b / (2 lambda^2) <= 240 (b <= 180 A^2, 20
-// keV): the change is at most c e = 4e-5 of a term of f0, so FP32 leaves 2e-12
-// of that term (1e-13 for the b ~ 1/s^2 that count at a reflection); f0's third
-// order (c e)^3 / 6 is 8e-15, the direction's second order in polarization and
-// decay below 1e-13 for P_pol > 1/4. Beyond the limit, with an analyser, at
-// P_pol < 1/4 and at the Q_cut edge every factor is evaluated per term as the
+// kernel holds the factor F there (f0 + f' + i f'', Debye-Waller, polarization)
+// and the first two derivatives of f0 in cos(2 theta); per term only the
+// CHANGE from the pixel's direction, 1 + eta, is formed in FP32 and multiplied
+// into the phasor, and F into the sum of a species' terms. At the limit, with c =
+// b / (2 lambda^2) <= 240 (b <= 180 A^2, 20 keV): the change is at most c e =
+// 4e-5 of a term of f0, so FP32 leaves 2e-12 of that term (1e-13 for the b ~
+// 1/s^2 that count at a reflection); f0's third order (c e)^3 / 6 is 8e-15, the
+// second order in polarization and decay below 1e-13 for P_pol > 1/4. Beyond
+// the limit, with an analyser, at P_pol < 1/4, at the Q_cut edge and where F is
+// too small beside its derivative every factor is evaluated per term as the
 // reference does.
-// There the sine and cosine of fmod(x, 2 pi) (2 pi the double) come from a
-// table: x = q h + d with h = 2 pi / 256, q h exact to d's last bit in one FMA
-// and q read off the low bits of x / h + 1.5 2^52 (|x| < 1e13); cos and sin of
-// d, |d| <= h / 2, are their Taylor polynomials to d^6 and d^5 (below 9e-18),
-// and those of the table's angle rotate them. Absolute error ~2e-16, next to
-// the 2e-6 rad that one ulp of the phase is worth.
-// The kernel is bound by the FP64 pipe (2 lane operations per clock and SM):
-// of ~320 operations a term most went to 5 exp, 2 divisions, 2 further square
-// roots, fmod and sincos (32,000 atoms x 1,920 pixels: 31.3 ms); with the
-// factors expanded 10.1 ms, with the table 7.2 ms.
+//
+// The phase k (a_x + r) keeps the reference's roundings bit for bit. r = the
+// rounded root of v = |P - a|^2 comes from a start r0 = R0 - u.a + (|a|^2 -
+// (u.a)^2) / 2 R0, its change from R0 in FP32: within |a| 2e-7 of r (240 ulps at
+// the limit), so that r0 + (v - r0^2) / (2 r0), one Newton step with the residue
+// from an FMA and 1 / r0 to 1e-14, is r to 1e-11 ulp before its rounding.
+// The sine and cosine of fmod(x, 2 pi) (2 pi the double) come from a table: x =
+// q h + d with h = 2 pi / 1024, q h exact to d's last bit in one FMA and q read
+// off the low bits of x / h + 1.5 2^52 (|x| < 1e13); the rotation by d is
+// 1 + i d in FP64, and its higher orders (d^2 / 2 <= 5e-6, d^3 / 6) in FP32,
+// 3e-13 at most, next to the 2e-6 rad that one ulp of the phase is worth.
+// FP32 values enter and leave FP64 by their bits: a conversion is an operation
+// of the FP64 pipe too.
+//
+// The kernel is bound by that pipe (2 lane operations per clock and SM). A term
+// was ~320 operations (5 exp, 2 divisions, 3 square roots, fmod, sincos):
+// 32,000 atoms x 1,920 pixels 31.3 ms; ~60 with the factors expanded and a sine
+// table of 256 angles and FP64 polynomials: 7.2 ms; 23 now (25 with complex
+// amplitudes): 3.0 ms.
 #define F64_FAR 1.5e-7f
 #define F64_PHASE_MAX 1e13   // largest phase the table's reduction takes [rad]
-#define F64_CS 256           // table angles
+#define F64_CS 1024          // table angles
+
+// A float's value by its bits; 0 below the smallest normal number.
+__device__ __forceinline__ double mk_widen(float f)
+{
+    const unsigned b = __float_as_uint(f);
+    const unsigned hi = (b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + (896u << 20));
+    return __hiloint2double((b & 0x7f800000u) ? (int)hi : 0, (b & 0x7f800000u) ? (int)(b << 29) : 0);
+}
+
+// A double in (1e-37, 1e38) or 0 rounded to float by its bits; smaller ones 0.
+__device__ __forceinline__ float mk_narrow(double d)
+{
+    const long long b = __double_as_longlong(d) + (1ll << 28);
+    const unsigned hi = (unsigned)(b >> 32), mag = hi & 0x7fffffffu;
+    const unsigned m = __funnelshift_l((unsigned)b, mag - (896u << 20), 3);
+    return __uint_as_float(mag > (897u << 20) ? (hi & 0x80000000u) | m : 0u);
+}
 
 template <bool FAR>
 __global__ void __launch_bounds__(F64_NT) mk_plain_f64_kernel(
@@ -74,12 +104,15 @@ __global__ void __launch_bounds__(F64_NT) mk_plain_f64_kernel(
     __shared__ double s_pos[F64_ATOMS][3];
     __shared__ double2 s_amp[F64_ATOMS];
     __shared__ float4 s_posf[F64_ATOMS];          // position in FP32, species (bits)
+    __shared__ float s_aa[F64_ATOMS];             // |a|^2
+    __shared__ int s_complex;                     // an amplitude of the step has an imaginary part
     __shared__ double s_ani[MK_MAX_SPECIES];
     __shared__ float s_wk[MK_MAX_SPECIES][11];
     __shared__ double2 s_cs[FAR ? F64_CS : 1];    // cos, sin of j 2 pi / F64_CS
+    __shared__ float2 s_csf[FAR ? F64_CS : 1];
     __shared__ unsigned s_far;                    // largest |a| of the step, float bits
-    extern __shared__ __align__(16) double s_f0[];           // FAR: [S][NT], then the derivatives
-    float2 *s_df = reinterpret_cast<float2 *>(s_f0 + (FAR ? A.sp.n * F64_NT : 0));
+    extern __shared__ __align__(16) double2 s_F[];           // FAR: [S][NT] F, then f0', f0''/2 and 1/F0
+    float4 *s_df = reinterpret_cast<float4 *>(s_F + (FAR ? A.sp.n * F64_NT : 0));
     const int p = blockIdx.x * F64_NT + threadIdx.x;
     const bool live = p < n_pix;
     for (int i = threadIdx.x; i < MK_MAX_SPECIES * 11; i += F64_NT)
@@ -96,19 +129,29 @@ __global__ void __launch_bounds__(F64_NT) mk_plain_f64_kernel(
 
     // the pixel's own direction: ux = cos(2 theta), and what changes with it
     bool expand = false, forward = false;
-    double ux = 0.0, scale0 = MK_R_E;
+    double scale0 = MK_R_E, half_inv = 0.0;
     float vx = 0.f, vy = 0.f, vz = 0.f, inv_R = 0.f, inv_P = 0.f, gx = 0.f, s2x = 0.f, ex = 0.f, ey = 0.f,
           ez = 0.f, eu = 0.f;
     if (FAR) {
-        for (int i = threadIdx.x; i < F64_CS; i += F64_NT) {
+        // every fourth angle by sincos, the three after it by rotation
+        double c1[3], s1[3];
+        for (int i = 0; i < 3; ++i) sincos((i + 1) * (MK_TWO_PI / F64_CS), &s1[i], &c1[i]);
+        for (int i = threadIdx.x; i < F64_CS / 4; i += F64_NT) {
             double sn, c;
-            sincos(i * (MK_TWO_PI / F64_CS), &sn, &c);
-            s_cs[i] = make_double2(c, sn);
+            sincos(i * (4.0 * MK_TWO_PI / F64_CS), &sn, &c);
+            for (int j = 0; j < 4; ++j) {
+                const double2 v = j == 0 ? make_double2(c, sn)
+                                         : make_double2(fma(c, c1[j - 1], -(sn * s1[j - 1])),
+                                                        fma(sn, c1[j - 1], c * s1[j - 1]));
+                s_cs[4 * i + j] = v;
+                s_csf[4 * i + j] = make_float2((float)v.x, (float)v.y);
+            }
         }
         __syncthreads();
         if (live && R0 > 0.0) {
             expand = A.k * R0 < 0.25 * F64_PHASE_MAX;       // x = k (a_x + r) < 2.1 k R0
-            ux = cx / R0;
+            const double ux = cx / R0;
+            half_inv = 0.5 / R0;
             const double uy = cy / R0, uz = cz / R0;
             vx = (float)ux; vy = (float)uy; vz = (float)uz;
             inv_R = (float)(1.0 / R0);
@@ -118,23 +161,6 @@ __global__ void __launch_bounds__(F64_NT) mk_plain_f64_kernel(
             if (A.remove_forward) {
                 forward = Q < qcut;
                 if (!(fabs(Q - qcut) > 1e-6 * A.k)) expand = false;   // Q changes by k e at most
-            }
-            for (int s = 0; s < A.sp.n; ++s) {
-                const float *wk = s_wk[s];
-                double f0 = wk[5], f1 = 0.0, f2 = 0.0;
-                for (int i = 0; i < 5; ++i) {
-                    const double b = (double)wk[6 + i], t = (double)wk[i] * exp(-b * s2), d = -b * ds2;
-                    f0 += t;
-                    f1 += t * d;
-                    f2 += t * d * d;
-                }
-                double fre = f0 + A.sp.anr[s];
-                if (forward) fre -= (double)A.sp.f0z[s] + A.sp.anr[s];
-                double w = 1.0;
-                if (A.sp.has_dw) w = exp(-(double)A.sp.dwb[s] * s2);
-                s_f0[s * F64_NT + threadIdx.x] = fre;
-                s_df[s * F64_NT + threadIdx.x] = make_float2((float)f1, (float)(0.5 * f2));
-                if (A.sp.has_dw) s_f0[(2 * A.sp.n + s) * F64_NT + threadIdx.x] = w;
             }
             if (A.apply_pol) {
                 const double e = A.ex * ux + A.ey * uy + A.ez * uz;
@@ -146,12 +172,38 @@ __global__ void __launch_bounds__(F64_NT) mk_plain_f64_kernel(
                 eu = (float)e;
                 ex = (float)A.ex; ey = (float)A.ey; ez = (float)A.ez;
             }
+            for (int s = 0; s < A.sp.n; ++s) {
+                const float *wk = s_wk[s];
+                double f0 = wk[5], f1 = 0.0, f2 = 0.0;
+                for (int i = 0; i < 5; ++i) {
+                    const double b = (double)wk[6 + i], t = (double)wk[i] * exp(-b * s2), d = -b * ds2;
+                    f0 += t;
+                    f1 += t * d;
+                    f2 += t * d * d;
+                }
+                double fre = f0 + A.sp.anr[s], fim = A.sp.ani[s];
+                if (forward) {
+                    fre -= (double)A.sp.f0z[s] + A.sp.anr[s];
+                    fim = 0.0;
+                }
+                // F0 + change as F0 (1 + change / F0): a change of 1 % at most
+                const double m2 = fre * fre + fim * fim;
+                if (!(f1 * f1 * 1e-13 < 1e-4 * m2)) expand = false;
+                double w = scale0;
+                if (A.sp.has_dw) w *= exp(-(double)A.sp.dwb[s] * s2);
+                s_F[s * F64_NT + threadIdx.x] = make_double2(fre * w, fim * w);
+                s_df[s * F64_NT + threadIdx.x] =
+                    make_float4((float)f1, (float)(0.5 * f2), (float)(fre / m2), (float)(-fim / m2));
+            }
         }
     }
     for (int64_t a0 = a_lo; a0 < a_hi; a0 += F64_ATOMS) {
         const int m = (int)min((int64_t)F64_ATOMS, a_hi - a0);
         __syncthreads();
-        if (threadIdx.x == 0) s_far = 0u;
+        if (threadIdx.x == 0) {
+            s_far = 0u;
+            s_complex = 0;
+        }
         __syncthreads();
         for (int j = threadIdx.x; j < m; j += F64_NT) {
             const double x = pos[3 * (a0 + j)], y = pos[3 * (a0 + j) + 1], z = pos[3 * (a0 + j) + 2];
@@ -162,56 +214,85 @@ __global__ void __launch_bounds__(F64_NT) mk_plain_f64_kernel(
             s_amp[j] = make_double2(e.x, e.y);
             s_posf[j] = make_float4((float)x, (float)y, (float)z, __int_as_float(species[a0 + j]));
             if (FAR) {
-                const float l = sqrtf((float)x * (float)x + (float)y * (float)y + (float)z * (float)z);
+                const float aa = (float)x * (float)x + (float)y * (float)y + (float)z * (float)z, l = sqrtf(aa);
+                s_aa[j] = aa;
+                if (e.y != 0.f) s_complex = 1;
                 atomicMax(&s_far, __float_as_uint(l <= 1e30f ? l : 1e30f));    // NaN: far out
             }
         }
         __syncthreads();
         if (!live) continue;
         if (FAR && expand && __uint_as_float(s_far) * inv_R < F64_FAR) {
-            for (int j = 0; j < m; ++j) {
-                const double ax = s_pos[j][0], ay = s_pos[j][1], az = s_pos[j][2];
-                const float4 pf = s_posf[j];
-                const int s = __float_as_int(pf.w);
-                const double dx = cx - ax, dy = cy - ay, dz = cz - az;
-                const double r = sqrt(dx * dx + dy * dy + dz * dz);
-                // cos and sin of the phase mod 2 pi
-                const double x = A.k * (ax + r), magic = 6755399441055744.0;
-                const double t52 = fma(x, F64_CS / MK_TWO_PI, magic);
-                const double d = fma(-(t52 - magic), MK_TWO_PI / F64_CS, x);
-                const double2 cs = s_cs[__double2loint(t52) & (F64_CS - 1)];
-                const double d2 = d * d;
-                const double sd = fma(d * d2, fma(d2, 1.0 / 120.0, -1.0 / 6.0), d);
-                const double cd = d2 * fma(d2, fma(d2, -1.0 / 720.0, 1.0 / 24.0), -0.5);   // cos d - 1
-                const double c = fma(cs.x, cd, fma(-cs.y, sd, cs.x));
-                const double sn = fma(cs.y, cd, fma(cs.x, sd, cs.y));
-                const float ua = fmaf(vz, pf.z, fmaf(vy, pf.y, vx * pf.x));
-                // change of cos(2 theta): (dx - ux r) / r, the difference in FP64
-                const float t = (float)(dx - ux * r) * inv_R;
-                const float2 df = s_df[s * F64_NT + threadIdx.x];
-                const double fre = s_f0[s * F64_NT + threadIdx.x] + (double)(fmaf(df.y, t, df.x) * t);
-                const double fim = forward ? 0.0 : s_ani[s];
-                float sig = A.decay ? ua * inv_R : 0.f;      // R0 / r - 1
-                if (A.apply_pol) {
-                    // P_pol's change over P_pol, and its root's; e.u' changes by te
-                    const float te = -(fmaf(ez, pf.z, fmaf(ey, pf.y, ex * pf.x)) - ua * eu) * inv_R;
-                    const float pd = (float)A.pdeg;
-                    const float q = (t * fmaf(0.5f * (1.f - pd), t, gx) - pd * te * fmaf(2.f, eu, te)) * inv_P;
-                    const float h = q * fmaf(-0.125f, q, 0.5f);
-                    sig = fmaf(h, sig, h + sig);
+            auto terms = [&](auto complex_amp) {
+                double sr = 0.0, si = 0.0;
+                int species = __float_as_int(s_posf[0].w);
+                float4 df = s_df[species * F64_NT + threadIdx.x];
+                auto flush = [&]() {
+                    const double2 F = s_F[species * F64_NT + threadIdx.x];
+                    acc_r = fma(F.x, sr, fma(-F.y, si, acc_r));
+                    acc_i = fma(F.x, si, fma(F.y, sr, acc_i));
+                };
+                for (int j = 0; j < m; ++j) {
+                    const double ax = s_pos[j][0], ay = s_pos[j][1], az = s_pos[j][2];
+                    const float4 pf = s_posf[j];
+                    const int s = __float_as_int(pf.w);
+                    if (s != species) {            // uniform across the block
+                        flush();
+                        sr = si = 0.0;
+                        species = s;
+                        df = s_df[species * F64_NT + threadIdx.x];
+                    }
+                    const double dx = cx - ax, dy = cy - ay, dz = cz - az;
+                    const double v = dx * dx + dy * dy + dz * dz;
+                    const float ua = fmaf(vz, pf.z, fmaf(vy, pf.y, vx * pf.x)), across = fmaf(-ua, ua, s_aa[j]);
+                    const float dr = fmaf(0.5f * inv_R, across, -ua);        // r - R0
+                    const double r0 = R0 + mk_widen(dr);
+                    const double r = fma(fma(-r0, r0, v), fma(half_inv, mk_widen(-dr * inv_R), half_inv), r0);
+                    // cos and sin of the phase mod 2 pi
+                    const double x = A.k * (ax + r), magic = 6755399441055744.0;
+                    const double t52 = fma(x, F64_CS / MK_TWO_PI, magic);
+                    const double d = fma(-(t52 - magic), MK_TWO_PI / F64_CS, x);
+                    const int q = __double2loint(t52) & (F64_CS - 1);
+                    const double2 cs = s_cs[q];
+                    const float2 cf = s_csf[q];
+                    const float d1 = mk_narrow(d), d2 = d1 * d1;
+                    const float cd = d2 * fmaf(d2, 1.f / 24.f, -0.5f), sd = d1 * d2 * (-1.f / 6.f);   // cos d - 1, sin d - d
+                    const float hc = fmaf(cf.x, cd, -cf.y * sd), hs = fmaf(cf.y, cd, cf.x * sd);
+                    const float c1 = fmaf(-cf.y, d1, cf.x) + hc, s1 = fmaf(cf.x, d1, cf.y) + hs;
+                    // change of cos(2 theta), to second order in e = a / R0
+                    const float ue = ua * inv_R, exx = pf.x * inv_R;
+                    const float t = fmaf(-exx, ue, fmaf(vx, ue, -exx)) +
+                                    vx * fmaf(ue, ue, -0.5f * across * inv_R * inv_R);
+                    float sig = A.decay ? ue : 0.f;      // R0 / r - 1
+                    if (A.apply_pol) {
+                        // P_pol's change over P_pol, and its root's; e.u' changes by te
+                        const float te = -(fmaf(ez, pf.z, fmaf(ey, pf.y, ex * pf.x)) - ua * eu) * inv_R;
+                        const float pd = (float)A.pdeg;
+                        const float g = (t * fmaf(0.5f * (1.f - pd), t, gx) - pd * te * fmaf(2.f, eu, te)) * inv_P;
+                        const float h = g * fmaf(-0.125f, g, 0.5f);
+                        sig = fmaf(h, sig, h + sig);
+                    }
+                    if (A.sp.has_dw) {
+                        const float b = -A.sp.dwb[s] * s2x * t, h = b * fmaf(0.5f, b, 1.f);
+                        sig = fmaf(h, sig, h + sig);
+                    }
+                    // 1 + eta = (1 + change of f0 / F0) (1 + sig)
+                    const float df0 = fmaf(df.y, t, df.x) * t, fr = df0 * df.z, fi = df0 * df.w;
+                    const float er = fmaf(fr, sig, fr + sig), ei = fmaf(fi, sig, fi);
+                    const double c = fma(-cs.y, d, cs.x) + mk_widen(fmaf(c1, er, fmaf(-s1, ei, hc)));
+                    const double sn = fma(cs.x, d, cs.y) + mk_widen(fmaf(s1, er, fmaf(c1, ei, hs)));
+                    const double2 E = s_amp[j];
+                    sr = fma(E.x, c, sr);
+                    si = fma(E.x, sn, si);
+                    if constexpr (decltype(complex_amp)::value) {
+                        sr = fma(-E.y, sn, sr);
+                        si = fma(E.y, c, si);
+                    }
                 }
-                double sc = scale0;
-                if (A.sp.has_dw) {
-                    const float d = -A.sp.dwb[s] * s2x * t, h = d * fmaf(0.5f, d, 1.f);
-                    sig = fmaf(h, sig, h + sig);
-                    sc *= s_f0[(2 * A.sp.n + s) * F64_NT + threadIdx.x];
-                }
-                const double scale = fma(sc, (double)sig, sc);
-                const double er = s_amp[j].x, ei = s_amp[j].y;
-                const double tr = er * fre - ei * fim, ti = er * fim + ei * fre;
-                acc_r += (tr * c - ti * sn) * scale;
-                acc_i += (tr * sn + ti * c) * scale;
-            }
+                flush();
+            };
+            if (s_complex) terms(std::true_type{});
+            else terms(std::false_type{});
             continue;
         }
         for (int j = 0; j < m; ++j) {
@@ -327,8 +408,8 @@ extern "C" int mk_kin_plain_f64(int64_t n, const double *pos, const int *species
     const int ns_eff = (int)((n + per - 1) / per);
     dim3 grid((n_pix + F64_NT - 1) / F64_NT, ns_eff);
     double2 *part = static_cast<double2 *>(workspace);
-    // expansions per (species, pixel): f0, its derivatives and the Debye-Waller factor
-    const size_t smem = A.analyser ? 0 : (A.sp.has_dw ? 3 : 2) * sizeof(double) * (size_t)A.sp.n * F64_NT;
+    // expansions per (species, pixel): the factor and its derivatives
+    const size_t smem = A.analyser ? 0 : (sizeof(double2) + sizeof(float4)) * (size_t)A.sp.n * F64_NT;
     auto fn = A.analyser ? mk_plain_f64_kernel<false> : mk_plain_f64_kernel<true>;
     MK_CHECK_CUDA(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     fn<<<grid, F64_NT, smem, st>>>(n, per, pos, species, reinterpret_cast<const float2 *>(amp), n_pix, px->xyz,

@@ -26,32 +26,100 @@ __device__ __forceinline__ float mk_tsc(double d)
 // The float32 lab position [A] that mk_atoms_lab divided by 1e10: the double
 // quotient times 1e10 is within two double ulps of it, so the cast recovers it.
 __device__ __forceinline__ float mk_lab_A(double m) { return (float)(m * 1e10); }
+// The same by floats: m = h + l, times 1e10 (a float's 24 bits hold it).
+__device__ __forceinline__ float mk_lab_A2(double m)
+{
+    const float h = (float)m, l = (float)(m - (double)h);
+    const float p = h * 1e10f;
+    return p + fmaf(l, 1e10f, fmaf(h, 1e10f, -p));
+}
 
+// A value as an unevaluated sum of two floats.
+struct MkF2 {
+    float h, l;
+};
+// h + l renormalised, |h| >= |l|.
+__device__ __forceinline__ MkF2 mk_fast2(float h, float l)
+{
+    const float s = h + l;
+    return MkF2{s, l - (s - h)};
+}
+
+// Beam-grid coordinate x / d + c of a float32 lab position x [A], to 2^-46 of it
+// (~1e-11 cells): i the nearest cell, f the rest. False within 1e-6 cells of a
+// cell's edge or of the grid's (n cells), and off the grid by more than half a
+// cell: the FP64 formula decides there.
+__device__ __forceinline__ bool mk_cell(float x, MkF2 inv, MkF2 c, int n, int *i, MkF2 *f)
+{
+    const float q = x * inv.h;
+    const float qe = fmaf(x, inv.l, fmaf(x, inv.h, -q));
+    const float s = q + c.h, b = s - q;
+    const float e = (q - (s - b)) + (c.h - b) + qe + c.l;        // two-sum, then the low parts
+    const float r = rintf(s);
+    if (!(fabsf(r) < 4e6f)) return false;
+    *f = mk_fast2(s - r, e);                                      // s - r is exact
+    *i = (int)r;
+    return fabsf(f->h) < 0.5f - 1e-6f && s > 1e-6f && s < (float)(n - 1) - 1e-6f;
+}
+
+// The three weights of cells i - 1, i, i + 1, rounded once as the FP64 formula's
+// are: 0.75 - f^2 and (0.5 -+ f)^2 / 2.
+__device__ __forceinline__ void mk_tsc3(MkF2 f, float (&w)[3])
+{
+    const float p = f.h * f.h, pe = fmaf(f.h, f.h, -p) + 2.f * f.h * f.l;
+    const MkF2 a = mk_fast2(0.75f, -p);
+    w[1] = a.h + (a.l - pe);
+#pragma unroll
+    for (int k = 0; k < 3; k += 2) {
+        MkF2 t = mk_fast2(0.5f, k ? f.h : -f.h);
+        t.l += k ? f.l : -f.l;
+        const float q = t.h * t.h;
+        w[k] = 0.5f * (q + (fmaf(t.h, t.h, -q) + 2.f * t.h * t.l));
+    }
+}
+
+// One atom a thread. In FP64 throughout (two divisions, six weights a thread of
+// ~15 operations each) the kernel was bound by that pipe's two lanes a clock: 479
+// us for 2M atoms on a 256 x 256 grid. The grid coordinates in two-float
+// arithmetic leave one FP64 subtraction a coordinate and the float atomics: 153
+// us.
 __global__ void mk_column_deposit_kernel(int64_t n, const double *__restrict__ pos,
                                          const int *__restrict__ species,
                                          const float2 *__restrict__ fwd, int ny, int nz,
-                                         double du, double dv, double uc, double vc,
-                                         float *__restrict__ sr, float *__restrict__ si)
+                                         double du, double dv, double uc, double vc, MkF2 idu, MkF2 idv,
+                                         MkF2 ucf, MkF2 vcf, float *__restrict__ sr, float *__restrict__ si)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     // +x beam: the transverse basis is (y, z)
-    const double iu = (double)mk_lab_A(pos[3 * i + 1]) / du + uc;
-    const double iv = (double)mk_lab_A(pos[3 * i + 2]) / dv + vc;
-    if (!(iu >= 0.0 && iu <= (double)(ny - 1) && iv >= 0.0 && iv <= (double)(nz - 1))) return;
+    const double y = pos[3 * i + 1], z = pos[3 * i + 2];
+    int ic, jc;
+    float wx[3], wy[3];
+    MkF2 fu, fv;
+    if (mk_cell(mk_lab_A2(y), idu, ucf, ny, &ic, &fu) && mk_cell(mk_lab_A2(z), idv, vcf, nz, &jc, &fv)) {
+        mk_tsc3(fu, wx);
+        mk_tsc3(fv, wy);
+    } else {
+        const double iu = (double)mk_lab_A(y) / du + uc, iv = (double)mk_lab_A(z) / dv + vc;
+        if (!(iu >= 0.0 && iu <= (double)(ny - 1) && iv >= 0.0 && iv <= (double)(nz - 1))) return;
+        ic = (int)floor(iu + 0.5);
+        jc = (int)floor(iv + 0.5);
+        for (int d = -1; d <= 1; ++d) {
+            wx[d + 1] = mk_tsc(fabs(iu - (double)(ic + d)));
+            wy[d + 1] = mk_tsc(fabs(iv - (double)(jc + d)));
+        }
+    }
     const float2 f = fwd[species[i]];
-    const long long ic = (long long)floor(iu + 0.5), jc = (long long)floor(iv + 0.5);
 #pragma unroll
     for (int dx = -1; dx <= 1; ++dx) {
-        const long long ii = ic + dx;
-        const float wx = mk_tsc(fabs(iu - (double)ii));
+        const int ii = ic + dx;
 #pragma unroll
         for (int dy = -1; dy <= 1; ++dy) {
-            const long long jj = jc + dy;
-            const float fac = __fmul_rn(wx, mk_tsc(fabs(iv - (double)jj)));
+            const int jj = jc + dy;
+            const float fac = __fmul_rn(wx[dx + 1], wy[dy + 1]);
             if (ii < 0 || ii >= ny || jj < 0 || jj >= nz || !(fac > 0.f)) continue;
-            atomicAdd(&sr[ii * nz + jj], __fmul_rn(f.x, fac));
-            atomicAdd(&si[ii * nz + jj], __fmul_rn(f.y, fac));
+            atomicAdd(&sr[(long long)ii * nz + jj], __fmul_rn(f.x, fac));
+            atomicAdd(&si[(long long)ii * nz + jj], __fmul_rn(f.y, fac));
         }
     }
 }
@@ -70,10 +138,12 @@ extern "C" int mk_beam_column_sums(int64_t n, const double *pos_lab, const int *
     MK_CHECK_CUDA(cudaMemsetAsync(sum_re, 0, m * sizeof(float), st));
     MK_CHECK_CUDA(cudaMemsetAsync(sum_im, 0, m * sizeof(float), st));
     if (n == 0) return MK_OK;
+    auto two = [](double x) { return MkF2{(float)x, (float)(x - (double)(float)x)}; };
     const int th = 256;
     mk_column_deposit_kernel<<<(unsigned)((n + th - 1) / th), th, 0, st>>>(
         n, pos_lab, species, reinterpret_cast<const float2 *>(fwd), grid_ny, grid_nz, grid[0],
-        grid[1], grid[2], grid[3], sum_re, sum_im);
+        grid[1], grid[2], grid[3], two(1.0 / grid[0]), two(1.0 / grid[1]), two(grid[2]), two(grid[3]), sum_re,
+        sum_im);
     MK_CHECK_CUDA(cudaGetLastError());
     return MK_OK;
 }

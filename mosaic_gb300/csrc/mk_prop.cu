@@ -23,22 +23,28 @@ __device__ __forceinline__ double mk_fftfreq(int i, int n, double d)
 }
 
 // Pad (nz, ny) into (nz2, ny2) centred at (z0, y0): edge replication
-// (mode 0) or a constant (mode 1).
+// (mode 0) or a constant (mode 1). PTS points a thread: two where rows have an
+// even number of points and start on 16 bytes.
+template <int PTS>
 __global__ void mk_prop_pad_kernel(const float2 *__restrict__ in, int ny, int nz,
                                    float2 *__restrict__ out, int ny2, int nz2, int y0, int z0,
                                    int mode, float2 cval)
 {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    const int x0 = PTS * (blockIdx.x * blockDim.x + threadIdx.x);
     const int y = blockIdx.y;
-    if (x >= ny2 || y >= nz2) return;
-    const int sx = x - y0, sz = y - z0;
-    float2 v;
-    if (mode == 1 && (sx < 0 || sx >= ny || sz < 0 || sz >= nz)) {
-        v = cval;
-    } else {
-        v = in[min(max(sz, 0), nz - 1) * ny + min(max(sx, 0), ny - 1)];
+    if (x0 >= ny2 || y >= nz2) return;
+    const int sz = y - z0;
+    const bool off = mode == 1 && (sz < 0 || sz >= nz);
+    const float2 *row = in + (size_t)min(max(sz, 0), nz - 1) * ny;
+    float2 v[PTS];
+#pragma unroll
+    for (int i = 0; i < PTS; ++i) {
+        const int sx = x0 + i - y0;
+        v[i] = off || (mode == 1 && (sx < 0 || sx >= ny)) ? cval : row[min(max(sx, 0), ny - 1)];
     }
-    out[(size_t)y * ny2 + x] = v;
+    float2 *o = out + (size_t)y * ny2 + x0;
+    if (PTS == 2) *reinterpret_cast<float4 *>(o) = make_float4(v[0].x, v[0].y, v[PTS - 1].x, v[PTS - 1].y);
+    else o[0] = v[0];
 }
 
 __global__ void mk_prop_mul_kernel(float2 *__restrict__ F, int ny2, int nz2, double dy, double dz,
@@ -108,8 +114,11 @@ __global__ void mk_prop_crop_kernel(const float2 *__restrict__ G, int ny2, int n
 // neighbouring points) on different banks at every stride; in place and
 // unpadded, radix-2 stages fused by threes with a bit-reversal pass between
 // the transforms ran 8-way conflicts and took 299 us for the 2048 x 4096
-// spectrum of a 2048 x 1500 field; this 91 us (98 MB at copy bandwidth: 15).
-// Twiddles come from a table of exp(-2 pi i t / N) made in FP64. The transfer
+// spectrum of a 2048 x 1500 field; this 81 us (98 MB at copy bandwidth: 15).
+// Twiddles exp(-2 pi i i k / M) of a pass over lines of M points come from a
+// table made in FP64, its M / 8 values of one k side by side: a warp's i are
+// neighbours. From one table of exp(-2 pi i t / N), read k 8^pass entries apart,
+// the same passes took 91 us. The transfer
 // function is formed in FP32 as the reference's prop_mul_kernel does
 // (Beam.py:4763-4830), with the two large constant phases, z (k - k_axis) and
 // -z k_axis, reduced mod 2 pi in FP64 on the host.
@@ -212,6 +221,7 @@ __global__ void __launch_bounds__(MK_FFT_NT, 2) mk_prop_cols_kernel(const __grid
     const int logw = 31 - __clz(W), items = W * (N >> 3);
     const int c0 = blockIdx.x * W;
     // forward passes
+    const float2 *tw = A.tw;
     for (int p = 0; p < P; ++p) {
         const int logm = A.logn - 3 * (p + 1), m = 1 << logm;
         for (int t = threadIdx.x; t < items; t += MK_FFT_NT) {
@@ -226,8 +236,9 @@ __global__ void __launch_bounds__(MK_FFT_NT, 2) mk_prop_cols_kernel(const __grid
             line[mk_pad8(base)] = v[0];
 #pragma unroll
             for (int k = 1; k < 8; ++k)
-                line[mk_pad8(base + (k << logm))] = mk_cmul(v[k], __ldg(A.tw + ((i * k) << (3 * p))));
+                line[mk_pad8(base + (k << logm))] = mk_cmul(v[k], __ldg(tw + (k - 1) * m + i));
         }
+        tw += 7 * m;
         __syncthreads();
     }
     // last radix, H, and back: 8 consecutive positions a thread
@@ -257,6 +268,7 @@ __global__ void __launch_bounds__(MK_FFT_NT, 2) mk_prop_cols_kernel(const __grid
     // inverse passes
     for (int p = P - 1; p >= 0; --p) {
         const int logm = A.logn - 3 * (p + 1), m = 1 << logm;
+        tw -= 7 * m;
         for (int t = threadIdx.x; t < items; t += MK_FFT_NT) {
             const int c = t & (W - 1), q = t >> logw;
             const int i = q & (m - 1), base = ((q >> logm) << (logm + 3)) + i;
@@ -265,7 +277,7 @@ __global__ void __launch_bounds__(MK_FFT_NT, 2) mk_prop_cols_kernel(const __grid
             v[0] = line[mk_pad8(base)];
 #pragma unroll
             for (int k = 1; k < 8; ++k) {
-                float2 w = __ldg(A.tw + ((i * k) << (3 * p)));
+                float2 w = __ldg(tw + (k - 1) * m + i);
                 w.y = -w.y;
                 v[k] = mk_cmul(line[mk_pad8(base + (k << logm))], w);
             }
@@ -305,17 +317,26 @@ __global__ void mk_prop_cols_short_kernel(const __grid_constant__ MkColsArgs A)
     }
 }
 
-// The tables of a column pass: twiddles exp(-2 pi i t / nz2) from FP64
-// sincospi, and 2 pi fftfreq + offset of every column and row as float32
-// (numpy ordering, in FP64).
+// The tables of a column pass: the passes' twiddles exp(-2 pi i i k / M), (7, M / 8)
+// of every M = nz2, nz2 / 8, .. >= 8, from FP64 sincospi, and 2 pi fftfreq +
+// offset of every column and row as float32 (numpy ordering, in FP64). A warp a
+// block: the FP64 pipe of every SM.
 __global__ void mk_prop_tables_kernel(float2 *__restrict__ tw, float *__restrict__ ky, float *__restrict__ kz,
                                       int ny2, int nz2, double dy, double dz, double offy, double offz)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < nz2) {
-        double s, c;
-        sincospi(-2.0 * (double)i / (double)nz2, &s, &c);
-        tw[i] = make_float2((float)c, (float)s);
+        int M = nz2, e = i;
+        while (M >= 8 && e >= 7 * (M / 8)) {
+            e -= 7 * (M / 8);
+            M /= 8;
+        }
+        if (M >= 8) {
+            const int k = e / (M / 8) + 1, t = (e % (M / 8)) * k * (nz2 / M);
+            double s, c;
+            sincospi(-2.0 * (double)t / (double)nz2, &s, &c);
+            tw[i] = make_float2((float)c, (float)s);
+        }
         kz[i] = (float)(MK_TWO_PI * mk_fftfreq(i, nz2, dz) + offz);
     }
     if (i < ny2) ky[i] = (float)(MK_TWO_PI * mk_fftfreq(i, ny2, dy) + offy);
@@ -373,7 +394,7 @@ extern "C" int mk_prop_cols_rows(float *spectrum, int ny2, int nz2, int z0, int 
     float2 *tw = reinterpret_cast<float2 *>(workspace);
     float *ky = reinterpret_cast<float *>(tw + nz2);
     float *kz = ky + ny2;
-    mk_prop_tables_kernel<<<(std::max(ny2, nz2) + 255) / 256, 256, 0, st>>>(tw, ky, kz, ny2, nz2, dy, dz,
+    mk_prop_tables_kernel<<<(std::max(ny2, nz2) + 31) / 32, 32, 0, st>>>(tw, ky, kz, ny2, nz2, dy, dz,
                                                                            k_perp_y, k_perp_z);
     MK_CHECK_CUDA(cudaGetLastError());
     MkColsArgs A;
@@ -426,10 +447,12 @@ extern "C" int mk_prop_pad(const float *field, int ny, int nz, float *padded, in
                "mk_prop_pad: bad arguments");
     MK_REQUIRE(y0 >= 0 && z0 >= 0 && y0 + ny <= ny2 && z0 + nz <= nz2, "mk_prop_pad: bad offsets");
     MK_REQUIRE(mode == 0 || mode == 1, "mk_prop_pad: mode must be 0 (edge) or 1 (constant)");
-    dim3 g((ny2 + 255) / 256, nz2);
-    mk_prop_pad_kernel<<<g, 256, 0, mk_stream(stream)>>>(
-        reinterpret_cast<const float2 *>(field), ny, nz, reinterpret_cast<float2 *>(padded), ny2,
-        nz2, y0, z0, mode, make_float2(cval_re, cval_im));
+    const bool two = ny2 % 2 == 0 && ((uintptr_t)padded & 15) == 0;
+    dim3 g((ny2 / (two ? 2 : 1) + 255) / 256, nz2);
+    auto fn = two ? mk_prop_pad_kernel<2> : mk_prop_pad_kernel<1>;
+    fn<<<g, 256, 0, mk_stream(stream)>>>(reinterpret_cast<const float2 *>(field), ny, nz,
+                                         reinterpret_cast<float2 *>(padded), ny2, nz2, y0, z0, mode,
+                                         make_float2(cval_re, cval_im));
     MK_CHECK_CUDA(cudaGetLastError());
     return MK_OK;
 }

@@ -1173,8 +1173,8 @@ __global__ void __launch_bounds__(256) mk_node_leaf_kernel(const MkNodeArgs A, c
 // coarse patch). An eighth wider than its nodes take (and every eighth of a
 // tile that keeps the |d|^2 term) is added term by term at the tile's nodes.
 // NS^2 terms an atom instead of N0^2: still bound by the MUFU. 10,321 tiles
-// on four 20 x 20 node patches 3.88 ms directly, 2.32 so; 15,814 on one of 16 x 16
-// 0.95 and 0.57 (all of them on 14 x 14 and 12 x 12 nodes: 2.78 and 0.74).
+// on four 20 x 20 node patches 3.88 ms directly, 2.07 so; 15,814 on one of 16 x 16
+// 0.95 and 0.56 (all of them on 14 x 14 and 12 x 12 nodes: 2.78 and 0.74).
 struct MkSubArgs {
     const int *list, *rows;              // tiles and the rows of their fields
     const MkNodeRec *rec;                // the eighths' nodes
@@ -1182,32 +1182,58 @@ struct MkSubArgs {
     float radius;                        // widest eighth [cycles]
     int patches;                         // of a block
 };
-// 256 threads, but 96 where there are only 288 eighth nodes (6 x 6; 466 us with
-// 288 threads, 436 with 96). Blocks of 16 NS threads for the others too, which
-// leave no round part empty, hold fewer warps an SM: 573 us instead of 524 for
-// 10 x 10.
+// Threads: 96 for the 288 nodes of 6 x 6 (a thread one: 603 us for 64 frames; two
+// 639), else 256, a thread two nodes (5.3M atoms on 12 x 12 and 14 x 14: 2.32 ->
+// 2.07 ms). Blocks that the node count divides into (224, 288, 416) hold fewer
+// warps an SM and were 1 to 25 % slower.
 __host__ __device__ constexpr int mk_leaf8_threads(int ns) { return ns == 6 ? 96 : 256; }
+// Sum of atom pairs' terms at direction w [cycles], phases relative to lin0, two
+// atoms a packed instruction.
+struct MkLeafSum {
+    mk_f2 wx, wy, wz, l0, re, im;
+    MkLeafSum() = default;
+    __device__ __forceinline__ MkLeafSum(const float3 &w, float lin0)
+        : wx(f2_splat(w.x)), wy(f2_splat(w.y)), wz(f2_splat(w.z)), l0(f2_splat(-lin0)), re(0ull), im(0ull) {}
+    __device__ __forceinline__ void add(const ulonglong2 &a, const ulonglong2 &b, const ulonglong2 &e)
+    {
+        const mk_f2 magic = f2_splat(MK_ROUND_MAGIC), two_pi = f2_splat(TWO_PI_F), m_one = f2_splat(-1.f);
+        const mk_f2 lin = f2_fma(b.x, wz, f2_fma(a.y, wy, f2_fma(a.x, wx, l0)));
+        const float2 r = f2_unpack(f2_mul(f2_sub(lin, f2_sub(f2_add(lin, magic), magic)), two_pi));
+        float s0, c0, s1, c1;
+        __sincosf(r.x, &s0, &c0);
+        __sincosf(r.y, &s1, &c1);
+        const mk_f2 c = f2_pack(c0, c1), s = f2_pack(s0, s1);
+        re = f2_fma(e.x, c, f2_fma(f2_mul(e.y, m_one), s, re));
+        im = f2_fma(e.x, s, f2_fma(e.y, c, im));
+    }
+    __device__ __forceinline__ float2 sum() const
+    {
+        const float2 r = f2_unpack(re), i = f2_unpack(im);
+        return make_float2(mk_unshort(r.x + r.y), mk_unshort(i.x + i.y));
+    }
+};
+
 template <int N0, int NS>
 __global__ void __launch_bounds__(mk_leaf8_threads(NS)) mk_node_leaf8_kernel(const MkNodeArgs A, const MkSubArgs B,
                                                                              const MkNodeRec *__restrict__ rec,
                                                                              long long n_nodes,
                                                                              float2 *__restrict__ V)
 {
-    constexpr int SQ = NS * NS, NT = mk_leaf8_threads(NS);
+    constexpr int SQ = NS * NS, NT = mk_leaf8_threads(NS), RW = N0 % 4 == 0 ? 4 : 2, ND = NS == 6 ? 1 : 2;
     extern __shared__ __align__(16) unsigned char leaf_smem[];
     const int T = A.tile_atoms, pairs = T / 16;          // atom pairs of an eighth
     float4 *s_pos = reinterpret_cast<float4 *>(leaf_smem);
     float4 *s_amp = s_pos + T;
     float2 *s_v = reinterpret_cast<float2 *>(s_amp + T / 2);        // [8][SQ]
     float2 *s_t = s_v + 8 * SQ;                                     // [8][N0][NS]
-    float *s_w = reinterpret_cast<float *>(s_t + 8 * N0 * NS);      // [N0][NS]
+    float *s_w = reinterpret_cast<float *>(s_t + 8 * N0 * NS);      // [NS][N0]
     __shared__ float4 s_c[8];                            // centre; 1 where the eighth has nodes
     const int t = B.list[blockIdx.x];
     const float4 *gp = A.tpos + (size_t)t * T;
     const float4 *ga = reinterpret_cast<const float4 *>(A.tamp + (size_t)t * T);
     for (int i = threadIdx.x; i < T; i += NT) s_pos[i] = gp[i];
     for (int i = threadIdx.x; i < T / 2; i += NT) s_amp[i] = ga[i];
-    for (int i = threadIdx.x; i < N0 * NS; i += NT) s_w[i] = B.w[i];
+    for (int i = threadIdx.x; i < N0 * NS; i += NT) s_w[i % NS * N0 + i / NS] = B.w[i];
     __syncthreads();
     const double4 o = A.origin[t];
     const float ox = (float)o.x, oy = (float)o.y, oz = (float)o.z;
@@ -1241,27 +1267,14 @@ __global__ void __launch_bounds__(mk_leaf8_threads(NS)) mk_node_leaf8_kernel(con
             s_c[s] = make_float4(c[0], c[1], c[2], !fr && r2 <= B.radius * B.radius ? 1.f : 0.f);
     }
     __syncthreads();
-    const mk_f2 magic = f2_splat(MK_ROUND_MAGIC), two_pi = f2_splat(TWO_PI_F), m_one = f2_splat(-1.f);
     const ulonglong2 *P2 = reinterpret_cast<const ulonglong2 *>(s_pos);
     const ulonglong2 *E2 = reinterpret_cast<const ulonglong2 *>(s_amp);
-    // pairs [p0, p1) at direction w, phases relative to the phase lin0 [cycles]
-    auto terms = [&](int p0, int p1, float wx_, float wy_, float wz_, float lin0) {
-        const mk_f2 wx = f2_splat(wx_), wy = f2_splat(wy_), wz = f2_splat(wz_), l0 = f2_splat(-lin0);
-        mk_f2 ar = 0ull, ai = 0ull;
+    // pairs [p0, p1) at direction w
+    auto terms = [&](int p0, int p1, const float3 &w) {
+        MkLeafSum a(w, 0.f);
 #pragma unroll 4
-        for (int p = p0; p < p1; ++p) {
-            const ulonglong2 a = P2[2 * p], b = P2[2 * p + 1], e = E2[p];
-            const mk_f2 lin = f2_fma(b.x, wz, f2_fma(a.y, wy, f2_fma(a.x, wx, l0)));
-            const float2 r = f2_unpack(f2_mul(f2_sub(lin, f2_sub(f2_add(lin, magic), magic)), two_pi));
-            float s0, c0, s1, c1;
-            __sincosf(r.x, &s0, &c0);
-            __sincosf(r.y, &s1, &c1);
-            const mk_f2 c = f2_pack(c0, c1), s = f2_pack(s0, s1);
-            ar = f2_fma(e.x, c, f2_fma(f2_mul(e.y, m_one), s, ar));
-            ai = f2_fma(e.x, s, f2_fma(e.y, c, ai));
-        }
-        const float2 r2 = f2_unpack(ar), i2 = f2_unpack(ai);
-        return make_float2(mk_unshort(r2.x + r2.y), mk_unshort(i2.x + i2.y));
+        for (int p = p0; p < p1; ++p) a.add(P2[2 * p], P2[2 * p + 1], E2[p]);
+        return a.sum();
     };
     // w = b - u', u' the direction from the tile's origin
     auto direction = [&](const float4 &w4, const float4 &u4) {
@@ -1272,24 +1285,52 @@ __global__ void __launch_bounds__(mk_leaf8_threads(NS)) mk_node_leaf8_kernel(con
     const int patches = (int)(n_nodes / (N0 * N0)), p_end = min((int)(blockIdx.y + 1) * B.patches, patches);
     for (int patch = blockIdx.y * B.patches; patch < p_end; ++patch) {
         const MkNodeRec *rs = B.rec + (long long)patch * SQ;
-        for (int i = threadIdx.x; i < 8 * SQ; i += NT) {
-            const int s = i / SQ, q = i - s * SQ;
+        // ND nodes a thread: an atom pair's 48 bytes from shared memory serve them all
+        for (int i = threadIdx.x; i < 8 * (SQ / ND); i += NT) {
+            const int s = i / (SQ / ND), q = i - s * (SQ / ND);
             const float4 c = s_c[s];
+            float2 *v = s_v + s * SQ + q;
             if (c.w == 0.f) {
-                s_v[i] = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int k = 0; k < ND; ++k) v[k * (SQ / ND)] = make_float2(0.f, 0.f);
                 continue;
             }
-            const float3 w = direction(rs[q].w, rs[q].u);
-            s_v[i] = terms(s * pairs, (s + 1) * pairs, w.x, w.y, w.z, fmaf(c.z, w.z, fmaf(c.y, w.y, c.x * w.x)));
+            MkLeafSum a[ND];
+#pragma unroll
+            for (int k = 0; k < ND; ++k) {
+                const MkNodeRec &R = rs[q + k * (SQ / ND)];
+                const float3 w = direction(R.w, R.u);
+                a[k] = MkLeafSum(w, fmaf(c.z, w.z, fmaf(c.y, w.y, c.x * w.x)));
+            }
+#pragma unroll 4 / ND
+            for (int p = s * pairs; p < (s + 1) * pairs; ++p) {
+                const ulonglong2 xy = P2[2 * p], z = P2[2 * p + 1], e = E2[p];
+#pragma unroll
+                for (int k = 0; k < ND; ++k) a[k].add(xy, z, e);
+            }
+#pragma unroll
+            for (int k = 0; k < ND; ++k) v[k * (SQ / ND)] = a[k].sum();
         }
         __syncthreads();
-        for (int i = threadIdx.x; i < 8 * N0 * NS; i += NT) {
-            const int s = i / (N0 * NS), r = i - s * N0 * NS, row = r / NS, c = r - row * NS;
-            mk_f2 a = 0ull;
+        // along z: RW rows a thread share the eighth's column and read their weights at once
+        for (int i = threadIdx.x; i < 8 * (N0 / RW) * NS; i += NT) {
+            const int s = i / (N0 / RW * NS), r = i - s * (N0 / RW * NS), row = r / NS * RW, c = r % NS;
+            mk_f2 a[RW];
 #pragma unroll
-            for (int j = 0; j < NS; ++j)
-                a = f2_fma(f2_splat(s_w[row * NS + j]), *reinterpret_cast<const mk_f2 *>(&s_v[s * SQ + j * NS + c]), a);
-            *reinterpret_cast<mk_f2 *>(&s_t[i]) = a;
+            for (int k = 0; k < RW; ++k) a[k] = 0ull;
+#pragma unroll
+            for (int j = 0; j < NS; ++j) {
+                alignas(16) float w[RW];
+                if constexpr (RW == 4)
+                    *reinterpret_cast<float4 *>(w) = *reinterpret_cast<const float4 *>(s_w + j * N0 + row);
+                else
+                    *reinterpret_cast<float2 *>(w) = *reinterpret_cast<const float2 *>(s_w + j * N0 + row);
+                const mk_f2 v = *reinterpret_cast<const mk_f2 *>(&s_v[s * SQ + j * NS + c]);
+#pragma unroll
+                for (int k = 0; k < RW; ++k) a[k] = f2_fma(f2_splat(w[k]), v, a[k]);
+            }
+#pragma unroll
+            for (int k = 0; k < RW; ++k) *reinterpret_cast<mk_f2 *>(&s_t[(s * N0 + row + k) * NS + c]) = a[k];
         }
         __syncthreads();
         const MkNodeRec *rn = rec + (long long)patch * N0 * N0;
@@ -1298,7 +1339,9 @@ __global__ void __launch_bounds__(mk_leaf8_threads(NS)) mk_node_leaf8_kernel(con
             const int row = g / N0, col = g - row * N0;
             const float4 w4 = rn[g].w, u4 = rn[g].u;
             const float3 w = direction(w4, u4);
-            float re = 0.f, im = 0.f;
+            float re = 0.f, im = 0.f, wy[NS];
+#pragma unroll
+            for (int i = 0; i < NS; ++i) wy[i] = s_w[i * N0 + col];
             for (int s = 0; s < 8; ++s) {
                 const float4 c = s_c[s];
                 if (c.w == 0.f) {               // uniform across the block
@@ -1326,7 +1369,7 @@ __global__ void __launch_bounds__(mk_leaf8_threads(NS)) mk_node_leaf8_kernel(con
                         }
                         v = make_float2(mk_unshort(v.x), mk_unshort(v.y));
                     } else {
-                        v = terms(s * pairs, (s + 1) * pairs, w.x, w.y, w.z, 0.f);
+                        v = terms(s * pairs, (s + 1) * pairs, w);
                     }
                     re += v.x;
                     im += v.y;
@@ -1334,7 +1377,6 @@ __global__ void __launch_bounds__(mk_leaf8_threads(NS)) mk_node_leaf8_kernel(con
                 }
                 mk_f2 v = 0ull;
                 const ulonglong2 *t2 = reinterpret_cast<const ulonglong2 *>(s_t + (s * N0 + row) * NS);
-                const float *wy = s_w + col * NS;
 #pragma unroll
                 for (int i = 0; i < NS / 2; ++i) {
                     const ulonglong2 tt = t2[i];

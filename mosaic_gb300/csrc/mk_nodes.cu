@@ -46,7 +46,7 @@
 #include "mk_split.cuh"
 
 #define MK_NODE_MAX 20       // nodes per axis at most (fine nodes: 16)
-#define MK_NODE_SB 4         // sources staged per step
+#define MK_NODE_SB(n) ((n) > 16 ? 4 : (n) == 16 ? 6 : 8)   // sources staged per step, within 48 KB
 #define MK_MERGE_NT 128      // threads of a merge block
 #define MK_PIX_COLS 32       // pixel block: 32 columns x 16 rows, 4 rows a thread
 #define MK_PIX_ROWS 16
@@ -834,12 +834,12 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
     plan->patches1 = patch;
     plan->weights = wf;
     // slices of sources: enough blocks for every SM several times over, at
-    // least two staging steps a slice
+    // least eight sources a slice
     int sms = 152, devid = 0;
     if (cudaGetDevice(&devid) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, devid);
     const long long want = (12ll * sms + pblk - 1) / pblk;
     plan->slices = (int)std::max<long long>(1, std::min<long long>(std::min<long long>(want, 256),
-                                                                   plan->n_src / (2 * MK_NODE_SB)));
+                                                                   plan->n_src / 8));
     plan->src_per_slice = (plan->n_src + plan->slices - 1) / plan->slices;
     plan->slices = (plan->n_src + plan->src_per_slice - 1) / plan->src_per_slice;
     for (int f = 0; f < n_frames; ++f) fr[f].part_off = fr[f].pix_off * plan->slices;
@@ -1446,15 +1446,17 @@ __device__ __forceinline__ void mk_stage_fields(float2 (*s_v)[N * N], const floa
 // N0^2 / n1 packed FMAs a node, made again for every patch of a row) it took
 // 6.72 ms for N0 = 20, n1 = 12 on the 1024 x 1024 detector and 1.46 ms for N0 =
 // 16 on the 512 x 512 one; here 2.34 and 0.70 ms (4.5 and 5.2 ps a (tile, fine
-// node)).
+// node)). Six or eight sources a step instead of four: 0.44 -> 0.42 ms for 15,814 tiles
+// into runs on 16 x 16 middle nodes (at N0 = 20 slower).
 template <int N0, int ROWS>
 __global__ void __launch_bounds__(MK_MERGE_NT) mk_node_merge_kernel(const MkMergeArgs A)
 {
+    constexpr int SB = MK_NODE_SB(N0);
     constexpr int MAXR = 16;                 // rows of a block at most
-    __shared__ __align__(16) float2 s_v[2][MK_NODE_SB][N0 * N0];
-    __shared__ __align__(16) float2 s_t[MK_NODE_SB][MAXR][N0];
+    __shared__ __align__(16) float2 s_v[2][SB][N0 * N0];
+    __shared__ __align__(16) float2 s_t[SB][MAXR][N0];
     __shared__ float s_wz[MAXR][N0];
-    __shared__ __align__(16) float s_d[2][MK_NODE_SB][8];
+    __shared__ __align__(16) float s_d[2][SB][8];
     const long long it = A.item_base + blockIdx.x % A.items;
     const int grp = (int)(blockIdx.x / A.items);
     const int n1 = A.n_out;
@@ -1511,7 +1513,7 @@ __global__ void __launch_bounds__(MK_MERGE_NT) mk_node_merge_kernel(const MkMerg
     const long long first = S.first;
     const int count = S.count;
     auto stage = [&](int s0, int buf) {
-        const int m = min(MK_NODE_SB, count - s0);
+        const int m = min(SB, count - s0);
         mk_stage_fields<N0>(s_v[buf], V, A.in_patches * N0 * N0, first + s0, m);
         mk_cp_commit();
         if ((int)threadIdx.x < m) {
@@ -1530,10 +1532,10 @@ __global__ void __launch_bounds__(MK_MERGE_NT) mk_node_merge_kernel(const MkMerg
         }
     };
     stage(0, 0);
-    for (int s0 = 0, buf = 0; s0 < count; s0 += MK_NODE_SB, buf ^= 1) {
-        const int m = min(MK_NODE_SB, count - s0);
-        if (s0 + MK_NODE_SB < count) {
-            stage(s0 + MK_NODE_SB, buf ^ 1);
+    for (int s0 = 0, buf = 0; s0 < count; s0 += SB, buf ^= 1) {
+        const int m = min(SB, count - s0);
+        if (s0 + SB < count) {
+            stage(s0 + SB, buf ^ 1);
             mk_cp_wait<1>();
         } else {
             mk_cp_wait<0>();
@@ -1590,8 +1592,9 @@ __global__ void __launch_bounds__(MK_MERGE_NT) mk_node_merge_kernel(const MkMerg
 template <int N>
 __global__ void __launch_bounds__(128) mk_node_pixels_kernel(const MkNodeArgs A)
 {
-    __shared__ __align__(16) float2 s_v[2][MK_NODE_SB][N * N];
-    __shared__ __align__(16) float2 s_t[MK_NODE_SB][MK_PIX_ROWS][N];
+    constexpr int SB = MK_NODE_SB(N);
+    __shared__ __align__(16) float2 s_v[2][SB][N * N];
+    __shared__ __align__(16) float2 s_t[SB][MK_PIX_ROWS][N];
     __shared__ float s_wz[MK_PIX_ROWS][N];
     const long long blk = A.pblk_base + blockIdx.x;
     const int f = mk_find_frame(A.f_lo, A.f_hi, blk, [&](int i) { return A.frames[i].pblk_off; });
@@ -1642,12 +1645,12 @@ __global__ void __launch_bounds__(128) mk_node_pixels_kernel(const MkNodeArgs A)
             accr[r] = acci[r] = cr[r] = ci[r] = 0.f;
         }
     };
-    mk_stage_fields<N>(s_v[0], V, ld, s_lo, min(MK_NODE_SB, s_hi - s_lo));
+    mk_stage_fields<N>(s_v[0], V, ld, s_lo, min(SB, s_hi - s_lo));
     mk_cp_commit();
-    for (int s0 = s_lo, buf = 0; s0 < s_hi; s0 += MK_NODE_SB, buf ^= 1) {
-        const int m = min(MK_NODE_SB, s_hi - s0);
-        if (s0 + MK_NODE_SB < s_hi) {
-            mk_stage_fields<N>(s_v[buf ^ 1], V, ld, s0 + MK_NODE_SB, min(MK_NODE_SB, s_hi - s0 - MK_NODE_SB));
+    for (int s0 = s_lo, buf = 0; s0 < s_hi; s0 += SB, buf ^= 1) {
+        const int m = min(SB, s_hi - s0);
+        if (s0 + SB < s_hi) {
+            mk_stage_fields<N>(s_v[buf ^ 1], V, ld, s0 + SB, min(SB, s_hi - s0 - SB));
             mk_cp_commit();
             mk_cp_wait<1>();
         } else {

@@ -5,7 +5,8 @@
 
 One step = one full kinematic exposure of the workload: stage transform and
 incident amplitudes, species + Hilbert tiling, per-pixel prologue, the FP32
-split-phase sum and the FP64 reduction. `value` is measured with the atom
+sum in the form the entry point takes (nodes where admitted, with their plan;
+else the split kernel on every (atom, pixel)) and the FP64 reduction. `value` is measured with the atom
 positions already resident in HBM; `e2e` goes through the public entry point
 ``beam.atomic_scattering_kinematic`` with host arrays (host->device copies and
 the device->host read of the field inside the timed region).
@@ -19,8 +20,8 @@ shards into independent exposures; there is no data-path collective) and
 
 Besides the timed steps, rank 0 reports (outside the timed region): the FP64
 plain kernel on 1,029 pixels spread over the whole detector (speed and error
-reference), the batched scan (all 724 frames of the 4M-atom rocking scan in
-one graph-captured launch), the surrogate-assisted 101 x 101 theta x chi scan
+reference), the split kernel and the node form's kernels alone, the batched
+scan (all 724 frames of the 4M-atom rocking scan, one graph replay), the surrogate-assisted 101 x 101 theta x chi scan
 (frames/s against the exact batched scan of all 10,201 frames, which is run
 and timed too, and every returned frame's error against it) and the CPU
 baseline.
@@ -288,7 +289,7 @@ def probe_pipes(dev):
 def scan_leg(args, dev):
     """Batched scan: the 724 frames of the 4M-atom rocking x chi scan (181
     theta steps x 4 chi offsets, ROI sides cycling 64/128/256/512), all in
-    one persistent launch captured in a CUDA graph; frames/s of one replay.
+    one CUDA graph (the node form's launches, or one persistent split launch); frames/s of one replay.
     The scan's tile size and launch shape come from the autotuner (tuned on
     a probe of the first frames when not cached); the kernels are warmed on
     an 8-frame scan of the same staged atoms, so the whole scan runs once,
@@ -324,7 +325,7 @@ def scan_leg(args, dev):
             "launch_source": scan.launch_source, "tile_atoms": scan.tiles.tile_atoms,
             "autotune": [[float(t), c] for t, c in scan.tune_results], "clocks": sampler.summary(),
             "note": "the 181 theta x 4 chi rocking scan; ROI sides 64/128/256/512 by frame index; "
-                    "atoms staged once, all frames one persistent launch, one timed graph replay"}
+                    "atoms staged once, all frames in one graph, one timed replay"}
 
 
 def surrogate_leg(args, dev):
@@ -565,6 +566,45 @@ def run_reference(args):
     print(json.dumps(line))
 
 
+def own_launches(step):
+    """Launches of this library's kernels (mk_*) in one step, by the profiler;
+    0 where it sees none."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    for _ in range(2):                  # the profiler's first session may miss device events
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            step()
+            torch.cuda.synchronize()
+    return sum(1 for e in prof.events() if "mk_" in e.name)
+
+
+def node_leg(B, engine, atoms, pix, phys, table, mufu_per_s):
+    """The node form's kernels alone (its plan made once): time, the leaf
+    terms they evaluate and what share of the MUFU rate (two results a term)
+    those are."""
+    import torch
+    tiles = engine.Tiles(atoms, B.k, engine.DEFAULT_TILE_ATOMS, device=atoms.pos.device)
+    tol = min(float(B._kernel_phase_tol_rad), float(B._phase_tol_rad))
+    plan = engine.NodePlan.make(tiles, pix, B.k, tuple(phys.beam_dir), tol)
+    _, fresnel, _, diag = B.split_budget(tiles, pix.r0_min())
+    ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+    ms = []
+    for _ in range(4):
+        ev[0].record()
+        engine.run_nodes(plan, tiles, pix, phys, table, fresnel=int(fresnel),
+                         fresnel_radius=diag["fresnel_radius_m"])
+        ev[1].record()
+        ev[1].synchronize()
+        ms.append(ev[0].elapsed_time(ev[1]))
+    terms = plan.leaf_terms()
+    t = float(np.median(ms[1:])) * 1e-3
+    return {"ms": 1e3 * t, "leaf_terms": terms, "bound": "mufu", "achieved": terms / t / 1e9,
+            "peak": mufu_per_s / MUFU_PER_TERM / 1e9, "unit": "Gterm/s",
+            "frac": terms / t / (mufu_per_s / MUFU_PER_TERM), **plan.info(),
+            "note": "all of the form's kernels against the time their leaf terms' sines and cosines "
+                    "take: the merges and the pixel step are in the time, not in the terms"}
+
+
 def run_ours(args):
     import torch
     import torch.distributed as dist
@@ -599,9 +639,14 @@ def run_ours(args):
     n_atoms, n_pix = pos_h.shape[0], ny * nz
     terms = float(n_atoms) * n_pix
 
-    # Tile size and launch shape: autotuned once on a probe (tile sizes 512,
-    # 1024 and 2048, each with the pixel forms its geometry allows), cached
-    # on disk; the entry point then finds the same choice in the cache.
+    # The step takes the form the entry point takes: nodes where admitted. A
+    # switch that fixes a launch or a pixel form, and the kernel profile, take
+    # the split kernel on every (atom, pixel).
+    nodes = not (args.launch or args.profile or args.tile_atoms or args.no_pairs or args.no_quads or
+                 args.no_octets or args.no_squares or args.no_factor_table)
+    # The split kernel's tile size and launch shape: autotuned once on a probe
+    # (tile sizes 512, 1024 and 2048, each with the pixel forms its geometry
+    # allows), cached on disk.
     atoms = engine.atoms_lab(pos_d, idx_h, w.stage.rotation, w.stage.translation, table,
                              e0=B._beam_E0_map, grid=B._beam_grid(), device=dev)
     pix = engine.Pixels(coords_m, ny, nz, phys, device=dev)
@@ -644,16 +689,19 @@ def run_ours(args):
     fresnel = su.fresnel
     B._kernel_tile_atoms = T
     launch = engine.grouping_launch(launch, level, tiles, pix, B.k, ginfo)
-    B._kernel_launch = launch
+    if not nodes:
+        B._kernel_launch = launch
     amp_real = tiles.amp_is_real()
     # the per-(species, pixel) factor table where the geometry admits it,
     # decided once (the check reads back the tile and pixel extents)
     ftab = (not args.no_factor_table) and engine.factor_table_ok(tiles, pix, phys)
     split_times = []
 
-    def step(record=False):
+    def step(record=False, nodes=nodes):
         a = engine.atoms_lab(pos_d, idx_d, w.stage.rotation, w.stage.translation, table,
                              e0=B._beam_E0_map, grid=B._beam_grid(), device=dev, counts=counts)
+        if nodes:
+            return B._scatter_once(a, engine.Pixels(coords_d, ny, nz, phys, device=dev), phys)
         t = engine.Tiles(a, B.k, T, device=dev)
         p = engine.Pixels(coords_d, ny, nz, phys, device=dev)
         if record:
@@ -667,8 +715,15 @@ def run_ours(args):
             split_times.append((e0, e1))
         return out
 
-    for _ in range(args.warmup):
+    if nodes:
+        B._kernel_tile_atoms = int(args.tile_atoms)       # the entry point's own choice
         step()
+        nodes = B.last_run.get("launch_source") == "nodes"
+        if not nodes:
+            B._kernel_tile_atoms, B._kernel_launch = T, launch
+    run_info = dict(B.last_run) if nodes else None
+    for _ in range(args.warmup):
+        step(nodes=nodes)
     barrier()
     sampler = ClockSampler(local)
     with sampler:
@@ -676,7 +731,7 @@ def run_ours(args):
         ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         ev0.record()
         for _ in range(args.steps):
-            out = step(record=True)
+            out = step(record=True, nodes=nodes)
         ev1.record()
         barrier()
     engine.sync()
@@ -685,6 +740,10 @@ def run_ours(args):
         t = torch.tensor([ms], device=dev)
         dist.all_reduce(t, op=dist.ReduceOp.MAX)
         ms = float(t.item())
+    if nodes:           # the split kernel beside it, outside the timed region
+        for _ in range(2):
+            step(record=True, nodes=False)
+        engine.sync()
     split_ms = float(np.mean([a.elapsed_time(b) for a, b in split_times]))
     value = terms * world / (ms * 1e-3) / 1e9
     clocks = sampler.summary()
@@ -743,7 +802,9 @@ def run_ours(args):
     form_bound = "mufu" if mufu / mufu_pt <= fma / fp32_pt else "fp32"
     traffic = profiled_traffic(args.config, n_pix, launch)
     achieved = terms / (split_ms * 1e-3)
-    gpu_launches = args.steps * (8 + int(bool(ftab)))
+    node_form = node_leg(B, engine, atoms, pix, phys, table, mufu * n_sm * clk * 1e6) if nodes else None
+    per_step = own_launches(lambda: step(nodes=nodes)) or 8 + int(bool(ftab))
+    gpu_launches = args.steps * per_step
 
     configs = configs_leg(args, dev) if (rank == 0 and not args.no_configs) else None
     scan = scan_leg(args, dev) if (rank == 0 and args.scan_frames > 0) else None
@@ -757,8 +818,11 @@ def run_ours(args):
             "scaling": "weak", "vs_baseline": None, "dtype": "f32 (FP64 origins and reduction)",
             "data": "synthetic",
             "config": {"workload": args.config, "atoms": n_atoms, "pixels": n_pix,
-                       "terms_per_step": terms, "tile_atoms": B._kernel_tile_atoms,
+                       "terms_per_step": terms, "tile_atoms": run_info["tile_atoms"] if nodes else T,
                        "launch": launch, "fresnel_term": bool(fresnel), "factor_table": bool(ftab),
+                       "form": "nodes" if nodes else "split",
+                       "nodes": {k: run_info[k] for k in ("nodes", "groups", "single_tiles", "wide_tiles",
+                                                          "tile_atoms")} if nodes else None,
                        "l2": "inputs larger than L2 (positions + tiles ~300 MB); no flush",
                        "parallelism": f"replicas x{world}"},
             "e2e": {"value": terms * world / e2e_s / 1e9, "unit": "Gatom*pixel/s",
@@ -786,10 +850,13 @@ def run_ours(args):
                                                "savings ratio, not a roofline fraction -- the "
                                                "executed form shares sin/cos between pixels"},
                          "pipe_probe_ops_per_clk_per_sm": pipes,
-                         "split_kernel_ms": split_ms},
+                         "split_kernel_ms": split_ms,
+                         "note": "the split kernel on every (atom, pixel)" +
+                                 (", timed beside the step, which takes the node form" if nodes else "")},
+            "node_form": node_form,
             "fp64_plain": {"value": fp64_rate, "unit": "Gatom*pixel/s",
                            "subset": f"{m} pixels spread over the whole detector, all atoms",
-                           "speedup_fp32_vs_fp64": (achieved / 1e9) / fp64_rate},
+                           "speedup_fp32_vs_fp64": value / world / fp64_rate},
             "accuracy": {"rel_err_max_over_peak": chk["rel_err_max_over_peak"],
                          "rel_err_l2": chk["rel_err_l2"],
                          "rel_err_corners_and_edge_midpoints":
@@ -817,7 +884,8 @@ def run_ours(args):
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
-    ap.add_argument("--steps", type=int, default=5)
+    ap.add_argument("--steps", type=int, default=None,
+                    help="timed steps (default 100; 5 for the reference and the kernel profile)")
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--config", default="nacl_screw_8m")
@@ -860,6 +928,8 @@ def main():
     ap.add_argument("--profile", action="store_true",
                     help="kernel-profile run: cached launch shape, timed steps only")
     args = ap.parse_args()
+    if args.steps is None:      # a step in node form is a few ms: enough of them to sample the clocks
+        args.steps = 5 if args.impl == "reference" or args.profile else 100
     if args.profile_gemm:
         gemm_profile_case()
         return

@@ -951,7 +951,7 @@ class NodePlan:
     DIRECT_S_PER_TERM = 0.18e-12
 
     def __init__(self, plan, buf, tiles):
-        self.plan, self.buf = plan, buf
+        self.plan, self.buf, self.tile_atoms = plan, buf, tiles.tile_atoms
         self.dev = torch.from_numpy(buf[: plan.buf_bytes]).to(tiles.origin.device)
         self.wide = None
         if plan.n_wide:
@@ -979,9 +979,17 @@ class NodePlan:
         check(rc)
         return cls(plan, buf, tiles)
 
+    def leaf_terms(self):
+        """Terms the leaves evaluate, every eighth taken to fit its nodes."""
+        p, n0 = self.plan, self.plan.n0
+        wide = p.ns[1] or n0
+        per = p.patches0 * (p.n_narrow * p.ns[0] ** 2 + (p.n_members - p.n_narrow) * wide ** 2) \
+            if p.ns[0] else p.patches0 * p.n_members * n0 ** 2
+        return self.tile_atoms * (per + p.n_msingle * p.patchesm * p.nm ** 2 + p.n_mid * p.patches1 * p.n1 ** 2)
+
     def info(self):
         p = self.plan
-        return dict(form="nodes", nodes=(p.n0, p.n1), groups=p.n_groups, single_tiles=p.n_mid,
+        return dict(form="nodes", nodes=tuple(n for n in (p.n0, p.nm, p.n1) if n), groups=p.n_groups, single_tiles=p.n_mid,
                     wide_tiles=p.n_wide, group_radius_m=p.radius2_m)
 
 

@@ -426,7 +426,8 @@ extern "C" int mk_prop_cols_rows(float *spectrum, int ny2, int nz2, int z0, int 
     const size_t smem = sizeof(float2) * (size_t)A.W * (size_t)A.ld;
     const int last = logn % 3 == 0 ? 3 : logn % 3;
     auto fn = last == 1 ? mk_prop_cols_kernel<1> : (last == 2 ? mk_prop_cols_kernel<2> : mk_prop_cols_kernel<3>);
-    MK_CHECK_CUDA(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > (48u << 10))
+        MK_CHECK_CUDA(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     fn<<<ny2 / A.W, MK_FFT_NT, smem, st>>>(A);
     MK_CHECK_CUDA(cudaGetLastError());
     return MK_OK;

@@ -9,12 +9,15 @@ error behaviour (ValueError for a non-+x beam or size mismatches,
 MemoryError when scratch cannot be allocated).
 
 Arithmetic runs on the GPU in libmosaic_kin.so:
-  * ``_use_fast_kernel`` True (default): FP32 split-phase sum
-    (``mk_kin_split_f32``); it declines to the FP64 sum when the geometry
+  * ``_use_fast_kernel`` True (default): FP32 sum, in node form
+    (``mk_kin_nodes_f32``) for large sums on plane detectors, else the
+    split-phase kernel (``mk_kin_split_f32``); it declines to the FP64 sum when the geometry
     leaves its error budget (extreme near field), as the reference's fast
     kernel declines to its general kernel (Beam.py:1376-1441).
   * ``_use_fast_kernel`` False: FP64 plain sum (``mk_kin_plain_f64``), the
-    reference CPU kernel's arithmetic term for term.
+    reference CPU kernel's arithmetic with its rounding of the phase; the
+    slowly varying factors are expanded about each pixel's direction where
+    the sample is small against the distance (to ~1e-14 of the sum).
 There is no CPU path: ``use_gpu=False`` and a missing GPU raise.
 """
 from __future__ import annotations
@@ -597,9 +600,11 @@ class beam:
             self.apply_depth_ein(atoms)
         pix = self._pixels_for(coords, Ny, Nz, phys)
         out = self.scatter_device(atoms, pix, phys)
+        field = torch.view_as_complex(out)
+        if not return_double:           # rounded on the device: half the copy, no pass on the host
+            field = field.to(torch.complex64)
         engine.sync()
-        field = torch.view_as_complex(out).cpu().numpy().reshape(Nz, Ny)
-        return field if return_double else field.astype(np.complex64)
+        return field.cpu().numpy().reshape(Nz, Ny)
 
     def _pixels_for(self, coords, Ny, Nz, phys):
         """The prepared pixels of these coordinates and physics: kept from

@@ -22,8 +22,6 @@
 // and returns.
 #include <cuda_bf16.h>
 
-#include <atomic>
-
 #include "mk_tc.cuh"
 
 #define MK_TCG_BM 128
@@ -406,15 +404,8 @@ template <int BN>
 static int mk_tcg_launch(const MkTcGemm &g, dim3 grid, cudaStream_t st, int *status)
 {
     const size_t smem = 2048 + (size_t)MK_TCG_STAGES(BN) * (MK_TCG_BM + BN) * MK_TCG_BK * 2;
-    // the attribute is set once per device: it belongs to the loaded function
-    static std::atomic<unsigned long long> done{0};
-    int dev = 0;
-    MK_CHECK_CUDA(cudaGetDevice(&dev));
-    if (dev >= 64 || !(done.load(std::memory_order_acquire) >> dev & 1ull)) {
-        MK_CHECK_CUDA(cudaFuncSetAttribute((const void *)mk_gemm_tc_kernel<BN>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        if (dev < 64) done.fetch_or(1ull << dev, std::memory_order_release);
-    }
+    MK_CHECK_CUDA(cudaFuncSetAttribute((const void *)mk_gemm_tc_kernel<BN>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     mk_gemm_tc_kernel<BN><<<grid, MK_TCG_NT, smem, st>>>(g, status);
     MK_CHECK_CUDA(cudaGetLastError());
     return MK_OK;

@@ -31,11 +31,11 @@
 // 1/20 of the FP64 pipe's cost (2 FP64 operations per clock and SM).
 //
 // Measured against the split kernel on every (atom, pixel), through the entry
-// point: 8.19M atoms x 512^2 349 -> 9.2 ms, 5.3M x 1024^2 at 0.5 m 1040 ->
-// 14 ms, 2M x 256^2 29.0 -> 6.1 ms, 32k x 128^2 1.38 -> 0.96 ms; a staged scan
-// of 16 frames x 500k atoms 103.4 -> 1.34 ms. Error against FP64 at 64 pixels
-// spread over the detector: peak-relative intensity 3.5e-7 (split kernel
-// 8.5e-7) on the first, 1.4e-6 (2.0e-6) on the second.
+// point: 8.19M atoms x 512^2 354 -> 7.6 ms, 5.3M x 1024^2 at 0.5 m 1042 ->
+// 9.6 ms, 2M x 256^2 29.1 -> 5.3 ms, 32k x 128^2 1.43 -> 0.91 ms; a staged scan
+// of 16 frames x 500k atoms 103 -> 1.0 ms. Error against FP64 at 64 pixels
+// spread over the detector: peak-relative intensity 4 to 6e-7 (split kernel
+// 8.5e-7) on the first, 1.6 to 1.8e-6 (1.6 to 2.0e-6) on the second.
 //
 // Interpolation weights are FP64 Lagrange products rounded once; the pixel
 // coordinates they are taken at are the pixels' own (projected on the

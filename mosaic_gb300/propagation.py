@@ -7,7 +7,7 @@ exact free-space transfer function with the carrier removed, transformed
 back and centre-cropped; distances the padded grid cannot sample without
 aliasing are split into equal alias-free steps. Here the 2-D transform is
 split by dimension: the row (y) transforms, over contiguous rows, are cuFFT
-through torch.fft, and one libmosaic_kin kernel (``mk_prop_cols``) does the
+through torch.fft, and one libmosaic_kin kernel (``mk_prop_cols_rows``) does the
 column transform, the transfer-function multiply and the inverse column
 transform for groups of neighbouring columns in shared memory, so the
 spectrum makes one round trip through HBM between the row transforms

@@ -1,4 +1,4 @@
-"""Batched scans: every step of a motor scan in one persistent launch.
+"""Batched scans: every step of a motor scan in one batch of launches.
 
 The reference runs a scan as one full exposure per step
 (experiment.scan_nD, Experiment.py:285-336): reload and re-stage every chunk,
@@ -11,8 +11,10 @@ vector, all moved into the sample frame by the inverse stage transform:
 
 k (b_f . a + |P'_f - a|) is then exactly the phase of atom a at pixel P_f
 with the sample at (R_f, t_f). All frames (each with its own ROI, of any
-size) become work items of one persistent kernel (``mk_kin_scan_f32``);
-the launch sequence can be captured in a CUDA graph and replayed.
+size) take one plan of the node form (``engine.NodePlan``) where it is
+admitted, else become work items of one persistent kernel
+(``mk_kin_scan_f32``); the launch sequence can be captured in a CUDA graph and
+replayed.
 
 The incident amplitude must not depend on the frame: the beam profile must
 be uniform and cover the sample in every frame (checked; otherwise run the
@@ -54,7 +56,7 @@ def roi_indices(det_shape, side, centre=None):
 
 
 class BatchedScan:
-    """All frames of a scan as one launch over atoms staged once.
+    """All frames of a scan in one batch over atoms staged once.
 
     Args:
         beam: a configured ``mosaic_gb300.beam``.

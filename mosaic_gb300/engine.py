@@ -160,6 +160,8 @@ class Pixels:
         sh = _stream_handle(stream)
         self.spans = [(0, P)]
         self.shapes = [(self.ny, self.nz)]
+        # frames whose direction is not the physics': no single factor table
+        self.rotated = any(tuple(map(float, b)) != tuple(phys.beam_dir) for _, _, b in frames or ())
         if frames is None:
             check(L.mk_pixels_prepare(ctypes.byref(self.abi), ctypes.byref(phys), sh))
             return
@@ -206,6 +208,7 @@ class Pixels:
             rec[i, 9:12] = np.asarray(f.translation, dtype=np.float64).reshape(3)
             rec[i, 12:15] = beam_dirs[i]
             rec[i, 15:19] = offs[i], *self.shapes[i], first[id(f.pixels)]
+        self.rotated = bool((rec[:, :9] != np.eye(3).reshape(9)).any())
         lab = torch.empty(size, **dd)
         for a, px in arrays:
             t = torch.from_numpy(np.array(px, dtype=np.float64, order="C")).view(-1)   # a copy: may be read-only
@@ -1021,7 +1024,7 @@ def run_nodes(np_, tiles, pix, phys, table, out=None, accumulate=False, fresnel=
               factor=None, sums=None, ws=None, stream=None):
     """Node-form sum of a plan's groups and single tiles (``mk_kin_nodes_f32``;
     the plan's wide tiles are the caller's); float64 (P, 2). ``factor``: the
-    factor table (default: ``Pixels.factor_table`` of single exposures)."""
+    factor table (default: ``Pixels.factor_table``, for single exposures only)."""
     L = _require_cuda()
     if out is None:
         out = torch.empty((pix.n, 2), dtype=torch.float64, device=pix.xyz.device)
@@ -1029,6 +1032,8 @@ def run_nodes(np_, tiles, pix, phys, table, out=None, accumulate=False, fresnel=
     if ws is None:
         ws = torch.empty(np_.plan.ws_bytes, dtype=torch.uint8, device=pix.xyz.device)
     if factor is None:
+        if pix.rotated:
+            raise ValueError("run_nodes: frames of their own directions need their factor table")
         factor = pix.factor_table(table, phys, stream)
     pabi = MkPixels.from_buffer_copy(pix.abi)
     pabi.factor = factor.data_ptr()

@@ -179,6 +179,9 @@ class BatchedScan:
             # nothing for the split kernel: a plan of its simplest shape keeps
             # the frame table the factor table reads
             self.replan(self.tiles, Setup(self.tiles, 0, {}), engine.default_launch(0), workspace=False)
+        # the groups' factors: the plan admits their radius, whatever the wide
+        # tiles allow the split kernel
+        self.ftab = self._frame_factors(self._frame_records)
         self.nodes = plan
         self._node_ws = torch.empty(plan.plan.ws_bytes, dtype=torch.uint8, device=self._dev)
         self.diag = dict(self.diag, **plan.info())
@@ -245,23 +248,12 @@ class BatchedScan:
         self.n_items, self.n_partial = int(n_items.value), int(n_part.value)
         raw = np.frombuffer(bytes(desc), dtype=np.uint8).copy()
         self.frames_dev = torch.as_tensor(raw).to(self._dev)
+        self._frame_records = bytes(raw)
         # per-(species, pixel) factors at every frame's pixel directions,
         # where the tile origins allow it (engine.factor_table_ok)
         self.pix_abi, self.ftab = self.pix.abi, None
         if engine.factor_table_ok(tiles, self.pix, self.phys):
-            key = (self.table.key(), bytes(raw))
-            if getattr(self, "_ftab_key", None) == key and self._ftab is not None:
-                self.ftab = self._ftab
-            else:
-                self.ftab = torch.empty((len(self.table.labels), self.pix.n, 2),
-                                        dtype=torch.float32, device=self._dev)
-                abi = MkPixels.from_buffer_copy(self.pix.abi)
-                abi.factor = self.ftab.data_ptr()
-                sp = self.table.abi()
-                check(self.L.mk_factor_table(ctypes.byref(abi), ctypes.byref(sp),
-                                             ctypes.byref(self.phys), nf,
-                                             self.frames_dev.data_ptr(), engine._stream_handle()))
-                self._ftab_key, self._ftab = key, self.ftab
+            self.ftab = self._frame_factors(self._frame_records)
             self.pix_abi = MkPixels.from_buffer_copy(self.pix.abi)
             self.pix_abi.factor = self.ftab.data_ptr()
         need = int(self.L.mk_scan_workspace_size(self.n_partial))
@@ -269,6 +261,23 @@ class BatchedScan:
             self.ws = torch.empty(need, dtype=torch.uint8, device=self._dev)
             self.ws_bytes = need
         self._graph = None
+
+    def _frame_factors(self, frames):
+        """(n_species, P, 2) scattering factors at every frame's own pixel
+        directions, for the planned frame records ``frames`` (the bytes
+        of ``frames_dev``); kept for the last species table and records."""
+        key = (self.table.key(), frames)
+        if self._ftab_key != key or self._ftab is None:
+            self._ftab = torch.empty((len(self.table.labels), self.pix.n, 2), dtype=torch.float32,
+                                     device=self._dev)
+            abi = MkPixels.from_buffer_copy(self.pix.abi)
+            abi.factor = self._ftab.data_ptr()
+            sp = self.table.abi()
+            check(self.L.mk_factor_table(ctypes.byref(abi), ctypes.byref(sp), ctypes.byref(self.phys),
+                                         len(self.frames), self.frames_dev.data_ptr(),
+                                         engine._stream_handle()))
+            self._ftab_key = key
+        return self._ftab
 
     def _check_uniform_beam(self, pos):
         B = self.beam

@@ -507,6 +507,10 @@ class beam:
             return None
         cfg = engine.default_launch(4 if pix.squares_fit() else 2, tiles.tile_atoms)
         info, factor, edge, full = {}, True, None, phys
+        # scatter_device sums the atoms in halves into the same field when
+        # memory runs out: everything is allocated, and the edge pixels
+        # summed, before the field is first written
+        ws = torch.empty(plan.plan.ws_bytes, dtype=torch.uint8, device=pix.xyz.device)
         if phys.analyser:
             masked = engine.analyser_mask(tiles, pix, phys, atoms.table)
             if masked is None:
@@ -515,24 +519,28 @@ class beam:
             phys = type(full).from_buffer_copy(full)
             phys.analyser = 0
             info["edge_pixels"] = int(edge.numel())
+        if edge is not None and edge.numel():
+            sub = engine.Pixels(pix.xyz[edge].t(), int(edge.numel()), 1, full, device=pix.xyz.device)
+            edge_sum = engine.run_plain(atoms, sub, full)
+        table = pix.factor_table(atoms.table, phys) if factor is True else factor
+        if out is None:
+            out, accumulate = torch.empty((pix.n, 2), dtype=torch.float64, device=pix.xyz.device), False
         if plan.wide is not None:
             su, diag = self.split_setup(plan.wide, pix, phys)
             if su is None:
                 return None
             cfg = engine.grouping_launch(engine.default_launch(su.level, tiles.tile_atoms), su.level,
                                          plan.wide, pix, self.k, su.info)
-            out = engine.run_split(plan.wide, pix, phys, atoms.table, launch=cfg, fresnel=su.fresnel,
-                                   out=out, accumulate=accumulate, fresnel_radius=su.fresnel_radius,
-                                   factor_table=factor)
+            engine.run_split(plan.wide, pix, phys, atoms.table, launch=cfg, fresnel=su.fresnel, out=out,
+                             accumulate=accumulate, fresnel_radius=su.fresnel_radius, factor_table=factor)
             accumulate = True
             info.update(su.info)
         _, fresnel, _, diag = self.split_budget(tiles, pix.r0_min())
         res = engine.run_nodes(plan, tiles, pix, phys, atoms.table, out=out, accumulate=accumulate,
-                               fresnel=int(fresnel), fresnel_radius=diag["fresnel_radius_m"],
-                               factor=None if factor is True else factor)
+                               fresnel=int(fresnel), fresnel_radius=diag["fresnel_radius_m"], factor=table,
+                               ws=ws)
         if edge is not None and edge.numel():
-            sub = engine.Pixels(pix.xyz[edge].t(), int(edge.numel()), 1, full, device=pix.xyz.device)
-            res[edge] += engine.run_plain(atoms, sub, full)
+            res.index_add_(0, edge, edge_sum)
         self.last_run = dict(path="split_f32", n_tiles=tiles.n_tiles, tile_atoms=tiles.tile_atoms,
                              fresnel=bool(fresnel), factor_table=True, launch=dict(cfg),
                              launch_source="nodes", **plan.info(), **info, **diag)

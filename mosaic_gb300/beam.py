@@ -506,7 +506,10 @@ class beam:
         if plan is None:
             return None
         cfg = engine.default_launch(4 if pix.squares_fit() else 2, tiles.tile_atoms)
-        info, factor, edge, full = {}, True, None, phys
+        # a top-hat's mask lives in the factor table: all tiles have to take it
+        if phys.analyser and plan.wide is not None and not engine.factor_table_ok(plan.wide, pix, phys):
+            return None
+        info, factor, edge, full = {}, None, None, phys
         # scatter_device sums the atoms in halves into the same field when
         # memory runs out: everything is allocated, and the edge pixels
         # summed, before the field is first written
@@ -522,7 +525,7 @@ class beam:
         if edge is not None and edge.numel():
             sub = engine.Pixels(pix.xyz[edge].t(), int(edge.numel()), 1, full, device=pix.xyz.device)
             edge_sum = engine.run_plain(atoms, sub, full)
-        table = pix.factor_table(atoms.table, phys) if factor is True else factor
+        table = pix.factor_table(atoms.table, phys) if factor is None else factor
         if out is None:
             out, accumulate = torch.empty((pix.n, 2), dtype=torch.float64, device=pix.xyz.device), False
         if plan.wide is not None:
@@ -534,7 +537,7 @@ class beam:
             engine.run_split(plan.wide, pix, phys, atoms.table, launch=cfg, fresnel=su.fresnel, out=out,
                              accumulate=accumulate, fresnel_radius=su.fresnel_radius, factor_table=factor)
             accumulate = True
-            info.update(su.info)
+            info.update(su.info, wide_factor_table=engine.factor_table_ok(plan.wide, pix, phys))
         _, fresnel, _, diag = self.split_budget(tiles, pix.r0_min())
         res = engine.run_nodes(plan, tiles, pix, phys, atoms.table, out=out, accumulate=accumulate,
                                fresnel=int(fresnel), fresnel_radius=diag["fresnel_radius_m"], factor=table,

@@ -53,3 +53,28 @@ def test_scan_with_wide_tiles_takes_every_frames_own_factors(cuda):
     # a rotated frame's pixels have no single factor table to fall back on
     with pytest.raises(ValueError):
         engine.run_nodes(scan.nodes, scan.tiles, scan.pix, scan.phys, scan.table)
+
+
+@pytest.mark.parametrize("analyser", [False, True])
+def test_wide_tiles_take_the_factor_table_by_its_rule(cuda, monkeypatch, analyser):
+    """An exposure's wide tiles beyond the factor table's bound take the factor
+    per tile; under a top-hat analyser, whose mask is in the table, the sum is
+    not the node form's to take."""
+    w, sample = _dilute()
+    B, st, D = w.beam, StaticStage(w.stage.rotation, w.stage.translation), _det(w, (200, 180))
+    plans, runs = [], []
+    make, split = engine.NodePlan.make.__func__, engine.run_split
+    monkeypatch.setattr(engine.NodePlan, "make", classmethod(
+        lambda cls, *a, **k: plans.append(make(cls, *a, **k)) or plans[-1]))
+    monkeypatch.setattr(engine, "run_split", lambda *a, **k: runs.append((a, k)) or split(*a, **k))
+    kw = dict(apply_polarization=True, return_double=True)
+    if analyser:
+        kw.update(analyser_mode="top-hat", analyser_acceptance_angle_rad=0.05)
+    got = B.atomic_scattering_kinematic(sample, D, st, **kw)
+    wide, (tiles, pix, phys, *_), opts = plans[-1].wide, *runs[-1]
+    assert wide is not None and not engine.factor_table_ok(wide, pix, phys)
+    assert (B.last_run["launch_source"] == "nodes") == (not analyser)
+    assert (tiles is wide) == (not analyser) and opts.get("factor_table") is None
+    B._use_fast_kernel = False
+    ref = B.atomic_scattering_kinematic(sample, D, st, **kw)
+    assert rel_intensity(got, ref) <= 1e-4, rel_intensity(got, ref)

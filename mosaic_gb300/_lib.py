@@ -195,6 +195,11 @@ SIGNATURES = {
     "mk_tiles_build": (ctypes.c_int, [ctypes.c_int64, _vp, _vp, _vp, ctypes.c_int,
                                       ctypes.POINTER(ctypes.c_int64), ctypes.c_double,
                                       ctypes.POINTER(MkTiles), _vp, ctypes.c_size_t, _vp]),
+    "mk_tiles_workspace_size_keys": (ctypes.c_size_t, [ctypes.c_int64, ctypes.c_int]),
+    "mk_tiles_build_keys": (ctypes.c_int, [ctypes.c_int64, _vp, _vp, _vp, ctypes.c_int,
+                                           ctypes.POINTER(ctypes.c_int64), ctypes.c_double,
+                                           ctypes.POINTER(MkTiles), ctypes.c_int, _vp, _vp,
+                                           ctypes.c_size_t, _vp]),
     "mk_sum_workspace_size": (ctypes.c_size_t, [ctypes.c_int, ctypes.c_int]),
     "mk_kin_plain_f64": (ctypes.c_int, [ctypes.c_int64, _vp, _vp, _vp, ctypes.POINTER(MkSpecies),
                                         ctypes.POINTER(MkPhysics), ctypes.POINTER(MkPixels),

@@ -320,8 +320,9 @@ __device__ __forceinline__ double mk_unordered(unsigned long long o)
     return __longlong_as_double(b);
 }
 
-__global__ void mk_bbox_init(unsigned long long *bb)
+__global__ void mk_bbox_init(unsigned long long *bb, int *crowded)
 {
+    if (threadIdx.x == 0 && crowded) *crowded = 0;
     if (threadIdx.x < 3) bb[threadIdx.x] = ~0ull;       // min
     else if (threadIdx.x < 6) bb[threadIdx.x] = 0ull;   // max
 }
@@ -356,10 +357,10 @@ __global__ void __launch_bounds__(MK_BBOX_NT) mk_bbox_kernel(int64_t n, const do
 // Unlike a Z-order (Morton) curve, consecutive cells are always face
 // neighbours, so a run of consecutive atoms never spans two distant corners
 // of the sample and every tile stays compact.
-#define MK_HILBERT_BITS 10   // per axis inside one cube, at most
 #define MK_MAX_CUBES 128     // 7 bits of cube index at most
 
-__device__ __forceinline__ uint32_t mk_hilbert3(uint32_t x, uint32_t y, uint32_t z, int bits)
+template <class Key>
+__device__ __forceinline__ Key mk_hilbert3(uint32_t x, uint32_t y, uint32_t z, int bits)
 {
     uint32_t X[3] = {x, y, z};
     for (uint32_t Q = 1u << (bits - 1); Q > 1; Q >>= 1) {
@@ -383,7 +384,7 @@ __device__ __forceinline__ uint32_t mk_hilbert3(uint32_t x, uint32_t y, uint32_t
     X[0] ^= t;
     X[1] ^= t;
     X[2] ^= t;
-    uint32_t h = 0;
+    Key h = 0;
     for (int b = bits - 1; b >= 0; --b) {
         h = (h << 1) | ((X[0] >> b) & 1u);
         h = (h << 1) | ((X[1] >> b) & 1u);
@@ -395,13 +396,13 @@ __device__ __forceinline__ uint32_t mk_hilbert3(uint32_t x, uint32_t y, uint32_t
 // The cubes and the key's layout, from the bounding box, once per build.
 struct MkKeyGrid {
     double lo[3];
-    float inv[3];        // 1 / cube side, per axis
+    double inv[3];       // 1 / cube side, per axis
     int nc[3];           // cubes per axis
     int bits;            // Hilbert bits per axis
     int cube_bits;
 };
 
-__global__ void mk_key_grid_kernel(const unsigned long long *__restrict__ bb, int key_bits,
+__global__ void mk_key_grid_kernel(const unsigned long long *__restrict__ bb, int key_bits, int axis_bits,
                                    int species_bits, MkKeyGrid *__restrict__ out)
 {
     MkKeyGrid G;
@@ -423,10 +424,10 @@ __global__ void mk_key_grid_kernel(const unsigned long long *__restrict__ bb, in
         if (!(all > MK_MAX_CUBES)) break;
         side *= 1.25;
     }
-    for (int c = 0; c < 3; ++c) G.inv[c] = span[c] > 0.0 ? (float)(G.nc[c] / span[c]) : 0.f;
+    for (int c = 0; c < 3; ++c) G.inv[c] = span[c] > 0.0 ? G.nc[c] / span[c] : 0.0;
     G.cube_bits = 0;
     while ((1 << G.cube_bits) < G.nc[0] * G.nc[1] * G.nc[2]) ++G.cube_bits;
-    G.bits = min(MK_HILBERT_BITS, (key_bits - species_bits - G.cube_bits) / 3);
+    G.bits = min(axis_bits, (key_bits - species_bits - G.cube_bits) / 3);
     *out = G;
 }
 
@@ -441,31 +442,41 @@ __global__ void mk_key_grid_kernel(const unsigned long long *__restrict__ bb, in
 // longer extents as cubes of their own, a few atoms thick, and every tile
 // that crossed one spanned the sample (5.4M atoms of a cubic polycrystal: 14
 // tiles too wide for the node form, 2.1 ms in the split kernel at 1024^2).
-// The key has 32 bits, or 24 below MK_SHORT_KEY_ATOMS atoms (four or three
-// radix passes): the cells then still outnumber the atoms. 62-bit keys
-// (17 Hilbert bits an axis, cut in FP64 by every thread) took 1355 us to make
-// and 551 us to sort for 8.19M atoms, and eight passes, 63 us, for 32k.
+// Short keys have 32 bits, or 24 below MK_SHORT_KEY_ATOMS atoms (four or three
+// radix passes, at most 10 Hilbert bits an axis): in a filled box the cells then
+// outnumber the atoms. Long ones have 62 (17 bits an axis, 8 passes) and resolve
+// samples whose box is mostly empty -- particles far apart, an atom far off --
+// where short cells hold many atoms each, in input order: the tile build reports
+// more than MK_CROWD atoms of a species in one cell. Long keys, then cut in FP64
+// by every thread, took 1355 us to make and 551 us to sort for 8.19M atoms, and
+// 63 us to sort 32k.
 #define MK_SHORT_KEY_ATOMS (1 << 17)
+#define MK_LONG_KEY_BITS 62
+#define MK_CROWD 8
+
+// Real: what the cell coordinates are formed in; 17 bits of up to 128 cubes
+// need FP64.
+template <class Key, class Real>
 __global__ void mk_keys_kernel(int64_t n, const double *__restrict__ pos,
                                const int *__restrict__ species, const MkKeyGrid *__restrict__ grid,
-                               uint32_t *__restrict__ keys, int *__restrict__ idx)
+                               Key *__restrict__ keys, int *__restrict__ idx)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const MkKeyGrid &G = *grid;
     const int bits = G.bits;
-    const float top = (float)((1u << bits) - 1);
+    const Real top = (Real)((1u << bits) - 1);
     uint32_t q[3];
     int cube[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        const float t = (float)(pos[3 * i + c] - G.lo[c]) * G.inv[c];
-        cube[c] = min(G.nc[c] - 1, max(0, (int)floorf(t)));
-        const float f = fminf(fmaxf(t - (float)cube[c], 0.f), 1.f);
+        const Real t = (Real)(pos[3 * i + c] - G.lo[c]) * (Real)G.inv[c];
+        cube[c] = min(G.nc[c] - 1, max(0, (int)floor(t)));
+        const Real f = fmin(fmax(t - (Real)cube[c], (Real)0), (Real)1);
         q[c] = (uint32_t)(f * top);
     }
-    const uint32_t ci = (uint32_t)((cube[2] * G.nc[1] + cube[1]) * G.nc[0] + cube[0]);
-    keys[i] = ((((uint32_t)species[i] << G.cube_bits) | ci) << (3 * bits)) | mk_hilbert3(q[0], q[1], q[2], bits);
+    const Key ci = (Key)((cube[2] * G.nc[1] + cube[1]) * G.nc[0] + cube[0]);
+    keys[i] = ((((Key)species[i] << G.cube_bits) | ci) << (3 * bits)) | mk_hilbert3<Key>(q[0], q[1], q[2], bits);
     idx[i] = (int)i;
 }
 
@@ -484,12 +495,14 @@ struct MkTileMap {
 // stay off the FP64 pipe (2 lane operations per clock and SM), which bound
 // the build at 39 operations an atom (645 us for 8.19M atoms; here 358). Tiles of
 // up to 2 NT atoms hold their positions in registers, larger ones gather them
-// again for the offsets.
+// again for the offsets. `keys` (short ones, or null): *crowded is set where
+// atoms MK_CROWD apart in the order have the same key.
 template <int NT, bool HOLD>
 __global__ void __launch_bounds__(NT) mk_tile_kernel(MkTileMap M, double kappa,
                                                       const double *__restrict__ pos,
                                                       const float2 *__restrict__ amp,
                                                       const int *__restrict__ order,
+                                                      const uint32_t *__restrict__ keys, int *crowded,
                                                       double4 *__restrict__ origin,
                                                       int *__restrict__ tspecies,
                                                       float4 *__restrict__ tpos,
@@ -502,6 +515,9 @@ __global__ void __launch_bounds__(NT) mk_tile_kernel(MkTileMap M, double kappa,
     const long long end = M.run_start[s] + M.run_count[s];
     __shared__ float red[6][NT / 32];
     __shared__ float rad2[NT / 32];
+    if (keys)
+        for (long long i = first + (long long)threadIdx.x * MK_CROWD; i < first + M.tile_atoms; i += NT * MK_CROWD)
+            if (i + MK_CROWD < end && keys[i] == keys[i + MK_CROWD]) *crowded = 1;
     const long long a0 = order[first];
     const double fx = pos[3 * a0], fy = pos[3 * a0 + 1], fz = pos[3 * a0 + 2];
 
@@ -615,24 +631,61 @@ __global__ void __launch_bounds__(NT) mk_tile_kernel(MkTileMap M, double kappa,
 
 static size_t mk_align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
+template <class Key>
 static size_t mk_cub_temp_bytes(int64_t n)
 {
     size_t tb = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, tb, (uint32_t *)nullptr, (uint32_t *)nullptr, (int *)nullptr,
-                                    (int *)nullptr, (int)n, 0, 32);
+    cub::DeviceRadixSort::SortPairs(nullptr, tb, (Key *)nullptr, (Key *)nullptr, (int *)nullptr, (int *)nullptr,
+                                    (int)n, 0, sizeof(Key) == 8 ? MK_LONG_KEY_BITS : 32);
     return tb;
 }
 
-extern "C" size_t mk_tiles_workspace_size(int64_t n)
+extern "C" size_t mk_tiles_workspace_size_keys(int64_t n, int long_keys)
 {
     if (n <= 0) return 256;
-    return mk_align256(64) + mk_align256(sizeof(MkKeyGrid)) + 4 * mk_align256(4 * (size_t)n) +
-           mk_align256(mk_cub_temp_bytes(n));
+    const size_t key = long_keys ? 8 : 4;
+    return mk_align256(64) + mk_align256(sizeof(MkKeyGrid)) + 2 * mk_align256(key * (size_t)n) +
+           2 * mk_align256(4 * (size_t)n) +
+           mk_align256(long_keys ? mk_cub_temp_bytes<unsigned long long>(n) : mk_cub_temp_bytes<uint32_t>(n));
+}
+
+extern "C" size_t mk_tiles_workspace_size(int64_t n) { return mk_tiles_workspace_size_keys(n, 1); }
+
+// Sorted keys and order of the atoms, in the workspace `w`.
+template <class Key, class Real>
+static int mk_sort_atoms(int64_t n, const double *pos, const int *species, const MkKeyGrid *grid, char *w,
+                         int key_bits, cudaStream_t st, const Key **keys, const int **order)
+{
+    Key *k_in = reinterpret_cast<Key *>(w);
+    w += mk_align256(sizeof(Key) * (size_t)n);
+    Key *k_out = reinterpret_cast<Key *>(w);
+    w += mk_align256(sizeof(Key) * (size_t)n);
+    int *i_in = reinterpret_cast<int *>(w);
+    w += mk_align256(4 * (size_t)n);
+    int *i_out = reinterpret_cast<int *>(w);
+    w += mk_align256(4 * (size_t)n);
+    size_t temp = mk_cub_temp_bytes<Key>(n);
+    const int th = 256;
+    mk_keys_kernel<Key, Real><<<(unsigned)((n + th - 1) / th), th, 0, st>>>(n, pos, species, grid, k_in, i_in);
+    MK_CHECK_CUDA(cudaGetLastError());
+    MK_CHECK_CUDA(cub::DeviceRadixSort::SortPairs(w, temp, k_in, k_out, i_in, i_out, (int)n, 0, key_bits, st));
+    *keys = k_out;
+    *order = i_out;
+    return MK_OK;
 }
 
 extern "C" int mk_tiles_build(int64_t n, const double *pos, const int *species, const float *amp,
                               int n_species, const int64_t *counts, double k, mk_tiles *tiles,
                               void *workspace, size_t ws_bytes, void *stream)
+{
+    return mk_tiles_build_keys(n, pos, species, amp, n_species, counts, k, tiles, 1, nullptr, workspace,
+                               ws_bytes, stream);
+}
+
+extern "C" int mk_tiles_build_keys(int64_t n, const double *pos, const int *species, const float *amp,
+                                   int n_species, const int64_t *counts, double k, mk_tiles *tiles,
+                                   int long_keys, int *crowded, void *workspace, size_t ws_bytes,
+                                   void *stream)
 {
     MK_REQUIRE(tiles && counts, "mk_tiles_build: null argument");
     MK_REQUIRE(n_species >= 1 && n_species <= MK_MAX_SPECIES, "mk_tiles_build: 1..%d species",
@@ -664,7 +717,7 @@ extern "C" int mk_tiles_build(int64_t n, const double *pos, const int *species, 
                (long long)n);
     MK_REQUIRE(tiles->n_tiles == tiles_needed, "mk_tiles_build: n_tiles %d, layout needs %d",
                tiles->n_tiles, tiles_needed);
-    const size_t need = mk_tiles_workspace_size(n);
+    const size_t need = mk_tiles_workspace_size_keys(n, long_keys);
     if (!workspace || ws_bytes < need) {
         mk_set_error("mk_tiles_build: workspace %zu bytes, need %zu", ws_bytes, need);
         return MK_ENOMEM;
@@ -674,32 +727,25 @@ extern "C" int mk_tiles_build(int64_t n, const double *pos, const int *species, 
     w += mk_align256(64);
     MkKeyGrid *grid = reinterpret_cast<MkKeyGrid *>(w);
     w += mk_align256(sizeof(MkKeyGrid));
-    uint32_t *k_in = reinterpret_cast<uint32_t *>(w);
-    w += mk_align256(4 * (size_t)n);
-    uint32_t *k_out = reinterpret_cast<uint32_t *>(w);
-    w += mk_align256(4 * (size_t)n);
-    int *i_in = reinterpret_cast<int *>(w);
-    w += mk_align256(4 * (size_t)n);
-    int *i_out = reinterpret_cast<int *>(w);
-    w += mk_align256(4 * (size_t)n);
-    size_t temp = mk_cub_temp_bytes(n);
     cudaStream_t st = mk_stream(stream);
-
-    const int key_bits = n <= MK_SHORT_KEY_ATOMS ? 24 : 32;
+    const int key_bits = long_keys ? MK_LONG_KEY_BITS : n <= MK_SHORT_KEY_ATOMS ? 24 : 32;
     int species_bits = 0;
     while ((1 << species_bits) < n_species) ++species_bits;
-    mk_bbox_init<<<1, 32, 0, st>>>(bb);
+    mk_bbox_init<<<1, 32, 0, st>>>(bb, crowded);
     const int nb = (int)std::min<int64_t>((3 * n + 4 * MK_BBOX_NT - 1) / (4 * MK_BBOX_NT), 152 * 10);
     mk_bbox_kernel<<<nb, MK_BBOX_NT, 0, st>>>(n, pos, bb);
-    mk_key_grid_kernel<<<1, 1, 0, st>>>(bb, key_bits, species_bits, grid);
-    const int th = 256;
-    mk_keys_kernel<<<(unsigned)((n + th - 1) / th), th, 0, st>>>(n, pos, species, grid, k_in, i_in);
-    MK_CHECK_CUDA(cudaGetLastError());
-    MK_CHECK_CUDA(cub::DeviceRadixSort::SortPairs(w, temp, k_in, k_out, i_in, i_out, (int)n, 0, key_bits, st));
+    mk_key_grid_kernel<<<1, 1, 0, st>>>(bb, key_bits, long_keys ? 17 : 10, species_bits, grid);
+    const uint32_t *keys = nullptr;
+    const unsigned long long *keys64 = nullptr;
+    const int *order = nullptr;
+    const int rc = long_keys ? mk_sort_atoms<unsigned long long, double>(n, pos, species, grid, w, key_bits, st,
+                                                                         &keys64, &order)
+                             : mk_sort_atoms<uint32_t, float>(n, pos, species, grid, w, key_bits, st, &keys, &order);
+    if (rc != MK_OK) return rc;
     if (tiles_needed > 0) {
         auto fn = T <= 512 ? mk_tile_kernel<256, true> : mk_tile_kernel<256, false>;
         fn<<<tiles_needed, 256, 0, st>>>(
-            M, k / MK_TWO_PI, pos, reinterpret_cast<const float2 *>(amp), i_out,
+            M, k / MK_TWO_PI, pos, reinterpret_cast<const float2 *>(amp), order, crowded ? keys : nullptr, crowded,
             reinterpret_cast<double4 *>(tiles->origin), tiles->species,
             reinterpret_cast<float4 *>(tiles->pos), reinterpret_cast<float2 *>(tiles->amp));
         MK_CHECK_CUDA(cudaGetLastError());

@@ -569,7 +569,11 @@ def ein_depth(atoms, e0, grid, tau, phi, s_min, s_max, stream=None):
 
 
 class Tiles:
-    """Species-partitioned, Morton-ordered atom tiles (mk_tiles_build)."""
+    """Species-partitioned, Hilbert-ordered atom tiles (mk_tiles_build_keys).
+    The order is built from short keys; the read-back of the tile origins,
+    which every plan and bound starts from, also says where those left many
+    atoms in one cell, and the tiles are then built again from long ones. (In
+    a stream capture, which allows no read-back: long ones at once.)"""
 
     def __init__(self, atoms: Atoms, k, tile_atoms=DEFAULT_TILE_ATOMS, device="cuda", stream=None):
         L = _require_cuda()
@@ -577,7 +581,8 @@ class Tiles:
         counts = np.ascontiguousarray(atoms.counts, dtype=np.int64)
         n_tiles = int(sum((int(c) + T - 1) // T for c in counts))
         self.n_tiles, self.tile_atoms = n_tiles, T
-        self.origin = torch.empty((max(n_tiles, 1), 4), dtype=torch.float64, device=device)
+        rows = torch.empty((max(n_tiles, 1) + 1, 4), dtype=torch.float64, device=device)
+        self.origin = rows[:-1]                     # the last row: the crowding flag
         self.species = torch.empty(max(n_tiles, 1), dtype=torch.int32, device=device)
         self.pos = torch.empty((max(n_tiles, 1) * T, 4), dtype=torch.float32, device=device)
         self.amp = torch.empty((max(n_tiles, 1) * T, 2), dtype=torch.float32, device=device)
@@ -586,13 +591,23 @@ class Tiles:
         self.table, self.counts = atoms.table, counts
         if atoms.n == 0:
             return
-        ws_n = L.mk_tiles_workspace_size(atoms.n)
-        ws = torch.empty(ws_n, dtype=torch.uint8, device=device)
-        check(L.mk_tiles_build(atoms.n, _ptr(atoms.pos), _ptr(atoms.species), _ptr(atoms.amp),
-                               len(counts), counts.ctypes.data_as(ctypes.POINTER(ctypes.c_int64)),
-                               float(k), ctypes.byref(self.abi), _ptr(ws), ws_n,
-                               _stream_handle(stream)))
-        self._ws = ws   # keep until the stream has consumed it
+        capturing = torch.cuda.is_current_stream_capturing()
+        for long_keys in ((1,) if capturing else (0, 1)):
+            ws_n = L.mk_tiles_workspace_size_keys(atoms.n, long_keys)
+            ws = torch.empty(ws_n, dtype=torch.uint8, device=device)
+            check(L.mk_tiles_build_keys(atoms.n, _ptr(atoms.pos), _ptr(atoms.species), _ptr(atoms.amp),
+                                        len(counts), counts.ctypes.data_as(ctypes.POINTER(ctypes.c_int64)),
+                                        float(k), ctypes.byref(self.abi), long_keys, _ptr(rows[-1]),
+                                        _ptr(ws), ws_n, _stream_handle(stream)))
+            self._ws = ws   # keep until the stream has consumed it
+            if capturing:
+                break
+            with torch.cuda.stream(stream):         # None: the current one
+                host = rows.cpu().numpy()
+            if not host[-1].view(np.int32)[0]:
+                break
+        if not capturing:
+            self._origins_host = host[:-1]
 
     def _extents(self):
         """(largest tile radius, largest origin norm), from the origins read

@@ -459,15 +459,23 @@ class beam:
         from . import autotune
         return autotune.tile_atoms(n_pix, kind)
 
-    def choose_split(self, atoms, pix, phys, launch=None):
+    def choose_split(self, atoms, pix, phys, launch=None, built=None):
         """Tiles, set-up and launch shape of the FP32 split sum for these
         atoms and pixels: an explicit ``launch`` or ``_kernel_launch`` (tile
         size ``_kernel_tile_atoms`` or the cached one), else the autotuner's
         cached choice for this detector size, else -- when ``_autotune`` --
         tuned now over tile sizes and launch shapes (the result is cached),
         else the defaults. Returns (setup or None when the geometry declines
-        the split form, launch dict, where it came from, diagnostics)."""
+        the split form, launch dict, where it came from, diagnostics).
+        ``built``: tiles of these atoms made already, used where their size
+        is the one wanted."""
         from . import autotune
+
+        def tiles_of(T):
+            if built is not None and built.tile_atoms == T:
+                return built
+            return engine.Tiles(atoms, self.k, T, device=atoms.pos.device)
+
         explicit = launch or self._kernel_launch
         if not explicit and not phys.analyser and self._autotune and \
                 autotune.cached(pix.n) is None:
@@ -475,8 +483,7 @@ class beam:
                      else list(autotune.TILE_SIZES))
             setups, diags = {}, {}
             for T in sizes:
-                su, diag = self.split_setup(engine.Tiles(atoms, self.k, T, device=atoms.pos.device),
-                                            pix, phys)
+                su, diag = self.split_setup(tiles_of(T), pix, phys)
                 diags[T] = diag
                 if su is not None:
                     setups[T] = su
@@ -485,7 +492,7 @@ class beam:
             best, self.last_tune = autotune.tune(setups, pix, phys, atoms.table)
             T = int(best.pop("tile_atoms"))
             return setups[T], best, "tuned", diags[T]
-        tiles = engine.Tiles(atoms, self.k, self.tile_atoms_for(pix.n), device=atoms.pos.device)
+        tiles = tiles_of(self.tile_atoms_for(pix.n))
         su, diag = self.split_setup(tiles, pix, phys)
         if su is None:
             return None, None, "declined", diag
@@ -494,13 +501,16 @@ class beam:
         src = "cached" if autotune.cached(pix.n) is not None else "default"
         return su, tuned_launch(pix.n, su.level, tiles.tile_atoms), src, diag
 
-    def _scatter_nodes(self, atoms, pix, phys, out, accumulate):
+    def _scatter_nodes(self, atoms, tiles, pix, phys, out, accumulate):
         """The node form of the FP32 sum (detectors on a plane grid, no Darwin
         analyser, no remove_forward), its wide tiles through the split kernel
         and the pixels a top-hat's edge cuts through the FP64 sum; None where
-        its plan declines."""
-        tiles = engine.Tiles(atoms, self.k, int(self._kernel_tile_atoms or engine.DEFAULT_TILE_ATOMS),
-                             device=atoms.pos.device)
+        its plan, or a top-hat that cuts too many pixels, declines."""
+        masked = None
+        if phys.analyser:
+            masked = engine.analyser_mask(tiles, pix, phys, atoms.table)
+            if masked is None:
+                return None
         tol = min(float(self._kernel_phase_tol_rad), float(self._phase_tol_rad))
         plan = engine.NodePlan.make(tiles, pix, self.k, tuple(phys.beam_dir), tol)
         if plan is None:
@@ -514,10 +524,7 @@ class beam:
         # memory runs out: everything is allocated, and the edge pixels
         # summed, before the field is first written
         ws = torch.empty(plan.plan.ws_bytes, dtype=torch.uint8, device=pix.xyz.device)
-        if phys.analyser:
-            masked = engine.analyser_mask(tiles, pix, phys, atoms.table)
-            if masked is None:
-                return None
+        if masked is not None:
             factor, edge = masked
             phys = type(full).from_buffer_copy(full)
             phys.analyser = 0
@@ -550,14 +557,18 @@ class beam:
         return res
 
     def _scatter_once(self, atoms, pix, phys, out=None, accumulate=False, launch=None):
+        tiles = None
         if self._use_fast_kernel and self._use_nodes and not (launch or self._kernel_launch) and \
                 phys.analyser != 2 and not phys.remove_forward and \
-                float(atoms.n) * pix.n >= engine.NODES_MIN_TERMS:
-            res = self._scatter_nodes(atoms, pix, phys, out, accumulate)
+                float(atoms.n) * pix.n >= engine.NODES_MIN_TERMS and \
+                pix.plane_grid(self.k, self._kernel_phase_tol_rad):
+            tiles = engine.Tiles(atoms, self.k, int(self._kernel_tile_atoms or engine.DEFAULT_TILE_ATOMS),
+                                 device=atoms.pos.device)
+            res = self._scatter_nodes(atoms, tiles, pix, phys, out, accumulate)
             if res is not None:
                 return res
         if self._use_fast_kernel and atoms.n > 0:
-            su, cfg, src, diag = self.choose_split(atoms, pix, phys, launch)
+            su, cfg, src, diag = self.choose_split(atoms, pix, phys, launch, built=tiles)
             if su is not None:
                 tiles = su.tiles
                 cfg = engine.grouping_launch(cfg, su.level, tiles, pix, self.k, su.info)

@@ -261,8 +261,21 @@ class Pixels:
                                                int((shapes[:, 1] * shapes[:, 2]).max()),
                                                _ptr(self.xyz), _ptr(fit), _stream_handle(stream)))
             self._fit = (shapes, fit.cpu().numpy())
-            self._r0_min = float(self._fit[1][:, 10].min())
+            f = self._fit[1]
+            self._r0_min = float(f[:, 10].min())
+            with np.errstate(invalid="ignore", divide="ignore", over="ignore"):
+                self._plane = (bool(((f[:, 11] <= 0.25) & (f[:, 10] > 0.0)).all()),
+                               float((f[:, 9] / f[:, 10]).max()))       # NaN: no plane
         return self._fit
+
+    def plane_grid(self, k, phase_tol):
+        """Whether every frame is a plane grid of pixels as ``mk_nodes_plan``
+        asks, known before any tiles are built: within a quarter pixel of even
+        steps, and so little off the plane that atoms 0.1 nm apart -- any tile
+        is wider -- keep their phase within ``phase_tol``."""
+        self.plane_fit()
+        even, off_plane = self._plane
+        return even and 1e-10 * k * off_plane <= phase_tol
 
     def r0_min(self):
         """Smallest pixel distance (one read-back per Pixels object)."""

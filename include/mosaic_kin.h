@@ -300,13 +300,13 @@ int mk_tiles_build(int64_t n, const double *pos, const int *species, const float
                    void *workspace, size_t ws_bytes, void *stream);
 /* mk_tiles_build with the order's resolution given: long keys (17 bits an axis,
  * mk_tiles_build's) or short ones (at most 10), whose build is faster.
- * crowded (device int, may be NULL): 1 where short keys left more than a few
+ * crowded (device double, may be NULL): 1 where short keys left more than a few
  * atoms in one cell, in input order, so that the tiles may be wider than need
  * be: build again with long ones. */
 size_t mk_tiles_workspace_size_keys(int64_t n, int long_keys);
 int mk_tiles_build_keys(int64_t n, const double *pos, const int *species, const float *amp,
                         int n_species, const int64_t *counts, double k, mk_tiles *tiles,
-                        int long_keys, int *crowded, void *workspace, size_t ws_bytes, void *stream);
+                        int long_keys, double *crowded, void *workspace, size_t ws_bytes, void *stream);
 
 /* --- sums ------------------------------------------------------------- */
 /* Bytes of workspace the sums need (partial fields of `slices` slices). */

@@ -320,9 +320,9 @@ __device__ __forceinline__ double mk_unordered(unsigned long long o)
     return __longlong_as_double(b);
 }
 
-__global__ void mk_bbox_init(unsigned long long *bb, int *crowded)
+__global__ void mk_bbox_init(unsigned long long *bb, double *crowded)
 {
-    if (threadIdx.x == 0 && crowded) *crowded = 0;
+    if (threadIdx.x == 0 && crowded) *crowded = 0.0;
     if (threadIdx.x < 3) bb[threadIdx.x] = ~0ull;       // min
     else if (threadIdx.x < 6) bb[threadIdx.x] = 0ull;   // max
 }
@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(NT) mk_tile_kernel(MkTileMap M, double kappa,
                                                       const double *__restrict__ pos,
                                                       const float2 *__restrict__ amp,
                                                       const int *__restrict__ order,
-                                                      const uint32_t *__restrict__ keys, int *crowded,
+                                                      const uint32_t *__restrict__ keys, double *crowded,
                                                       double4 *__restrict__ origin,
                                                       int *__restrict__ tspecies,
                                                       float4 *__restrict__ tpos,
@@ -517,7 +517,7 @@ __global__ void __launch_bounds__(NT) mk_tile_kernel(MkTileMap M, double kappa,
     __shared__ float rad2[NT / 32];
     if (keys)
         for (long long i = first + (long long)threadIdx.x * MK_CROWD; i < first + M.tile_atoms; i += NT * MK_CROWD)
-            if (i + MK_CROWD < end && keys[i] == keys[i + MK_CROWD]) *crowded = 1;
+            if (i + MK_CROWD < end && keys[i] == keys[i + MK_CROWD]) *crowded = 1.0;
     const long long a0 = order[first];
     const double fx = pos[3 * a0], fy = pos[3 * a0 + 1], fz = pos[3 * a0 + 2];
 
@@ -684,7 +684,7 @@ extern "C" int mk_tiles_build(int64_t n, const double *pos, const int *species, 
 
 extern "C" int mk_tiles_build_keys(int64_t n, const double *pos, const int *species, const float *amp,
                                    int n_species, const int64_t *counts, double k, mk_tiles *tiles,
-                                   int long_keys, int *crowded, void *workspace, size_t ws_bytes,
+                                   int long_keys, double *crowded, void *workspace, size_t ws_bytes,
                                    void *stream)
 {
     MK_REQUIRE(tiles && counts, "mk_tiles_build: null argument");

@@ -594,13 +594,15 @@ class Tiles:
         counts = np.ascontiguousarray(atoms.counts, dtype=np.int64)
         n_tiles = int(sum((int(c) + T - 1) // T for c in counts))
         self.n_tiles, self.tile_atoms = n_tiles, T
-        rows = torch.empty((max(n_tiles, 1) + 1, 4), dtype=torch.float64, device=device)
-        self.origin = rows[:-1]                     # the last row: the crowding flag
+        # origins and radii; the last row's first value is the crowding flag,
+        # read back with them
+        self._rows = torch.empty((max(n_tiles, 1) + 1, 4), dtype=torch.float64, device=device)
+        at = self._rows.data_ptr()
         self.species = torch.empty(max(n_tiles, 1), dtype=torch.int32, device=device)
         self.pos = torch.empty((max(n_tiles, 1) * T, 4), dtype=torch.float32, device=device)
         self.amp = torch.empty((max(n_tiles, 1) * T, 2), dtype=torch.float32, device=device)
-        self.abi = MkTiles(n_tiles, T, self.origin.data_ptr(), self.species.data_ptr(),
-                           self.pos.data_ptr(), self.amp.data_ptr())
+        self.abi = MkTiles(n_tiles, T, at, self.species.data_ptr(), self.pos.data_ptr(),
+                           self.amp.data_ptr())
         self.table, self.counts = atoms.table, counts
         if atoms.n == 0:
             return
@@ -610,17 +612,24 @@ class Tiles:
             ws = torch.empty(ws_n, dtype=torch.uint8, device=device)
             check(L.mk_tiles_build_keys(atoms.n, _ptr(atoms.pos), _ptr(atoms.species), _ptr(atoms.amp),
                                         len(counts), counts.ctypes.data_as(ctypes.POINTER(ctypes.c_int64)),
-                                        float(k), ctypes.byref(self.abi), long_keys, _ptr(rows[-1]),
+                                        float(k), ctypes.byref(self.abi), long_keys, at + 32 * n_tiles,
                                         _ptr(ws), ws_n, _stream_handle(stream)))
             self._ws = ws   # keep until the stream has consumed it
             if capturing:
                 break
-            with torch.cuda.stream(stream):         # None: the current one
-                host = rows.cpu().numpy()
-            if not host[-1].view(np.int32)[0]:
-                break
-        if not capturing:
+            if stream is None:
+                host = self._rows.cpu().numpy()
+            else:
+                with torch.cuda.stream(stream):
+                    host = self._rows.cpu().numpy()
             self._origins_host = host[:-1]
+            if not host[-1, 0]:
+                break
+
+    @property
+    def origin(self):
+        """(n_tiles, 4) float64: FP64 origin and radius of every tile."""
+        return self._rows[:-1]
 
     def _extents(self):
         """(largest tile radius, largest origin norm), from the origins read
@@ -983,7 +992,7 @@ class NodePlan:
 
     def __init__(self, plan, buf, tiles):
         self.plan, self.buf, self.tile_atoms = plan, buf, tiles.tile_atoms
-        self.dev = torch.from_numpy(buf[: plan.buf_bytes]).to(tiles.origin.device)
+        self.dev = torch.from_numpy(buf[: plan.buf_bytes]).to(tiles.species.device)
         self.wide = None
         if plan.n_wide:
             idx = np.frombuffer(buf, dtype=np.int32, count=plan.n_wide, offset=plan.off_wide)
@@ -1130,7 +1139,7 @@ class TilesView:
     @classmethod
     def gather(cls, tiles, idx):
         """The tiles ``idx`` (host int32) copied into arrays of their own."""
-        i = torch.from_numpy(np.ascontiguousarray(idx, dtype=np.int64)).to(tiles.origin.device)
+        i = torch.from_numpy(np.ascontiguousarray(idx, dtype=np.int64)).to(tiles.species.device)
         n, T = tiles.n_tiles, tiles.tile_atoms
         v = types.SimpleNamespace(
             tile_atoms=T, table=tiles.table, origin=tiles.origin[i], species=tiles.species[i],

@@ -462,7 +462,7 @@ class SurrogateScan:
         chi0 = float(stage.motor_value[stage.motor_index("chi")])
         self.steps = [dict(mu=mu0 + self.theta[i], chi=chi0 + self.chi[j]) for i, j in self.ij]
         self._staged = None
-        self._side, self._keep = None, []
+        self._side, self._keep, self._last_sum = None, [], None
 
     def prepare(self):
         """Stage the atoms and tiles once (setup shared by every exact call,
@@ -579,11 +579,13 @@ class SurrogateScan:
                                nodes=not direct, **self.kw)
             self._staged = self._staged or scan
             side.wait_stream(cur)
+            begin, done = (torch.cuda.Event(enable_timing=True) for _ in range(2))
             with torch.cuda.stream(side):
+                begin.record(side)
                 f, _ = scan.run(side)
                 out[a:b] = (f * f).sum(1).reshape(len(frames), -1)[: len(sub)].float()
-                done = torch.cuda.Event()
                 done.record(side)
+            self._last_sum = (begin, done)
             # a batch's buffers stay alive until the side stream is done with
             # them; two batches back it long is
             while len(self._keep) >= 2:
@@ -593,16 +595,23 @@ class SurrogateScan:
         cur.wait_stream(side)
         return out
 
+    DIRECT_FRAMES = 64      # frames the direct sum is timed and checked on (one batch)
+
     def run(self, verify=0, exact_all=False):
-        """Run the scan. ``exact_all`` also computes every frame by the direct
-        sum over (atom, pixel) pairs (the exact-only scan, timed), which the
-        true error of every returned frame is measured against -- a reference
-        that shares neither the surrogate's frames nor the node form they are
-        summed with; otherwise the exact-only time is the exact launch's
-        per-frame time times the frame count, and ``verify`` > 0 computes that
-        many unjudged predicted frames directly (untimed) to measure their
-        true error. Where the node form is admitted an exact scan of every
-        frame (``exact(np.arange(n))``) costs less than the networks' fit."""
+        """Run the scan. ``exact_all`` also computes every frame exactly, as
+        ``exact`` does for any user (the exact-only scan, timed), and the
+        error of every returned frame against it; otherwise its time is the
+        exact launch's per-frame time times the frame count, and ``verify`` > 0
+        computes that many unjudged predicted frames directly (untimed) to
+        measure their true error. DIRECT_FRAMES random frames by the direct
+        sum over (atom, pixel) pairs are timed in either case, and with
+        ``exact_all`` compared (``direct_err``): the exact scan's own check.
+
+        ``exact_seconds``, ``gain_vs_exact``: the exact-only scan, and how
+        many times faster this one was; ``direct_seconds``, ``gain``: the same
+        against the direct sum of every frame, at the rate of those frames.
+        Where the node form is admitted an exact scan of every frame costs
+        less than the networks' fit."""
         sync = torch.cuda.synchronize
         n = len(self.ij)
         t = {}
@@ -712,13 +721,20 @@ class SurrogateScan:
                    judge_err=err_j, judge_err_base=err_jb, times=t, setup_seconds=setup_s,
                    seconds=total, frames_per_s=n / total,
                    final_loss=float(self.losses[-1][-1]), params=self.net.n_params, rank=r)
+        rng = np.random.default_rng(self.seed + 2)
+        some = np.sort(rng.choice(n, size=min(n, self.DIRECT_FRAMES), replace=False))
+        I_some = self.exact(some, direct=True)
+        sync()
+        # the sum alone: a long scan's set-up runs beside it
+        res["direct_seconds"] = 1e-3 * self._last_sum[0].elapsed_time(self._last_sum[1]) * n / len(some)
         if exact_all:
-            sync()
             t0 = time.perf_counter()
-            I_all = self.exact(np.arange(n), direct=True)
+            I_all = self.exact(np.arange(n))
             sync()
             ex_s = time.perf_counter() - t0
             res.update(exact_seconds=ex_s, exact_measured=True)
+            res["direct_err"] = frame_rel_error(I_all[torch.as_tensor(some, device=self.dev)],
+                                                I_some).cpu().numpy()
             pi = torch.as_tensor(pred_idx, device=self.dev)
             # the prediction of every predicted frame (judged ones by the
             # network that did not see them), and the spline's alone
@@ -731,7 +747,9 @@ class SurrogateScan:
         else:
             res.update(exact_seconds=n * t["exact"] / (len(tr) + len(judged)), exact_measured=False)
         res["exact_frames_per_s"] = n / res["exact_seconds"]
-        res["gain"] = res["exact_seconds"] / total
+        res["gain_vs_exact"] = res["exact_seconds"] / total
+        res["direct_frames_per_s"] = n / res["direct_seconds"]
+        res["gain"] = res["direct_seconds"] / total
         sync()
         self._keep = []
         if verify and not exact_all:

@@ -198,16 +198,17 @@ class Pixels:
         rec = np.zeros((len(frames), 20))
         arrays, first, size = [], {}, 0       # frames may share a pixel array: uploaded once
         for i, f in enumerate(frames):
-            if np.shape(f.pixels) != (3, sizes[i]):
-                raise ValueError(f"frame {i}: pixels {np.shape(f.pixels)} do not match its shape {self.shapes[i]}")
-            if id(f.pixels) not in first:
-                first[id(f.pixels)] = size
-                arrays.append((size, f.pixels))
+            px = f.source() if hasattr(f, "source") else f.pixels
+            if np.shape(px) != (3, sizes[i]):
+                raise ValueError(f"frame {i}: pixels {np.shape(px)} do not match its shape {self.shapes[i]}")
+            if id(px) not in first:
+                first[id(px)] = size
+                arrays.append((size, px))
                 size += 3 * sizes[i]
             rec[i, :9] = np.asarray(f.rotation, dtype=np.float64).reshape(9)
             rec[i, 9:12] = np.asarray(f.translation, dtype=np.float64).reshape(3)
             rec[i, 12:15] = beam_dirs[i]
-            rec[i, 15:19] = offs[i], *self.shapes[i], first[id(f.pixels)]
+            rec[i, 15:19] = offs[i], *self.shapes[i], first[id(px)]
         self.rotated = bool((rec[:, :9] != np.eye(3).reshape(9)).any())
         lab = torch.empty(size, **dd)
         for a, px in arrays:

@@ -43,6 +43,29 @@ class Frame:
     shape: tuple
 
 
+class RoiFrame(Frame):
+    """A frame of a region of interest: given the ROI's array, which its other
+    frames are given too, its ``pixels`` are a copy of its own from the first
+    time they are read (``source`` reads them without one)."""
+
+    def __init__(self, rotation, translation, pixels, shape):
+        self.rotation, self.translation, self.shape = rotation, translation, shape
+        self._roi, self._own = pixels, None
+
+    @property
+    def pixels(self):
+        if self._own is None:
+            self._own = self._roi.copy()
+        return self._own
+
+    @pixels.setter
+    def pixels(self, value):
+        self._own = value
+
+    def source(self):
+        return self._roi if self._own is None else self._own
+
+
 def roi_indices(det_shape, side, centre=None):
     """Pixel indices (iz*Ny + iy) of a square ROI of ``side`` pixels centred
     on the detector (or on ``centre`` = (iy, iz)), clipped to the detector."""
@@ -364,23 +387,21 @@ def frames_from_motors(stage, detector, steps, rois=None):
     saved = stage._motor_value.copy()
     out = []
     full = np.asarray(detector.pixel_coordinates)
-    roi_pixels = {}             # the frames of one ROI share its pixel array (read-only)
+    roi_pixels = {}             # gathered once for the frames of one ROI
     try:
         for i, st in enumerate(steps):
             stage._motor_value[:] = saved
             for name, v in st.items():
                 stage._motor_value[stage.motor_index(name)] = float(v)
             R, t = stage.get_rotation().copy(), stage.get_translation().copy()
-            coords, shape = full, tuple(detector.shape)
-            if rois is not None and rois[i] is not None:
-                side = int(rois[i])
-                if side not in roi_pixels:
-                    sel, shape = roi_indices(detector.shape, side)
-                    coords = full[:, sel]
-                    coords.flags.writeable = False
-                    roi_pixels[side] = (coords, shape)
-                coords, shape = roi_pixels[side]
-            out.append(Frame(R, t, coords, shape))
+            if rois is None or rois[i] is None:
+                out.append(Frame(R, t, full, tuple(detector.shape)))
+                continue
+            side = int(rois[i])
+            if side not in roi_pixels:
+                sel, shape = roi_indices(detector.shape, side)
+                roi_pixels[side] = (full[:, sel], shape)
+            out.append(RoiFrame(R, t, *roi_pixels[side]))
     finally:
         stage._motor_value[:] = saved
         stage.get_rotation()

@@ -45,14 +45,18 @@ struct MkPlainArgs {
 // kernel holds the factor F there (f0 + f' + i f'', Debye-Waller, polarization)
 // and the first two derivatives of f0 in cos(2 theta); per term only the
 // CHANGE from the pixel's direction, 1 + eta, is formed in FP32 and multiplied
-// into the phasor, and F into the sum of a species' terms. At the limit, with c =
-// b / (2 lambda^2) <= 240 (b <= 180 A^2, 20 keV): the change is at most c e =
-// 4e-5 of a term of f0, so FP32 leaves 2e-12 of that term (1e-13 for the b ~
-// 1/s^2 that count at a reflection); f0's third order (c e)^3 / 6 is 8e-15, the
-// second order in polarization and decay below 1e-13 for P_pol > 1/4. Beyond
-// the limit, with an analyser, at P_pol < 1/4, at the Q_cut edge and where F is
-// too small beside its derivative every factor is evaluated per term as the
-// reference does.
+// into the phasor, and F into the sum of a species' terms. With e = |a| / |P|, d_i =
+// b_i / (2 lambda^2) and f_i the Gaussians of f0, the change of f0 is at most sum
+// |f_i| d_i (sin(2 theta) e + e^2); FP32 forms the change of cos(2 theta) to 3
+// roundings of e and the product to 4 of itself. The expansion is taken where that
+// stays below 1e-12 of |F|, the third order below 2e-13 and the Debye-Waller
+// factor's roundings below 5e-13 of theirs (tested per pixel and species: it
+// holds for tabulated atoms at 8 to 20 keV, and fails near forward at high
+// energies, for very wide electron clouds and where F cancels). Polarization and
+// decay change by e at most, their second order is below 1e-13 for P_pol > 1/4;
+// with the sine and cosine below, a term is within 2e-12 of its size. Beyond
+// the limit, with an analyser, at P_pol < 1/4 and at the Q_cut edge every factor
+// is evaluated per term as the reference does.
 //
 // The phase k (a_x + r) keeps the reference's roundings bit for bit. r = the
 // rounded root of v = |P - a|^2 comes from a start r0 = R0 - u.a + (|a|^2 -
@@ -155,6 +159,7 @@ __global__ void __launch_bounds__(F64_NT) mk_plain_f64_kernel(
             const double uy = cy / R0, uz = cz / R0;
             vx = (float)ux; vy = (float)uy; vz = (float)uz;
             inv_R = (float)(1.0 / R0);
+            const float across0 = sqrtf(fmaf(vz, vz, vy * vy));          // sin(2 theta)
             const double g = fmax(2.0 * (1.0 - ux), 0.0), Q = A.k * sqrt(g);
             const double sk = s_fac * A.k, s2 = sk * sk * g, ds2 = -2.0 * sk * sk;   // d s2 / d ux
             s2x = (float)ds2;
@@ -174,23 +179,32 @@ __global__ void __launch_bounds__(F64_NT) mk_plain_f64_kernel(
             }
             for (int s = 0; s < A.sp.n; ++s) {
                 const float *wk = s_wk[s];
-                double f0 = wk[5], f1 = 0.0, f2 = 0.0;
+                double f0 = wk[5], f1 = 0.0, f2 = 0.0, f1_abs = 0.0;
+                float b_max = 0.f;
                 for (int i = 0; i < 5; ++i) {
-                    const double b = (double)wk[6 + i], t = (double)wk[i] * exp(-b * s2), d = -b * ds2;
+                    const double b = (double)wk[6 + i], t = (double)wk[i] * exp(-b * s2), d = -b * ds2, td = t * d;
                     f0 += t;
-                    f1 += t * d;
-                    f2 += t * d * d;
+                    f1 += td;
+                    f1_abs += fabs(td);
+                    f2 += td * d;
+                    b_max = fmaxf(b_max, fabsf(wk[6 + i]));
                 }
                 double fre = f0 + A.sp.anr[s], fim = A.sp.ani[s];
                 if (forward) {
                     fre -= (double)A.sp.f0z[s] + A.sp.anr[s];
                     fim = 0.0;
                 }
-                // F0 + change as F0 (1 + change / F0): a change of 1 % at most
+                // F0 + change as F0 (1 + change / F0), each remainder against F0
                 const double m2 = fre * fre + fim * fim;
-                if (!(f1 * f1 * 1e-13 < 1e-4 * m2)) expand = false;
+                const double round = f1_abs * (F64_FAR * 0x1p-24) * (double)(3.f + 4.f * across0);
+                const double d_e = (double)(b_max * -s2x * F64_FAR), third = f1_abs * F64_FAR * d_e * d_e / 6.0;
+                if (!(round * round <= 1e-24 * m2 && third * third <= 4e-26 * m2)) expand = false;
                 double w = scale0;
-                if (A.sp.has_dw) w *= exp(-(double)A.sp.dwb[s] * s2);
+                if (A.sp.has_dw) {
+                    w *= exp(-(double)A.sp.dwb[s] * s2);
+                    if (!(fabsf(A.sp.dwb[s] * s2x) * (F64_FAR * 0x1p-24f) * (3.f + 4.f * across0) <= 5e-13f))
+                        expand = false;
+                }
                 s_F[s * F64_NT + threadIdx.x] = make_double2(fre * w, fim * w);
                 s_df[s * F64_NT + threadIdx.x] =
                     make_float4((float)f1, (float)(0.5 * f2), (float)(fre / m2), (float)(-fim / m2));

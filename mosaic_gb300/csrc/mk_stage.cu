@@ -91,7 +91,9 @@ __global__ void mk_pixels_kernel(int ny, int nz, const double *__restrict__ xyz,
 }
 
 // A scan's frames: lab pixels (A) into the sample frame, P' = R^T (P - t) /
-// 1e10, and their prologue, all frames in one launch. `frames`: 20 doubles
+// 1e10, and their prologue, all frames in one launch. The product is rounded as
+// NumPy's matrix product rounds it (first term, then one FMA each): k |P| is
+// ~5e10 rad, where an ulp of a position turns a frame's phase by ~1e-5 rad. `frames`: 20 doubles
 // each -- R (9), t (3), b (3), first pixel, ny, nz, lab offset, 1 unused -- and
 // lab holds a frame's (3, ny nz) coordinates from that offset on (frames of one
 // ROI may share them). FP64 pipe:
@@ -119,7 +121,7 @@ __global__ void __launch_bounds__(256) mk_scan_pixels_kernel(const double *__res
             const int i = j == 0 ? p : (j == 1 ? i0 : i1);
             const double x = L[i] - F[9], y = L[n + i] - F[10], z = L[2ll * n + i] - F[11];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) P[j][c] = mk_metres(F[c] * x + F[3 + c] * y + F[6 + c] * z);
+            for (int c = 0; c < 3; ++c) P[j][c] = mk_metres(fma(F[6 + c], z, fma(F[3 + c], y, __dmul_rn(F[c], x))));
         }
         const MkPixelOut o = mk_pixel(P[0], P[1], P[2], kappa, k, b);
         const long long g = off + p;

@@ -7,13 +7,13 @@
 // strides: the same operand conventions as mk_gemm_bf16, so one kernel
 // serves the MLP's forward pass, its input and weight gradients and the
 // decoding of predicted frames). A CTA of 8 warps owns a 128 x BN tile of C:
-// the K loop runs in chunks of 64 through MK_TCG_STAGES shared-memory
+// the K loop runs in chunks of 64 through S (3 or 5) shared-memory
 // stages, two chunks ahead of the tensor core: every thread stages part of
 // a chunk into the K-major core-matrix layout of mk_tc.cuh (k-contiguous
 // operands by asynchronous 16-byte cp.async copies, row-contiguous ones by
 // batched 16-byte loads repacked in registers), one elected thread issues
 // the chunk's four tcgen05.mma (K = 16 each) and commits them to the
-// stage's mbarrier, which frees the stage for the chunk MK_TCG_STAGES
+// stage's mbarrier, which frees the stage for the chunk S
 // later. The epilogue reads the accumulator back with tcgen05.ld (warp w:
 // TMEM lanes 32 (w % 4) .. + 31 = tile rows, columns of half w / 4), one
 // row per thread. Split-K over gridDim.z adds partial tiles into C with atomics.
@@ -26,11 +26,13 @@
 
 #define MK_TCG_BM 128
 #define MK_TCG_BK 64
-// Stages: wide outputs (BN 128, the frame decode) 3, which lets two CTAs share
-// an SM; 64-column tiles 5, so that all four chunks of a 256-deep layer are in
-// flight before its first MMA (few CTAs, latency-bound: 11.0 -> 10.1 us a launch of
-// two 1272 x 256 x 256 networks).
-#define MK_TCG_STAGES(BN) ((BN) >= 128 ? 3 : 5)
+// Stages of the ring: 3 let three CTAs of 64-column tiles (two of 128) share an
+// SM; 5, one CTA an SM, where no more CTAs than SMs are launched, so that all
+// four chunks of a 256-deep layer are in flight before its first MMA. Two
+// networks' M x 256 x 256 layer, 3 and 5 stages: M = 1272 (80 CTAs) 9.9 and 8.9
+// us, 2048 (128) 10.1 and 9.0, 4864 (304) 15.1 and 17.2, 40000 (2504) 102 and 134.
+#define MK_TCG_STAGES 3
+#define MK_TCG_STAGES_FEW 5
 #define MK_TCG_NT 256
 
 #define MK_GEMM_ACCUMULATE 1
@@ -186,17 +188,16 @@ __device__ __forceinline__ void mk_tcg_load16(float (&d)[16], const float *p, in
     }
 }
 
-template <int BN>
+template <int BN, int S>
 __global__ void __launch_bounds__(MK_TCG_NT) mk_gemm_tc_kernel(MkTcGemm g, int *status)
 {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     // 1024-byte aligned base for the operand stages
     unsigned char *smem = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem);            // MK_TCG_STAGES barriers
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem);            // S barriers
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + 64);
     unsigned char *stages = smem + 1024;
-    constexpr int S = MK_TCG_STAGES(BN);
     constexpr int A_BYTES = MK_TCG_BM * MK_TCG_BK * 2;
     constexpr int STAGE_BYTES = A_BYTES + BN * MK_TCG_BK * 2;
     constexpr uint32_t NCOLS = BN < 32 ? 32u : (uint32_t)BN;
@@ -400,13 +401,13 @@ static int mk_tcg_read_status(cudaStream_t st)
     return MK_OK;
 }
 
-template <int BN>
+template <int BN, int S>
 static int mk_tcg_launch(const MkTcGemm &g, dim3 grid, cudaStream_t st, int *status)
 {
-    const size_t smem = 2048 + (size_t)MK_TCG_STAGES(BN) * (MK_TCG_BM + BN) * MK_TCG_BK * 2;
-    MK_CHECK_CUDA(cudaFuncSetAttribute((const void *)mk_gemm_tc_kernel<BN>,
+    const size_t smem = 2048 + (size_t)S * (MK_TCG_BM + BN) * MK_TCG_BK * 2;
+    MK_CHECK_CUDA(cudaFuncSetAttribute((const void *)mk_gemm_tc_kernel<BN, S>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    mk_gemm_tc_kernel<BN><<<grid, MK_TCG_NT, smem, st>>>(g, status);
+    mk_gemm_tc_kernel<BN, S><<<grid, MK_TCG_NT, smem, st>>>(g, status);
     MK_CHECK_CUDA(cudaGetLastError());
     return MK_OK;
 }
@@ -473,7 +474,12 @@ extern "C" int mk_gemm_tc_groups(int groups, const long long *group_strides, int
     }
     MK_REQUIRE((long long)groups * g.slices < 65536, "mk_gemm_tc: too many groups");
     grid.z = (unsigned)(groups * g.slices);
-    return bn == 128 ? mk_tcg_launch<128>(g, grid, st, status) : mk_tcg_launch<64>(g, grid, st, status);
+    int dev = 0, sms = 0;
+    MK_CHECK_CUDA(cudaGetDevice(&dev));
+    MK_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (bn == 128) return mk_tcg_launch<128, MK_TCG_STAGES>(g, grid, st, status);
+    return (long long)grid.x * grid.y * grid.z <= sms ? mk_tcg_launch<64, MK_TCG_STAGES_FEW>(g, grid, st, status)
+                                                      : mk_tcg_launch<64, MK_TCG_STAGES>(g, grid, st, status);
 }
 
 extern "C" int mk_gemm_tc(int M, int N, int K, const void *A, long long sam, long long sak,

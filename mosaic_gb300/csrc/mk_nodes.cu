@@ -1855,13 +1855,20 @@ static int mk_merge(const MkMergeArgs &A, int n_in, int n_runs, cudaStream_t st)
     return MK_OK;
 }
 
+// A tile's atoms in shared memory. The kernels' limit is set to that of the
+// largest tiles with every launch: threads with smaller ones must not lower it
+// between another's setting it and its launch.
+#define MK_TILE_ATOMS_MAX 4096
+static size_t leaf_bytes(int tile_atoms) { return (size_t)tile_atoms * 24; }
+
 template <int N0, int NS>
 static int mk_launch_leaf8(const MkNodeArgs &A, MkSubArgs B, int n_list, const MkNodeRec *rec,
                            long long nodes, float2 *V, cudaStream_t st)
 {
-    const size_t smem = (size_t)A.tile_atoms * 24 + 8 * 8 * (size_t)NS * (NS + N0) + 4 * (size_t)N0 * NS;
+    const size_t fixed = 8 * 8 * (size_t)NS * (NS + N0) + 4 * (size_t)N0 * NS, smem = leaf_bytes(A.tile_atoms) + fixed;
     auto fn = mk_node_leaf8_kernel<N0, NS>;
-    MK_CHECK_CUDA(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MK_CHECK_CUDA(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(leaf_bytes(MK_TILE_ATOMS_MAX) + fixed)));
     // a block's patches share its tile's atoms and boxes; 16 blocks an SM first
     const int patches = (int)(nodes / (N0 * N0));
     B.patches = (int)std::max<long long>(1, std::min<long long>(8, (long long)n_list * patches / (16 * 152)));
@@ -1885,6 +1892,8 @@ extern "C" int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, c
     MK_REQUIRE(!phys->analyser && !phys->remove_forward && phys->k > 0.0,
                "mk_kin_nodes_f32: no analyser (a top-hat comes in the factor table, mk_analyser_mask) and "
                "no remove_forward here");
+    MK_REQUIRE(tiles->tile_atoms >= 128 && tiles->tile_atoms <= MK_TILE_ATOMS_MAX,
+               "mk_kin_nodes_f32: bad tile_atoms %d", tiles->tile_atoms);
     MK_REQUIRE(plan->n_src >= 1 && plan->n_frames >= 1 && (long long)px->ny * px->nz >= plan->n_pix,
                "mk_kin_nodes_f32: empty plan or too few pixels");
     if (!workspace || ws_bytes < (size_t)plan->ws_bytes) {
@@ -1964,12 +1973,11 @@ extern "C" int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, c
     mk_node_prep_kernel<<<dim3(plan->n_frames, prep.node_blocks + std::min((points + 3) / 4, most)), MK_PREP_NT, 0,
                           st>>>(prep);
     MK_CHECK_CUDA(cudaGetLastError());
-    const size_t leaf_smem = (size_t)T * 24;
-    MK_CHECK_CUDA(cudaFuncSetAttribute((const void *)mk_node_leaf_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)leaf_smem));
+    MK_CHECK_CUDA(cudaFuncSetAttribute((const void *)mk_node_leaf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)leaf_bytes(MK_TILE_ATOMS_MAX)));
     auto leaf = [&](const int *list, const int *rows, int n_list, const MkNodeRec *rec, long long nodes, float2 *V) {
         const int th = (int)std::min<long long>(256, (nodes + 31) / 32 * 32);
-        mk_node_leaf_kernel<<<dim3(n_list, (unsigned)((nodes + th - 1) / th)), th, leaf_smem, st>>>(
+        mk_node_leaf_kernel<<<dim3(n_list, (unsigned)((nodes + th - 1) / th)), th, leaf_bytes(T), st>>>(
             A, list, rows, rec, nodes, V);
     };
     // passes of whole frames whose node fields and partials fit the chunk

@@ -125,6 +125,7 @@ __global__ void mk_prop_crop_kernel(const float2 *__restrict__ G, int ny2, int n
 #define MK_FFT_NT 512
 #define MK_FFT_MAX 8192
 #define MK_FFT_SMEM (74 << 10)    // a block's lines where three blocks fit an SM
+#define MK_FFT_SMEM_MAX (227u << 10)
 
 __device__ __forceinline__ float2 mk_cmul(float2 a, float2 b)
 {
@@ -358,7 +359,7 @@ static int mk_prop_cols_width(int ny2, int nz2)
 {
     int W = 16;
     while (W > 4 && sizeof(float2) * (size_t)W * mk_prop_ld(nz2, W) > MK_FFT_SMEM) W /= 2;
-    while (W > 1 && sizeof(float2) * (size_t)W * mk_prop_ld(nz2, W) > (227u << 10)) W /= 2;
+    while (W > 1 && sizeof(float2) * (size_t)W * mk_prop_ld(nz2, W) > MK_FFT_SMEM_MAX) W /= 2;
     return std::max(1, std::min(W, ny2));
 }
 
@@ -426,8 +427,11 @@ extern "C" int mk_prop_cols_rows(float *spectrum, int ny2, int nz2, int z0, int 
     const size_t smem = sizeof(float2) * (size_t)A.W * (size_t)A.ld;
     const int last = logn % 3 == 0 ? 3 : logn % 3;
     auto fn = last == 1 ? mk_prop_cols_kernel<1> : (last == 2 ? mk_prop_cols_kernel<2> : mk_prop_cols_kernel<3>);
+    // the same value with every launch: another thread's smaller transform must not
+    // lower the limit before this one's launch
     if (smem > (48u << 10))
-        MK_CHECK_CUDA(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        MK_CHECK_CUDA(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)MK_FFT_SMEM_MAX));
     fn<<<ny2 / A.W, MK_FFT_NT, smem, st>>>(A);
     MK_CHECK_CUDA(cudaGetLastError());
     return MK_OK;

@@ -425,7 +425,10 @@ extern "C" int mk_kin_plain_f64(int64_t n, const double *pos, const int *species
     // expansions per (species, pixel): the factor and its derivatives
     const size_t smem = A.analyser ? 0 : (sizeof(double2) + sizeof(float4)) * (size_t)A.sp.n * F64_NT;
     auto fn = A.analyser ? mk_plain_f64_kernel<false> : mk_plain_f64_kernel<true>;
-    MK_CHECK_CUDA(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // the same value with every launch: threads with fewer species must not lower
+    // the limit between another's setting it and its launch
+    MK_CHECK_CUDA(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)((sizeof(double2) + sizeof(float4)) * MK_MAX_SPECIES * F64_NT)));
     fn<<<grid, F64_NT, smem, st>>>(n, per, pos, species, reinterpret_cast<const float2 *>(amp), n_pix, px->xyz,
                                    px->r0, reinterpret_cast<const double4 *>(px->q), A, part);
     MK_CHECK_CUDA(cudaGetLastError());

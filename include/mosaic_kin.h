@@ -185,6 +185,7 @@ typedef struct {
     int n_wide;             /* tiles left to the split kernel (their indices at off_wide) */
     int n_src;              /* n_groups + n_mid */
     int slices, src_per_slice, passes;
+    int sms;                /* SMs of the device it was planned for */
     int ns[2];              /* nodes per axis of a tile's eighths, narrow tiles and others (0: tiles
                              evaluated whole) */
     int n_narrow;           /* narrow tiles (the first of off_leaf) */

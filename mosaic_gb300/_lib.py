@@ -154,7 +154,7 @@ class MkLaunch(ctypes.Structure):
 class MkNodePlan(ctypes.Structure):
     _fields_ = [(n, ctypes.c_int) for n in
                 ("n_frames", "n_tiles", "n0", "n1", "group_tiles", "n_groups", "n_members", "n_mid",
-                 "n_wide", "n_src", "slices", "src_per_slice", "passes")] + \
+                 "n_wide", "n_src", "slices", "src_per_slice", "passes", "sms")] + \
                [("ns", ctypes.c_int * 2)] + [(n, ctypes.c_int) for n in ("n_narrow", "nm", "n_msrc", "n_msingle")] + \
                [(n, ctypes.c_longlong) for n in ("patches0", "patchesm", "patches1", "weights", "n_pix")] + \
                [("sub_w_off", ctypes.c_longlong * 2)] + \

@@ -809,6 +809,9 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
             item[m] += (long long)F.pz[to] * F.py[in] * M.strips * M.chunks;
         }
     }
+    int sms = 152, devid = 0;               // 152: planned without a device
+    if (cudaGetDevice(&devid) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, devid);
+    plan->sms = sms;
     const long long patch = patches[MK_FINE];
     plan->patches0 = patches[MK_COARSE];
     plan->patchesm = patches[MK_MIDDLE];
@@ -818,7 +821,7 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
         const int ns = sub_nodes(best.n0, tile_atoms, c == 0);
         if (!sub_nodes(best.n0, tile_atoms, true)) break;
         // a second launch pays where both fill the chip: eight blocks an SM
-        const bool two = (long long)members.size() * plan->patches0 >= 8 * 152;
+        const bool two = (long long)members.size() * plan->patches0 >= 8ll * sms;
         const double split_at = two ? narrow_radius(best.n0, sub_nodes(best.n0, tile_atoms, true), best.r1) : -1.0;
         for (size_t i = 0; i < members.size(); ++i)
             if ((rad[members[i]] <= split_at) == (c == 0)) {
@@ -835,8 +838,6 @@ extern "C" int mk_nodes_plan(int n_tiles, int tile_atoms, int n_species, const i
     plan->weights = wf;
     // slices of sources: enough blocks for every SM several times over, at
     // least eight sources a slice
-    int sms = 152, devid = 0;
-    if (cudaGetDevice(&devid) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, devid);
     const long long want = (12ll * sms + pblk - 1) / pblk;
     plan->slices = (int)std::max<long long>(1, std::min<long long>(std::min<long long>(want, 256),
                                                                    plan->n_src / 8));
@@ -1863,7 +1864,7 @@ static size_t leaf_bytes(int tile_atoms) { return (size_t)tile_atoms * 24; }
 
 template <int N0, int NS>
 static int mk_launch_leaf8(const MkNodeArgs &A, MkSubArgs B, int n_list, const MkNodeRec *rec,
-                           long long nodes, float2 *V, cudaStream_t st)
+                           long long nodes, float2 *V, int sms, cudaStream_t st)
 {
     const size_t fixed = 8 * 8 * (size_t)NS * (NS + N0) + 4 * (size_t)N0 * NS, smem = leaf_bytes(A.tile_atoms) + fixed;
     auto fn = mk_node_leaf8_kernel<N0, NS>;
@@ -1871,7 +1872,7 @@ static int mk_launch_leaf8(const MkNodeArgs &A, MkSubArgs B, int n_list, const M
                                        (int)(leaf_bytes(MK_TILE_ATOMS_MAX) + fixed)));
     // a block's patches share its tile's atoms and boxes; 16 blocks an SM first
     const int patches = (int)(nodes / (N0 * N0));
-    B.patches = (int)std::max<long long>(1, std::min<long long>(8, (long long)n_list * patches / (16 * 152)));
+    B.patches = (int)std::max<long long>(1, std::min<long long>(8, (long long)n_list * patches / (16ll * sms)));
     fn<<<dim3(n_list, (patches + B.patches - 1) / B.patches), mk_leaf8_threads(NS), smem, st>>>(A, B, rec, nodes, V);
     return MK_OK;
 }
@@ -1894,7 +1895,7 @@ extern "C" int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, c
                "no remove_forward here");
     MK_REQUIRE(tiles->tile_atoms >= 128 && tiles->tile_atoms <= MK_TILE_ATOMS_MAX,
                "mk_kin_nodes_f32: bad tile_atoms %d", tiles->tile_atoms);
-    MK_REQUIRE(plan->n_src >= 1 && plan->n_frames >= 1 && (long long)px->ny * px->nz >= plan->n_pix,
+    MK_REQUIRE(plan->n_src >= 1 && plan->n_frames >= 1 && plan->sms >= 1 && (long long)px->ny * px->nz >= plan->n_pix,
                "mk_kin_nodes_f32: empty plan or too few pixels");
     if (!workspace || ws_bytes < (size_t)plan->ws_bytes) {
         mk_set_error("mk_kin_nodes_f32: workspace %zu bytes, need %lld", ws_bytes, plan->ws_bytes);
@@ -1965,7 +1966,7 @@ extern "C" int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, c
                                       (F.mg[0].ratio_y + F.mg[0].ratio_z) * nm);
     }
     for (int l = 0; l < 5; ++l) prep.cheb[l].fill(prep.n[l]);
-    const int most = std::max(1, 1216 / plan->n_frames);
+    const int most = std::max(1, 8 * plan->sms / plan->n_frames);
     prep.node_blocks = std::min((nodes + MK_PREP_NT - 1) / MK_PREP_NT, most);
     prep.kappa = A.kappa_d;
     prep.xyz = px->xyz;
@@ -2011,14 +2012,14 @@ extern "C" int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, c
                 B.rec = rec[3 + c] + F.off[MK_COARSE] * ns * ns;
                 int rc = MK_OK;
                 switch (n0 * 100 + ns) {
-                case 2014: rc = mk_launch_leaf8<20, 14>(A, B, n, r0, nodes0, V[0], st); break;
-                case 2012: rc = mk_launch_leaf8<20, 12>(A, B, n, r0, nodes0, V[0], st); break;
-                case 1612: rc = mk_launch_leaf8<16, 12>(A, B, n, r0, nodes0, V[0], st); break;
-                case 1610: rc = mk_launch_leaf8<16, 10>(A, B, n, r0, nodes0, V[0], st); break;
-                case 1210: rc = mk_launch_leaf8<12, 10>(A, B, n, r0, nodes0, V[0], st); break;
-                case 1208: rc = mk_launch_leaf8<12, 8>(A, B, n, r0, nodes0, V[0], st); break;
-                case 1008: rc = mk_launch_leaf8<10, 8>(A, B, n, r0, nodes0, V[0], st); break;
-                case 806: rc = mk_launch_leaf8<8, 6>(A, B, n, r0, nodes0, V[0], st); break;
+                case 2014: rc = mk_launch_leaf8<20, 14>(A, B, n, r0, nodes0, V[0], plan->sms, st); break;
+                case 2012: rc = mk_launch_leaf8<20, 12>(A, B, n, r0, nodes0, V[0], plan->sms, st); break;
+                case 1612: rc = mk_launch_leaf8<16, 12>(A, B, n, r0, nodes0, V[0], plan->sms, st); break;
+                case 1610: rc = mk_launch_leaf8<16, 10>(A, B, n, r0, nodes0, V[0], plan->sms, st); break;
+                case 1210: rc = mk_launch_leaf8<12, 10>(A, B, n, r0, nodes0, V[0], plan->sms, st); break;
+                case 1208: rc = mk_launch_leaf8<12, 8>(A, B, n, r0, nodes0, V[0], plan->sms, st); break;
+                case 1008: rc = mk_launch_leaf8<10, 8>(A, B, n, r0, nodes0, V[0], plan->sms, st); break;
+                case 806: rc = mk_launch_leaf8<8, 6>(A, B, n, r0, nodes0, V[0], plan->sms, st); break;
                 default: leaf(B.list, B.rows, n, r0, nodes0, V[0]);
                 }
                 if (rc != MK_OK) return rc;

@@ -17,7 +17,8 @@ Arithmetic runs on the GPU in libmosaic_kin.so:
   * ``_use_fast_kernel`` False: FP64 plain sum (``mk_kin_plain_f64``), the
     reference CPU kernel's arithmetic with its rounding of the phase; the
     slowly varying factors are expanded about each pixel's direction where
-    the sample is small against the distance (to ~1e-14 of the sum).
+    the sample is small against the distance (each term to 2e-12 of its size;
+    the phase's own rounding is worth ~2e-6).
 There is no CPU path: ``use_gpu=False`` and a missing GPU raise.
 """
 from __future__ import annotations

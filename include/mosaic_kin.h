@@ -435,7 +435,7 @@ int mk_kin_nodes_f32(const mk_tiles *tiles, const mk_physics *phys, const mk_pix
  * `excursion` [rad] of the pixel's own is accepted and 0 elsewhere; pixels the
  * acceptance edge may cut are 0 too and listed in edge (device, 1 + edge_cap
  * ints: how many there are, then the first edge_cap of them, in any order),
- * for mk_kin_plain_f64 to sum. */
+ * to be summed with the analyser per atom (mk_kin_split_f32, mk_kin_plain_f64). */
 int mk_analyser_mask(const mk_pixels *px, const mk_physics *phys, double excursion, int n_species,
                      float *factor_out, int *edge, int edge_cap, void *stream);
 

@@ -1783,8 +1783,8 @@ __global__ void mk_node_sums_final_kernel(int n_frames, const double *__restrict
 // |u' - c|^2 is within 2 sqrt(x) exc + exc^2 of the pixel's: a pixel whose own
 // x is farther than that from the acceptance edge takes one factor, 0 or 1,
 // for every atom, which its factor-table entries carry; the others (the edge
-// passes them within 1e-7 rad: a pixel or two of a detector) are zeroed and
-// listed for the FP64 sum. FP64, one pass: 24 B read, 16 B a species.
+// passes them within 1e-7 rad: a few of a detector) are zeroed and listed for
+// the split kernel's per-atom test. FP64, one pass: 24 B read, 16 B a species.
 __global__ void __launch_bounds__(256) mk_analyser_mask_kernel(long long n, const double *__restrict__ xyz,
                                                                double cx, double cy, double cz, double x_acc,
                                                                double exc, int n_species,

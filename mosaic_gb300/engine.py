@@ -1034,7 +1034,7 @@ class NodePlan:
                     wide_tiles=p.n_wide, group_radius_m=p.radius2_m)
 
 
-EDGE_PIXELS = 1024      # pixels the acceptance edge may cut that the FP64 sum takes
+EDGE_PIXELS = 1024      # pixels the acceptance edge may cut beside the node form
 
 
 def analyser_mask(tiles, pix, phys, table, stream=None):
@@ -1055,7 +1055,7 @@ def analyser_mask(tiles, pix, phys, table, stream=None):
     n = int(edge[0])
     if n > EDGE_PIXELS:
         return None
-    return out, edge[1:1 + n].long()
+    return out, edge[1:1 + n].sort().values.long()      # listed in any order
 
 
 def run_nodes(np_, tiles, pix, phys, table, out=None, accumulate=False, fresnel=0, fresnel_radius=0.0,

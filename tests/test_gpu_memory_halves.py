@@ -72,14 +72,17 @@ def test_top_hat_edge_pixels_are_added_once(cuda, monkeypatch):
     _always_nodes(monkeypatch)
     whole = B.atomic_scattering_kinematic(sample, D, st, **kw)
     assert B.last_run["launch_source"] == "nodes" and B.last_run["edge_pixels"] >= 1
-    plain, failed = engine.run_plain, []
+    split, plain, failed = engine.run_split, engine.run_plain, []
 
-    def failing(*a, **k):
-        if len(failed) < 2:
-            failed.append(1)
-            raise torch.cuda.OutOfMemoryError("test")
-        return plain(*a, **k)
-    monkeypatch.setattr(engine, "run_plain", failing)
+    def failing(run):           # the edge pixels' sum, whichever kernel it takes
+        def call(*a, **k):
+            if len(failed) < 2:
+                failed.append(1)
+                raise torch.cuda.OutOfMemoryError("test")
+            return run(*a, **k)
+        return call
+    monkeypatch.setattr(engine, "run_split", failing(split))
+    monkeypatch.setattr(engine, "run_plain", failing(plain))
     parts = B.atomic_scattering_kinematic(sample, D, st, **kw)
     assert len(failed) == 2 and B.last_run["memory_splits"] >= 1
     assert rel_max(parts, whole) <= 2e-5, rel_max(parts, whole)

@@ -1083,11 +1083,16 @@ def run_nodes(np_, tiles, pix, phys, table, out=None, accumulate=False, fresnel=
     return out
 
 
-def plain_slices(n, bx, sms):
+def plain_slices(n, bx, sms, warps=4):
     """Slices of n atoms for bx blocks of pixels: the FP64 pipe is shared by an
     SM's blocks, five at a time, so what counts is that every SM gets as many
     of them, and the ~40 atoms' time a block takes to set up. 32,000 atoms x
-    1,920 pixels in 50 slices (4.9 blocks an SM) 2.7 ms, in 63 (6.2) 3.0."""
+    1,920 pixels in 50 slices (4.9 blocks an SM) 2.7 ms, in 63 (6.2) 3.0. Sums
+    too small for five blocks an SM take fewer, larger slices where the most
+    laden SM has less to do (one block an SM takes 1.2 of a shared one's time):
+    1,600 atoms x 5,568 pixels in 3 slices (0.87 blocks an SM) instead of 4
+    (1.16), per-term factors 5.6 -> 4.1 ms. (Not for a block of fewer than four
+    live ``warps``, which leave parts of an SM's FP64 pipe to other blocks.)"""
     most = max(1, min((n + 511) // 512, 4096))
     best, ns = 0.0, 1
     for waves in range(1, 7):
@@ -1096,7 +1101,15 @@ def plain_slices(n, bx, sms):
         fill = blocks / math.ceil(blocks) * (n / (n + 40.0 * s))
         if fill > best:
             best, ns = fill, s
-    return ns
+
+    def laden(s):
+        per_sm = math.ceil(bx * s / sms)
+        return per_sm * (n / s + 40.0) * (1.2 if per_sm == 1 else 1.0)
+
+    if warps < 4:
+        return ns
+    few = min((min(max(per_sm * sms // bx, 1), most) for per_sm in range(1, 5)), key=laden)
+    return few if laden(few) < 0.9 * laden(ns) else ns
 
 
 def run_plain(atoms: Atoms, pix: Pixels, phys, slices=0, out=None, accumulate=False, stream=None):
@@ -1107,7 +1120,7 @@ def run_plain(atoms: Atoms, pix: Pixels, phys, slices=0, out=None, accumulate=Fa
         ns = int(slices)
     else:
         sms = torch.cuda.get_device_properties(pix.xyz.device).multi_processor_count
-        ns = plain_slices(n, (pix.n + 127) // 128, sms)
+        ns = plain_slices(n, (pix.n + 127) // 128, sms, warps=min(4, (pix.n + 31) // 32))
     ws_n = L.mk_sum_workspace_size(pix.n, ns)
     ws = torch.empty(ws_n, dtype=torch.uint8, device=pix.xyz.device)
     if out is None:

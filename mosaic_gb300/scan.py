@@ -191,6 +191,10 @@ class BatchedScan:
         plan = engine.NodePlan.make(self.tiles, self.pix, B.k, self._bd, tol)
         if plan is None:
             return False
+        try:
+            ws = torch.empty(plan.plan.ws_bytes, dtype=torch.uint8, device=self._dev)
+        except torch.cuda.OutOfMemoryError:     # up to 16 GB; the split kernel's is far smaller
+            return False
         _, fresnel, _, self.diag = B.split_budget(self.tiles, self.pix.r0_min())
         self._node_fresnel = (int(fresnel), self.diag["fresnel_radius_m"])
         if plan.wide is not None:
@@ -205,8 +209,7 @@ class BatchedScan:
         # the groups' factors: the plan admits their radius, whatever the wide
         # tiles allow the split kernel
         self.ftab = self._frame_factors(self._frame_records)
-        self.nodes = plan
-        self._node_ws = torch.empty(plan.plan.ws_bytes, dtype=torch.uint8, device=self._dev)
+        self.nodes, self._node_ws = plan, ws
         self.diag = dict(self.diag, **plan.info())
         return True
 

@@ -537,6 +537,8 @@ int mk_relu_backward(long long n, const float *grad, const float *pre, float *go
 int mk_bias_grad(int M, int N, const float *g, float *db, void *stream);
 int mk_bias_grad_groups(int groups, int M, int N, const float *g, long long g_stride, float *db,
                         long long db_stride, void *stream);
+/* Device memory set to zero bytes (what the added-into gradients start from). */
+int mk_zero(void *p, size_t bytes, void *stream);
 /* mk_bias_grad_groups added into db. */
 int mk_bias_grad_add_groups(int groups, int M, int N, const float *g, long long g_stride, float *db,
                             long long db_stride, void *stream);

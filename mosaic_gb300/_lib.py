@@ -167,6 +167,7 @@ class MkNodePlan(ctypes.Structure):
 
 # name -> (restype, argtypes)
 SIGNATURES = {
+    "mk_zero": (ctypes.c_int, [_vp, ctypes.c_size_t, _vp]),
     "mk_analyser_mask": (ctypes.c_int, [ctypes.POINTER(MkPixels), ctypes.POINTER(MkPhysics),
                                         ctypes.c_double, ctypes.c_int, _vp, _vp, ctypes.c_int, _vp]),
     "mk_scan_pixels": (ctypes.c_int, [ctypes.c_int, _vp, ctypes.c_int, _vp, ctypes.c_double, _vp,

@@ -292,6 +292,13 @@ static int mk_bias_grad_run(int groups, int M, int N, const float *g, long long 
     return MK_OK;
 }
 
+extern "C" int mk_zero(void *p, size_t bytes, void *stream)
+{
+    MK_REQUIRE(p || bytes == 0, "mk_zero: null argument");
+    MK_CHECK_CUDA(cudaMemsetAsync(p, 0, bytes, mk_stream(stream)));
+    return MK_OK;
+}
+
 extern "C" int mk_bias_grad_groups(int groups, int M, int N, const float *g, long long g_stride,
                                    float *db, long long db_stride, void *stream)
 {

@@ -158,7 +158,8 @@ class MLP:
         gradient of a hidden layer carries the ReLU derivative in its
         GEMM's epilogue (the layer's outputs as the mask)."""
         B = int(G.shape[-2])
-        self.gP.zero_()     # every layer's gradient is added into the flat buffer
+        # every layer's gradient is added into the flat buffer
+        check(self.L.mk_zero(_p(self.gP), 4 * self.gP.numel(), engine._stream_handle()))
         for l in range(len(self.dims) - 2, -1, -1):
             K, N = self.dims[l], self.dims[l + 1]
             gx = 0 if (l == 0 and acts[0].dim() == 2) else B * K

@@ -301,8 +301,8 @@ int mk_tiles_build(int64_t n, const double *pos, const int *species, const float
                    void *workspace, size_t ws_bytes, void *stream);
 /* mk_tiles_build with the order's resolution given: long keys (17 bits an axis,
  * mk_tiles_build's) or short ones (at most 10), whose build is faster.
- * crowded (device double, may be NULL): 1 where short keys left more than a few
- * atoms in one cell, in input order, so that the tiles may be wider than need
+ * crowded (device double, may be NULL): 1 where short keys left more than a
+ * quarter of a tile in one cell, in input order, so that the tiles may be wider than need
  * be: build again with long ones. */
 size_t mk_tiles_workspace_size_keys(int64_t n, int long_keys);
 int mk_tiles_build_keys(int64_t n, const double *pos, const int *species, const float *amp,

@@ -449,12 +449,14 @@ __global__ void mk_key_grid_kernel(const unsigned long long *__restrict__ bb, in
 // outnumber the atoms. Long ones have 62 (17 bits an axis, 8 passes) and resolve
 // samples whose box is mostly empty -- particles far apart, an atom far off --
 // where short cells hold many atoms each, in input order: the tile build reports
-// more than MK_CROWD atoms of a species in one cell. Long keys, then cut in FP64
+// more than a quarter of a tile in one cell. Fewer do not widen the tiles: two
+// particles of 32,000 atoms 0.3 um apart, ~110 atoms a cell, have 2.04 nm tiles,
+// 2.02 with long keys, whose build adds 230 us to a call of 1.44 ms; with 1,600 a
+// cell they are 1.5 times as wide. Long keys, then cut in FP64
 // by every thread, took 1355 us to make and 551 us to sort for 8.19M atoms, and
 // 63 us to sort 32k.
 #define MK_SHORT_KEY_ATOMS (1 << 17)
 #define MK_LONG_KEY_BITS 62
-#define MK_CROWD 8
 
 // Real: what the cell coordinates are formed in; 17 bits of up to 128 cubes
 // need FP64.
@@ -498,7 +500,7 @@ struct MkTileMap {
 // the build at 39 operations an atom (645 us for 8.19M atoms; here 358). Tiles of
 // up to 2 NT atoms hold their positions in registers, larger ones gather them
 // again for the offsets. `keys` (short ones, or null): *crowded is set where
-// atoms MK_CROWD apart in the order have the same key.
+// atoms a quarter of a tile apart in the order have the same key.
 template <int NT, bool HOLD>
 __global__ void __launch_bounds__(NT) mk_tile_kernel(MkTileMap M, double kappa,
                                                       const double *__restrict__ pos,
@@ -517,9 +519,10 @@ __global__ void __launch_bounds__(NT) mk_tile_kernel(MkTileMap M, double kappa,
     const long long end = M.run_start[s] + M.run_count[s];
     __shared__ float red[6][NT / 32];
     __shared__ float rad2[NT / 32];
-    if (keys)
-        for (long long i = first + (long long)threadIdx.x * MK_CROWD; i < first + M.tile_atoms; i += NT * MK_CROWD)
-            if (i + MK_CROWD < end && keys[i] == keys[i + MK_CROWD]) *crowded = 1.0;
+    if (keys && threadIdx.x < 8) {
+        const long long i = first + (long long)threadIdx.x * (M.tile_atoms >> 3), j = i + (M.tile_atoms >> 2);
+        if (j < end && keys[i] == keys[j]) *crowded = 1.0;
+    }
     const long long a0 = order[first];
     const double fx = pos[3 * a0], fy = pos[3 * a0 + 1], fz = pos[3 * a0 + 2];
 

@@ -60,3 +60,27 @@ def test_build_on_another_stream_and_read_back(cuda):
     assert np.array_equal(engine.origins_host(a), engine.origins_host(b))
     assert np.array_equal(engine.origins_host(b), b.origin.cpu().numpy())
     assert torch.equal(a.pos, b.pos)
+
+
+@pytest.mark.parametrize("apart, again", [(0.0, False), (3.0e3, False), (2.0e4, True)])
+def test_built_again_only_where_it_pays(cuda, monkeypatch, apart, again):
+    """A few dozen atoms a cell leave the tiles as they are; hundreds do not."""
+    rng = np.random.default_rng(3)
+    one = (rng.random((30000, 3)) - 0.5) * 70.0
+    pos = np.concatenate([one, one + apart / np.sqrt(3.0)])[rng.permutation(60000)]
+    L = engine._require_cuda()
+    keys = []
+
+    class Spy:
+        def __getattr__(self, name):
+            return getattr(L, name)
+
+        def mk_tiles_build_keys(self, *a):
+            keys.append(a[8])
+            return L.mk_tiles_build_keys(*a)
+    table = engine.SpeciesTable.build(["Cu"], ScatteringTables(), 10000.0)
+    atoms = engine.atoms_lab(pos.astype(np.float32), np.zeros(60000, np.int32), np.eye(3), np.zeros(3), table,
+                             device=cuda)
+    monkeypatch.setattr(engine, "_require_cuda", lambda: Spy())
+    engine.Tiles(atoms, 5e10, 512, device=cuda)
+    assert keys == ([0, 1] if again else [0])

@@ -507,6 +507,8 @@ class beam:
         analyser, no remove_forward), its wide tiles and the pixels a top-hat's
         edge cuts through the split kernel; None where
         its plan, or a top-hat that cuts too many pixels, declines."""
+        if not pix.plane_grid(self.k, self._kernel_phase_tol_rad):
+            return None
         masked = None
         if phys.analyser:
             masked = engine.analyser_mask(tiles, pix, phys, atoms.table)
@@ -579,7 +581,7 @@ class beam:
         if self._use_fast_kernel and self._use_nodes and not (launch or self._kernel_launch) and \
                 phys.analyser != 2 and not phys.remove_forward and \
                 float(atoms.n) * pix.n >= engine.NODES_MIN_TERMS and \
-                pix.plane_grid(self.k, self._kernel_phase_tol_rad):
+                pix.may_be_plane(self.k, self._kernel_phase_tol_rad):
             tiles = engine.Tiles(atoms, self.k, int(self._kernel_tile_atoms or engine.DEFAULT_TILE_ATOMS),
                                  device=atoms.pos.device)
             res = self._scatter_nodes(atoms, tiles, pix, phys, out, accumulate)

@@ -248,11 +248,10 @@ class Pixels:
         self._ftab = (key, ftab)
         return ftab
 
-    def plane_fit(self, stream=None):
-        """(shapes (F, 3) int64, fit (F, 12) float64) on the host: every
-        frame's pixel grid as ``mk_plane_fit`` describes it (one read-back per
-        Pixels object)."""
-        if getattr(self, "_fit", None) is None:
+    def start_plane_fit(self, stream=None):
+        """Launch ``mk_plane_fit`` (once per Pixels object): other work can be
+        queued behind it before ``plane_fit`` reads it back."""
+        if getattr(self, "_fit_dev", None) is None:
             shapes = np.array([(off, ny, nz) for (off, _), (ny, nz) in zip(self.spans, self.shapes)],
                               dtype=np.int64)
             dev = self.xyz.device
@@ -261,7 +260,15 @@ class Pixels:
             check(_require_cuda().mk_plane_fit(len(shapes), _ptr(sd),
                                                int((shapes[:, 1] * shapes[:, 2]).max()),
                                                _ptr(self.xyz), _ptr(fit), _stream_handle(stream)))
-            self._fit = (shapes, fit.cpu().numpy())
+            self._fit_dev = (shapes, sd, fit)
+
+    def plane_fit(self, stream=None):
+        """(shapes (F, 3) int64, fit (F, 12) float64) on the host: every
+        frame's pixel grid as ``mk_plane_fit`` describes it (one read-back per
+        Pixels object)."""
+        if getattr(self, "_fit", None) is None:
+            self.start_plane_fit(stream)
+            self._fit = (self._fit_dev[0], self._fit_dev[2].cpu().numpy())
             f = self._fit[1]
             self._r0_min = float(f[:, 10].min())
             with np.errstate(invalid="ignore", divide="ignore", over="ignore"):
@@ -271,12 +278,19 @@ class Pixels:
 
     def plane_grid(self, k, phase_tol):
         """Whether every frame is a plane grid of pixels as ``mk_nodes_plan``
-        asks, known before any tiles are built: within a quarter pixel of even
-        steps, and so little off the plane that atoms 0.1 nm apart -- any tile
-        is wider -- keep their phase within ``phase_tol``."""
+        asks, known without any tiles: within a quarter pixel of even steps,
+        and so little off the plane that atoms 0.1 nm apart -- any tile is
+        wider -- keep their phase within ``phase_tol``."""
         self.plane_fit()
         even, off_plane = self._plane
         return even and 1e-10 * k * off_plane <= phase_tol
+
+    def may_be_plane(self, k, phase_tol):
+        """``plane_grid`` where it is known; until then True, its fit launched."""
+        if getattr(self, "_fit", None) is None:
+            self.start_plane_fit()
+            return True
+        return self.plane_grid(k, phase_tol)
 
     def r0_min(self):
         """Smallest pixel distance (one read-back per Pixels object)."""

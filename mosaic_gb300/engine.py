@@ -260,7 +260,9 @@ class Pixels:
             check(_require_cuda().mk_plane_fit(len(shapes), _ptr(sd),
                                                int((shapes[:, 1] * shapes[:, 2]).max()),
                                                _ptr(self.xyz), _ptr(fit), _stream_handle(stream)))
-            self._fit_dev = (shapes, sd, fit)
+            done = torch.cuda.Event()
+            done.record(stream or torch.cuda.current_stream())
+            self._fit_dev = (shapes, sd, fit, done)
 
     def plane_fit(self, stream=None):
         """(shapes (F, 3) int64, fit (F, 12) float64) on the host: every
@@ -268,6 +270,7 @@ class Pixels:
         Pixels object)."""
         if getattr(self, "_fit", None) is None:
             self.start_plane_fit(stream)
+            torch.cuda.current_stream().wait_event(self._fit_dev[3])    # another stream may have launched it
             self._fit = (self._fit_dev[0], self._fit_dev[2].cpu().numpy())
             f = self._fit[1]
             self._r0_min = float(f[:, 10].min())
